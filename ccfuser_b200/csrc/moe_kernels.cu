@@ -338,19 +338,24 @@ __global__ void combine_reduce_kernel(const void* comb, const int* slot_row, voi
 // ---------------------------------------------------------------------------------------------------
 // bias gradients: out[g, n] = sum over the rows of group g of x[r, n]. Block = 128 columns (16 lanes x 16 bytes) x 16
 // row lanes, four rows in flight per thread: the kernel streams the matrix once and has to keep enough loads in
-// flight to do so at the memory rate.
+// flight to do so at the memory rate. With few groups and columns one block per (column block, group) leaves most of the
+// chip idle (4 groups x 4096 columns: 128 blocks that each walk 4096 rows), so up to 8 blocks of a cluster share the rows
+// and the cluster's first block adds their partial sums, read over distributed shared memory in a fixed order: no atomics,
+// no workspace, the same result every time.
 // ---------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) colsum_grouped_kernel(const void* x, long long ld, int n, const int* group_base,
                                                              const int* group_rows, void* out, int fp16) {
   __shared__ float red[16][128];
+  __shared__ float part[128];
   const int g = blockIdx.y;
+  const int split = blockIdx.z, splits = gridDim.z;   // the cluster spans the z dimension of the grid
   const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
   const int col = blockIdx.x * 128 + cx * 8;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col < n) {
     const int r0 = group_base[g], nr = group_rows[g];
     const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + static_cast<size_t>(r0) * ld + col;
-    for (int r = ry; r < nr; r += 64) {
+    for (int r = split * 64 + ry; r < nr; r += 64 * splits) {
       uint4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -372,15 +377,24 @@ __global__ void __launch_bounds__(256) colsum_grouped_kernel(const void* x, long
 #pragma unroll
   for (int i = 0; i < 8; ++i) red[ry][cx * 8 + i] = acc[i];
   __syncthreads();
+  float s = 0.f;
   if (threadIdx.x < 128) {
-    const int c = blockIdx.x * 128 + threadIdx.x;
-    if (c < n) {
-      float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) s += red[i][threadIdx.x];
-      if (fp16) reinterpret_cast<__half*>(out)[static_cast<size_t>(g) * n + c] = __float2half(s);
-      else reinterpret_cast<__nv_bfloat16*>(out)[static_cast<size_t>(g) * n + c] = __float2bfloat16(s);
+    for (int i = 0; i < 16; ++i) s += red[i][threadIdx.x];
+    part[threadIdx.x] = s;
+  }
+  if (splits > 1) {
+    cluster_sync_all();
+    if (split == 0 && threadIdx.x < 128) {
+      const uint32_t mine = smem_u32(&part[threadIdx.x]);
+      for (int r = 1; r < splits; ++r) s += ld_cluster_f32(map_to_cta(mine, r));
     }
+    cluster_sync_all();   // no block leaves while its partial sums may still be read
+  }
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (split == 0 && threadIdx.x < 128 && c < n) {
+    if (fp16) reinterpret_cast<__half*>(out)[static_cast<size_t>(g) * n + c] = __float2half(s);
+    else reinterpret_cast<__nv_bfloat16*>(out)[static_cast<size_t>(g) * n + c] = __float2bfloat16(s);
   }
 }
 
@@ -576,10 +590,25 @@ int ccf_combine_reduce(const void* comb, const int* slot_row, void* y, int T, in
 int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
                        void* out, int fp16, void* stream) {
   if (n % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;   // 16-byte loads
-  dim3 grid((n + 127) / 128, groups);
-  ccf::colsum_grouped_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(x, ld, n, group_base,
-                                                                                        group_rows, out, fp16);
-  return last_err();
+  const int blocks = (n + 127) / 128 * groups;
+  if (groups < 1 || blocks < 1) return -2;
+  // Rows are shared by a cluster while the launch has fewer than four blocks per SM: below that the loads in flight do not
+  // cover the memory latency; above it a cluster only adds its two barriers.
+  int splits = 1;
+  while (splits < 8 && blocks * splits < 4 * 148) splits *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((n + 127) / 128, groups, splits);
+  cfg.blockDim = dim3(256);
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = splits;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, ccf::colsum_grouped_kernel, x, ld, n, group_base, group_rows, out, fp16);
+  return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 int ccf_sgd_step(void* p, const void* g, long long n, float lr, float wd, int fp16, void* stream) {
