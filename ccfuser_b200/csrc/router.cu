@@ -10,6 +10,11 @@
 // rows per stage), warp 1 = MMA issuer (tcgen05.mma M128 x N x K16, N = E rounded up to 32, accumulator in TMEM),
 // warps 2..5 = epilogue, one per TMEM lane quarter. Router rows beyond E are zero-filled by TMA and masked out of the
 // selection. Every wait is bounded and reports through the status word.
+//
+// One CTA streams its 128 rows at what its stages in flight allow (about 0.4 us per 64-deep k-block), so with few row tiles
+// the walk over d is the kernel's time: a cluster of up to 8 CTAs then shares the k-blocks of one row tile. Each CTA
+// leaves its partial logits in its shared memory, and every CTA of the cluster finishes 128 / splits of the rows: it adds
+// the partial sums over distributed shared memory in a fixed order and selects from them.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -79,7 +84,42 @@ struct RouterArgs {
   int* status;
   unsigned long long wait_limit_ns;
   int tokens, d, e, n_pad, k, fp16, stages, tmem_cols;
+  int ctrl_off;            // bytes of shared memory in front of the control block
+  int splits;              // CTAs of the cluster that share a row tile (gridDim.y); 1 = no cluster
 };
+
+// Adds column e's logit of one row to the running selection.
+__device__ __forceinline__ void router_offer(const RouterArgs& a, float (&tv)[kRtMaxK], int (&ti)[kRtMaxK], bool& has_nan, float v,
+                                             int row, int e) {
+  if (a.logits != nullptr && row < a.tokens && e < a.e) a.logits[static_cast<size_t>(row) * a.e + e] = v;
+  if (e < a.e) {
+    if (v != v) { has_nan = true; v = -INFINITY; }
+    topk_offer(tv, ti, v, e);
+  }
+}
+
+// Columns part, part + kSplits, ... of row r of this CTA's share: the cluster's partial logits added in CTA order. `mine` is
+// the row's address in column 0 of this CTA's partial logits (the same place in every CTA). Four columns at a time, so that
+// 4 * kSplits remote reads are in flight per thread.
+template <int kSplits>
+__device__ __forceinline__ void router_add_splits(uint32_t mine, float* sums, int part, int r, int n_pad) {
+  constexpr int kRows = BM / kSplits, kCols = 4;
+  for (int c0 = part; c0 < n_pad; c0 += kSplits * kCols) {    // n_pad is a multiple of 32
+    float v[kCols][kSplits];
+#pragma unroll
+    for (int u = 0; u < kCols; ++u)
+#pragma unroll
+      for (int p = 0; p < kSplits; ++p)
+        v[u][p] = ld_cluster_f32(map_to_cta(mine + static_cast<uint32_t>((c0 + u * kSplits) * BM) * 4u, p));
+#pragma unroll
+    for (int u = 0; u < kCols; ++u) {
+      float t = v[u][0];
+#pragma unroll
+      for (int p = 1; p < kSplits; ++p) t += v[u][p];
+      sums[(c0 + u * kSplits) * kRows + r] = t;
+    }
+  }
+}
 
 __global__ void __launch_bounds__(kRtThreads, 1)
 router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
@@ -87,13 +127,16 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stage_bytes = kRtABytes + a.n_pad * 128;
-  RouterCtrl* ctrl = reinterpret_cast<RouterCtrl*>(smem + a.stages * stage_bytes);
+  RouterCtrl* ctrl = reinterpret_cast<RouterCtrl*>(smem + a.ctrl_off);
   const uint32_t smem_base = smem_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_word = &ctrl->abort_word;
   const uint64_t limit = fail_fast_limit(a.status, a.wait_limit_ns);
   const int row0 = blockIdx.x * BM;
-  const int kblocks = (a.d + BK - 1) / BK;
+  const int kblocks_all = (a.d + BK - 1) / BK;
+  const int per_split = (kblocks_all + a.splits - 1) / a.splits;
+  const int kb0 = static_cast<int>(blockIdx.y) * per_split;          // this CTA's share of the k-blocks (never empty)
+  const int kblocks = min(per_split, kblocks_all - kb0);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
@@ -135,8 +178,8 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         const uint32_t fullb = smem_u32(&ctrl->full[stage]);
         const uint32_t sa = smem_base + stage * stage_bytes;
         mbar_arrive_expect_tx(fullb, static_cast<uint32_t>(stage_bytes));
-        tma_load_2d(sa, &tmX, fullb, kb * BK, row0);            // rows past T and columns past d read as zero
-        tma_load_2d(sa + kRtABytes, &tmW, fullb, kb * BK, 0);   // all router rows (box of n_pad rows)
+        tma_load_2d(sa, &tmX, fullb, (kb0 + kb) * BK, row0);            // rows past T and columns past d read as zero
+        tma_load_2d(sa + kRtABytes, &tmW, fullb, (kb0 + kb) * BK, 0);   // all router rows (box of n_pad rows)
       }
       __syncwarp();
       if (++stage == a.stages) { stage = 0; phase ^= 1; }
@@ -168,38 +211,69 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // ======================= epilogue: one token row per thread =======================
     const int q = warp & 3;   // TMEM lane quarter this warp may read
     const int row = row0 + q * 32 + lane;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     if (mbar_wait(smem_u32(&ctrl->acc_full), 0, abort_word, limit)) {
       tc_fence_after();
-      // running top-8 in registers, best first; a candidate enters only if it is strictly greater than the current
-      // last entry and bubbles up past strictly smaller ones, so equal logits keep the lower expert id first
-      float tv[kRtMaxK];
-      int ti[kRtMaxK];
+      if (a.splits == 1) {
+        // running top-8 in registers, best first; a candidate enters only if it is strictly greater than the current
+        // last entry and bubbles up past strictly smaller ones, so equal logits keep the lower expert id first
+        float tv[kRtMaxK];
+        int ti[kRtMaxK];
 #pragma unroll
-      for (int j = 0; j < kRtMaxK; ++j) { tv[j] = -INFINITY; ti[j] = -1; }
-      bool has_nan = false;   // a NaN logit is ranked as -inf and turns the row's weights into NaN
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-      for (int c = 0; c < a.n_pad; c += 32) {
-        uint32_t racc[32];
-        tmem_ld32(t_row + c, racc);
-        tmem_ld_wait();
+        for (int j = 0; j < kRtMaxK; ++j) { tv[j] = -INFINITY; ti[j] = -1; }
+        bool has_nan = false;   // a NaN logit is ranked as -inf and turns the row's weights into NaN
+        for (int c = 0; c < a.n_pad; c += 32) {
+          uint32_t racc[32];
+          tmem_ld32(t_row + c, racc);
+          tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int e = c + i;
-          float v = __uint_as_float(racc[i]) + ctrl->bias[e];
-          if (a.logits != nullptr && row < a.tokens && e < a.e) a.logits[static_cast<size_t>(row) * a.e + e] = v;
-          if (e < a.e) {
-            if (v != v) { has_nan = true; v = -INFINITY; }
-            topk_offer(tv, ti, v, e);
-          }
+          for (int i = 0; i < 32; ++i)
+            router_offer(a, tv, ti, has_nan, __uint_as_float(racc[i]) + ctrl->bias[c + i], row, c + i);
+        }
+        if (row < a.tokens)
+          topk_finish(tv, ti, a.k, a.idx + static_cast<size_t>(row) * a.k, a.w + static_cast<size_t>(row) * a.k, has_nan);
+      } else {
+        // partial logits, [column][row], over the operand stages: every MMA that read them has completed
+        for (int c = 0; c < a.n_pad; c += 32) {
+          uint32_t racc[32];
+          tmem_ld32(t_row + c, racc);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) reinterpret_cast<uint32_t*>(smem)[(c + i) * BM + q * 32 + lane] = racc[i];
         }
       }
-      if (row < a.tokens)
-        topk_finish(tv, ti, a.k, a.idx + static_cast<size_t>(row) * a.k, a.w + static_cast<size_t>(row) * a.k, has_nan);
     } else {
       report_status(a.status, CCF_ERR_MBAR_TIMEOUT, 0x42);
     }
   }
 
+  if (a.splits > 1) {
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int rank = static_cast<int>(blockIdx.y), rows = BM / a.splits;
+      const int i = (warp - 2) * 32 + lane, r = i % rows, part = i / rows;   // `splits` threads share a row's columns
+      float* sums = reinterpret_cast<float*>(smem) + a.n_pad * BM;           // [column][rows of this CTA]
+      const uint32_t mine = smem_base + static_cast<uint32_t>(rank * rows + r) * 4u;
+      if (a.splits == 8) router_add_splits<8>(mine, sums, part, r, a.n_pad);
+      else if (a.splits == 4) router_add_splits<4>(mine, sums, part, r, a.n_pad);
+      else router_add_splits<2>(mine, sums, part, r, a.n_pad);
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps
+      if (i < rows) {
+        const int row = row0 + rank * rows + i;
+        float tv[kRtMaxK];
+        int ti[kRtMaxK];
+#pragma unroll
+        for (int j = 0; j < kRtMaxK; ++j) { tv[j] = -INFINITY; ti[j] = -1; }
+        bool has_nan = false;
+        for (int c = 0; c < a.e; ++c) router_offer(a, tv, ti, has_nan, sums[c * rows + i] + ctrl->bias[c], row, c);
+        if (row < a.tokens)
+          topk_finish(tv, ti, a.k, a.idx + static_cast<size_t>(row) * a.k, a.w + static_cast<size_t>(row) * a.k, has_nan);
+      }
+      __syncwarp();
+    }
+    cluster_sync_all();   // no CTA leaves while its partial sums may still be read
+  }
   tc_fence_before();
   __syncthreads();
   if (ctrl->abort_word) {
@@ -371,12 +445,26 @@ int ccf_router_topk(const void* x, const void* wg, const void* bias, int tokens,
   a.tmem_cols = 32;
   while (a.tmem_cols < a.n_pad) a.tmem_cols *= 2;
   const int stage_bytes = kRtABytes + a.n_pad * 128;
+  const int kblocks = (d + BK - 1) / BK;
+  const int tiles = (tokens + BM - 1) / BM;
+  // Share a row tile among as many CTAs as still fit the chip in one wave (a CTA fills an SM's shared memory); each keeps at
+  // least two k-blocks, and none is left without any.
+  a.splits = 8;
+  while (a.splits > 1 && (tiles * a.splits > 148 || kblocks < 2 * a.splits ||
+                          (a.splits - 1) * ((kblocks + a.splits - 1) / a.splits) >= kblocks))
+    a.splits /= 2;
+  const int per_split = (kblocks + a.splits - 1) / a.splits;
   a.stages = 200 * 1024 / stage_bytes;
   if (a.stages > kRtMaxStages) a.stages = kRtMaxStages;
-  const int kblocks = (d + BK - 1) / BK;
-  if (a.stages > kblocks) a.stages = kblocks;
+  if (a.stages > per_split) a.stages = per_split;
   if (a.stages < 1) return -3;
-  const int smem_bytes = 1024 + a.stages * stage_bytes + static_cast<int>(sizeof(RouterCtrl));
+  int body_bytes = a.stages * stage_bytes;
+  if (a.splits > 1) {            // partial logits of 128 rows and the sums of 128 / splits rows take the stages' place
+    const int sum_bytes = a.n_pad * (BM + BM / a.splits) * 4;
+    if (body_bytes < sum_bytes) body_bytes = (sum_bytes + 15) / 16 * 16;
+  }
+  a.ctrl_off = body_bytes;
+  const int smem_bytes = 1024 + body_bytes + static_cast<int>(sizeof(RouterCtrl));
   CUtensorMap tmx, tmw;
   int rc;
   if ((rc = make_tmap(&tmx, x, tokens, d, 64, BM, fp16))) return rc;
@@ -389,9 +477,19 @@ int ccf_router_topk(const void* x, const void* wg, const void* bias, int tokens,
     if (err != cudaSuccess) return -static_cast<int>(err);
     configured[cur & 63] = true;
   }
-  const int grid = (tokens + BM - 1) / BM;
-  router_topk_kernel<<<grid, kRtThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream_v)>>>(tmx, tmw, a);
-  cudaError_t err = cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles, a.splits);
+  cfg.blockDim = dim3(kRtThreads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream_v);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = a.splits;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.splits > 1 ? 1 : 0;
+  cudaError_t err = cudaLaunchKernelEx(&cfg, router_topk_kernel, tmx, tmw, a);
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }
 
