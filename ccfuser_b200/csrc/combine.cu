@@ -1,0 +1,218 @@
+// Last kernels of a pass over one layer: the slot reduction (forward output, input gradient) and the router's backward.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "combine.h"
+#include "dispatch.cuh"
+#include "gemm_args.h"
+#include "sm100.cuh"
+
+namespace ccf {
+
+constexpr int kMaxK = 8;
+constexpr int kReduceThreads = 256;
+constexpr int kReducePieces = 2;   // 16-byte pieces of the result per thread
+
+__device__ __forceinline__ void add_piece(float (&acc)[8], const uint4& x, float scale, int fp16) {
+  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float2 f = unpack2(w[q], fp16);
+    acc[2 * q] = fmaf(scale, f.x, acc[2 * q]);
+    acc[2 * q + 1] = fmaf(scale, f.y, acc[2 * q + 1]);
+  }
+}
+
+// y[t, :] = sum_j keep(t, j) * comb[t * k + j, :] in fp32, one rounding. Bound by reading k rows and writing one per token;
+// a block takes whole tokens (512 pieces of 16 bytes) and kK is a template argument so that all rows of a token are
+// requested before the first is used. With kRouter the same pass adds the router's share of the input gradient,
+// sum_j g_j Wg[idx_j, :] (Wg is small and stays in L2), which as a kernel of its own wrote and re-read a [T, d] matrix.
+template <int kK, bool kRouter>
+__global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __grid_constant__ CcfReduceArgs a) {
+  const int vecs = a.d >> 3, K = kK > 0 ? kK : a.top_k, fp16 = a.fp16;
+  if (blockIdx.x == 0 && a.done != nullptr) {
+    if (threadIdx.x == 0) {
+      const int target = *a.cum + *a.sent_rows * a.n_tiles + 1;
+      if (!wait_flag_ge(a.done, target, fail_fast_limit(a.status, a.wait_limit_ns)))
+        report_status(a.status, CCF_ERR_FLAG_TIMEOUT, 0x400000);
+      *a.cum = target;
+    }
+    for (int i = threadIdx.x; i < a.zero_count; i += kReduceThreads) a.zero_words[i] = 0;
+  }
+  const int per_block = max(1, kReduceThreads * kReducePieces / vecs);   // tokens of this block
+  const int t0 = static_cast<int>(blockIdx.x) * per_block;
+  const int items = min(per_block, a.tokens - t0) * vecs;
+  const uint4* comb = reinterpret_cast<const uint4*>(a.comb);
+  const uint4* wg = reinterpret_cast<const uint4*>(a.wg);
+#pragma unroll kReducePieces
+  for (int i = threadIdx.x; i < items; i += kReduceThreads) {
+    const int lt = i / vecs, v = i - lt * vecs, t = t0 + lt;
+    const size_t s0 = static_cast<size_t>(t) * K;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    constexpr int kN = kK > 0 ? kK : kMaxK;
+    bool on[kN];
+    for (int j0 = 0; j0 < K; j0 += kN) {   // once, except for more than kMaxK slots per token
+      uint4 x[kN];
+#pragma unroll
+      for (int j = 0; j < kN; ++j) {
+        on[j] = j0 + j < K && __ldg(a.slot_row + s0 + j0 + j) >= 0;
+        x[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (on[j]) x[j] = comb[(s0 + j0 + j) * vecs + v];
+      }
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+        if (on[j]) add_piece(acc, x[j], 1.f, fp16);
+    }
+    if constexpr (kRouter) {
+      float w[kN], dw[kN];
+      float dot = 0.f;
+#pragma unroll
+      for (int j = 0; j < kN; ++j) {
+        w[j] = j < K ? __ldg(a.w + s0 + j) : 0.f;
+        dw[j] = on[j] ? a.dw[s0 + j] : 0.f;
+        dot = fmaf(w[j], dw[j], dot);
+      }
+#pragma unroll
+      for (int j = 0; j < kN; ++j) {
+        if (j >= K) continue;
+        const int e = __ldg(a.idx + s0 + j);
+        const bool routed = e >= 0 && e < a.e;
+        const float g = routed ? w[j] * (dw[j] - dot) : 0.f;
+        if (v == 0) a.g[s0 + j] = g;
+        if (routed) add_piece(acc, __ldg(wg + static_cast<size_t>(e) * vecs + v), g, fp16);
+      }
+    }
+    uint4 o;
+    o.x = pack2(acc[0], acc[1], fp16);
+    o.y = pack2(acc[2], acc[3], fp16);
+    o.z = pack2(acc[4], acc[5], fp16);
+    o.w = pack2(acc[6], acc[7], fp16);
+    reinterpret_cast<uint4*>(a.y)[static_cast<size_t>(t) * vecs + v] = o;
+  }
+}
+
+// The gradient of the logits is non-zero only in the k selected columns, so dWg is a sum of scaled token rows per expert.
+// The routing kernel left the slots listed by expert: a block sums 128 columns over one expert's list (16 row lanes, four
+// rows in flight per thread), and a cluster of up to 8 blocks shares a long list, its first block adding their partial sums
+// in a fixed order. x is read top_k times, from L2 after the first; products and sums are fp32 and the result is
+// rounded once, where scattering into shared memory needed atomics, a zeroed fp32 result and a conversion pass, and the
+// dense [T, 128] gradient for a tensor-core product needed ten small launches around it.
+__global__ void __launch_bounds__(256) router_dw_kernel(const int* __restrict__ raw_order, const int* __restrict__ count_raw,
+                                                        const float* __restrict__ g_slot, const void* __restrict__ x, void* dwg,
+                                                        void* db, int d, int top_k, int fp16) {
+  __shared__ float red[16][128];
+  __shared__ float redg[16];
+  __shared__ float part[128];
+  __shared__ float partg;
+  const int e = blockIdx.y, split = blockIdx.z, splits = gridDim.z;
+  const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
+  const int col = blockIdx.x * 128 + cx * 8;
+  const int* list = raw_order + CCF_MAX_GROUPS + raw_order[e];
+  const int nr = count_raw[e];
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  float sum_g = 0.f;
+  const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + col;
+  for (int r = split * 64 + ry; r < nr; r += 64 * splits) {
+    float g[4];
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int rr = r + 16 * u;
+      const int s = rr < nr ? __ldg(list + rr) : 0;
+      g[u] = rr < nr ? __ldg(g_slot + s) : 0.f;
+      v[u] = rr < nr && col < d ? __ldg(reinterpret_cast<const uint4*>(base + static_cast<size_t>(s / top_k) * d))
+                                : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      add_piece(acc, v[u], g[u], fp16);
+      sum_g += g[u];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) red[ry][cx * 8 + i] = acc[i];
+  if (cx == 0) redg[ry] = sum_g;
+  __syncthreads();
+  float s = 0.f, sg = 0.f;
+  if (threadIdx.x < 128) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { s += red[i][threadIdx.x]; sg += redg[i]; }
+    part[threadIdx.x] = s;
+    if (threadIdx.x == 0) partg = sg;
+  }
+  if (splits > 1) {
+    cluster_sync_all();
+    if (split == 0 && threadIdx.x < 128) {
+      const uint32_t mine = smem_u32(&part[threadIdx.x]), mineg = smem_u32(&partg);
+      for (int r = 1; r < splits; ++r) {
+        s += ld_cluster_f32(map_to_cta(mine, r));
+        if (threadIdx.x == 0) sg += ld_cluster_f32(map_to_cta(mineg, r));
+      }
+    }
+    cluster_sync_all();   // no block leaves while its partial sums may still be read
+  }
+  if (split != 0 || threadIdx.x >= 128) return;
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c < d) {
+    if (fp16) reinterpret_cast<__half*>(dwg)[static_cast<size_t>(e) * d + c] = __float2half(s);
+    else reinterpret_cast<__nv_bfloat16*>(dwg)[static_cast<size_t>(e) * d + c] = __float2bfloat16(s);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && db != nullptr) {
+    if (fp16) reinterpret_cast<__half*>(db)[e] = __float2half(sg);
+    else reinterpret_cast<__nv_bfloat16*>(db)[e] = __float2bfloat16(sg);
+  }
+}
+
+}  // namespace ccf
+
+extern "C" {
+
+int ccf_reduce(const CcfReduceArgs* a, void* stream) {
+  using namespace ccf;
+  if (a->d < 8 || a->d % 8 != 0 || a->top_k < 0) return -2;
+  if (a->wg != nullptr && (a->top_k > kMaxK || a->top_k < 1)) return -2;
+  if (a->tokens == 0 && a->done == nullptr) return 0;
+  const int vecs = a->d >> 3;
+  const int per_block = kReduceThreads * kReducePieces / vecs > 1 ? kReduceThreads * kReducePieces / vecs : 1;
+  int blocks = (a->tokens + per_block - 1) / per_block;
+  if (blocks < 1) blocks = 1;    // a call without tokens still consumes its completion count
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+#define CCF_REDUCE(K)                                                                       \
+  do {                                                                                      \
+    if (a->wg != nullptr) combine_reduce_kernel<K, true><<<blocks, kReduceThreads, 0, st>>>(*a);  \
+    else combine_reduce_kernel<K, false><<<blocks, kReduceThreads, 0, st>>>(*a);            \
+  } while (0)
+  if (a->top_k == 1) CCF_REDUCE(1);
+  else if (a->top_k == 2) CCF_REDUCE(2);
+  else CCF_REDUCE(0);
+#undef CCF_REDUCE
+  cudaError_t err = cudaGetLastError();
+  return err == cudaSuccess ? 0 : -static_cast<int>(err);
+}
+
+int ccf_router_dw(const int* raw_order, const int* count_raw, const float* g, const void* x, void* dwg, void* db, int slots, int d,
+                  int e, int top_k, int fp16, void* stream) {
+  using namespace ccf;
+  if (d < 8 || d % 8 != 0 || e < 1 || e > CCF_MAX_GROUPS || top_k < 1 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;
+  const int blocks = (d + 127) / 128 * e;
+  // as in ccf_colsum_grouped: share an expert's rows until there are four blocks per SM, four passes of 64 rows at least
+  int splits = 1;
+  while (splits < 8 && blocks * splits < 4 * 148 && slots / e >= 2 * splits * 256) splits *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((d + 127) / 128, e, splits);
+  cfg.blockDim = dim3(256);
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = splits;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  cudaError_t err = cudaLaunchKernelEx(&cfg, router_dw_kernel, raw_order, count_raw, g, x, dwg, db, d, top_k, fp16);
+  return err == cudaSuccess ? 0 : -static_cast<int>(err);
+}
+
+}  // extern "C"

@@ -8,8 +8,10 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "combine.h"
 #include "dispatch.cuh"
 #include "gemm_args.h"
+#include "plan.cuh"
 #include "sm100.cuh"
 
 namespace ccf {
@@ -177,91 +179,11 @@ __global__ void route_pos_kernel(const int* __restrict__ expert, int S, int E, c
 }
 
 // ---------------------------------------------------------------------------------------------------
-// count exchange + plan. One CTA. Every rank writes its kept counts into every rank's table (peer
-// stores + release flag carrying the step epoch), waits (bounded) for all rows of its own table, then
-// computes the row layout of every owner's receive buffer:
-//   rows of expert e start at base[e] (multiple of 128) on owner e / E_loc,
-//   rows sent by source r start at base[e] + sum_{r' < r} count[r'][e].
-// Replaces the NCCL all-gather + .cpu() + Python block planner of the reference
-// (mix_moe/csrc/cuda/global_exchange.cpp:139-177, mix_moe/mix_moe/transformer.py:150-250).
+// count exchange + plan (plan.cuh) as kernels of their own: calls whose slots do not fit the one-kernel routing (route.cu)
 // ---------------------------------------------------------------------------------------------------
 using PlanArgs = ::CcfPlanArgs;   // gemm_args.h
 
-__device__ __forceinline__ void plan_body(const PlanArgs& a, const int epoch) {
-  __shared__ int rows[CCF_MAX_GROUPS];
-  __shared__ int myoff[CCF_MAX_GROUPS];
-  __shared__ int base[CCF_MAX_GROUPS];
-  __shared__ int failed;
-  const int tid = threadIdx.x;
-  if (tid == 0) failed = 0;
-  // 1. publish my counts
-  for (int i = tid; i < a.world * a.e_total; i += blockDim.x) {
-    const int p = i / a.e_total, e = i - p * a.e_total;
-    a.peer_table[p][a.my_rank * a.e_total + e] = a.count_kept[e];
-  }
-  __threadfence_system();
-  __syncthreads();
-  if (tid < a.world) st_release_sys(a.peer_flag[tid] + a.my_rank, epoch);
-  // 2. wait for everyone's counts (my own table, local memory)
-  if (tid < a.world) {
-    if (!wait_flag_ge(a.peer_flag[a.my_rank] + tid, epoch, fail_fast_limit(a.status, a.wait_limit_ns))) {
-      report_status(a.status, CCF_ERR_FLAG_TIMEOUT, 0x800000 | tid);
-      failed = 1;
-    }
-  }
-  __syncthreads();
-  if (failed) {
-    for (int e = tid; e < a.e_total; e += blockDim.x) a.dst_base[e] = 0;
-    for (int e = tid; e < a.e_loc; e += blockDim.x) {
-      a.group_base[e] = 0;
-      a.group_rows[e] = 0;
-      if (a.local_begin != nullptr) { a.local_begin[e] = 0; a.local_rows[e] = 0; }
-    }
-    if (tid < a.world) a.sent_rows[tid] = 0;
-    return;
-  }
-  // 3. plan
-  const int* table = a.peer_table[a.my_rank];
-  for (int e = tid; e < a.e_total; e += blockDim.x) {
-    int tot = 0, off = 0;
-    for (int r = 0; r < a.world; ++r) {
-      const int c = ld_relaxed_sys(table + r * a.e_total + e);
-      if (a.table_copy) a.table_copy[r * a.e_total + e] = c;
-      if (r < a.my_rank) off += c;
-      tot += c;
-    }
-    rows[e] = tot;
-    myoff[e] = off;
-  }
-  __syncthreads();
-  if (tid < a.world) {
-    int run = 0, sent = 0;
-    for (int i = 0; i < a.e_loc; ++i) {
-      const int e = tid * a.e_loc + i;
-      base[e] = run;
-      run += (rows[e] + 127) & ~127;
-      // rows of mine that fit into the owner's buffer: the rest is rejected by the dispatch role and must not be
-      // waited for (source and owner derive the same limit from the same table)
-      const int first = run - ((rows[e] + 127) & ~127) + myoff[e];
-      sent += max(0, min(a.count_kept[e], a.max_rows - first));
-    }
-    a.sent_rows[tid] = sent;
-    if (run > a.max_rows) report_status(a.status, CCF_ERR_OVERFLOW, tid);
-  }
-  __syncthreads();
-  for (int e = tid; e < a.e_total; e += blockDim.x) a.dst_base[e] = base[e] + myoff[e];
-  for (int i = tid; i < a.e_loc; i += blockDim.x) {
-    const int e = a.my_rank * a.e_loc + i;
-    a.group_base[i] = base[e];
-    a.group_rows[i] = min(rows[e], max(0, a.max_rows - base[e]));
-    if (a.local_begin != nullptr) {
-      a.local_begin[i] = myoff[e];
-      a.local_rows[i] = max(0, min(a.count_kept[e], a.max_rows - (base[e] + myoff[e])));
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) plan_kernel(const __grid_constant__ PlanArgs a) { plan_body(a, a.epoch); }
+__global__ void __launch_bounds__(256) plan_kernel(const __grid_constant__ PlanArgs a) { plan_body(a, a.epoch, a.count_kept); }
 
 // Same, with the call's epoch taken from a counter in device memory (previous value + 1, written back at the end)
 // instead of a launch argument: a captured CUDA graph replays with fixed arguments, so a host-side epoch would
@@ -270,7 +192,7 @@ __global__ void __launch_bounds__(256) plan_kernel_dev_epoch(const __grid_consta
   __shared__ int epoch;
   if (threadIdx.x == 0) epoch = *epoch_counter + 1;
   __syncthreads();
-  plan_body(a, epoch);
+  plan_body(a, epoch, a.count_kept);
   __syncthreads();
   if (threadIdx.x == 0) *epoch_counter = epoch;
 }
@@ -293,8 +215,8 @@ __global__ void __launch_bounds__(256) dispatch_kernel(const __grid_constant__ C
 }
 
 // ---------------------------------------------------------------------------------------------------
-// combine: wait until every owner has stored all rows of this rank (and finished its kernel), then
-// sum the top-k slots of each token. Counters are monotonic; `cum` holds the value already consumed.
+// combine: wait until every owner has stored all rows of this rank (and finished its kernel). Counters are monotonic; `cum`
+// holds the value already consumed. The sum of the top-k slots of each token follows in combine.cu.
 // ---------------------------------------------------------------------------------------------------
 __global__ void combine_wait_kernel(const int* done, int* cum, const int* sent_rows, int n_tiles, int world,
                                     unsigned long long limit_ns, int* status) {
@@ -304,35 +226,6 @@ __global__ void combine_wait_kernel(const int* done, int* cum, const int* sent_r
   if (!wait_flag_ge(done + o, target, fail_fast_limit(status, limit_ns)))
     report_status(status, CCF_ERR_FLAG_TIMEOUT, 0x400000 | o);
   cum[o] = target;
-}
-
-// y[t, :] = sum_j keep(t, j) * comb[t * k + j, :]; one thread per 16-byte piece of an output row, fp32 accumulate.
-// (A warp per token made the kernel latency-bound for small batches: d / 256 dependent iterations per warp.)
-__global__ void combine_reduce_kernel(const void* comb, const int* slot_row, void* y, int T, int K, int d, int fp16) {
-  const int vecs = d >> 3;
-  const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (gid >= static_cast<long long>(T) * vecs) return;
-  const int t = static_cast<int>(gid / vecs), v = static_cast<int>(gid - static_cast<long long>(t) * vecs);
-  const uint4* c = reinterpret_cast<const uint4*>(comb);
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int j = 0; j < K; ++j) {
-    const int s = t * K + j;
-    if (__ldg(slot_row + s) < 0) continue;
-    const uint4 x = c[static_cast<size_t>(s) * vecs + v];
-    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float2 f = unpack2(w[q], fp16);
-      acc[2 * q] += f.x;
-      acc[2 * q + 1] += f.y;
-    }
-  }
-  uint4 o;
-  o.x = pack2(acc[0], acc[1], fp16);
-  o.y = pack2(acc[2], acc[3], fp16);
-  o.z = pack2(acc[4], acc[5], fp16);
-  o.w = pack2(acc[6], acc[7], fp16);
-  reinterpret_cast<uint4*>(y)[static_cast<size_t>(t) * vecs + v] = o;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -578,24 +471,29 @@ int ccf_combine_wait(const int* done, int* cum, const int* sent_rows, int n_tile
 int ccf_combine_reduce(const void* comb, const int* slot_row, void* y, int T, int K, int d, int fp16, void* stream) {
   if (d % 8 != 0) return -2;
   if (T == 0) return 0;
-  const long long pieces = static_cast<long long>(T) * (d >> 3);
-  const int threads = 256;
-  const long long blocks = (pieces + threads - 1) / threads;
-  if (blocks > 0x7fffffffLL) return -2;
-  ccf::combine_reduce_kernel<<<static_cast<unsigned>(blocks), threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      comb, slot_row, y, T, K, d, fp16);
-  return last_err();
+  CcfReduceArgs a;
+  memset(&a, 0, sizeof(a));
+  a.comb = comb;
+  a.slot_row = slot_row;
+  a.y = y;
+  a.tokens = T;
+  a.top_k = K;
+  a.d = d;
+  a.fp16 = fp16;
+  return ccf_reduce(&a, stream);
 }
 
-int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
-                       void* out, int fp16, void* stream) {
+// `rows_hint`: expected rows per group, or 0 when the caller does not know
+int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                            void* out, int fp16, int rows_hint, void* stream) {
   if (n % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;   // 16-byte loads
   const int blocks = (n + 127) / 128 * groups;
   if (groups < 1 || blocks < 1) return -2;
-  // Rows are shared by a cluster while the launch has fewer than four blocks per SM: below that the loads in flight do not
-  // cover the memory latency; above it a cluster only adds its two barriers.
+  // Rows are shared by a cluster while the launch has fewer than four blocks per SM (below that the loads in flight do not
+  // cover the memory latency) and every block keeps at least four passes of 64 rows: 16 groups of 188 rows took 10.5 us
+  // unshared and 15.1 us in clusters of 2 and 8, 4 groups of 4096 rows 103 us and 43 us (both for 4 d + d columns).
   int splits = 1;
-  while (splits < 8 && blocks * splits < 4 * 148) splits *= 2;
+  while (splits < 8 && blocks * splits < 4 * 148 && (rows_hint <= 0 || rows_hint >= 2 * splits * 256)) splits *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((n + 127) / 128, groups, splits);
   cfg.blockDim = dim3(256);
@@ -609,6 +507,11 @@ int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int
   cfg.numAttrs = splits > 1 ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, ccf::colsum_grouped_kernel, x, ld, n, group_base, group_rows, out, fp16);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
+}
+
+int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                       void* out, int fp16, void* stream) {
+  return ccf_colsum_grouped_hint(x, ld, n, groups, group_base, group_rows, out, fp16, 0, stream);
 }
 
 int ccf_sgd_step(void* p, const void* g, long long n, float lr, float wd, int fp16, void* stream) {

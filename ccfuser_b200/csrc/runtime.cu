@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include "combine.h"
+#include "route.h"
 #include "runtime.h"
 
 extern "C" {
@@ -17,9 +19,8 @@ int ccf_plan(const CcfPlanArgs* a, void* stream);
 int ccf_plan_dev_epoch(const CcfPlanArgs* a, int* epoch_counter, void* stream);
 int ccf_combine_wait(const int* done, int* cum, const int* sent_rows, int n_tiles, int world,
                      unsigned long long limit_ns, int* status, void* stream);
-int ccf_combine_reduce(const void* comb, const int* slot_row, void* y, int T, int K, int d, int fp16, void* stream);
-int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
-                       void* out, int fp16, void* stream);
+int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                            void* out, int fp16, int rows_hint, void* stream);
 }
 
 namespace {
@@ -132,16 +133,49 @@ int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
   return ccf_gemm_launch(&g, stream);
 }
 
-int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, int bn, Dry* dry, void* stream) {
+// Wait for the owners and sum the k slots of each token. With G (backward) and a router in the call, the sum also carries
+// the gradient through the gate weights.
+int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, int bn, const CcfLayerGrads* G, const int* idx,
+                    const float* gate_w, Dry* dry, void* stream) {
   if (dry != nullptr) return 0;
-  int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model, bn), L->world, L->wait_limit_ns,
-                            L->status, stream);
-  if (rc) return rc;
-  return ccf_combine_reduce(comb, L->slot_row, out, tokens, L->top_k, L->d_model, L->fp16, stream);
+  CcfReduceArgs r;
+  memset(&r, 0, sizeof(r));
+  r.comb = comb;
+  r.slot_row = L->slot_row;
+  r.y = out;
+  r.tokens = tokens;
+  r.top_k = L->top_k;
+  r.d = L->d_model;
+  r.fp16 = L->fp16;
+  if (L->world == 1) {
+    r.done = L->done;
+    r.cum = L->done_cum;
+    r.sent_rows = L->sent_rows;
+    r.n_tiles = combine_units(L->d_model, bn);
+    r.status = L->status;
+    r.wait_limit_ns = L->wait_limit_ns;
+    r.zero_words = L->tile_flags;
+    r.zero_count = L->max_rows / 128 + 1;
+  } else {
+    const int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model, bn), L->world,
+                                    L->wait_limit_ns, L->status, stream);
+    if (rc) return rc;
+  }
+  if (G != nullptr && G->router_w != nullptr) {
+    r.idx = idx;
+    r.w = gate_w;
+    r.dw = G->dgate;
+    r.wg = G->router_w;
+    r.g = G->slot_grad;
+    r.e = L->e_total;
+  }
+  return ccf_reduce(&r, stream);
 }
 
+// The arrival counters return to zero between the kernel that waits on them and this rank's finish token: peers push the
+// next pass's rows only after that token. A single rank has no peers, and its reduce kernel, the last of the pass, does it.
 int zero_tile_flags(const CcfLayer* L, Dry* dry, void* stream) {
-  if (dry != nullptr) return 0;
+  if (dry != nullptr || L->world == 1) return 0;
   cudaError_t e = cudaMemsetAsync(L->tile_flags, 0, sizeof(int) * (L->max_rows / 128 + 1),
                                   reinterpret_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
@@ -175,12 +209,7 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
   }
   if (dry == nullptr) {
     if (L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
-    // 1. positions, kept counts, destination order of this rank's slots
-    rc = ccf_route_ordered(idx, tokens * L->top_k, L->e_total, capacity, L->slot_pos, L->block_hist, L->block_off,
-                           L->count_raw, L->count_kept, L->ticket, L->order_off, L->sorted_slot, L->slot_row,
-                           L->rank * e_loc, stream);
-    if (rc) return rc;
-    // 2. count exchange with all ranks + row layout
+    // 1. positions, kept counts, destination order of this rank's slots; count exchange with all ranks + row layout
     CcfPlanArgs p;
     memset(&p, 0, sizeof(p));
     p.count_kept = L->count_kept;
@@ -203,7 +232,16 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
     p.e_loc = e_loc;
     p.epoch = epoch;
     p.max_rows = L->max_rows;
-    rc = epoch >= 0 ? ccf_plan(&p, stream) : ccf_plan_dev_epoch(&p, L->epoch_dev, stream);
+    int* epoch_dev = epoch >= 0 ? nullptr : L->epoch_dev;
+    rc = ccf_route_plan(idx, tokens * L->top_k, L->e_total, capacity, L->slot_pos, L->count_raw, L->count_kept, L->order_off,
+                        L->sorted_slot, L->slot_row, L->rank * e_loc, save_pre ? L->raw_order : nullptr, &p, epoch_dev, stream);
+    if (rc == 1) {   // no slots, or more than the one-kernel form holds
+      rc = ccf_route_ordered(idx, tokens * L->top_k, L->e_total, capacity, L->slot_pos, L->block_hist, L->block_off,
+                             L->count_raw, L->count_kept, L->ticket, L->order_off, L->sorted_slot, L->slot_row,
+                             L->rank * e_loc, stream);
+      if (rc) return rc;
+      rc = epoch_dev == nullptr ? ccf_plan(&p, stream) : ccf_plan_dev_epoch(&p, epoch_dev, stream);
+    }
     if (rc) return rc;
   }
   // 3. dispatch + GEMM-1 (+ bias + activation)
@@ -248,7 +286,7 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
-  rc = wait_and_reduce(L, L->comb, y, tokens, gemm2_bn, dry, stream);
+  rc = wait_and_reduce(L, L->comb, y, tokens, gemm2_bn, nullptr, nullptr, nullptr, dry, stream);
   if (dry_count != nullptr) *dry_count = dry_state.n;
   return rc;
 }
@@ -265,6 +303,7 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
   // decides: there the one-CTA kernel is faster than CTA pairs.
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
   const int wgrad_two_cta = rows_per_expert > 512 ? L->two_cta : 0;
+  const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
   const int row_two_cta = rows_per_expert > L->small_rows ? L->two_cta : 0;
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
   // GEMM. w2 may be at any group size (dgrad-2 above it is its last reader). w1 / wg only on a single rank: dgrad-1 reads
@@ -313,7 +352,7 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
     if ((rc = issue(g, dry, stream))) return rc;
   }
   if (G->db2 != nullptr && dry == nullptr) {
-    if ((rc = ccf_colsum_grouped(L->grecv, d, d, e_loc, L->group_base, L->group_rows, G->db2, L->fp16, stream))) return rc;
+    if ((rc = ccf_colsum_grouped_hint(L->grecv, d, d, e_loc, L->group_base, L->group_rows, G->db2, L->fp16, rows_hint, stream))) return rc;
   }
   // 4. wgrad-1: dW1[e] = dh^T x_e  [f, d]  (SwiGLU: gate projection from dh, up projection from dh2)
   auto wgrad1 = [&](const void* a0, void* out) {
@@ -360,20 +399,23 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
     if ((rc = wgrad1(G->dh2, sgd ? const_cast<void*>(L->w1) : G->dw1))) return rc;
     if (dry == nullptr) {
       if (G->db1 != nullptr &&
-          (rc = ccf_colsum_grouped(G->dh2, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, stream)))
+          (rc = ccf_colsum_grouped_hint(G->dh2, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, rows_hint, stream)))
         return rc;
       if (G->dbg != nullptr &&
-          (rc = ccf_colsum_grouped(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->dbg, L->fp16, stream)))
+          (rc = ccf_colsum_grouped_hint(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->dbg, L->fp16, rows_hint, stream)))
         return rc;
     }
   } else {
     if ((rc = wgrad1(G->dh, sgd ? const_cast<void*>(L->w1) : G->dw1))) return rc;
     if (dry == nullptr && G->db1 != nullptr &&
-        (rc = ccf_colsum_grouped(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, stream)))
+        (rc = ccf_colsum_grouped_hint(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, rows_hint, stream)))
       return rc;
   }
   if (!sgd && (rc = dgrad1())) return rc;
-  rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, 256, dry, stream);
+  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, 256, G, idx, gate_w, dry, stream))) return rc;
+  if (G->router_dw != nullptr && dry == nullptr)
+    rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d, L->e_total, L->top_k,
+                       L->fp16, stream);
   if (dry_count != nullptr) *dry_count = dry_state.n;
   return rc;
 }

@@ -33,6 +33,7 @@ struct CcfLayer {
   int* group_rows;
   int* sent_rows;
   int* table_copy;
+  int* raw_order;   // [CCF_MAX_GROUPS + max_slots] all routed slots by expert (dropped ones too), for the router's gradient
   // buffers shared by the layers of one expert-parallel group
   void* grecv;      // [max_rows, d] rows received in backward (symmetric)
   void* gcomb;      // [max_slots, d] input-gradient rows returned to this rank (symmetric)
@@ -89,6 +90,13 @@ struct CcfLayerGrads {
   // the old w1 / wg runs before them.
   float sgd_lr;
   float sgd_wd;
+  // The router's part of the backward pass (router_w non-null: the layer call included the router): dx also gets the
+  // gradient through the gate weights, and router_dw / router_db are written from the routing kernel's slot lists.
+  const void* router_w;   // [e_total, d]
+  const void* x;          // [tokens, d] the layer's input
+  float* slot_grad;       // [tokens * top_k] scratch
+  void* router_dw;        // [e_total, d]; null = not wanted
+  void* router_db;        // [e_total]; null = no bias
 };
 
 extern "C" {

@@ -88,6 +88,8 @@ class MoELayer(nn.Module):
         if backend == "fused":
             fused = self._fused_impl()
             x = x.contiguous()
+            if token_mask is None and cfg.shadow_experts == 0 and fused.one_node(x):
+                return self._finish(fused.route_and_run(x), x, None, shape)
             idx, score = fused.route(x)
         else:
             idx, score = self.gate(x)
@@ -113,6 +115,9 @@ class MoELayer(nn.Module):
             y = moe_forward_a2a(x, idx, score, self.experts, num_experts=cfg.num_experts,
                                 capacity=cfg.capacity(x.shape[0]), group=group, stats=self.last_stats)
             y = y.to(inp.dtype)
+        return self._finish(y, x, y_shadow, shape)
+
+    def _finish(self, y, x, y_shadow, shape):
         if y_shadow is not None:
             y = y + y_shadow.to(y.dtype)
         if self.shared is not None:

@@ -14,6 +14,7 @@ import torch
 
 MAX_RANKS = 8
 MAX_GROUPS = 256
+ROUTE_CLUSTER_SLOTS = 65536   # csrc/route.h: slots that the one-kernel routing + plan holds
 
 EPI_STORE, EPI_BIAS_ACT, EPI_SWIGLU, EPI_COMBINE, EPI_DACT, EPI_DSWIGLU = range(6)
 ACT_NONE, ACT_GELU, ACT_RELU = range(3)
@@ -102,7 +103,7 @@ class Layer(C.Structure):
         ("xrecv", _vp), ("comb", _vp), ("h_act", _vp), ("h_pre", _vp), ("h_pre2", _vp),
         ("slot_pos", _vp), ("slot_row", _vp), ("sorted_slot", _vp), ("order_off", _vp), ("local_begin", _vp),
         ("local_rows", _vp), ("count_raw", _vp), ("count_kept", _vp), ("dst_base", _vp), ("group_base", _vp),
-        ("group_rows", _vp), ("sent_rows", _vp), ("table_copy", _vp),
+        ("group_rows", _vp), ("sent_rows", _vp), ("table_copy", _vp), ("raw_order", _vp),
         ("grecv", _vp), ("gcomb", _vp), ("row_src", _vp), ("row_gate", _vp), ("tile_flags", _vp), ("done", _vp),
         ("done_cum", _vp), ("block_hist", _vp), ("block_off", _vp), ("ticket", _vp), ("sched", _vp), ("status", _vp),
         ("epoch_dev", _vp),
@@ -121,7 +122,8 @@ class Layer(C.Structure):
 class LayerGrads(C.Structure):
     """Mirror of CcfLayerGrads (csrc/runtime.h)."""
     _fields_ = [("dgate", _vp), ("dh", _vp), ("dh2", _vp), ("dw1", _vp), ("db1", _vp), ("dwg", _vp), ("dbg", _vp),
-                ("dw2", _vp), ("db2", _vp), ("dx", _vp), ("sgd_lr", C.c_float), ("sgd_wd", C.c_float)]
+                ("dw2", _vp), ("db2", _vp), ("dx", _vp), ("sgd_lr", C.c_float), ("sgd_wd", C.c_float),
+                ("router_w", _vp), ("x", _vp), ("slot_grad", _vp), ("router_dw", _vp), ("router_db", _vp)]
 
 
 _lib = None
@@ -191,6 +193,8 @@ def _declare(lib):
         "ccf_topk_softmax_bwd": ([p, p, p, i, i, i, p, i, i, p], i),
         "ccf_route": ([p, i, i, i, p, p, p, p, p, p, p], i),
         "ccf_route_ordered": ([p, i, i, i, p, p, p, p, p, p, p, p, p, i, p], i),
+        "ccf_route_plan": ([p, i, i, i, p, p, p, p, p, p, i, p, C.POINTER(PlanArgs), p, p], i),
+        "ccf_router_dw": ([p, p, p, p, p, p, i, i, i, i, i, p], i),
         "ccf_layer_forward": ([C.POINTER(Layer), p, p, p, p, i, i, i, i, p, p, i, p], i),
         "ccf_layer_backward": ([C.POINTER(Layer), p, p, p, C.POINTER(LayerGrads), i, i, p, p, i, p], i),
         "ccf_flag_barrier": ([C.POINTER(BarrierArgs), p], i),

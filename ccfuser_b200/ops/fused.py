@@ -262,6 +262,7 @@ class FusedMoE:
         self.group_rows = torch.zeros(e_loc, **i32)
         self.sent_rows = torch.zeros(N.MAX_RANKS, **i32)
         self.table_copy = torch.zeros(self.world, cfg.num_experts, **i32)
+        self.raw_order = torch.zeros(N.MAX_GROUPS + self.max_slots, **i32)   # slots by expert before the capacity clamp
         self.check_every_call = bool(env_flag("CHECK_STATUS", 0))
         self.fused_router = bool(env_flag("FUSED_ROUTER", 1))   # one-kernel router (ops/router.py) wherever it applies
         self._save_pre = True   # whether the next forward stores the pre-activations (set per call by run_experts)
@@ -277,8 +278,47 @@ class FusedMoE:
     # ------------------------------------------------------------------------------------------
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         x = x.contiguous()
+        if self.one_node(x):
+            return self.route_and_run(x)
         idx, w = self.route(x)
         return self.run_experts(x, idx, w)
+
+    def _aux_coefs(self):
+        gate = self.layer.gate
+        return getattr(gate, "aux_loss_coef", 0.0), getattr(gate, "z_loss_coef", 0.0)
+
+    def one_node(self, x: torch.Tensor) -> bool:
+        """Whether router and experts of this call run as one autograd node (route_and_run): the one-kernel router
+        applies, no auxiliary loss asks for the logits, and the call's slots fit the one-kernel routing, which lists them
+        by expert for the router's weight gradient. Then the input gradient through the gate weights is added in the slot
+        reduction that ends the backward pass, instead of in a kernel of its own and an addition of two [T, d] matrices."""
+        cfg, layer = self.cfg, self.layer
+        lin = getattr(layer.gate, "gate", None)
+        coef, zcoef = self._aux_coefs()
+        return (self.native_runtime and self.fused_router and isinstance(lin, torch.nn.Linear)
+                and not (coef and coef > 0) and not (zcoef and zcoef > 0) and x.shape[0] <= cfg.max_tokens
+                and x.shape[0] * cfg.top_k <= N.ROUTE_CLUSTER_SLOTS and R.supported(x, lin.weight, cfg.top_k)
+                and lin.weight.shape[0] == cfg.num_experts and (lin.bias is None or lin.bias.dtype == x.dtype))
+
+    def _expert_tensors(self):
+        ex, gated = self.layer.experts, self.cfg.activation == "swiglu"
+        return (ex.htoh4.weight, ex.htoh4.bias, ex.htoh4_gate.weight if gated else None,
+                ex.htoh4_gate.bias if gated else None, ex.h4toh.weight, ex.h4toh.bias)
+
+    def route_and_run(self, x: torch.Tensor) -> torch.Tensor:
+        """Router and experts as one autograd node; for calls that ``one_node`` accepts."""
+        lin = self.layer.gate.gate
+        if hasattr(self.layer.gate, "set_loss"):
+            self.layer.gate.set_loss(None)
+        tensors = (x, lin.weight, lin.bias) + self._expert_tensors()
+        self._save_pre = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+        try:
+            y = _FusedLayerFn.apply(*tensors, self)
+        finally:
+            self._save_pre = True
+        if self.check_every_call:
+            self.ctx.check_status("fused MoE forward")
+        return y
 
     def route(self, x: torch.Tensor):
         """Router logits -> (idx [T, k] int32, weights [T, k] fp32) with the top-k softmax kernel; also sets the gate's
@@ -286,8 +326,7 @@ class FusedMoE:
         cfg, layer = self.cfg, self.layer
         if x.shape[0] > cfg.max_tokens:
             raise ValueError(f"{x.shape[0]} tokens exceed config.max_tokens={cfg.max_tokens}")
-        coef = getattr(layer.gate, "aux_loss_coef", 0.0)
-        zcoef = getattr(layer.gate, "z_loss_coef", 0.0)
+        coef, zcoef = self._aux_coefs()
         lin = getattr(layer.gate, "gate", None)
         if self.fused_router and isinstance(lin, torch.nn.Linear) and R.supported(x, lin.weight, cfg.top_k):
             # linear layer + top-k + softmax in one kernel. The logits are written (fp32) only when an auxiliary loss
@@ -315,16 +354,13 @@ class FusedMoE:
     def run_experts(self, x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """The expert-parallel part for given routing decisions. A slot whose expert id is negative is not routed
         (the routing kernels drop it, its gate weight gets a zero gradient from here)."""
-        cfg, layer = self.cfg, self.layer
         x = x.contiguous()
-        ex = layer.experts
-        wg = ex.htoh4_gate.weight if cfg.activation == "swiglu" else None
-        bg = ex.htoh4_gate.bias if cfg.activation == "swiglu" else None
-        tensors = (x, w, ex.htoh4.weight, ex.htoh4.bias, wg, bg, ex.h4toh.weight, ex.h4toh.bias)
+        experts = self._expert_tensors()
+        tensors = (x, w) + experts
         # without a backward pass to come the pre-activations need not be stored (inference / no_grad)
         self._save_pre = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
         try:
-            y = _FusedMoEFn.apply(x, w, idx, ex.htoh4.weight, ex.htoh4.bias, wg, bg, ex.h4toh.weight, ex.h4toh.bias, self)
+            y = _FusedMoEFn.apply(x, w, idx, *experts, self)
         finally:
             self._save_pre = True
         if self.check_every_call:
@@ -346,7 +382,7 @@ class FusedMoE:
         L.xrecv, L.comb = self.xrecv.data_ptr(), self.comb.data_ptr()
         L.h_act, L.h_pre, L.h_pre2 = self.h_act.data_ptr(), self.h_pre.data_ptr(), N.ptr(self.h_pre2)
         for name in ("slot_pos", "slot_row", "sorted_slot", "order_off", "local_begin", "local_rows", "count_raw",
-                     "count_kept", "dst_base", "group_base", "group_rows", "sent_rows", "table_copy"):
+                     "count_kept", "dst_base", "group_base", "group_rows", "sent_rows", "table_copy", "raw_order"):
             setattr(L, name, getattr(self, name).data_ptr())
         for name in ("grecv", "gcomb", "row_src", "row_gate", "tile_flags", "done", "done_cum", "block_hist", "block_off",
                      "ticket", "epoch_dev"):
@@ -604,6 +640,92 @@ class GraphedForwardPool:
         raise ValueError(f"{n} tokens exceed the largest bucket ({self.graphs[-1].tokens})")
 
 
+def _native_forward(fm: FusedMoE, x: torch.Tensor, idx: torch.Tensor, gate_w: torch.Tensor) -> torch.Tensor:
+    cfg, cc = fm.cfg, fm.ctx
+    t = x.shape[0]
+    y = torch.empty_like(x)
+    if not cc.device_epoch:
+        cc.epoch += 1
+    with nvtx_range("moe.forward_native"):
+        N.check(N.load().ccf_layer_forward(C.byref(fm.native_desc()), x.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
+                                           y.data_ptr(), t, cfg.capacity(t), int(fm._save_pre),
+                                           -1 if cc.device_epoch else cc.epoch, N.stream_ptr(), None, 0, None),
+                "ccf_layer_forward")
+    # kernels: route + plan (three where the slots do not fit one), dispatch + GEMM-1, GEMM-2 + combine, reduce; with peers
+    # also the wait
+    N.count(4 + int(fm.world > 1) + (2 if t * cfg.top_k > N.ROUTE_CLUSTER_SLOTS else 0))
+    return y
+
+
+def _native_backward(fm: FusedMoE, dy, idx, gate_w, dgate, w1, wg, w2, has_bias, router=None):
+    """Backward pass of the experts in one C call -> (dx, (dw1, db1, dwg, dbg, dw2, db2)). ``router = (wt, x, dwt, db)``:
+    the call included the router; dx then also carries the gradient through the gate weights, and dwt / db are written."""
+    cfg, cc = fm.cfg, fm.ctx
+    t, d, f, e_loc = dy.shape[0], cfg.d_model, cfg.d_ffn, cfg.experts_per_rank
+    swiglu = cfg.activation == "swiglu"
+    sgd2 = fm.sgd if (fm.sgd is not None and fm.sgd[0] != 0.0) else None
+    sgd = sgd2 if fm.world == 1 else None
+    has_b1, has_bg, has_b2 = has_bias
+    mk = torch.empty_like
+    bias = lambda n: torch.empty(e_loc, n, dtype=cfg.dtype, device=dy.device)   # noqa: E731
+    g = N.LayerGrads()
+    dh = torch.empty(fm.max_rows, f, dtype=cfg.dtype, device=dy.device)
+    dh2 = mk(dh) if swiglu else None
+    dw2 = None if sgd2 is not None else mk(w2)
+    dw1, dwg = (None, None) if sgd is not None else (mk(w1), (mk(wg) if swiglu else None))
+    db1, db2, dbg = (bias(f) if has_b1 else None), (bias(d) if has_b2 else None), (bias(f) if has_bg else None)
+    dx = mk(dy)
+    g.dgate, g.dh, g.dh2 = dgate.data_ptr(), dh.data_ptr(), N.ptr(dh2)
+    g.dw1, g.db1, g.dwg, g.dbg, g.dw2, g.db2, g.dx = (N.ptr(v) for v in (dw1, db1, dwg, dbg, dw2, db2, dx))
+    if sgd2 is not None:
+        g.sgd_lr, g.sgd_wd = float(sgd2[0]), float(sgd2[1])
+    if router is not None:
+        wt, x, dwt, drb = router
+        slot_grad = torch.empty(t * cfg.top_k, dtype=torch.float32, device=dy.device)
+        g.router_w, g.x, g.slot_grad = wt.data_ptr(), x.data_ptr(), slot_grad.data_ptr()
+        g.router_dw, g.router_db = N.ptr(dwt), N.ptr(drb)
+    N.check(N.load().ccf_layer_backward(C.byref(fm.native_desc()), dy.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
+                                        C.byref(g), t, cfg.capacity(t), N.stream_ptr(), None, 0, None), "ccf_layer_backward")
+    # kernels: dy dispatch + dgrad-2, wgrad-2, wgrad-1 (two for SwiGLU), dgrad-1 + combine, reduce, column sums, the router's
+    # weight gradient; with peers also the wait
+    N.count(5 + int(fm.world > 1) + int(swiglu) + int(has_b1) + int(has_b2) + int(has_bg)
+            + int(router is not None and router[2] is not None))
+    if fm.check_every_call:
+        cc.check_status("fused MoE backward")
+    return dx, (dw1, db1, dwg, dbg, dw2, db2)
+
+
+class _FusedLayerFn(torch.autograd.Function):
+    """Router and experts of one call as one node (FusedMoE.one_node says when)."""
+
+    @staticmethod
+    def forward(ctx, x, rw, rb, w1, b1, wg, bg, w2, b2, fm: FusedMoE):
+        fm.ctx.ws.enter()
+        fm.claim_buffers(ctx)
+        rw = rw.contiguous()
+        idx, gate_w, _ = R.route_topk(x, rw, None if rb is None else rb.contiguous(), fm.cfg.top_k)
+        y = _native_forward(fm, x, idx, gate_w)
+        ctx.fm = fm
+        ctx.save_for_backward(x, rw, idx, gate_w, w1, wg, w2)
+        ctx.has_bias = (b1 is not None, bg is not None, b2 is not None)
+        ctx.has_router_bias = rb is not None
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        fm: FusedMoE = ctx.fm
+        fm.ctx.ws.enter()
+        fm.release_buffers(ctx)
+        x, rw, idx, gate_w, w1, wg, w2 = ctx.saved_tensors
+        need_rw, need_rb = ctx.needs_input_grad[1], ctx.has_router_bias and ctx.needs_input_grad[2]
+        # the gate gradient of a dropped slot stays unwritten: the reduction takes it as zero
+        dgate = torch.empty(gate_w.numel(), dtype=torch.float32, device=dy.device)
+        drw = torch.empty_like(rw) if (need_rw or need_rb) else None
+        drb = torch.empty(rw.shape[0], dtype=rw.dtype, device=dy.device) if need_rb else None
+        dx, grads = _native_backward(fm, dy.contiguous(), idx, gate_w, dgate, w1, wg, w2, ctx.has_bias, (rw, x, drw, drb))
+        return (dx, drw if need_rw else None, drb) + grads + (None,)
+
+
 class _FusedMoEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate_w, idx, w1, b1, wg, bg, w2, b2, fm: FusedMoE):
@@ -614,16 +736,7 @@ class _FusedMoEFn(torch.autograd.Function):
         fm.ctx.ws.enter()
         fm.claim_buffers(ctx)
         if fm.native_runtime:
-            y = torch.empty(t, d, dtype=x.dtype, device=x.device)
-            cc = fm.ctx
-            if not cc.device_epoch:
-                cc.epoch += 1
-            with nvtx_range("moe.forward_native"):
-                N.check(N.load().ccf_layer_forward(C.byref(fm.native_desc()), x.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
-                                                   y.data_ptr(), t, cfg.capacity(t), int(fm._save_pre),
-                                                   -1 if cc.device_epoch else cc.epoch, N.stream_ptr(), None, 0, None),
-                        "ccf_layer_forward")
-            N.count(7)   # kernels: route (2), plan, dispatch + GEMM-1, GEMM-2 + combine, wait, reduce
+            y = _native_forward(fm, x, idx, gate_w)
             ctx.fm = fm
             ctx.tokens = t
             ctx.save_for_backward(idx, gate_w, w1, wg, w2)
@@ -664,27 +777,8 @@ class _FusedMoEFn(torch.autograd.Function):
         sgd2 = fm.sgd if (fm.sgd is not None and fm.sgd[0] != 0.0) else None
         sgd = sgd2 if fm.world == 1 else None
         if fm.native_runtime:
-            has_b1, has_bg, has_b2 = ctx.has_bias
-            mk = lambda like: torch.empty_like(like)                       # noqa: E731
-            bias = lambda n: torch.empty(e_loc, n, dtype=cfg.dtype, device=dy.device)   # noqa: E731
-            g = N.LayerGrads()
-            dh = torch.empty(fm.max_rows, f, dtype=cfg.dtype, device=dy.device)
-            dh2 = torch.empty_like(dh) if swiglu else None
-            dw2 = None if sgd2 is not None else mk(w2)
-            dw1, dwg = (None, None) if sgd is not None else (mk(w1), (mk(wg) if swiglu else None))
-            db1, db2, dbg = (bias(f) if has_b1 else None), (bias(d) if has_b2 else None), (bias(f) if has_bg else None)
-            dx = torch.empty(t, d, dtype=dy.dtype, device=dy.device)
-            g.dgate, g.dh, g.dh2 = dgate.data_ptr(), dh.data_ptr(), N.ptr(dh2)
-            g.dw1, g.db1, g.dwg, g.dbg, g.dw2, g.db2, g.dx = (N.ptr(v) for v in (dw1, db1, dwg, dbg, dw2, db2, dx))
-            if sgd2 is not None:
-                g.sgd_lr, g.sgd_wd = float(sgd2[0]), float(sgd2[1])
-            N.check(lib.ccf_layer_backward(C.byref(fm.native_desc()), dy.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
-                                           C.byref(g), t, cfg.capacity(t), st, None, 0, None), "ccf_layer_backward")
-            # kernels: dy dispatch + dgrad-2, wgrad-2, wgrad-1 (two for SwiGLU), dgrad-1 + combine, wait, reduce, column sums
-            N.count(6 + int(swiglu) + int(has_b1) + int(has_b2) + int(has_bg))
-            if fm.check_every_call:
-                cc.check_status("fused MoE backward")
-            return dx, dgate.view(t, cfg.top_k), None, dw1, db1, dwg, dbg, dw2, db2, None
+            dx, grads = _native_backward(fm, dy, idx, gate_w, dgate, w1, wg, w2, ctx.has_bias)
+            return (dx, dgate.view(t, cfg.top_k), None) + grads + (None,)
         # 1+2. push g*dy rows (dispatch role) + dgrad-2 with the activation derivative in the epilogue
         disp = fm._dispatch_args(dy, t, idx, gate_w, backward=True, dgate=dgate)
         common = dict(group_base=fm.group_base, group_rows=fm.group_rows, num_groups=e_loc, wait_ns=cc.wait_ns,

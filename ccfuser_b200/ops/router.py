@@ -23,26 +23,31 @@ from . import gemm as G
 from .gemm import Workspace
 
 
+def route_topk(x: torch.Tensor, wt: torch.Tensor, bias, k: int, want_logits: bool = False):
+    """The router kernel on contiguous operands of one type -> (idx, w, fp32 logits or None); no autograd."""
+    t, d = x.shape
+    e = wt.shape[0]
+    idx = torch.empty(t, k, dtype=torch.int32, device=x.device)
+    w = torch.empty(t, k, dtype=torch.float32, device=x.device)
+    logits = torch.empty(t, e, dtype=torch.float32, device=x.device) if want_logits else None
+    ws = Workspace.get(x.device)
+    dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
+    N.check(N.load().ccf_router_topk(x.data_ptr(), wt.data_ptr(), N.ptr(bias), t, d, e, k, int(x.dtype == torch.float16),
+                                     idx.data_ptr(), w.data_ptr(), N.ptr(logits), ws.status.data_ptr(),
+                                     5_000_000_000, dev, N.stream_ptr()), "ccf_router_topk")
+    N.count(1)
+    return idx, w, logits
+
+
 class _FusedRouter(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, k, want_logits):
-        lib = N.load()
-        t, d = x.shape
-        e = weight.shape[0]
         if x.dtype not in (torch.bfloat16, torch.float16) or weight.dtype != x.dtype:
             raise TypeError("fused router: x and the router weight must both be bf16 or both fp16")
         x = x.contiguous()
         wt = weight.contiguous()
         b = None if bias is None else bias.to(x.dtype).contiguous()
-        idx = torch.empty(t, k, dtype=torch.int32, device=x.device)
-        w = torch.empty(t, k, dtype=torch.float32, device=x.device)
-        logits = torch.empty(t, e, dtype=torch.float32, device=x.device) if want_logits else None
-        ws = Workspace.get(x.device)
-        dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
-        N.check(lib.ccf_router_topk(x.data_ptr(), wt.data_ptr(), N.ptr(b), t, d, e, k, int(x.dtype == torch.float16),
-                                    idx.data_ptr(), w.data_ptr(), N.ptr(logits), ws.status.data_ptr(),
-                                    5_000_000_000, dev, N.stream_ptr()), "ccf_router_topk")
-        N.count(1)
+        idx, w, logits = route_topk(x, wt, b, k, want_logits)
         ctx.save_for_backward(x, wt, idx, w)
         ctx.has_bias = bias is not None
         ctx.mark_non_differentiable(idx)

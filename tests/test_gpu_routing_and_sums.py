@@ -1,8 +1,139 @@
-"""Column sums and the router's split over d at the edges of their blocks and clusters, against fp64 sums."""
+"""Routing + plan in one kernel, slot reduction, router weight gradient, column sums and the router's split over d: at the
+edges of their blocks, clusters and dispatch rules, against fp64 sums or the separate kernels they replace."""
+import ctypes as C
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+def _plan_args(N, e, kept, max_rows, epoch):
+    i32 = dict(dtype=torch.int32, device="cuda")
+    out = {k: torch.full((e,), -7, **i32) for k in ("dst_base", "group_base", "group_rows", "local_begin", "local_rows")}
+    out["sent_rows"], out["table_copy"] = torch.full((8,), -7, **i32), torch.full((e,), -7, **i32)
+    keep = {"table": torch.zeros(e, **i32), "flag": torch.zeros(8, **i32), "status": torch.zeros(2, **i32)}
+    p = N.PlanArgs()
+    p.count_kept = kept.data_ptr()
+    p.peer_table[0], p.peer_flag[0] = keep["table"].data_ptr(), keep["flag"].data_ptr()
+    for k, t in out.items():
+        setattr(p, k, t.data_ptr())
+    p.status, p.wait_limit_ns = keep["status"].data_ptr(), 1_000_000_000
+    p.world, p.my_rank, p.e_total, p.e_loc, p.epoch, p.max_rows = 1, 0, e, e, epoch, max_rows
+    return p, out, keep
+
+
+@pytest.mark.parametrize("slots,e,cap,first", [(1, 1, 1, 0), (31, 4, 100, 2), (1024, 64, 20, 0), (1025, 256, 1 << 20, 255),
+                                              (4097, 64, 50, 3), (16384, 8, 2000, 0), (32768, 64, 1 << 20, 0),
+                                              (40000, 16, 2600, 5), (65536, 256, 300, 128)])
+def test_route_plan_equals_the_separate_kernels(slots, e, cap, first):
+    """Every output of the one-kernel form is the one of ccf_route_ordered + ccf_plan, with a receive buffer that some rows
+    do not fit and ids outside the table; raw_order lists all routed slots by expert in slot order."""
+    from ccfuser_b200 import native as N
+    lib = N.load()
+    g = torch.Generator(device="cuda").manual_seed(slots)
+    expert = torch.randint(-1, e + 1, (slots,), dtype=torch.int32, device="cuda", generator=g)   # -1 and e: not routed
+    i32 = dict(dtype=torch.int32, device="cuda")
+    nb = (slots + 1023) // 1024
+    max_rows = max(128, slots // 2 // 128 * 128)
+    res = []
+    for one in (False, True):
+        t = {"pos": torch.zeros(slots, **i32), "raw": torch.zeros(e, **i32), "kept": torch.zeros(e, **i32),
+             "order_off": torch.zeros(e + 1, **i32), "sorted_slot": torch.full((slots,), -1, **i32),
+             "slot_row": torch.zeros(slots, **i32)}
+        p, out, keep = _plan_args(N, e, t["kept"], max_rows, 3)
+        if one:
+            raw_order = torch.full((N.MAX_GROUPS + slots,), -1, **i32)
+            N.check(lib.ccf_route_plan(expert.data_ptr(), slots, e, cap, t["pos"].data_ptr(), t["raw"].data_ptr(),
+                                       t["kept"].data_ptr(), t["order_off"].data_ptr(), t["sorted_slot"].data_ptr(),
+                                       t["slot_row"].data_ptr(), first, raw_order.data_ptr(), C.byref(p), None,
+                                       N.stream_ptr()), "ccf_route_plan")
+        else:
+            bh, bo, ticket = torch.zeros(nb * e, **i32), torch.zeros(nb * e, **i32), torch.zeros(1, **i32)
+            N.check(lib.ccf_route_ordered(expert.data_ptr(), slots, e, cap, t["pos"].data_ptr(), bh.data_ptr(), bo.data_ptr(),
+                                          t["raw"].data_ptr(), t["kept"].data_ptr(), ticket.data_ptr(),
+                                          t["order_off"].data_ptr(), t["sorted_slot"].data_ptr(), t["slot_row"].data_ptr(),
+                                          first, N.stream_ptr()), "ccf_route_ordered")
+            N.check(lib.ccf_plan(C.byref(p), N.stream_ptr()), "ccf_plan")
+        torch.cuda.synchronize()
+        res.append({**t, **out, "status": keep["status"]})
+    for k in res[0]:
+        assert torch.equal(res[0][k], res[1][k]), k
+    # the layout itself, from the counts
+    kept = res[1]["kept"].cpu()
+    padded = (kept + 127) // 128 * 128
+    base = torch.cumsum(padded, 0) - padded
+    assert torch.equal(res[1]["group_base"].cpu().long(), base)
+    assert int(res[1]["sent_rows"][0]) == int(torch.minimum(kept, (max_rows - base).clamp(min=0)).sum())
+    ids = expert.cpu()
+    for k in range(e):
+        ex = (first + k) % e
+        want = (ids == ex).nonzero().flatten().int()
+        start = int(raw_order[ex])
+        assert torch.equal(raw_order[N.MAX_GROUPS + start:N.MAX_GROUPS + start + want.numel()].cpu(), want)
+
+
+def test_route_plan_leaves_other_sizes_to_the_separate_kernels():
+    from ccfuser_b200 import native as N
+    kept = torch.zeros(4, dtype=torch.int32, device="cuda")
+    p, _, _ = _plan_args(N, 4, kept, 128, 1)
+    for slots in (0, N.ROUTE_CLUSTER_SLOTS + 1):
+        assert N.load().ccf_route_plan(0, slots, 4, 1, 0, 0, 0, 0, 0, 0, 0, 0, C.byref(p), None, N.stream_ptr()) == 1
+
+
+@pytest.mark.parametrize("tokens,k,d,fp16", [(1, 1, 64, False), (129, 2, 768, True), (77, 3, 4096, False), (33, 8, 512, True),
+                                            (40, 9, 256, False), (65, 2, 8192, False)])
+def test_combine_reduce(tokens, k, d, fp16):
+    from ccfuser_b200 import native as N
+    dt = torch.float16 if fp16 else torch.bfloat16
+    torch.manual_seed(tokens)
+    comb = torch.randn(tokens * k, d, device="cuda").to(dt)
+    row = torch.randint(-1, 5, (tokens * k,), dtype=torch.int32, device="cuda")
+    comb[row < 0] = float("nan")                                     # rows of dropped slots are never read
+    y = torch.empty(tokens, d, dtype=dt, device="cuda")
+    N.check(N.load().ccf_combine_reduce(comb.data_ptr(), row.data_ptr(), y.data_ptr(), tokens, k, d, int(fp16),
+                                        N.stream_ptr()), "ccf_combine_reduce")
+    ref = torch.where((row >= 0).unsqueeze(1), comb.double(), torch.zeros((), dtype=torch.float64, device="cuda"))
+    ref = ref.view(tokens, k, d).sum(1)
+    # one rounding to the element type after fp32 sums: with 8 (bf16) or 11 (fp16) significant bits half a unit in the last
+    # place is at most 2^-8 or 2^-11 of the value
+    ulp = 2.0 ** (-11 if fp16 else -8)
+    assert ((y.double() - ref).abs() <= ref.abs() * ulp * 1.01 + 1e-6).all()
+
+
+@pytest.mark.parametrize("act,e,k,t,cf,dtype", [("gelu", 4, 2, 300, None, torch.bfloat16), ("relu", 16, 1, 129, 1.0, torch.float16),
+                                               ("swiglu", 8, 3, 1000, 0.5, torch.bfloat16),
+                                               ("gelu", 64, 2, 4500, 1.25, torch.bfloat16), ("gelu", 2, 2, 1, None, torch.float16)])
+def test_one_node_layer_equals_router_then_experts(act, e, k, t, cf, dtype):
+    """Router and experts as one autograd node against the two nodes (same kernels for everything but the router's
+    backward): outputs are the same bits, dx differs by roundings of its two addends, the router's gradients by the
+    rounding of the dense logit gradient the two-node form multiplies with."""
+    from ccfuser_b200 import MoEConfig, MoELayer
+    torch.manual_seed(e + t)
+    d, f = 256, 512
+    cfg = MoEConfig(d_model=d, d_ffn=f, num_experts=e, top_k=k, capacity_factor=cf, activation=act, dtype=dtype,
+                    backend="fused", max_tokens=t)
+    layer = MoELayer(cfg, device="cuda")
+    fm = layer._fused_impl()
+    x = torch.randn(t, d, device="cuda", dtype=dtype).requires_grad_()
+    gy = torch.randn(t, d, device="cuda", dtype=dtype)
+    got = []
+    for one in (False, True):
+        assert fm.one_node(x)
+        for p in [x, *layer.parameters()]:
+            p.grad = None
+        y = layer(x) if one else fm.run_experts(x, *fm.route(x))
+        y.backward(gy)
+        got.append({"y": y.detach(), "x": x.grad, **{n: p.grad for n, p in layer.named_parameters()}})
+    layer.check_status()
+    eps = 2.0 ** (-10 if dtype == torch.float16 else -7)
+    for n in got[0]:
+        a, b = got[0][n].double(), got[1][n].double()
+        if n.startswith("experts") or n == "y":
+            assert torch.equal(a, b), n
+        else:
+            assert (a - b).norm() <= 2 * eps * a.norm() + 1e-6, n
+    layer.release()
 
 
 @pytest.mark.parametrize("t,d,e,k,dtype,bias", [(1, 128, 3, 2, torch.bfloat16, True), (127, 256, 8, 2, torch.float16, False),
