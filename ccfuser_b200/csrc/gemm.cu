@@ -55,6 +55,8 @@ struct __align__(16) Ctrl {
   int pad;
   int sched_tile[kSchedSlots];
   int mt_prefix[CCF_MAX_GROUPS + 1];
+  int base[CCF_MAX_GROUPS];   // first row and number of rows of each group: every role decodes every tile, and a global
+  int rows[CCF_MAX_GROUPS];   // read per decode would sit in front of each tile's first load
 };
 
 constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kEpiWarps * kEpiStageBytes + static_cast<int>(sizeof(Ctrl));
@@ -74,8 +76,8 @@ __device__ __forceinline__ Tile decode_tile(int t, const CcfGemmArgs& a, const C
     const int mt_g = c->mt_prefix[lo + 1] - c->mt_prefix[lo];
     const int local = t - nt * c->mt_prefix[lo];
     const int j = local / mt_g, i = local - j * mt_g;
-    const int rows = a.group_rows[lo];
-    ti.row0 = a.group_base[lo] + i * BM;
+    const int rows = c->rows[lo];
+    ti.row0 = c->base[lo] + i * BM;
     ti.rows_valid = min(BM, rows - i * BM);
     ti.n0 = j * bn_out;
     ti.kblocks = a.kseg * ((a.k + BK - 1) / BK);
@@ -89,16 +91,55 @@ __device__ __forceinline__ Tile decode_tile(int t, const CcfGemmArgs& a, const C
     ti.row0 = i * BM;
     ti.rows_valid = BM;
     ti.n0 = j * BN;
-    ti.kblocks = (a.group_rows[ti.g] + BK - 1) / BK;
-    ti.krow0 = a.group_base[ti.g];
+    ti.kblocks = (c->rows[ti.g] + BK - 1) / BK;
+    ti.krow0 = c->base[ti.g];
   }
   return ti;
+}
+
+// Tile tables of one launch, filled by one warp of every CTA at start-up: 32 groups at a time, prefix sums by shuffles.
+// One thread walking the groups paid a global-memory latency for every few groups, in every CTA of every launch.
+template <bool kKGroup>
+__device__ __forceinline__ void tile_tables_warp(const CcfGemmArgs& args, Ctrl* ctrl, int bn_out, int lane) {
+  const int nt = (args.n + bn_out - 1) / bn_out;
+  int acc = 0, rows = 0;
+  for (int g0 = 0; g0 < args.num_groups; g0 += 32) {
+    const int g = g0 + lane;
+    int gr = 0;
+    if (g < args.num_groups) {
+      gr = args.group_rows[g];
+      ctrl->rows[g] = gr;
+      ctrl->base[g] = args.group_base[g];
+    }
+    if constexpr (!kKGroup) {
+      const int mt = (gr + BM - 1) / BM;
+      int sm = mt, sr = gr;   // inclusive scans
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int vm = __shfl_up_sync(0xffffffffu, sm, off), vr = __shfl_up_sync(0xffffffffu, sr, off);
+        if (lane >= off) { sm += vm; sr += vr; }
+      }
+      if (g < args.num_groups) ctrl->mt_prefix[g] = acc + sm - mt;
+      acc += __shfl_sync(0xffffffffu, sm, 31);
+      rows += __shfl_sync(0xffffffffu, sr, 31);
+    }
+  }
+  if (lane == 0) {
+    ctrl->n_tiles = nt;
+    if constexpr (!kKGroup) {
+      ctrl->mt_prefix[args.num_groups] = acc;
+      ctrl->total_tiles = acc * nt;
+      ctrl->total_rows = rows;
+    } else {
+      ctrl->total_tiles = args.num_groups * (args.m_per_group / BM) * nt;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------------------------------
-template <int kAMajor, int kBMajor, int kEpi, bool kKGroup>
+template <int kAMajor, int kBMajor, int kEpi, bool kKGroup, int kFp16>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
@@ -129,22 +170,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
       mbar_init(smem_u32(&ctrl->sched_empty[s]), 1 + kEpiWarps);
     }
     ctrl->abort_word = 0;
-    const int nt = (args.n + bn_out - 1) / bn_out;
-    ctrl->n_tiles = nt;
-    if constexpr (!kKGroup) {
-      int acc = 0;
-      for (int g = 0; g < args.num_groups; ++g) {
-        ctrl->mt_prefix[g] = acc;
-        acc += (args.group_rows[g] + BM - 1) / BM;
-      }
-      ctrl->mt_prefix[args.num_groups] = acc;
-      ctrl->total_tiles = acc * nt;
-      int rows = 0;
-      for (int g = 0; g < args.num_groups; ++g) rows += args.group_rows[g];
-      ctrl->total_rows = rows;
-    } else {
-      ctrl->total_tiles = args.num_groups * (args.m_per_group / BM) * nt;
-    }
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&tmA0);
@@ -158,6 +183,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
     tmem_alloc(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish();
   }
+  if (warp == 2) tile_tables_warp<kKGroup>(args, ctrl, bn_out, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -360,7 +386,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + ti.row0;
       else row_base = ti.row0;
-      const CombineDest cd = epilogue_tile<kEpi>(args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane);
+      const CombineDest cd = epilogue_tile<kEpi, kFp16>(args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane);
       if (warp == 2 && lane == 0) trace_ev(args, seq, 7);
       if (have_acc) {
         // all TMEM reads of this accumulator stage are complete: hand it back to the MMA warp
@@ -489,9 +515,9 @@ int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, 
   return 0;
 }
 
-template <int A, int B, int E, bool KG>
-static int launch_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
-  auto kern = grouped_gemm_kernel<A, B, E, KG>;
+template <int A, int B, int E, bool KG, int FP16>
+static int launch_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+  auto kern = grouped_gemm_kernel<A, B, E, KG, FP16>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
   int dev = 0;
@@ -504,6 +530,11 @@ static int launch_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int gr
   kern<<<grid, kThreads, kSmemBytes, stream>>>(tm[0], tm[1], tm[2], tm[3], args);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
+}
+
+template <int A, int B, int E, bool KG>
+static int launch_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+  return args.fp16 ? launch_variant_of<A, B, E, KG, 1>(tm, args, grid, stream) : launch_variant_of<A, B, E, KG, 0>(tm, args, grid, stream);
 }
 
 }  // namespace ccf

@@ -37,6 +37,8 @@ struct __align__(16) Ctrl2 {
   int tiles_a;                          // pair tiles (x n-tiles) of phase A: made only of rows this rank pushed itself
   int mt_prefix[CCF_MAX_GROUPS + 1];    // phase B (all other pair tiles), prefix over groups
   int mta_prefix[CCF_MAX_GROUPS + 1];   // phase A, prefix over groups
+  int base[CCF_MAX_GROUPS];             // first row and number of rows of each group: every role decodes every tile, and a
+  int rows[CCF_MAX_GROUPS];             // global read per decode would sit in front of each tile's first load
   short a0[CCF_MAX_GROUPS];             // first phase-A pair tile of each group
   short na[CCF_MAX_GROUPS];             // number of phase-A pair tiles of each group
 };
@@ -144,8 +146,8 @@ __host__ __device__ __forceinline__ PairTile decode_pair_tile(int t, const CcfGe
     int i = local - j * mt_g;
     if (phase_a) i += c->a0[lo];
     else if (i >= c->a0[lo]) i += c->na[lo];
-    ti.row0 = a.group_base[lo] + i * PM;
-    ti.rows_pair = min(PM, a.group_rows[lo] - i * PM);
+    ti.row0 = c->base[lo] + i * PM;
+    ti.rows_pair = min(PM, c->rows[lo] - i * PM);
     ti.n0 = j * bn_out;
     ti.kblocks = a.kseg * ((a.k + BK - 1) / BK);
     ti.krow0 = 0;
@@ -158,42 +160,39 @@ __host__ __device__ __forceinline__ PairTile decode_pair_tile(int t, const CcfGe
     ti.row0 = i * PM;
     ti.rows_pair = PM;
     ti.n0 = j * BN;
-    ti.kblocks = (a.group_rows[ti.g] + BK - 1) / BK;
-    ti.krow0 = a.group_base[ti.g];
+    ti.kblocks = (c->rows[ti.g] + BK - 1) / BK;
+    ti.krow0 = c->base[ti.g];
   }
   return ti;
 }
 
-// Tile tables of one launch, computed by one thread of every CTA at start-up (host-callable so that the tile order can
-// be checked exhaustively without a GPU): number of column tiles; pair tiles per group, split into phase A (tiles that
-// hold only rows this rank pushed itself) and phase B (the rest) with their prefix sums; total tiles and total rows.
+// Tile tables of one launch, filled by every CTA at start-up: number of column tiles; pair tiles per group, split into
+// phase A (tiles that hold only rows this rank pushed itself) and phase B (the rest) with their prefix sums; total tiles
+// and total rows. One group's share (host-callable so that the tile order can be checked exhaustively without a GPU):
+__host__ __device__ __forceinline__ void pair_group_tiles(const CcfGemmArgs& args, Ctrl2* ctrl, int g, int& n_a, int& n_b) {
+  const int gr = ctrl->rows[g];
+  const int mt = (gr + PM - 1) / PM;
+  int a0 = 0, na = 0;
+  if (args.local_begin != nullptr && args.tile_flags != nullptr) {
+    const int lb = args.local_begin[g], le = min(gr, lb + args.local_rows[g]);
+    a0 = (lb + PM - 1) / PM;
+    // a tile is local-only when it lies inside [lb, le); the last tile of the group also counts when le == gr
+    const int a1 = (le == gr) ? mt : le / PM;
+    na = max(0, a1 - a0);
+    if (na == 0) a0 = 0;
+  }
+  ctrl->a0[g] = static_cast<short>(a0);
+  ctrl->na[g] = static_cast<short>(na);
+  n_a = na;
+  n_b = mt - na;
+}
+
 template <bool kKGroup, int kEpi>
-__host__ __device__ __forceinline__ void pair_tile_tables(const CcfGemmArgs& args, Ctrl2* ctrl) {
+__host__ __device__ __forceinline__ void pair_tile_totals(const CcfGemmArgs& args, Ctrl2* ctrl, int acc_a, int acc_b, int rows) {
   constexpr int bn_out = (kEpi == CCF_EPI_SWIGLU) ? BN / 2 : BN;
   const int nt = (args.n + bn_out - 1) / bn_out;
   ctrl->n_tiles = nt;
   if constexpr (!kKGroup) {
-    int acc_a = 0, acc_b = 0, rows = 0;
-    for (int g = 0; g < args.num_groups; ++g) {
-      const int gr = args.group_rows[g];
-      const int mt = (gr + PM - 1) / PM;
-      int a0 = 0, na = 0;
-      if (args.local_begin != nullptr && args.tile_flags != nullptr) {
-        const int lb = args.local_begin[g], le = min(gr, lb + args.local_rows[g]);
-        a0 = (lb + PM - 1) / PM;
-        // a tile is local-only when it lies inside [lb, le); the last tile of the group also counts when le == gr
-        int a1 = (le == gr) ? mt : le / PM;
-        na = max(0, a1 - a0);
-        if (na == 0) a0 = 0;
-      }
-      ctrl->a0[g] = static_cast<short>(a0);
-      ctrl->na[g] = static_cast<short>(na);
-      ctrl->mta_prefix[g] = acc_a;
-      ctrl->mt_prefix[g] = acc_b;
-      acc_a += na;
-      acc_b += mt - na;
-      rows += gr;
-    }
     ctrl->mta_prefix[args.num_groups] = acc_a;
     ctrl->mt_prefix[args.num_groups] = acc_b;
     ctrl->tiles_a = acc_a * nt;
@@ -204,7 +203,59 @@ __host__ __device__ __forceinline__ void pair_tile_tables(const CcfGemmArgs& arg
   }
 }
 
-template <int kAMajor, int kBMajor, int kEpi, bool kKGroup>
+// The same by one warp: 32 groups at a time, prefix sums by shuffles. One thread walking the groups paid a global-memory
+// latency for every few groups, in every CTA of every launch.
+template <bool kKGroup, int kEpi>
+__device__ __forceinline__ void pair_tile_tables_warp(const CcfGemmArgs& args, Ctrl2* ctrl, int lane) {
+  int acc_a = 0, acc_b = 0, rows = 0;
+  for (int g0 = 0; g0 < args.num_groups; g0 += 32) {
+    const int g = g0 + lane;
+    int n_a = 0, n_b = 0, gr = 0;
+    if (g < args.num_groups) {
+      gr = args.group_rows[g];
+      ctrl->rows[g] = gr;
+      ctrl->base[g] = args.group_base[g];
+      if constexpr (!kKGroup) pair_group_tiles(args, ctrl, g, n_a, n_b);
+    }
+    if constexpr (!kKGroup) {
+      int sa = n_a, sb = n_b, sr = gr;   // inclusive scans
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int va = __shfl_up_sync(0xffffffffu, sa, off), vb = __shfl_up_sync(0xffffffffu, sb, off);
+        const int vr = __shfl_up_sync(0xffffffffu, sr, off);
+        if (lane >= off) { sa += va; sb += vb; sr += vr; }
+      }
+      if (g < args.num_groups) {
+        ctrl->mta_prefix[g] = acc_a + sa - n_a;
+        ctrl->mt_prefix[g] = acc_b + sb - n_b;
+      }
+      acc_a += __shfl_sync(0xffffffffu, sa, 31);
+      acc_b += __shfl_sync(0xffffffffu, sb, 31);
+      rows += __shfl_sync(0xffffffffu, sr, 31);
+    }
+  }
+  if (lane == 0) pair_tile_totals<kKGroup, kEpi>(args, ctrl, acc_a, acc_b, rows);
+}
+
+// host: the tables of a row-grouped launch
+template <int kEpi>
+static void pair_tile_tables_host(const CcfGemmArgs& args, Ctrl2* ctrl) {
+  int acc_a = 0, acc_b = 0, rows = 0;
+  for (int g = 0; g < args.num_groups; ++g) {
+    ctrl->rows[g] = args.group_rows[g];
+    ctrl->base[g] = args.group_base[g];
+    int n_a, n_b;
+    pair_group_tiles(args, ctrl, g, n_a, n_b);
+    ctrl->mta_prefix[g] = acc_a;
+    ctrl->mt_prefix[g] = acc_b;
+    acc_a += n_a;
+    acc_b += n_b;
+    rows += args.group_rows[g];
+  }
+  pair_tile_totals<false, kEpi>(args, ctrl, acc_a, acc_b, rows);
+}
+
+template <int kAMajor, int kBMajor, int kEpi, bool kKGroup, int kFp16>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                          const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
@@ -232,7 +283,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       mbar_init(smem_u32(&ctrl->acc_empty[s]), 2 * kEpiWarps);
     }
     ctrl->abort_word = 0;
-    pair_tile_tables<kKGroup, kEpi>(args, ctrl);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&tmA0);
@@ -246,6 +296,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
+  if (warp == 2) pair_tile_tables_warp<kKGroup, kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
@@ -426,7 +477,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + tt.row0;
       else row_base = tt.row0;
-      const CombineDest cd = epilogue_tile<kEpi>(args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane);
+      const CombineDest cd = epilogue_tile<kEpi, kFp16>(args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane);
       if (warp == 2 && lane == 0) trace_ev(args, seq, 7);
       if (have_acc) {
         tc_fence_before();
@@ -470,9 +521,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
   }
 }
 
-template <int A, int B, int E, bool KG>
-static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
-  auto kern = grouped_gemm_pair_kernel<A, B, E, KG>;
+template <int A, int B, int E, bool KG, int FP16>
+static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+  auto kern = grouped_gemm_pair_kernel<A, B, E, KG, FP16>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
   int dev = 0;
@@ -496,6 +547,12 @@ static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, i
   cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], args);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
+}
+
+template <int A, int B, int E, bool KG>
+static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+  return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1>(tm, args, grid, stream)
+                   : launch_pair_variant_of<A, B, E, KG, 0>(tm, args, grid, stream);
 }
 
 // Called by ccf_gemm_launch (gemm.cu) when the two-CTA kernel is requested. `key` encodes (A-major, B-major, epilogue,
@@ -550,7 +607,7 @@ extern "C" int ccf_debug_pair_tile_order(const int* group_base, const int* group
   Ctrl2* c = new Ctrl2;
   int total;
   if (swiglu) {
-    pair_tile_tables<false, CCF_EPI_SWIGLU>(a, c);
+    pair_tile_tables_host<CCF_EPI_SWIGLU>(a, c);
     total = c->total_tiles;
     for (int t = 0; t < total && t < cap; ++t) {
       const PairTile ti = decode_pair_tile<false, CCF_EPI_SWIGLU>(t, a, c);
@@ -558,7 +615,7 @@ extern "C" int ccf_debug_pair_tile_order(const int* group_base, const int* group
       memcpy(out + 5 * t, rec, sizeof(rec));
     }
   } else {
-    pair_tile_tables<false, CCF_EPI_STORE>(a, c);
+    pair_tile_tables_host<CCF_EPI_STORE>(a, c);
     total = c->total_tiles;
     for (int t = 0; t < total && t < cap; ++t) {
       const PairTile ti = decode_pair_tile<false, CCF_EPI_STORE>(t, a, c);

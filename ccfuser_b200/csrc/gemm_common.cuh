@@ -40,40 +40,48 @@ struct Tile {
 // erf as an odd polynomial: erf(z) ~= z * P(z^2) on |z| <= 3 (degree 8 in z^2, fitted minimax-style; |error| <= 2.6e-5
 // in fp32 Horner form, erf(3) = 1 - 2.2e-5 beyond the clamp), far below bf16 / fp16 resolution. No MUFU operation and
 // no branch: libm's erff and the exp/rcp-based forms kept the SFU pipe busy for ~4 k cycles per 128x256 tile.
-__device__ __forceinline__ float erf_poly(float z) {
-  z = fminf(fmaxf(z, -3.f), 3.f);
-  const float u = z * z;
-  float p = 4.074189994e-08f;
-  p = fmaf(p, u, -1.944814854e-06f);
-  p = fmaf(p, u, 4.106040073e-05f);
-  p = fmaf(p, u, -5.110358431e-04f);
-  p = fmaf(p, u, 4.235422620e-03f);
-  p = fmaf(p, u, -2.510284860e-02f);
-  p = fmaf(p, u, 1.110793178e-01f);
-  p = fmaf(p, u, -3.753148649e-01f);
-  p = fmaf(p, u, 1.128268424e+00f);
-  return p * z;
+// Two elements at a time (packed fp32 multiply-adds): the epilogue warps are bound by the instructions they issue, and the
+// polynomial is most of an activation epilogue's.
+__device__ __forceinline__ f32x2 erf_poly2(f32x2 z) {
+  float z0, z1;
+  upk2(z, z0, z1);
+  z = pk2(fminf(fmaxf(z0, -3.f), 3.f), fminf(fmaxf(z1, -3.f), 3.f));
+  const f32x2 u = mul2(z, z);
+  f32x2 p = bc2(4.074189994e-08f);
+  p = fma2(p, u, bc2(-1.944814854e-06f));
+  p = fma2(p, u, bc2(4.106040073e-05f));
+  p = fma2(p, u, bc2(-5.110358431e-04f));
+  p = fma2(p, u, bc2(4.235422620e-03f));
+  p = fma2(p, u, bc2(-2.510284860e-02f));
+  p = fma2(p, u, bc2(1.110793178e-01f));
+  p = fma2(p, u, bc2(-3.753148649e-01f));
+  p = fma2(p, u, bc2(1.128268424e+00f));
+  return mul2(p, z);
 }
 __device__ __forceinline__ float fast_rcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));  // branch-free, 1 ulp: keeps the element loops interleavable
   return y;
 }
-__device__ __forceinline__ float gelu_f(float x) {
-  const float hx = 0.5f * x;
-  return fmaf(hx, erf_poly(x * 0.70710678118654752f), hx);
+__device__ __forceinline__ void gelu2(float& x0, float& x1) {
+  const f32x2 x = pk2(x0, x1), hx = mul2(x, bc2(0.5f));
+  upk2(fma2(hx, erf_poly2(mul2(x, bc2(0.70710678118654752f))), hx), x0, x1);
 }
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  const float cdf = fmaf(0.5f, erf_poly(x * 0.70710678118654752f), 0.5f);
-  const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
-  return fmaf(x, pdf, cdf);
+// f *= gelu'(x)
+__device__ __forceinline__ void gelu_grad2(float& f0, float& f1, float x0, float x1) {
+  const f32x2 x = pk2(x0, x1);
+  const f32x2 cdf = fma2(bc2(0.5f), erf_poly2(mul2(x, bc2(0.70710678118654752f))), bc2(0.5f));
+  float e0, e1;
+  upk2(mul2(mul2(bc2(-0.5f), x), x), e0, e1);
+  const f32x2 pdf = mul2(bc2(0.3989422804014327f), pk2(__expf(e0), __expf(e1)));
+  upk2(mul2(pk2(f0, f1), fma2(x, pdf, cdf)), f0, f1);
 }
 // The activation switch sits outside the element loop: with a branch per element the compiler cannot
 // interleave the 32 independent dependency chains and the epilogue ran ~200 clocks per element.
 __device__ __forceinline__ void act32(float (&f)[32], int act) {
   if (act == CCF_ACT_GELU) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) f[i] = gelu_f(f[i]);
+    for (int i = 0; i < 32; i += 2) gelu2(f[i], f[i + 1]);
   } else if (act == CCF_ACT_RELU) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] = fmaxf(f[i], 0.f);
@@ -83,7 +91,7 @@ __device__ __forceinline__ void act32(float (&f)[32], int act) {
 __device__ __forceinline__ void act_grad32(float (&f)[32], const float (&pz)[32], int act) {
   if (act == CCF_ACT_GELU) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) f[i] *= gelu_grad_f(pz[i]);
+    for (int i = 0; i < 32; i += 2) gelu_grad2(f[i], f[i + 1], pz[i], pz[i + 1]);
   } else if (act == CCF_ACT_RELU) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] = pz[i] > 0.f ? f[i] : 0.f;
@@ -139,8 +147,8 @@ __device__ __forceinline__ void add_bias_raw(float (&f)[32], const uint4 (&raw)[
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 t = unpack2(w[j], fp16);
-      f[i * 8 + j * 2] += t.x;
-      f[i * 8 + j * 2 + 1] += t.y;
+      float &f0 = f[i * 8 + j * 2], &f1 = f[i * 8 + j * 2 + 1];
+      upk2(add2(pk2(f0, f1), pk2(t.x, t.y)), f0, f1);
     }
   }
 }
@@ -314,11 +322,13 @@ __device__ __forceinline__ void sgd_unstage(uint32_t stage, int lane, const uint
   __syncwarp();
 }
 
-template <int kEpi>
+// kFp16 is a template argument: as a run-time value every conversion of an element pair computed both types' results and
+// selected one, about a third of an epilogue's instructions.
+template <int kEpi, int kFp16>
 __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, const Tile& ti, long long row_base,
                                                      int rows_valid, int rows_store, bool have_acc, uint32_t t_row,
                                                      uint32_t stage, int q, int half, int lane) {
-  const int fp16 = args.fp16;
+  constexpr int fp16 = kFp16;
   const int r_in_tile = q * 32 + lane;
   const bool valid = r_in_tile < rows_valid;
   const long long orow = row_base + r_in_tile;
@@ -343,6 +353,31 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
   // 128-column narrow tile)
   const int n_chunks = (kEpi == CCF_EPI_SWIGLU || args.bn == 128) ? 2 : 4;
   const int chunk0 = half * n_chunks;
+  // A warp whose 32 rows all lie beyond the data has nothing to compute: with few rows per expert (decoding, the last tile
+  // of every group) most warps are of that kind and only held the others' issue slots. Outputs that a weight-gradient
+  // reduction may read get their zeros.
+  if (q * 32 >= rows_valid) {
+    if constexpr (kEpi != CCF_EPI_STORE && kEpi != CCF_EPI_COMBINE) {
+      const uint32_t zero[16] = {};
+      const int ok = min(32, max(0, rows_store - q * 32));
+      for (int c = 0; c < n_chunks; ++c) {
+        const int n = ti.n0 + (chunk0 + c) * 32;
+        if (n >= args.n || ok == 0) break;
+        auto put = [&](void* p) {
+          if (p != nullptr)
+            staged_store64_lin(stage, lane, zero, addr2(p, row_base + q * 32, args.ld_out, n),
+                               static_cast<unsigned long long>(args.ld_out) * 2ull, ok);
+        };
+        put(args.out0);
+        if constexpr (kEpi != CCF_EPI_DACT) put(args.out1);
+        if constexpr (kEpi == CCF_EPI_SWIGLU) put(args.out2);
+      }
+    }
+    CombineDest none;
+    none.rank = 0;
+    none.ok = false;
+    return none;
+  }
   uint32_t racc[32];  // one buffer: the next chunk is requested right after this one is copied out to f[]
   if (have_acc) tmem_ld32(t_row + chunk0 * 32, racc);
   constexpr bool kBias0Prefetch = (kEpi == CCF_EPI_STORE || kEpi == CCF_EPI_BIAS_ACT || kEpi == CCF_EPI_COMBINE);
@@ -422,9 +457,9 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
           staged_store64_lin(stage, lane, w, lin_of(args.out2) + n * 2ull, lin_stride, lin_rows_store);
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float sg = fast_rcp(1.f + __expf(-f[i]));
-          f[i] = f[i] * sg * u[i];
+        for (int i = 0; i < 32; i += 2) {
+          const f32x2 sg = pk2(fast_rcp(1.f + __expf(-f[i])), fast_rcp(1.f + __expf(-f[i + 1])));
+          upk2(mul2(mul2(pk2(f[i], f[i + 1]), sg), pk2(u[i], u[i + 1])), f[i], f[i + 1]);
         }
         pack32(f, w, fp16);
         staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
@@ -442,7 +477,10 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const float2 p = unpack2(w[j], fp16);
-            w[j] = pack2(p.x - lr * fmaf(wd, p.x, f[2 * j]), p.y - lr * fmaf(wd, p.y, f[2 * j + 1]), fp16);
+            const f32x2 p2 = pk2(p.x, p.y);
+            float n0, n1;
+            upk2(fma2(bc2(-lr), fma2(bc2(wd), p2, pk2(f[2 * j], f[2 * j + 1])), p2), n0, n1);
+            w[j] = pack2(n0, n1, fp16);
           }
           staged_store64_lin(stage, lane, w, lin_base + n * 2ull, lin_stride, lin_rows);
         } else {
@@ -465,7 +503,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
       } else if constexpr (kEpi == CCF_EPI_COMBINE) {
         if (has_b0) add_bias_raw(f, bcur, fp16);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] *= c_gate;
+        for (int i = 0; i < 32; i += 2) upk2(mul2(pk2(f[i], f[i + 1]), bc2(c_gate)), f[i], f[i + 1]);
         pack32(f, w, fp16);
         // peer stores over NVLink (or local when c_rank is this rank), 64 contiguous bytes per row
         staged_store64(stage, lane, w, c_ok ? addr2(args.peer_comb[c_rank], c_slot, args.ld_out, n) : 0ull);
@@ -489,10 +527,17 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const float2 gp = unpack2(w[j], fp16), up = unpack2(wu[j], fp16);
-          const float a0 = valid ? f[2 * j] : 0.f, a1 = valid ? f[2 * j + 1] : 0.f;
+          const f32x2 a = valid ? pk2(f[2 * j], f[2 * j + 1]) : 0ull;
+          const f32x2 g = pk2(gp.x, gp.y), u = pk2(up.x, up.y);
           const float s0 = fast_rcp(1.f + __expf(-gp.x)), s1 = fast_rcp(1.f + __expf(-gp.y));
-          w[j] = pack2(a0 * up.x * (s0 * (1.f + gp.x * (1.f - s0))), a1 * up.y * (s1 * (1.f + gp.y * (1.f - s1))), fp16);
-          wu[j] = pack2(a0 * gp.x * s0, a1 * gp.y * s1, fp16);
+          const f32x2 sg = pk2(s0, s1);
+          const f32x2 dg = mul2(mul2(a, u), mul2(sg, fma2(g, pk2(1.f - s0, 1.f - s1), bc2(1.f))));
+          const f32x2 du = mul2(mul2(a, g), sg);
+          float d0, d1;
+          upk2(dg, d0, d1);
+          w[j] = pack2(d0, d1, fp16);
+          upk2(du, d0, d1);
+          wu[j] = pack2(d0, d1, fp16);
         }
         staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
         staged_store64_lin(stage, lane, wu, lin_of(args.out1) + n * 2ull, lin_stride, lin_rows_store);

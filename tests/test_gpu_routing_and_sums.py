@@ -185,3 +185,30 @@ def test_column_sums_shared_by_a_cluster(rows, n, fp16):
     mag = torch.stack([x[b:b + r].double().abs().sum(0) for b, r in zip(base, rows)])
     ulp = 2.0 ** (-11 if fp16 else -8)
     assert ((outs[0].double() - ref).abs() <= ref.abs() * ulp + mag * 2.0 ** -16 + 1e-7).all()
+
+
+@pytest.mark.parametrize("two_cta", [False, True])
+@pytest.mark.parametrize("groups", [1, 31, 33, 64, 256])
+def test_tile_tables_of_many_groups(groups, two_cta):
+    """The warp-parallel tile tables of both GEMM kernels: ragged and empty groups across the 32-group scan steps."""
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(groups)
+    rows = torch.randint(0, 300, (groups,), generator=g)
+    rows[torch.randint(0, groups, (groups // 3,), generator=g)] = 0
+    rows[-1] = 129
+    padded = (rows + 127) // 128 * 128
+    base = torch.cumsum(padded, 0) - padded
+    total = int(padded.sum()) + 128
+    k, n = 64, 256
+    x = torch.randn(total, k, device="cuda").bfloat16()
+    w = (torch.randn(groups * n, k, device="cuda") * 0.1).bfloat16()
+    out = torch.zeros(total, n, dtype=torch.bfloat16, device="cuda")
+    gb, gr = base.int().cuda(), rows.int().cuda()
+    ws = G.launch(a0=x, b0=w, a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_STORE, n=n, k=k, group_base=gb, group_rows=gr,
+                  num_groups=groups, b_group_rows=n, out0=out, two_cta=two_cta)
+    ws.check("tables")
+    for i in range(groups):
+        b, r = int(base[i]), int(rows[i])
+        ref = x[b:b + r].double() @ w[i * n:(i + 1) * n].double().t()
+        assert ((out[b:b + r].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all(), i
