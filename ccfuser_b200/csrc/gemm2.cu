@@ -7,8 +7,7 @@
 //
 // Same modes, operand majors, epilogues, dispatch role and arrival-counter gating as gemm.cu; tiles are assigned
 // statically (tile = pair index + k * number of pairs) because both CTAs of a pair must walk the same sequence.
-// No TMA load in this file uses cluster multicast, and the stage hand-back uses two plain tcgen05.commit arrivals
-// (one per CTA) rather than a multicast commit.
+// No TMA load in this file uses cluster multicast; only the barrier arrival of a stage's hand-back goes to both CTAs.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -18,10 +17,17 @@
 
 namespace ccf {
 
-constexpr int k2Stages = 6;
+// A stage holds two k-blocks. Every hand-back of a stage (tcgen05.commit) costs the tensor pipe about 64 clocks per barrier it
+// arrives on, whatever the memory system does: with one k-block per stage and one commit per CTA of the pair a k-block took
+// 640 clocks instead of 512, also when every load hit the same lines. One multicast commit per two k-blocks is a quarter of that.
+// 32768 x 4096 x 14336, TFLOP/s (GELU forward / second projection): 1310 / 1359 before, 1361 / 1429 with the multicast commit
+// alone, 1416 / 1512 with two k-blocks per stage alone. Under the power cap the gain is smaller.
+constexpr int k2Stages = 3;
+constexpr int k2Sub = 2;                       // k-blocks per stage
 constexpr int k2ABytes = BM * BK * 2;          // this CTA's 128 rows of A
 constexpr int k2BBytes = (BN / 2) * BK * 2;    // this CTA's 128-column half of B
-constexpr int k2StageBytes = k2ABytes + k2BBytes;
+constexpr int k2SubBytes = k2ABytes + k2BBytes;
+constexpr int k2StageBytes = k2Sub * k2SubBytes;
 constexpr int PM = 2 * BM;                     // rows of a pair tile
 
 struct __align__(16) Ctrl2 {
@@ -108,9 +114,11 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// one arrival on the barrier at `cluster_addr` when every MMA issued so far by this thread has completed
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
+// one arrival on the barrier at this shared-memory offset of both CTAs when every MMA issued so far by this thread has
+// completed (the multicast of an arrival, not of data)
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(static_cast<uint16_t>(3))
                : "memory");
 }
 
@@ -340,7 +348,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       }
       if (lane == 0) trace_ev(args, seq, 1);
       const int kb_per_seg = kKGroup ? ti.kblocks : (args.k + BK - 1) / BK;
-      for (int kb = 0; kb < ti.kblocks; ++kb) {
+      for (int kb0 = 0; kb0 < ti.kblocks; kb0 += k2Sub) {
         if (!mbar_wait_cluster(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_word, limit)) {
           report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x22);
           ok = false;
@@ -348,34 +356,38 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
         }
         if (lane == 0) {
           const uint32_t full_leader = map_to_cta(smem_u32(&ctrl->full[stage]), 0);
-          const uint32_t sa = smem_base + stage * k2StageBytes;
-          const uint32_t sb = sa + k2ABytes;
-          if (cta == 0) mbar_arrive_expect_tx(smem_u32(&ctrl->full[stage]), 2 * k2StageBytes);
-          const int seg = kKGroup ? 0 : kb / kb_per_seg;
-          const int kk = kKGroup ? 0 : (kb - seg * kb_per_seg) * BK;
-          const CUtensorMap* ma = seg ? &tmA1 : &tmA0;
-          const CUtensorMap* mb = seg ? &tmB1 : &tmB0;
-          // A: this CTA's 128 rows
-          if constexpr (kAMajor == MAJ_K) {
-            tma_load_2d_pair(sa, ma, full_leader, kk, my_row0);
-          } else {
-            const int r = ti.krow0 + kb * BK;
-            tma_load_2d_pair(sa, ma, full_leader, my_row0, r);
-            tma_load_2d_pair(sa + 8192, ma, full_leader, my_row0 + 64, r);
-          }
-          // B: this CTA's half of the 256 columns
-          const int nh = static_cast<int>(cta) * (BN / 2);
-          if constexpr (kBMajor == MAJ_K) {
-            if constexpr (kEpi == CCF_EPI_SWIGLU) {
-              // leader loads the gate rows (accumulator columns [0,128)), the peer the up rows ([128,256))
-              tma_load_2d_pair(sb, cta == 0 ? &tmB1 : &tmB0, full_leader, kk, ti.g * args.b_group_rows + ti.n0);
+          const int n_sub = min(k2Sub, ti.kblocks - kb0);
+          if (cta == 0) mbar_arrive_expect_tx(smem_u32(&ctrl->full[stage]), static_cast<uint32_t>(n_sub) * 2 * k2SubBytes);
+          for (int u = 0; u < n_sub; ++u) {
+            const int kb = kb0 + u;
+            const uint32_t sa = smem_base + stage * k2StageBytes + u * k2SubBytes;
+            const uint32_t sb = sa + k2ABytes;
+            const int seg = kKGroup ? 0 : kb / kb_per_seg;
+            const int kk = kKGroup ? 0 : (kb - seg * kb_per_seg) * BK;
+            const CUtensorMap* ma = seg ? &tmA1 : &tmA0;
+            const CUtensorMap* mb = seg ? &tmB1 : &tmB0;
+            // A: this CTA's 128 rows
+            if constexpr (kAMajor == MAJ_K) {
+              tma_load_2d_pair(sa, ma, full_leader, kk, my_row0);
             } else {
-              tma_load_2d_pair(sb, mb, full_leader, kk, ti.g * args.b_group_rows + ti.n0 + nh);
+              const int r = ti.krow0 + kb * BK;
+              tma_load_2d_pair(sa, ma, full_leader, my_row0, r);
+              tma_load_2d_pair(sa + 8192, ma, full_leader, my_row0 + 64, r);
             }
-          } else {
-            const int r = kKGroup ? ti.krow0 + kb * BK : ti.g * args.b_group_rows + kk;
-            tma_load_2d_pair(sb, mb, full_leader, ti.n0 + nh, r);
-            tma_load_2d_pair(sb + 8192, mb, full_leader, ti.n0 + nh + 64, r);
+            // B: this CTA's half of the 256 columns
+            const int nh = static_cast<int>(cta) * (BN / 2);
+            if constexpr (kBMajor == MAJ_K) {
+              if constexpr (kEpi == CCF_EPI_SWIGLU) {
+                // leader loads the gate rows (accumulator columns [0,128)), the peer the up rows ([128,256))
+                tma_load_2d_pair(sb, cta == 0 ? &tmB1 : &tmB0, full_leader, kk, ti.g * args.b_group_rows + ti.n0);
+              } else {
+                tma_load_2d_pair(sb, mb, full_leader, kk, ti.g * args.b_group_rows + ti.n0 + nh);
+              }
+            } else {
+              const int r = kKGroup ? ti.krow0 + kb * BK : ti.g * args.b_group_rows + kk;
+              tma_load_2d_pair(sb, mb, full_leader, ti.n0 + nh, r);
+              tma_load_2d_pair(sb + 8192, mb, full_leader, ti.n0 + nh + 64, r);
+            }
           }
         }
         __syncwarp();
@@ -399,7 +411,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
         tc_fence_after();
         if (lane == 0) trace_ev(args, seq, 3);
         const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = 0; kb < ti.kblocks; ++kb) {
+        for (int kb0 = 0; kb0 < ti.kblocks; kb0 += k2Sub) {
           if (!mbar_wait_cluster(smem_u32(&ctrl->full[stage]), phase, abort_word, limit)) {
             report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x25);
             ok = false;
@@ -407,25 +419,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
           }
           tc_fence_after();
           if (lane == 0) {
-            if (kb == 0) trace_ev(args, seq, 4);
-            const uint32_t sa = smem_base + stage * k2StageBytes;
-            const uint32_t sb = sa + k2ABytes;
+            if (kb0 == 0) trace_ev(args, seq, 4);
+            const int n_sub = min(k2Sub, ti.kblocks - kb0);
+            for (int u = 0; u < n_sub; ++u) {
+              const uint32_t sa = smem_base + stage * k2StageBytes + u * k2SubBytes;
+              const uint32_t sb = sa + k2ABytes;
 #pragma unroll
-            for (int k = 0; k < BK / UK; ++k) {
-              const uint64_t da = (kAMajor == MAJ_K) ? make_smem_desc(sa + k * 32, 16, 1024)
-                                                     : make_smem_desc(sa + k * 2048, 8192, 1024);
-              const uint64_t db = (kBMajor == MAJ_K) ? make_smem_desc(sb + k * 32, 16, 1024)
-                                                     : make_smem_desc(sb + k * 2048, 8192, 1024);
-              umma_f16_pair(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < BK / UK; ++k) {
+                const uint64_t da = (kAMajor == MAJ_K) ? make_smem_desc(sa + k * 32, 16, 1024)
+                                                       : make_smem_desc(sa + k * 2048, 8192, 1024);
+                const uint64_t db = (kBMajor == MAJ_K) ? make_smem_desc(sb + k * 32, 16, 1024)
+                                                       : make_smem_desc(sb + k * 2048, 8192, 1024);
+                umma_f16_pair(d_tmem, da, db, idesc, (kb0 > 0 || u > 0 || k > 0) ? 1u : 0u);
+              }
             }
-            // hand the stage back to both producers
-            const uint32_t e0 = smem_u32(&ctrl->empty[stage]);
-            umma_commit_pair(map_to_cta(e0, 0));
-            umma_commit_pair(map_to_cta(e0, 1));
-            if (kb == ti.kblocks - 1) {
-              const uint32_t f0 = smem_u32(&ctrl->acc_full[as]);
-              umma_commit_pair(map_to_cta(f0, 0));
-              umma_commit_pair(map_to_cta(f0, 1));
+            umma_commit_pair(smem_u32(&ctrl->empty[stage]));   // hand the stage back to both producers
+            if (kb0 + k2Sub >= ti.kblocks) {
+              umma_commit_pair(smem_u32(&ctrl->acc_full[as]));
               trace_ev(args, seq, 5);
             }
           }
@@ -538,11 +548,7 @@ static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = k2SmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[1] = {cluster_attribute(2, 1, 1)};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], args);

@@ -498,11 +498,7 @@ int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, cons
   cfg.gridDim = dim3((n + 127) / 128, groups, splits);
   cfg.blockDim = dim3(256);
   cfg.stream = reinterpret_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = splits;
+  cudaLaunchAttribute attr[1] = {ccf::cluster_attribute(1, 1, splits)};
   cfg.attrs = attr;
   cfg.numAttrs = splits > 1 ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, ccf::colsum_grouped_kernel, x, ld, n, group_base, group_rows, out, fp16);

@@ -16,7 +16,7 @@ namespace ccf {
 // `kept`: this rank's kept rows per expert, readable by every thread of the block (global or shared memory).
 // A single rank skips the exchange: its own counts are the table. The prefix sums run one thread per expert over the
 // experts in front of it on the same owner (independent shared-memory reads) instead of one thread per owner over all of
-// them: with 64 experts on one owner the serial walk was most of the kernel's 7 us.
+// them.
 __device__ __forceinline__ void plan_body(const CcfPlanArgs& a, const int epoch, const int* kept) {
   __shared__ int rows[CCF_MAX_GROUPS];
   __shared__ int myoff[CCF_MAX_GROUPS];

@@ -26,6 +26,16 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
+// host: launch attribute of a cluster
+inline cudaLaunchAttribute cluster_attribute(unsigned x, unsigned y, unsigned z) {
+  cudaLaunchAttribute a;
+  a.id = cudaLaunchAttributeClusterDimension;
+  a.val.clusterDim.x = x;
+  a.val.clusterDim.y = y;
+  a.val.clusterDim.z = z;
+  return a;
+}
+
 // ----------------------------------------------------------------------------------------------
 // packed fp32 pairs: one instruction for two fused multiply-adds, each rounded as the scalar one
 // ----------------------------------------------------------------------------------------------
