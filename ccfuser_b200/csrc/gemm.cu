@@ -1,8 +1,8 @@
 // Grouped GEMM for sm_100a: TMA (local memory, no multicast) -> 128B-swizzled shared memory ->
 // tcgen05.mma with fp32 accumulators in TMEM -> tcgen05.ld epilogue. One persistent CTA per SM,
 // 10 warps: warp 0 = tile scheduler + TMA producer, warp 1 = MMA issuer (one elected thread),
-// warps 2..9 = epilogue (two per TMEM lane quarter, each taking half of the tile's columns). Tiles are 128 x 256 x 64, four shared-memory
-// stages, two TMEM accumulator stages (2 x 256 columns) so the epilogue of a tile overlaps the
+// warps 2..9 = epilogue (two per TMEM lane quarter, each taking half of the tile's columns). Tiles are 128 x 256 x 64, four to nine
+// shared-memory stages, two TMEM accumulator stages (2 x 256 columns) so the epilogue of a tile overlaps the
 // main loop of the next one.
 //
 // The kernel replaces the reference's wmma tile GEMM and its callers (mix_moe/csrc/cuda/mix_gemm.cu:22-244
@@ -34,15 +34,20 @@
 
 namespace ccf {
 
-constexpr int kStages = 4;
+// Pipeline memory: four 48 KB stages (128 rows of A, 256 columns of B). A bound on the rows of every group (args.a_rows) makes
+// the stages smaller and their number larger: a launch that streams weights for a handful of rows is limited by the weight
+// bytes it has in flight, and with 128-column tiles four fixed stages hold 64 KB of them per SM where nine 20 KB stages hold
+// 144 (GEMM-2 of 16 tokens, 16 experts, 1024 x 4096: 43 -> 39 us). Without the bound more stages only hurt: six 32 KB
+// stages for 128-column tiles took 236 us where four take 195 (128 tokens, 8 experts, 4096 x 14336).
 constexpr int kABytes = BM * BK * 2;
 constexpr int kBBytes = BN * BK * 2;
-constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kPipeBytes = 4 * (kABytes + kBBytes);
+constexpr int kMaxStages = 9;
 constexpr int kSchedSlots = 4;
 
 struct __align__(16) Ctrl {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t sched_full[kSchedSlots];
@@ -59,7 +64,7 @@ struct __align__(16) Ctrl {
   int rows[CCF_MAX_GROUPS];   // read per decode would sit in front of each tile's first load
 };
 
-constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kEpiWarps * kEpiStageBytes + static_cast<int>(sizeof(Ctrl));
+constexpr int kSmemBytes = 1024 + kPipeBytes + kEpiWarps * kEpiStageBytes + static_cast<int>(sizeof(Ctrl));
 
 template <bool kKGroup, int kEpi>
 __device__ __forceinline__ Tile decode_tile(int t, const CcfGemmArgs& a, const Ctrl* c) {
@@ -146,7 +151,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                     const __grid_constant__ CcfGemmArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem + kStages * kStageBytes + kEpiWarps * kEpiStageBytes);
+  Ctrl* ctrl = reinterpret_cast<Ctrl*>(smem + kPipeBytes + kEpiWarps * kEpiStageBytes);
   const uint32_t smem_base = smem_u32(smem);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -154,10 +159,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
   const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   const int bn_run = (!kKGroup && kBMajor == MAJ_K && kEpi != CCF_EPI_SWIGLU && args.bn == 128) ? 128 : BN;   // MMA N
   const int bn_out = (kEpi == CCF_EPI_SWIGLU) ? BN / 2 : bn_run;
+  constexpr bool kRowBound = !kKGroup && kAMajor == MAJ_K;
+  const int a_rows = kRowBound && args.a_rows > 0 ? args.a_rows : BM;   // rows of A per stage
+  const uint32_t a_bytes = static_cast<uint32_t>(a_rows * BK * 2);
+  const uint32_t stage_bytes = a_bytes + static_cast<uint32_t>(bn_run * BK * 2);
+  const int stages = a_rows < BM ? min(kMaxStages, static_cast<int>(kPipeBytes / stage_bytes)) : 4;
 
   // ---- set-up ------------------------------------------------------------------------------------
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(smem_u32(&ctrl->full[s]), 1);
       mbar_init(smem_u32(&ctrl->empty[s]), 1);
     }
@@ -243,6 +253,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         }
       }
       if (lane == 0) trace_ev(args, seq, 1);
+      if (kRowBound && ti.rows_valid > a_rows) report_status(args.status, CCF_ERR_BOUNDS, ti.row0 & 0xffffff);
       const int kb_per_seg = kKGroup ? ti.kblocks : (args.k + BK - 1) / BK;
       for (int kb = 0; kb < ti.kblocks; ++kb) {
         if (!mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_word, limit)) {
@@ -252,16 +263,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         }
         if (lane == 0) {
           const uint32_t fullb = smem_u32(&ctrl->full[stage]);
-          const uint32_t sa = smem_base + stage * kStageBytes;
-          const uint32_t sb = sa + kABytes;
-          mbar_arrive_expect_tx(fullb, kABytes + bn_run * BK * 2);
+          const uint32_t sa = smem_base + stage * stage_bytes;
+          const uint32_t sb = sa + a_bytes;
+          mbar_arrive_expect_tx(fullb, stage_bytes);
           const int seg = kKGroup ? 0 : kb / kb_per_seg;
           const int kk = kKGroup ? 0 : (kb - seg * kb_per_seg) * BK;
           const CUtensorMap* ma = seg ? &tmA1 : &tmA0;
           const CUtensorMap* mb = seg ? &tmB1 : &tmB0;
           // A operand
           if constexpr (kAMajor == MAJ_K) {
-            tma_load_2d(sa, ma, fullb, kk, ti.row0);
+            tma_load_2d(sa, ma, fullb, kk, ti.row0);   // a_rows rows: the MMA reads what follows them too, and those result rows
+                                                       // are never stored
           } else {
             const int r = ti.krow0 + kb * BK;
             tma_load_2d(sa, ma, fullb, ti.row0, r);
@@ -283,7 +295,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
           }
         }
         __syncwarp();
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (lane == 0) trace_ev(args, seq, 2);
       ++seq;
@@ -322,8 +334,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
         tc_fence_after();
         if (lane == 0) {
           if (kb == 0) trace_ev(args, seq, 4);
-          const uint32_t sa = smem_base + stage * kStageBytes;
-          const uint32_t sb = sa + kABytes;
+          const uint32_t sa = smem_base + stage * stage_bytes;
+          const uint32_t sb = sa + a_bytes;
 #pragma unroll
           for (int k = 0; k < BK / UK; ++k) {
             const uint64_t da = (kAMajor == MAJ_K) ? make_smem_desc(sa + k * 32, 16, 1024)
@@ -339,7 +351,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
           }
         }
         __syncwarp();
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
@@ -382,7 +394,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
       }
       if (warp == 2 && lane == 0) trace_ev(args, seq, 6);
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * BN;
-      const uint32_t stage = smem_base + kStages * kStageBytes + (warp - 2) * kEpiStageBytes;
+      const uint32_t stage = smem_base + kPipeBytes + (warp - 2) * kEpiStageBytes;
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + ti.row0;
       else row_base = ti.row0;
@@ -568,8 +580,12 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
   }
   CUtensorMap tm[4];
   const int fp16 = a.fp16;
-  const int a_box_rows = (L->a_major == MAJ_K) ? BM : BK;
   const bool pair = L->two_cta != 0;
+  if (a.a_rows != 0 && a.a_rows != BM) {
+    // the row bound exists in the one-CTA kernel for row-grouped launches with a K-major A operand
+    if ((a.a_rows != 32 && a.a_rows != 64) || pair || L->kgroup || L->a_major != MAJ_K) return -11;
+  }
+  const int a_box_rows = (L->a_major == MAJ_K) ? (a.a_rows > 0 ? a.a_rows : BM) : BK;
   if (pair && L->kgroup && (a.m_per_group % (2 * BM) != 0)) return -8;
   if (a.bn != 0 && a.bn != BN) {
     // the narrow tile exists in the one-CTA kernel for row-grouped launches with a K-major B operand

@@ -121,6 +121,10 @@ void set_combine(CcfGemmLaunch& g, const CcfLayer* L, void* const* peer_comb, co
   g.args.max_slots = L->max_slots;
 }
 
+// Bound on the rows of any expert of a single-rank call (its capacity, at most all slots of the call; other ranks may bring
+// any number of rows), rounded up to a pipeline geometry of the one-CTA kernel: 32, 64, or 0 for no bound.
+int row_bound(int capacity, int world) { return world != 1 || capacity > 64 ? 0 : capacity > 32 ? 64 : 32; }
+
 int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
   // the pair kernel needs 256-row output tiles in k-grouped mode
   if (g.kgroup && g.args.m_per_group % 256 != 0) g.two_cta = 0;
@@ -266,6 +270,7 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
     }
     set_dispatch(g, L, x, idx, gate_w, tokens, capacity, 0, nullptr);
     g.two_cta = row_two_cta;
+    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -282,6 +287,7 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
     g.args.ld_out = d;
     set_combine(g, L, L->peer_comb, L->row_gate);
     g.two_cta = row_two_cta;
+    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
     g.args.bn = gemm2_bn;
     if ((rc = issue(g, dry, stream))) return rc;
   }
@@ -332,6 +338,7 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
     }
     set_dispatch(g, L, dy, idx, gate_w, tokens, capacity, 1, G->dgate);
     g.two_cta = row_two_cta;
+    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -391,6 +398,7 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
     }
     set_combine(g, L, L->peer_gcomb, nullptr);
     g.two_cta = row_two_cta;
+    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
     return issue(g, dry, stream);
   };
   if (sgd && (rc = dgrad1())) return rc;

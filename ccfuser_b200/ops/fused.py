@@ -272,6 +272,7 @@ class FusedMoE:
         self._desc_key = None
         self.sgd = None         # (lr, weight decay): expert weights are updated by the weight-gradient GEMMs (fuse_sgd)
         self._call_bn = 256
+        self._call_rows = 0
         self._call_two_cta = None   # kernel choice of the current call's row-grouped launches (_row_two_cta)
         self._owed = None       # weak reference to the autograd node whose backward still needs this layer's buffers
 
@@ -486,6 +487,12 @@ class FusedMoE:
         rows = tokens * self.cfg.top_k * self.world // max(1, self.cfg.num_experts)
         return None if rows > G.SMALL_ROWS_DEFAULT else False
 
+    def _row_bound(self, tokens: int) -> int:
+        """Row bound of the row-grouped launches of a call with ``tokens`` tokens per rank (ops/gemm.py: row_bound)."""
+        if G.TWO_CTA_DEFAULT and self._row_two_cta(tokens) is None:
+            return 0
+        return G.row_bound(self.cfg.capacity(tokens), self.world)
+
     def _gemm2_bn(self, tokens: int) -> int:
         """Tile width of the forward GEMM-2 + combine launch of a call with ``tokens`` tokens per rank (ops/gemm.py:
         narrow_tiles); the source-side wait counts its completion units with the same width."""
@@ -549,8 +556,8 @@ class FusedMoE:
         common = dict(group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, tile_flags=cc.tile_flags,
                       dispatch=disp, n_comm_ctas=cc.n_comm, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace,
                       total_index=self.max_rows // TILE, local_begin=self.local_begin, local_rows=self.local_rows,
-                      two_cta=self._row_two_cta(t))
-        self._call_two_cta = common["two_cta"]
+                      two_cta=self._row_two_cta(t), a_rows=self._row_bound(t))
+        self._call_two_cta, self._call_rows = common["two_cta"], common["a_rows"]
         self._call_bn = self._gemm2_bn(t)
         if cfg.activation == "swiglu":
             G.launch(a0=self.xrecv, b0=w1.view(e_loc * f, d), b1=wg.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_K,
@@ -569,6 +576,7 @@ class FusedMoE:
         G.launch(a0=self.h_act, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_COMBINE, n=d, k=f,
                  group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, b_group_rows=d, bias0=b2,
                  ld_out=d, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace, two_cta=self._call_two_cta, bn=self._call_bn,
+                 a_rows=self._call_rows,
                  **self._combine_kw(self.buf.peer_ptrs(self.off_comb), cc.row_gate))
 
     def stage_reduce(self, tokens: int, out: torch.Tensor):
@@ -785,17 +793,17 @@ class _FusedMoEFn(torch.autograd.Function):
                       workspace=cc.ws)
         dh = torch.empty(fm.max_rows, f, dtype=cfg.dtype, device=dy.device)
         dh2 = torch.empty_like(dh) if swiglu else None
-        rt = fm._row_two_cta(t)
+        rt, ar = fm._row_two_cta(t), fm._row_bound(t)
         if swiglu:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DSWIGLU, n=f, k=d,
                      b_group_rows=d, out0=dh, out1=dh2, aux0=fm.h_pre, aux1=fm.h_pre2, tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, two_cta=rt, **common)
+                     local_rows=fm.local_rows, two_cta=rt, a_rows=ar, **common)
         else:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DACT, n=f, k=d,
                      b_group_rows=d, out0=dh, aux0=fm.h_pre, act=N.ACT_CODE[cfg.activation], tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, two_cta=rt, **common)
+                     local_rows=fm.local_rows, two_cta=rt, a_rows=ar, **common)
         cc.tile_flags.zero_()
         # 3. wgrad-2: dW2[e] = (g dy)^T h_act   [d, f]
         # With few rows per expert the reduction is only a handful of k-blocks and the per-tile latency chain decides:
@@ -819,11 +827,11 @@ class _FusedMoEFn(torch.autograd.Function):
             ck = fm._combine_kw(cc.peer("gcomb"), None)
             if swiglu:
                 G.launch(a0=dh, a1=dh2, b0=wg.view(e_loc * f, d), b1=w1.view(e_loc * f, d), a_major=N.MAJ_K,
-                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d, two_cta=rt,
+                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d, two_cta=rt, a_rows=ar,
                          **common, **ck)
             else:
                 G.launch(a0=dh, b0=w1.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f,
-                         b_group_rows=f, ld_out=d, two_cta=rt, **common, **ck)
+                         b_group_rows=f, ld_out=d, two_cta=rt, a_rows=ar, **common, **ck)
 
         if sgd is not None:
             dgrad1()            # reads w1 / wg before the weight-gradient GEMMs below overwrite them

@@ -212,3 +212,78 @@ def test_tile_tables_of_many_groups(groups, two_cta):
         b, r = int(base[i]), int(rows[i])
         ref = x[b:b + r].double() @ w[i * n:(i + 1) * n].double().t()
         assert ((out[b:b + r].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all(), i
+
+
+@pytest.mark.parametrize("a_rows,bn,two_cta,rows", [(32, 128, False, [1, 32, 0, 31, 7]), (32, 256, False, [32, 2]), (64, 128, False, [64, 33, 1]),
+                                                    (64, 256, False, [63, 0, 64]), (0, 128, False, [128, 97, 1, 65]),
+                                                    (0, 256, False, [33, 130, 300, 96]), (0, 256, True, [1, 129, 160, 257, 300, 512])])
+@pytest.mark.parametrize("k", [64, 1024])
+def test_row_bound(a_rows, bn, two_cta, rows, k):
+    """Pipeline geometries of the one-CTA kernel (rows of A per stage x tile width) and the CTA-pair kernel at ragged rows:
+    what the stages hold beyond a tile's rows must not reach a stored row. The rows of A outside the groups hold NaN."""
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops import gemm as G
+    torch.manual_seed(k + len(rows))
+    base, acc = [], 0
+    for r in rows:
+        base.append(acc)
+        acc += (r + 127) // 128 * 128
+    n, groups = 384, len(rows)
+    x = torch.full((max(acc, 128) + 128, k), float("nan"), device="cuda", dtype=torch.bfloat16)
+    for b, r in zip(base, rows):
+        x[b:b + r] = torch.randn(r, k, device="cuda").bfloat16()
+    w = (torch.randn(groups * n, k, device="cuda") * 0.1).bfloat16()
+    out = torch.full((x.shape[0], n), 7.0, dtype=torch.bfloat16, device="cuda")
+    ws = G.launch(a0=x, b0=w, a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_STORE, n=n, k=k,
+                  group_base=torch.tensor(base, dtype=torch.int32, device="cuda"),
+                  group_rows=torch.tensor(rows, dtype=torch.int32, device="cuda"), num_groups=groups, b_group_rows=n, out0=out,
+                  two_cta=two_cta, bn=bn, a_rows=a_rows)
+    ws.check("row bound")
+    for i, (b, r) in enumerate(zip(base, rows)):
+        ref = x[b:b + r].double() @ w[i * n:(i + 1) * n].double().t()
+        # bf16 result of fp32 sums of k products of order 0.1
+        assert ((out[b:b + r].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all(), i
+        assert (out[b + r:b + (r + 127) // 128 * 128] == 7.0).all()
+
+
+def test_row_bound_is_refused_where_it_does_not_exist():
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops import gemm as G
+    x = torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16)
+    gb, gr = G.single_group(32, "cuda")
+    for kw in (dict(two_cta=True, a_rows=32), dict(two_cta=False, a_rows=48), dict(two_cta=False, a_rows=32, a_major=N.MAJ_MN)):
+        kw = {"a_major": N.MAJ_K, **kw}
+        with pytest.raises(RuntimeError):
+            G.launch(a0=x, b0=x, b_major=N.MAJ_K, epi=N.EPI_STORE, n=128, k=64, group_base=gb, group_rows=gr, num_groups=1,
+                     b_group_rows=128, out0=x, **kw)
+
+
+@pytest.mark.parametrize("t,e,k,act", [(1, 16, 2, "gelu"), (16, 16, 2, "swiglu"), (40, 4, 1, "relu"), (64, 8, 1, "gelu"), (33, 64, 2, "gelu")])
+def test_few_token_layer_uses_the_bound_and_matches_the_oracle(t, e, k, act):
+    """Training and inference calls around the bounds of the small pipeline geometries, against the fp32 oracle on the same
+    routing decisions."""
+    from ccfuser_b200 import MoEConfig, MoELayer
+    from ccfuser_b200.ops.reference import dense_moe_oracle
+    torch.manual_seed(t * e)
+    cfg = MoEConfig(d_model=256, d_ffn=512, num_experts=e, top_k=k, activation=act, dtype=torch.bfloat16, backend="fused",
+                    max_tokens=128)
+    layer = MoELayer(cfg, device="cuda")
+    x = torch.randn(t, 256, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    fm = layer._fused_impl()
+    y = layer(x)
+    gy = torch.randn_like(y)
+    y.backward(gy)
+    layer.check_status()
+    with torch.no_grad():
+        assert torch.equal(layer(x.detach()), y)           # inference form: same kernels without the pre-activations
+        idx, w = fm.route(x.detach())
+    params = {n.replace("experts.", "").replace("gate.gate.", "gate."): p.detach().float().requires_grad_() for n, p in layer.named_parameters()}
+    xf = x.detach().float().requires_grad_()
+    sc = w.detach().clone()
+    (ref,) = dense_moe_oracle([xf], params, top_k=k, capacity=None, activation=act, routing=[(idx, sc)])
+    ref.backward(gy.float())
+    rel = lambda a, b: float((a.float() - b).norm() / b.norm().clamp_min(1e-6))   # noqa: E731
+    assert rel(y.detach(), ref.detach()) < 1e-2            # bf16 activations and results: 2^-8 each
+    assert rel(layer.experts.htoh4.weight.grad, params["htoh4.weight"].grad) < 1.5e-2
+    assert rel(layer.experts.h4toh.weight.grad, params["h4toh.weight"].grad) < 1.5e-2
+    layer.release()
