@@ -28,7 +28,8 @@ __device__ __forceinline__ void add_piece(float (&acc)[8], const uint4& x, float
 // y[t, :] = sum_j keep(t, j) * comb[t * k + j, :] in fp32, one rounding. Bound by reading k rows and writing one per token;
 // a block takes whole tokens (512 pieces of 16 bytes) and kK is a template argument so that all rows of a token are
 // requested before the first is used. With kRouter the same pass adds the router's share of the input gradient,
-// sum_j g_j Wg[idx_j, :] (Wg is small and stays in L2), which as a kernel of its own wrote and re-read a [T, d] matrix.
+// sum_j g_j Wg[idx_j, :] (Wg is small and stays in L2), which as a kernel of its own wrote and re-read a [T, d] matrix:
+// 16384 x 4096, top-2: 166 us for both, from 94 + 58 + 66 us (reduce, router dx, addition of the two gradients).
 template <int kK, bool kRouter>
 __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __grid_constant__ CcfReduceArgs a) {
   const int vecs = a.d >> 3, K = kK > 0 ? kK : a.top_k, fp16 = a.fp16;
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
         const int e = __ldg(a.idx + s0 + j);
         const bool routed = e >= 0 && e < a.e;
         const float g = routed ? w[j] * (dw[j] - dot) : 0.f;
-        if (v == 0) a.g[s0 + j] = g;
+        if (v == 0) a.g[s0 + j] = a.round_g ? unpack2(pack2(g, 0.f, fp16), fp16).x : g;
         if (routed) add_piece(acc, __ldg(wg + static_cast<size_t>(e) * vecs + v), g, fp16);
       }
     }
@@ -114,17 +115,24 @@ __global__ void __launch_bounds__(256) router_dw_kernel(const int* __restrict__ 
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   float sum_g = 0.f;
   const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + col;
+  // the slot ids are read one pass ahead: otherwise every pass waits for two dependent reads
+  int s_next[4];
+  auto fetch = [&](int r) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s_next[u] = r + 16 * u < nr ? __ldg(list + r + 16 * u) : -1;
+  };
+  fetch(split * 64 + ry);
   for (int r = split * 64 + ry; r < nr; r += 64 * splits) {
     float g[4];
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int rr = r + 16 * u;
-      const int s = rr < nr ? __ldg(list + rr) : 0;
-      g[u] = rr < nr ? __ldg(g_slot + s) : 0.f;
-      v[u] = rr < nr && col < d ? __ldg(reinterpret_cast<const uint4*>(base + static_cast<size_t>(s / top_k) * d))
-                                : make_uint4(0u, 0u, 0u, 0u);
+      const int s = s_next[u];
+      g[u] = s >= 0 ? __ldg(g_slot + s) : 0.f;
+      v[u] = s >= 0 && col < d ? __ldg(reinterpret_cast<const uint4*>(base + static_cast<size_t>(s / top_k) * d))
+                               : make_uint4(0u, 0u, 0u, 0u);
     }
+    fetch(r + 64 * splits);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       add_piece(acc, v[u], g[u], fp16);
@@ -178,16 +186,11 @@ int ccf_reduce(const CcfReduceArgs* a, void* stream) {
   const int per_block = kReduceThreads * kReducePieces / vecs > 1 ? kReduceThreads * kReducePieces / vecs : 1;
   int blocks = (a->tokens + per_block - 1) / per_block;
   if (blocks < 1) blocks = 1;    // a call without tokens still consumes its completion count
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-#define CCF_REDUCE(K)                                                                       \
-  do {                                                                                      \
-    if (a->wg != nullptr) combine_reduce_kernel<K, true><<<blocks, kReduceThreads, 0, st>>>(*a);  \
-    else combine_reduce_kernel<K, false><<<blocks, kReduceThreads, 0, st>>>(*a);            \
-  } while (0)
-  if (a->top_k == 1) CCF_REDUCE(1);
-  else if (a->top_k == 2) CCF_REDUCE(2);
-  else CCF_REDUCE(0);
-#undef CCF_REDUCE
+  auto kern = a->wg != nullptr ? (a->top_k == 1 ? combine_reduce_kernel<1, true> : a->top_k == 2 ? combine_reduce_kernel<2, true>
+                                                                                         : combine_reduce_kernel<0, true>)
+                               : (a->top_k == 1 ? combine_reduce_kernel<1, false> : a->top_k == 2 ? combine_reduce_kernel<2, false>
+                                                                                          : combine_reduce_kernel<0, false>);
+  kern<<<blocks, kReduceThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }
@@ -204,11 +207,7 @@ int ccf_router_dw(const int* raw_order, const int* count_raw, const float* g, co
   cfg.gridDim = dim3((d + 127) / 128, e, splits);
   cfg.blockDim = dim3(256);
   cfg.stream = reinterpret_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = splits;
+  cudaLaunchAttribute attr[1] = {cluster_attribute(1, 1, splits)};
   cfg.attrs = attr;
   cfg.numAttrs = splits > 1 ? 1 : 0;
   cudaError_t err = cudaLaunchKernelEx(&cfg, router_dw_kernel, raw_order, count_raw, g, x, dwg, db, d, top_k, fp16);
