@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "dispatch.cuh"   // pack2 / unpack2
+#include "sm100.cuh"
 
 namespace ccf {
 
@@ -86,143 +87,213 @@ __global__ void __launch_bounds__(kLnThreads) layernorm_fwd_kernel(const void* _
   }
 }
 
-// Backward, two kernels. With xh = (x - mean) * rstd and g = dy * gamma:
-//   dx = rstd * (g - mean_row(g) - xh * mean_row(g * xh))        one warp per row, like the forward pass
-//   dgamma = sum_rows dy * xh,   dbeta = sum_rows dy              a column reduction over all rows
-// Keeping both in one kernel meant a whole row's dgamma / dbeta partial sums in registers (255 per thread, one block
-// per SM); reading x and dy a second time for the column reduction costs less than that occupancy did.
-template <int kV>
-__global__ void __launch_bounds__(kLnThreads) layernorm_bwd_dx_kernel(const void* __restrict__ x, const void* __restrict__ dy,
-                                                                       const void* __restrict__ gamma,
-                                                                       const float* __restrict__ mean_in,
-                                                                       const float* __restrict__ rstd_in,
-                                                                       void* __restrict__ dx, int rows, int d, int fp16) {
-  const int row = blockIdx.x * kLnWarps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const int vecs = d >> 3;
-  const uint4* xr = reinterpret_cast<const uint4*>(x) + static_cast<size_t>(row) * vecs;
-  const uint4* dr = reinterpret_cast<const uint4*>(dy) + static_cast<size_t>(row) * vecs;
-  const uint4* gv = reinterpret_cast<const uint4*>(gamma);
-  const float mean = mean_in[row], rstd = rstd_in[row];
-  uint4 xv[kV], dv[kV];   // dv is overwritten with g = dy * gamma, packed again
-  float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-  for (int i = 0; i < kV; ++i) {
-    const int v = lane + 32 * i;
-    xv[i] = make_uint4(0, 0, 0, 0);
-    dv[i] = make_uint4(0, 0, 0, 0);
-    uint4 g4 = make_uint4(0, 0, 0, 0);
-    if (v < vecs) { xv[i] = __ldg(xr + v); dv[i] = __ldg(dr + v); g4 = __ldg(gv + v); }
-    const uint32_t xq[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w}, dq[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w};
-    const uint32_t gq[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 xf = unpack2(xq[j], fp16), df = unpack2(dq[j], fp16), gf = unpack2(gq[j], fp16);
-      const bool on = v < vecs;
-      const float h0 = on ? (xf.x - mean) * rstd : 0.f, h1 = on ? (xf.y - mean) * rstd : 0.f;
-      const float g0 = df.x * gf.x, g1 = df.y * gf.y;
-      s1 += g0 + g1;
-      s2 = fmaf(g0, h0, fmaf(g1, h1, s2));
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, off);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-  }
-  const float m1 = s1 / d, m2 = s2 / d;
-  uint4* outr = reinterpret_cast<uint4*>(dx) + static_cast<size_t>(row) * vecs;
-#pragma unroll
-  for (int i = 0; i < kV; ++i) {
-    const int v = lane + 32 * i;
-    if (v >= vecs) continue;
-    const uint4 g4 = __ldg(gv + v);
-    const uint32_t xq[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w}, dq[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w};
-    const uint32_t gq[4] = {g4.x, g4.y, g4.z, g4.w};
-    uint32_t o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 xf = unpack2(xq[j], fp16), df = unpack2(dq[j], fp16), gf = unpack2(gq[j], fp16);
-      const float h0 = (xf.x - mean) * rstd, h1 = (xf.y - mean) * rstd;
-      o[j] = pack2(rstd * (df.x * gf.x - m1 - h0 * m2), rstd * (df.y * gf.y - m1 - h1 * m2), fp16);
-    }
-    outr[v] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-}
-
-// Block (cx, ry): columns [128 cx, 128 cx + 128) (16 lanes x 16 bytes), rows ry * kLnParamRows ... (16 row lanes, four
-// rows in flight per thread). Partial sums meet in shared memory, then one fp32 atomic per column and block.
-constexpr int kLnParamRows = 512;
-__global__ void __launch_bounds__(256) layernorm_bwd_param_kernel(const void* __restrict__ x, const void* __restrict__ dy,
-                                                                  const float* __restrict__ mean_in,
-                                                                  const float* __restrict__ rstd_in,
-                                                                  float* __restrict__ dgamma, float* __restrict__ dbeta,
-                                                                  int rows, int d, int fp16) {
-  __shared__ float red[2][16][128];
-  const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
-  const int col = blockIdx.x * 128 + cx * 8;
-  const int r_begin = blockIdx.y * kLnParamRows, r_end = min(rows, r_begin + kLnParamRows);
+// Backward. With xh = (x - mean) * rstd and g = dy * gamma:
+//   dx = rstd * (g - mean_row(g) - xh * mean_row(g * xh)),   dgamma = sum_rows dy * xh,   dbeta = sum_rows dy.
+// Bound by reading x and dy and writing dx once. kW warps share a row, eight columns per thread, so that a thread meets
+// the same columns in every row it visits and its dgamma / dbeta sums are 16 registers (a warp per row needed a whole row's:
+// one block per SM, and a second pass over x and dy instead). The rows of a block arrive by bulk copies, up to kLnStages
+// pairs of row groups ahead: with loads to registers 16 warps per SM held 32 KB in flight, a third of what the memory
+// rate takes. The row sums meet in shared memory with one barrier per stage, which also frees the stage, and each block
+// leaves its partial dgamma / dbeta in `part` ([blocks, 2, d] fp32), which layernorm_bwd_finish_kernel adds in block order:
+// no atomics, no zeroed buffers, no conversion passes. 8192 x 2048 bf16: 39 + 7 us, where a dx kernel, a parameter kernel,
+// two fills and two conversions took 37 + 16 + 6 us and four launches more.
+constexpr int kLnRows = 2;       // rows per group and stage
+constexpr int kLnStages = 6;
+template <int kW>
+__global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ dy,
+                                                               const void* __restrict__ gamma, const float* __restrict__ mean_in,
+                                                               const float* __restrict__ rstd_in, void* __restrict__ dx,
+                                                               float* __restrict__ part, int rows, int d, int fp16) {
+  constexpr int kG = kLnWarps / kW;             // rows that a block works on side by side
+  constexpr int kStageRows = kG * kLnRows;      // consecutive rows: at most 8 KB each of x and dy
+  extern __shared__ __align__(16) uint8_t ln_ring[];   // [kLnStages][x rows, dy rows]
+  __shared__ float2 red[2][kG][kLnRows][kW];
+  __shared__ float psum[kG > 1 ? kG - 1 : 1][2][kW * 256];
+  __shared__ __align__(8) uint64_t full[kLnStages];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = warp / kW, wr = warp % kW;
+  const int v = wr * 32 + lane, vecs = d >> 3;  // this thread's 16-byte piece of a row
+  const bool col_on = v < vecs;
+  const uint32_t row_bytes = static_cast<uint32_t>(d) * 2u, half = kStageRows * row_bytes;
+  const uint32_t ring = smem_u32(ln_ring);
   float pg[8] = {0, 0, 0, 0, 0, 0, 0, 0}, pb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (col < d) {
-    const uint16_t* xb = reinterpret_cast<const uint16_t*>(x) + col;
-    const uint16_t* db = reinterpret_cast<const uint16_t*>(dy) + col;
-    for (int r = r_begin + ry; r < r_end; r += 64) {
-      uint4 xv[4], dv[4];
-      float mu[4], rs[4];
+  uint4 g4 = make_uint4(0, 0, 0, 0);
+  if (col_on) g4 = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+  const uint32_t gq[4] = {g4.x, g4.y, g4.z, g4.w};
+  const int step = static_cast<int>(gridDim.x) * kStageRows;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < kLnStages; ++k) mbar_init(smem_u32(&full[k]), 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  auto request = [&](int base, int slot) {      // thread 0
+    if (base >= rows) return;
+    const uint32_t bytes = static_cast<uint32_t>(min(kStageRows, rows - base)) * row_bytes, bar = smem_u32(&full[slot]);
+    const size_t off = static_cast<size_t>(base) * row_bytes;
+    mbar_arrive_expect_tx(bar, 2 * bytes);
+    bulk_load(ring + slot * 2 * half, reinterpret_cast<const uint8_t*>(x) + off, bytes, bar);
+    bulk_load(ring + slot * 2 * half + half, reinterpret_cast<const uint8_t*>(dy) + off, bytes, bar);
+  };
+  float mn[kLnRows], rn[kLnRows];
+  auto stats = [&](int base) {                  // one stage ahead of their use
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int rr = r + 16 * u;
-        const bool on = rr < r_end;
-        xv[u] = on ? __ldg(reinterpret_cast<const uint4*>(xb + static_cast<size_t>(rr) * d)) : make_uint4(0, 0, 0, 0);
-        dv[u] = on ? __ldg(reinterpret_cast<const uint4*>(db + static_cast<size_t>(rr) * d)) : make_uint4(0, 0, 0, 0);
-        mu[u] = on ? mean_in[rr] : 0.f;
-        rs[u] = on ? rstd_in[rr] : 0.f;
+    for (int u = 0; u < kLnRows; ++u) {
+      const int row = base + u * kG + grp;
+      mn[u] = row < rows ? __ldg(mean_in + row) : 0.f;
+      rn[u] = row < rows && col_on ? __ldg(rstd_in + row) : 0.f;   // 0: pieces outside contribute nothing below
+    }
+  };
+  int buf = 0, slot = 0, parity = 0;
+  int base = static_cast<int>(blockIdx.x) * kStageRows;
+  if (threadIdx.x == 0)
+    for (int k = 0; k < kLnStages; ++k) request(base + k * step, k);
+  stats(base);
+  for (; base < rows; base += step, buf ^= 1) {   // the same trips for every thread of the block
+    uint4 xv[kLnRows], dv[kLnRows];
+    float mu[kLnRows], rs[kLnRows];
+    // bounded; a copy that never arrives turns the rows into NaN instead of hanging
+    bool here = mbar_try_wait(smem_u32(&full[slot]), parity);
+    for (int tries = 0; !here && tries < (1 << 22); ++tries) here = mbar_try_wait(smem_u32(&full[slot]), parity);
+#pragma unroll
+    for (int u = 0; u < kLnRows; ++u) {
+      const int r = u * kG + grp;
+      xv[u] = make_uint4(0, 0, 0, 0);
+      dv[u] = make_uint4(0, 0, 0, 0);
+      if (base + r < rows && col_on) {
+        const uint8_t* at = ln_ring + slot * 2 * half + r * row_bytes + v * 16;
+        xv[u] = *reinterpret_cast<const uint4*>(at);
+        dv[u] = *reinterpret_cast<const uint4*>(at + half);
       }
+      mu[u] = here ? mn[u] : __int_as_float(0x7fc00000);
+      rs[u] = rn[u];
+    }
+    stats(base + step);
+    float s1[kLnRows], s2[kLnRows];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t xq[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w}, dq[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w};
+    for (int u = 0; u < kLnRows; ++u) {
+      const uint32_t xq[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w}, dq[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w};
+      s1[u] = s2[u] = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 xf = unpack2(xq[q], fp16), df = unpack2(dq[q], fp16);
-          pg[2 * q] = fmaf(df.x, (xf.x - mu[u]) * rs[u], pg[2 * q]);
-          pg[2 * q + 1] = fmaf(df.y, (xf.y - mu[u]) * rs[u], pg[2 * q + 1]);
-          pb[2 * q] += df.x;
-          pb[2 * q + 1] += df.y;
+      for (int j = 0; j < 4; ++j) {
+        const float2 xf = unpack2(xq[j], fp16), df = unpack2(dq[j], fp16), gf = unpack2(gq[j], fp16);
+        const float h0 = (xf.x - mu[u]) * rs[u], h1 = (xf.y - mu[u]) * rs[u];
+        const float g0 = df.x * gf.x, g1 = df.y * gf.y;
+        s1[u] += g0 + g1;
+        s2[u] = fmaf(g0, h0, fmaf(g1, h1, s2[u]));
+        pg[2 * j] = fmaf(df.x, h0, pg[2 * j]);
+        pg[2 * j + 1] = fmaf(df.y, h1, pg[2 * j + 1]);
+        pb[2 * j] += df.x;
+        pb[2 * j + 1] += df.y;
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+      for (int u = 0; u < kLnRows; ++u) {
+        s1[u] += __shfl_xor_sync(0xffffffffu, s1[u], off);
+        s2[u] += __shfl_xor_sync(0xffffffffu, s2[u], off);
+      }
+    }
+    if constexpr (kW > 1) {
+      if (lane == 0) {
+#pragma unroll
+        for (int u = 0; u < kLnRows; ++u) red[buf][grp][u][wr] = make_float2(s1[u], s2[u]);
+      }
+    }
+    __syncthreads();   // row sums are there and the stage has been read; `red`'s other half is written after the next one
+    if (threadIdx.x == 0) request(base + kLnStages * step, slot);
+    if (++slot == kLnStages) { slot = 0; parity ^= 1; }
+    if constexpr (kW > 1) {
+#pragma unroll
+      for (int u = 0; u < kLnRows; ++u) {
+        s1[u] = s2[u] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kW; ++k) {
+          const float2 r = red[buf][grp][u][k];
+          s1[u] += r.x;
+          s2[u] += r.y;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kLnRows; ++u) {
+      const int row = base + u * kG + grp;
+      if (row >= rows || !col_on) continue;
+      const float m1 = s1[u] / d, m2 = s2[u] / d;
+      const uint32_t xq[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w}, dq[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w};
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 xf = unpack2(xq[j], fp16), df = unpack2(dq[j], fp16), gf = unpack2(gq[j], fp16);
+        const float h0 = (xf.x - mu[u]) * rs[u], h1 = (xf.y - mu[u]) * rs[u];
+        o[j] = pack2(rs[u] * (df.x * gf.x - m1 - h0 * m2), rs[u] * (df.y * gf.y - m1 - h1 * m2), fp16);
+      }
+      reinterpret_cast<uint4*>(dx)[static_cast<size_t>(row) * vecs + v] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  // the block's row groups add up, then one partial row of dgamma and of dbeta per block
+  if constexpr (kG > 1) {
+    if (grp > 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        psum[grp - 1][0][i * (kW * 32) + v] = pg[i];
+        psum[grp - 1][1][i * (kW * 32) + v] = pb[i];
+      }
+    }
+    __syncthreads();
+    if (grp == 0) {
+      for (int k = 0; k < kG - 1; ++k) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          pg[i] += psum[k][0][i * (kW * 32) + v];
+          pb[i] += psum[k][1][i * (kW * 32) + v];
         }
       }
     }
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    red[0][ry][cx * 8 + i] = pg[i];
-    red[1][ry][cx * 8 + i] = pb[i];
-  }
-  __syncthreads();
-  if (threadIdx.x < 128) {
-    const int c = blockIdx.x * 128 + threadIdx.x;
-    if (c < d) {
-      float sg = 0.f, sb = 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) { sg += red[0][i][threadIdx.x]; sb += red[1][i][threadIdx.x]; }
-      atomicAdd(dgamma + c, sg);
-      if (dbeta != nullptr) atomicAdd(dbeta + c, sb);
-    }
+  if (grp == 0 && col_on) {
+    float4* og = reinterpret_cast<float4*>(part + static_cast<size_t>(blockIdx.x) * 2 * d) + 2 * v;
+    og[0] = make_float4(pg[0], pg[1], pg[2], pg[3]);
+    og[1] = make_float4(pg[4], pg[5], pg[6], pg[7]);
+    float4* ob = og + (d >> 2);
+    ob[0] = make_float4(pb[0], pb[1], pb[2], pb[3]);
+    ob[1] = make_float4(pb[4], pb[5], pb[6], pb[7]);
   }
 }
 
-template <int kV>
-static int launch_ln(bool fwd, const void* x, const void* dy, const void* gamma, const void* beta, void* out, float* mean,
-                     float* rstd, float* dgamma, float* dbeta, int rows, int d, float eps, int fp16, cudaStream_t st) {
-  if (fwd) {
-    const int blocks = (rows + kLnWarps - 1) / kLnWarps;
-    layernorm_fwd_kernel<kV><<<blocks, kLnThreads, 0, st>>>(x, gamma, beta, out, mean, rstd, rows, d, eps, fp16);
-  } else {
-    const int blocks = (rows + kLnWarps - 1) / kLnWarps;
-    layernorm_bwd_dx_kernel<kV><<<blocks, kLnThreads, 0, st>>>(x, dy, gamma, mean, rstd, out, rows, d, fp16);
-    dim3 grid((d + 127) / 128, (rows + kLnParamRows - 1) / kLnParamRows);
-    layernorm_bwd_param_kernel<<<grid, 256, 0, st>>>(x, dy, mean, rstd, dgamma, dbeta, rows, d, fp16);
+// Block: 32 columns of dgamma (blockIdx.y = 0) or dbeta (1), 8 lanes over the partial rows.
+__global__ void __launch_bounds__(256) layernorm_bwd_finish_kernel(const float* __restrict__ part, int blocks, int d, void* dgamma,
+                                                                   void* dbeta, int fp16) {
+  __shared__ float red[8][32];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), ly = threadIdx.x >> 5;
+  float s = 0.f;
+  if (c < d) {
+#pragma unroll 8
+    for (int b = ly; b < blocks; b += 8) s += __ldg(part + (static_cast<size_t>(b) * 2 + blockIdx.y) * d + c);
   }
+  red[ly][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (ly == 0 && c < d) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += red[k][threadIdx.x];
+    void* out = blockIdx.y == 0 ? dgamma : dbeta;
+    if (fp16) reinterpret_cast<__half*>(out)[c] = __float2half(s);
+    else reinterpret_cast<__nv_bfloat16*>(out)[c] = __float2bfloat16(s);
+  }
+}
+
+// blocks of the backward kernel = rows of its partial-sum buffer: two per SM, fewer for few rows
+static int ln_bwd_blocks(int rows, int d) {
+  const int w = (d + 255) / 256, kw = w <= 1 ? 1 : w <= 2 ? 2 : w <= 4 ? 4 : 8;
+  const int per = kLnWarps / kw * kLnRows, blocks = (rows + per - 1) / per;
+  return blocks < 2 * 148 ? blocks : 2 * 148;
+}
+
+template <int kV>
+static int launch_ln_fwd(const void* x, const void* gamma, const void* beta, void* out, float* mean, float* rstd, int rows, int d,
+                         float eps, int fp16, cudaStream_t st) {
+  const int blocks = (rows + kLnWarps - 1) / kLnWarps;
+  layernorm_fwd_kernel<kV><<<blocks, kLnThreads, 0, st>>>(x, gamma, beta, out, mean, rstd, rows, d, eps, fp16);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
@@ -241,20 +312,39 @@ int ccf_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* 
   using namespace ccf;
   if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (d <= 512) return launch_ln<2>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, rows, d, eps, fp16, st);
-  if (d <= 1024) return launch_ln<4>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, rows, d, eps, fp16, st);
-  return launch_ln<8>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, rows, d, eps, fp16, st);
+  if (d <= 512) return launch_ln_fwd<2>(x, gamma, beta, y, mean, rstd, rows, d, eps, fp16, st);
+  if (d <= 1024) return launch_ln_fwd<4>(x, gamma, beta, y, mean, rstd, rows, d, eps, fp16, st);
+  return launch_ln_fwd<8>(x, gamma, beta, y, mean, rstd, rows, d, eps, fp16, st);
 }
 
-// dx [rows, d] is written; dgamma and dbeta [d] (fp32, zero on entry; dbeta may be null) are accumulated into.
+// Rows of the partial-sum buffer that ccf_layernorm_bwd needs for this size.
+int ccf_layernorm_bwd_parts(int rows, int d) { return rows < 1 || d < 8 ? 0 : ccf::ln_bwd_blocks(rows, d); }
+
+// dx [rows, d], dgamma [d] and dbeta [d] (element type; dbeta may be null) are written. `part`: scratch of
+// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats, 16-byte aligned.
 int ccf_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
-                      float* dgamma, float* dbeta, int rows, int d, int fp16, void* stream) {
+                      float* part, void* dgamma, void* dbeta, int rows, int d, int fp16, void* stream) {
   using namespace ccf;
   if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (d <= 512) return launch_ln<2>(false, x, dy, gamma, nullptr, dx, const_cast<float*>(mean), const_cast<float*>(rstd), dgamma, dbeta, rows, d, 0.f, fp16, st);
-  if (d <= 1024) return launch_ln<4>(false, x, dy, gamma, nullptr, dx, const_cast<float*>(mean), const_cast<float*>(rstd), dgamma, dbeta, rows, d, 0.f, fp16, st);
-  return launch_ln<8>(false, x, dy, gamma, nullptr, dx, const_cast<float*>(mean), const_cast<float*>(rstd), dgamma, dbeta, rows, d, 0.f, fp16, st);
+  const int blocks = ln_bwd_blocks(rows, d);
+  const int w = (d + 255) / 256, kw = w <= 1 ? 1 : w <= 2 ? 2 : w <= 4 ? 4 : 8;
+  const int smem = kLnStages * 2 * (kLnWarps / kw * kLnRows) * d * 2;   // at most 96 KB
+  auto kern = d <= 256 ? layernorm_bwd_kernel<1> : d <= 512 ? layernorm_bwd_kernel<2> : d <= 1024 ? layernorm_bwd_kernel<4>
+                                                                                    : layernorm_bwd_kernel<8>;
+  static bool configured[64][4] = {};   // per device and instantiation: the attribute belongs to the (function, device) pair
+  int dev = 0;
+  cudaGetDevice(&dev);
+  bool& set = configured[dev & 63][kw == 1 ? 0 : kw == 2 ? 1 : kw == 4 ? 2 : 3];
+  if (!set) {
+    const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLnStages * 16384);
+    if (err != cudaSuccess) return -static_cast<int>(err);
+    set = true;
+  }
+  kern<<<blocks, 256, smem, st>>>(x, dy, gamma, mean, rstd, dx, part, rows, d, fp16);
+  layernorm_bwd_finish_kernel<<<dim3((d + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, st>>>(part, blocks, d, dgamma, dbeta, fp16);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 }  // extern "C"

@@ -43,13 +43,14 @@ class _LayerNormFn(torch.autograd.Function):
         rows, d = x2.shape
         dy2 = dy.reshape(rows, d).contiguous()
         dx = torch.empty_like(x2)
-        dg = torch.zeros(d, dtype=torch.float32, device=x2.device)
-        db = torch.zeros(d, dtype=torch.float32, device=x2.device) if ctx.has_bias else None
+        part = torch.empty(lib.ccf_layernorm_bwd_parts(rows, d), 2, d, dtype=torch.float32, device=x2.device)
+        dg = torch.empty_like(w)
+        db = torch.empty_like(w) if ctx.has_bias else None
         N.check(lib.ccf_layernorm_bwd(x2.data_ptr(), dy2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-                                      dx.data_ptr(), dg.data_ptr(), N.ptr(db), rows, d, int(x2.dtype == torch.float16),
-                                      N.stream_ptr()), "ccf_layernorm_bwd")
-        N.count(1)
-        return dx.view(ctx.shape), dg.to(w.dtype), (db.to(w.dtype) if db is not None else None), None
+                                      dx.data_ptr(), part.data_ptr(), dg.data_ptr(), N.ptr(db), rows, d,
+                                      int(x2.dtype == torch.float16), N.stream_ptr()), "ccf_layernorm_bwd")
+        N.count(2)
+        return dx.view(ctx.shape), dg, db, None
 
 
 def supported(x: torch.Tensor, normalized_shape, weight) -> bool:

@@ -60,3 +60,30 @@ def test_colsum_grouped(rows, n, groups, fp16):
                                         N.stream_ptr()), "ccf_colsum_grouped")
     ref = torch.stack([x[b:b + r].float().sum(0) for b, r in zip(base, rows)])
     assert torch.allclose(out.float(), ref, atol=0.15, rtol=2e-2)
+
+
+@pytest.mark.parametrize("rows,d,fp16", [(1, 8, False), (5, 256, True), (33, 264, False), (16, 520, True), (9473, 1024, False),
+                                        (2371, 2048, True), (4, 1032, False)])
+def test_layernorm_backward_split_rows(rows, d, fp16):
+    """One to eight warps per row, row groups side by side, fewer rows than blocks and a ragged last pass, against fp64;
+    the weight and bias gradients are the same bits every time (no atomics)."""
+    from ccfuser_b200.ops.norm import LayerNorm
+    dt = torch.float16 if fp16 else torch.bfloat16
+    torch.manual_seed(rows)
+    ln = LayerNorm(d, device="cuda", dtype=dt)
+    with torch.no_grad():
+        ln.weight.copy_(1 + 0.2 * torch.randn(d, device="cuda"))
+    x = (torch.randn(rows, d, device="cuda") * 2 + 0.5).to(dt).requires_grad_(True)
+    gy = torch.randn(rows, d, device="cuda").to(dt)
+    got = []
+    for _ in range(2):
+        x.grad = ln.weight.grad = ln.bias.grad = None
+        ln(x).backward(gy)
+        got.append((x.grad, ln.weight.grad, ln.bias.grad))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    xd = x.detach().double().requires_grad_(True)
+    wd, bd = ln.weight.detach().double().requires_grad_(True), ln.bias.detach().double().requires_grad_(True)
+    ref = torch.autograd.grad(torch.nn.functional.layer_norm(xd, (d,), wd, bd, ln.eps), (xd, wd, bd), gy.double())
+    eps = 2.0 ** (-11 if fp16 else -8)          # one rounding of each result; the fp32 sums are far below it
+    for a, r in zip(got[0], ref):
+        assert (a.double() - r).norm() <= eps * r.norm() + 1e-6
