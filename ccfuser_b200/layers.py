@@ -88,8 +88,9 @@ class MoELayer(nn.Module):
         if backend == "fused":
             fused = self._fused_impl()
             x = x.contiguous()
-            if token_mask is None and cfg.shadow_experts == 0 and fused.one_node(x):
-                return self._finish(fused.route_and_run(x), x, None, shape)
+            lin = fused.one_node(x) if token_mask is None and cfg.shadow_experts == 0 else None
+            if lin is not None:
+                return self._finish(fused.route_and_run(x, lin), x, None, shape)
             idx, score = fused.route(x)
         else:
             idx, score = self.gate(x)

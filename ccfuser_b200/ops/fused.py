@@ -279,8 +279,9 @@ class FusedMoE:
     # ------------------------------------------------------------------------------------------
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         x = x.contiguous()
-        if self.one_node(x):
-            return self.route_and_run(x)
+        lin = self.one_node(x)
+        if lin is not None:
+            return self.route_and_run(x, lin)
         idx, w = self.route(x)
         return self.run_experts(x, idx, w)
 
@@ -288,29 +289,34 @@ class FusedMoE:
         gate = self.layer.gate
         return getattr(gate, "aux_loss_coef", 0.0), getattr(gate, "z_loss_coef", 0.0)
 
-    def one_node(self, x: torch.Tensor) -> bool:
-        """Whether router and experts of this call run as one autograd node (route_and_run): the one-kernel router
+    def one_node(self, x: torch.Tensor):
+        """The router's linear layer if router and experts of this call run as one autograd node (route_and_run), else None:
+        the one-kernel router
         applies, no auxiliary loss asks for the logits, and the call's slots fit the one-kernel routing, which lists them
         by expert for the router's weight gradient. Then the input gradient through the gate weights is added in the slot
         reduction that ends the backward pass, instead of in a kernel of its own and an addition of two [T, d] matrices."""
-        cfg, layer = self.cfg, self.layer
-        lin = getattr(layer.gate, "gate", None)
+        cfg, gate, t = self.cfg, self.layer.gate, x.shape[0]
+        lin = getattr(gate, "gate", None)
+        if not (self.native_runtime and self.fused_router and isinstance(lin, torch.nn.Linear)
+                and t <= cfg.max_tokens and t * cfg.top_k <= N.ROUTE_CLUSTER_SLOTS):
+            return None
         coef, zcoef = self._aux_coefs()
-        return (self.native_runtime and self.fused_router and isinstance(lin, torch.nn.Linear)
-                and not (coef and coef > 0) and not (zcoef and zcoef > 0) and x.shape[0] <= cfg.max_tokens
-                and x.shape[0] * cfg.top_k <= N.ROUTE_CLUSTER_SLOTS and R.supported(x, lin.weight, cfg.top_k)
-                and lin.weight.shape[0] == cfg.num_experts and (lin.bias is None or lin.bias.dtype == x.dtype))
+        if (coef and coef > 0) or (zcoef and zcoef > 0):
+            return None
+        w, b = lin.weight, lin.bias
+        return lin if (R.supported(x, w, cfg.top_k) and w.shape[0] == cfg.num_experts
+                       and (b is None or b.dtype == x.dtype)) else None
 
     def _expert_tensors(self):
         ex, gated = self.layer.experts, self.cfg.activation == "swiglu"
         return (ex.htoh4.weight, ex.htoh4.bias, ex.htoh4_gate.weight if gated else None,
                 ex.htoh4_gate.bias if gated else None, ex.h4toh.weight, ex.h4toh.bias)
 
-    def route_and_run(self, x: torch.Tensor) -> torch.Tensor:
-        """Router and experts as one autograd node; for calls that ``one_node`` accepts."""
-        lin = self.layer.gate.gate
-        if hasattr(self.layer.gate, "set_loss"):
-            self.layer.gate.set_loss(None)
+    def route_and_run(self, x: torch.Tensor, lin: torch.nn.Linear) -> torch.Tensor:
+        """Router (its linear layer ``lin``) and experts as one autograd node; for calls that ``one_node`` accepts."""
+        gate = self.layer.gate
+        if hasattr(gate, "set_loss"):
+            gate.set_loss(None)
         tensors = (x, lin.weight, lin.bias) + self._expert_tensors()
         self._save_pre = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
         try:
@@ -368,14 +374,13 @@ class FusedMoE:
             self.ctx.check_status("fused MoE forward")
         return y
 
-    def native_desc(self) -> N.Layer:
+    def native_desc(self, params=None) -> N.Layer:
         """The layer's description for the native runtime (csrc/runtime.h: CcfLayer). Built once; rebuilt if a parameter
-        tensor has been replaced (its address changed)."""
-        cfg, cc, ex = self.cfg, self.ctx, self.layer.experts
+        tensor has been replaced (its address changed). ``params``: the expert tensors, where the caller has them in hand
+        (reading them from the modules costs several microseconds)."""
+        cfg, cc = self.cfg, self.ctx
         swiglu = cfg.activation == "swiglu"
-        params = (ex.htoh4.weight, ex.htoh4.bias, ex.htoh4_gate.weight if swiglu else None,
-                  ex.htoh4_gate.bias if swiglu else None, ex.h4toh.weight, ex.h4toh.bias)
-        key = tuple(N.ptr(t) for t in params)
+        key = tuple(N.ptr(t) for t in (params if params is not None else self._expert_tensors()))
         if self._desc is not None and self._desc_key == key:
             return self._desc
         L = N.Layer()
@@ -648,14 +653,14 @@ class GraphedForwardPool:
         raise ValueError(f"{n} tokens exceed the largest bucket ({self.graphs[-1].tokens})")
 
 
-def _native_forward(fm: FusedMoE, x: torch.Tensor, idx: torch.Tensor, gate_w: torch.Tensor) -> torch.Tensor:
+def _native_forward(fm: FusedMoE, x: torch.Tensor, idx: torch.Tensor, gate_w: torch.Tensor, params=None) -> torch.Tensor:
     cfg, cc = fm.cfg, fm.ctx
     t = x.shape[0]
     y = torch.empty_like(x)
     if not cc.device_epoch:
         cc.epoch += 1
     with nvtx_range("moe.forward_native"):
-        N.check(N.load().ccf_layer_forward(C.byref(fm.native_desc()), x.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
+        N.check(N.load().ccf_layer_forward(C.byref(fm.native_desc(params)), x.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
                                            y.data_ptr(), t, cfg.capacity(t), int(fm._save_pre),
                                            -1 if cc.device_epoch else cc.epoch, N.stream_ptr(), None, 0, None),
                 "ccf_layer_forward")
@@ -712,7 +717,7 @@ class _FusedLayerFn(torch.autograd.Function):
         fm.claim_buffers(ctx)
         rw = rw.contiguous()
         idx, gate_w, _ = R.route_topk(x, rw, None if rb is None else rb.contiguous(), fm.cfg.top_k)
-        y = _native_forward(fm, x, idx, gate_w)
+        y = _native_forward(fm, x, idx, gate_w, (w1, b1, wg, bg, w2, b2))
         ctx.fm = fm
         ctx.save_for_backward(x, rw, idx, gate_w, w1, wg, w2)
         ctx.has_bias = (b1 is not None, bg is not None, b2 is not None)

@@ -25,7 +25,9 @@ class Workspace:
     def __init__(self, device):
         self.sched = torch.zeros(8, dtype=torch.int32, device=device)
         self.status = torch.zeros(2, dtype=torch.int32, device=device)  # [first hard error, overflow count]
-        self._last_stream = None
+        self._last_stream, self._last_raw = None, None
+        self._on_gpu = self.sched.device.type == "cuda"
+        self._device_index = self.sched.device.index if self._on_gpu else -1
 
     @classmethod
     def get(cls, device) -> "Workspace":
@@ -44,8 +46,11 @@ class Workspace:
         workspace's scheduler words, so two calls may only follow each other on different streams if the earlier
         stream has drained (or the caller ordered the streams and says so with ``ordered_after``); work still pending
         on another stream means the two could run concurrently and corrupt each other's tile counters: that raises."""
-        if self.sched.device.type != "cuda":
+        if not self._on_gpu:
             return
+        raw = torch._C._cuda_getCurrentRawStream(self._device_index)
+        if self._last_stream is not None and raw == self._last_raw:
+            return                                # the stream of the previous call
         cur = torch.cuda.current_stream(self.sched.device)
         last = self._last_stream
         if last is not None and last != cur and not torch.cuda.is_current_stream_capturing() and not last.query():
@@ -54,7 +59,7 @@ class Workspace:
                 "still pending on another stream of the same device. The kernels of one device share scheduler words: "
                 "issue them on one stream, or order the streams (wait_stream / events) and call "
                 "Workspace.get(device).ordered_after() before switching.")
-        self._last_stream = cur
+        self._last_stream, self._last_raw = cur, raw
 
     def ordered_after(self):
         """The caller has ordered its next stream after all fused work issued so far (event or wait_stream)."""
