@@ -120,7 +120,7 @@ class MoEConfig:
             router += (mats * d * self.shared_ffn + ((mats - 1) * self.shared_ffn + d if self.bias else 0)) * esz
         per_layer = (rows * d + slots * d) * esz                                   # xrecv + comb (symmetric)
         per_layer += rows * f * esz * (mats if training else 1)                    # h_act (+ pre-activations)
-        per_layer += (3 * slots + 2 * self.num_experts + 6 * e_loc) * 4            # routing index arrays
+        per_layer += (4 * slots + 256 + 2 * self.num_experts + 6 * e_loc) * 4      # routing index arrays
         shared = (rows * d + slots * d) * esz + rows * 8                           # grecv + gcomb + row metadata
         transient = (rows * f * esz * (mats - 1) + weights) if training else 0     # dh(, dh2) + weight gradients of one layer
         out = {"parameters": layers * (weights + router), "gradients": layers * (weights + router) if training else 0,
