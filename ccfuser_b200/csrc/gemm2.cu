@@ -3,7 +3,7 @@
 // loads, the leader CTA issues one M = 256 MMA that reads both CTAs' shared memory and writes both CTAs' TMEM, and each
 // CTA runs the epilogue for its own 128 rows. Compared with the one-CTA kernel (gemm.cu) the B operand crosses the
 // L2 -> SM fabric once per pair instead of once per CTA: 64 KB instead of 96 KB per 128x256x64 worth of MMA work, and
-// six 32 KB pipeline stages fit where four 48 KB stages did.
+// six k-blocks (three stages of two) fit into shared memory where the one-CTA kernel holds four.
 //
 // Same modes, operand majors, epilogues, dispatch role and arrival-counter gating as gemm.cu; tiles are assigned
 // statically (tile = pair index + k * number of pairs) because both CTAs of a pair must walk the same sequence.

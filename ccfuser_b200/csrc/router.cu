@@ -30,11 +30,12 @@ constexpr int kRtABytes = BM * BK * 2;   // 128 rows x 128 bytes
 constexpr int kRtMaxK = 8;
 
 // Running top-kList selection, best first; the list is the shortest of 2, 4 and 8 that holds the k wanted entries: nearly every
-// candidate enters some lane's list, and bubbling through eight entries was most of a top-2 router's epilogue (8192 x 1024, 64 experts:
-// 21.6 us with eight, 13.7 with two; 16 tokens, 16 experts: 11.5 and 7.4). A candidate enters only if it is strictly greater than the current last
-// entry (or that entry is still empty, id -1) and bubbles up past strictly smaller or empty ones, so among equal logits
-// the lower expert id stays in front (candidates are offered in ascending id order) and a row of -inf logits still
-// yields the ids 0, 1, ... rather than none. Host-callable so that the rule can be tested without a GPU.
+// candidate enters some lane's list, and bubbling through eight entries was most of a top-2 router's epilogue (8192 x 1024,
+// 64 experts: 21.6 us with eight, 13.7 with two; 16 tokens, 16 experts: 11.5 and 7.4). A candidate enters only if it is
+// strictly greater than the current last entry (or that entry is still empty, id -1) and bubbles up past strictly smaller
+// or empty ones, so among equal logits the lower expert id stays in front (candidates are offered in ascending id order) and
+// a row of -inf logits still yields the ids 0, 1, ... rather than none. Host-callable so that the rule can be tested without
+// a GPU.
 template <int kList>
 __host__ __device__ __forceinline__ void topk_offer(float (&tv)[kList], int (&ti)[kList], float v, int e) {
   if (v > tv[kList - 1] || ti[kList - 1] < 0) {

@@ -96,7 +96,7 @@ class MoELayer(nn.Module):
             idx, score = self.gate(x)
         if token_mask is not None:
             keep = token_mask.reshape(-1, 1).to(device=idx.device, dtype=torch.bool)
-            idx = torch.where(keep, idx, torch.full_like(idx, -1))
+            idx = torch.where(keep, idx, -1)
         y_shadow = None
         if cfg.shadow_experts > 0:
             # the step's most popular experts are replicated: their slots leave the expert-parallel path
