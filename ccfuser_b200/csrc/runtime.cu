@@ -179,28 +179,29 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
   return ccf_reduce(&r, stream);
 }
 
-// The arrival counters return to zero between the kernel that waits on them and this rank's finish token: peers push the
-// next pass's rows only after that token. A single rank has no peers, and its reduce kernel, the last of the pass, does it.
-int zero_tile_flags(const CcfLayer* L, Dry* dry, void* stream) {
-  if (dry != nullptr || L->world == 1) return 0;
+int clear_arrivals(const CcfLayer* L, void* stream) {
   cudaError_t e = cudaMemsetAsync(L->tile_flags, 0, sizeof(int) * (L->max_rows / 128 + 1),
                                   reinterpret_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
-}  // namespace
+// The arrival counters return to zero between the kernel that waits on them and this rank's finish token: peers push the
+// next pass's rows only after that token. A single rank has no peers, and its reduce kernel, the last of the pass, does it.
+int zero_tile_flags(const CcfLayer* L, Dry* dry, void* stream) {
+  if (dry != nullptr || L->world == 1) return 0;
+  return clear_arrivals(L, stream);
+}
 
-extern "C" {
+// Result of a pass that ends with `rc`. A pass of a single rank that is given up at one of its launches never reaches the reduce
+// kernel: with the counters left full, every tile of the group's next pass would go through its gate before its rows have
+// arrived.
+int end_of_pass(const CcfLayer* L, int rc, Dry* dry, void* stream) {
+  if (rc != 0 && dry == nullptr && L->world == 1) clear_arrivals(L, stream);
+  return rc;
+}
 
-int ccf_sizeof_layer() { return static_cast<int>(sizeof(CcfLayer)); }
-int ccf_sizeof_layer_grads() { return static_cast<int>(sizeof(CcfLayerGrads)); }
-
-int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const float* gate_w, void* y, int tokens,
-                      int capacity, int save_pre, int epoch, void* stream, CcfGemmLaunch* dry_gemms, int dry_cap,
-                      int* dry_count) {
-  if (L == nullptr || L->world < 1 || L->world > CCF_MAX_RANKS || L->e_total > CCF_MAX_GROUPS) return -2;
-  Dry dry_state = {dry_gemms, dry_cap, 0};
-  Dry* dry = dry_gemms != nullptr ? &dry_state : nullptr;
+int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* gate_w, void* y, int tokens, int capacity,
+                 int save_pre, int epoch, void* stream, Dry* dry) {
   const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
   int rc = 0;
   // An expert that receives about one 256-row pair tile's worth of rows fills most second tiles with padding: such
@@ -295,16 +296,11 @@ int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const fl
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
-  rc = wait_and_reduce(L, L->comb, y, tokens, gemm2_bn, nullptr, nullptr, nullptr, dry, stream);
-  if (dry_count != nullptr) *dry_count = dry_state.n;
-  return rc;
+  return wait_and_reduce(L, L->comb, y, tokens, gemm2_bn, nullptr, nullptr, nullptr, dry, stream);
 }
 
-int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G,
-                       int tokens, int capacity, void* stream, CcfGemmLaunch* dry_gemms, int dry_cap, int* dry_count) {
-  if (L == nullptr || G == nullptr || L->world < 1 || L->world > CCF_MAX_RANKS) return -2;
-  Dry dry_state = {dry_gemms, dry_cap, 0};
-  Dry* dry = dry_gemms != nullptr ? &dry_state : nullptr;
+int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G, int tokens,
+                  int capacity, void* stream, Dry* dry) {
   const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
   int rc = 0;
   if (dry == nullptr && L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
@@ -427,8 +423,35 @@ int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const 
   if (G->router_dw != nullptr && dry == nullptr)
     rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d, L->e_total, L->top_k,
                        L->fp16, stream);
-  if (dry_count != nullptr) *dry_count = dry_state.n;
   return rc;
+}
+
+}  // namespace
+
+extern "C" {
+
+int ccf_sizeof_layer() { return static_cast<int>(sizeof(CcfLayer)); }
+int ccf_sizeof_layer_grads() { return static_cast<int>(sizeof(CcfLayerGrads)); }
+
+int ccf_layer_forward(const CcfLayer* L, const void* x, const int* idx, const float* gate_w, void* y, int tokens,
+                      int capacity, int save_pre, int epoch, void* stream, CcfGemmLaunch* dry_gemms, int dry_cap,
+                      int* dry_count) {
+  if (L == nullptr || L->world < 1 || L->world > CCF_MAX_RANKS || L->e_total > CCF_MAX_GROUPS) return -2;
+  Dry dry_state = {dry_gemms, dry_cap, 0};
+  Dry* dry = dry_gemms != nullptr ? &dry_state : nullptr;
+  const int rc = forward_pass(L, x, idx, gate_w, y, tokens, capacity, save_pre, epoch, stream, dry);
+  if (dry_count != nullptr) *dry_count = dry_state.n;
+  return end_of_pass(L, rc, dry, stream);
+}
+
+int ccf_layer_backward(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G,
+                       int tokens, int capacity, void* stream, CcfGemmLaunch* dry_gemms, int dry_cap, int* dry_count) {
+  if (L == nullptr || G == nullptr || L->world < 1 || L->world > CCF_MAX_RANKS) return -2;
+  Dry dry_state = {dry_gemms, dry_cap, 0};
+  Dry* dry = dry_gemms != nullptr ? &dry_state : nullptr;
+  const int rc = backward_pass(L, dy, idx, gate_w, G, tokens, capacity, stream, dry);
+  if (dry_count != nullptr) *dry_count = dry_state.n;
+  return end_of_pass(L, rc, dry, stream);
 }
 
 }  // extern "C"
