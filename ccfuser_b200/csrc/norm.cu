@@ -1,10 +1,10 @@
-// LayerNorm forward and backward for 2-byte activations, one warp per row, fp32 statistics.
+// LayerNorm forward and backward for 2-byte activations, fp32 statistics: one warp per row forward, up to eight backward.
 //
 // The transformer blocks around the MoE layers (the reference's example models are stock GPT-2 / BERT / Transformer-XL,
 // mix_moe/mix_moe/examples/models/moe_gpt.py, moe_bert.py, transformer-xl/mem_transformer_mix_moe.py) normalise a
 // [tokens, d_model] matrix twice per block. Both passes are bound by reading and writing that matrix once; the
-// backward also reduces the weight and bias gradients over all rows, which is done here with per-thread partial sums
-// over the rows a warp visits, one shared-memory reduction per block and one fp32 atomic per column and block.
+// backward also reduces the weight and bias gradients over all rows: per-thread partial sums over the rows a thread visits,
+// one partial row per block, added in block order by a second small kernel.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -95,7 +95,8 @@ __global__ void __launch_bounds__(kLnThreads) layernorm_fwd_kernel(const void* _
 // pairs of row groups ahead: with loads to registers 16 warps per SM held 32 KB in flight, a third of what the memory
 // rate takes. The row sums meet in shared memory with one barrier per stage, which also frees the stage, and each block
 // leaves its partial dgamma / dbeta in `part` ([blocks, 2, d] fp32), which layernorm_bwd_finish_kernel adds in block order:
-// no atomics, no zeroed buffers, no conversion passes. 8192 x 2048 bf16: 39 + 7 us, where a dx kernel, a parameter kernel,
+// no atomics, no zeroed buffers, no conversion passes. A copy that does not arrive within the limit ends the block: time-out
+// in the status word, no further requests, NaN in the rows it leaves undone and in its partial sums. 8192 x 2048 bf16: 39 + 7 us, where a dx kernel, a parameter kernel,
 // two fills and two conversions took 37 + 16 + 6 us and four launches more.
 constexpr int kLnRows = 2;       // rows per group and stage
 constexpr int kLnStages = 6;
@@ -103,13 +104,15 @@ template <int kW>
 __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ dy,
                                                                const void* __restrict__ gamma, const float* __restrict__ mean_in,
                                                                const float* __restrict__ rstd_in, void* __restrict__ dx,
-                                                               float* __restrict__ part, int rows, int d, int fp16) {
+                                                               float* __restrict__ part, int rows, int d, int fp16,
+                                                               int* status, unsigned long long wait_limit_ns) {
   constexpr int kG = kLnWarps / kW;             // rows that a block works on side by side
   constexpr int kStageRows = kG * kLnRows;      // consecutive rows: at most 8 KB each of x and dy
   extern __shared__ __align__(16) uint8_t ln_ring[];   // [kLnStages][x rows, dy rows]
   __shared__ float2 red[2][kG][kLnRows][kW];
   __shared__ float psum[kG > 1 ? kG - 1 : 1][2][kW * 256];
   __shared__ __align__(8) uint64_t full[kLnStages];
+  __shared__ int abort_word, lost_at;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = warp / kW, wr = warp % kW;
   const int v = wr * 32 + lane, vecs = d >> 3;  // this thread's 16-byte piece of a row
@@ -122,6 +125,8 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
   const uint32_t gq[4] = {g4.x, g4.y, g4.z, g4.w};
   const int step = static_cast<int>(gridDim.x) * kStageRows;
   if (threadIdx.x == 0) {
+    abort_word = 0;
+    lost_at = 0x7fffffff;
     for (int k = 0; k < kLnStages; ++k) mbar_init(smem_u32(&full[k]), 1);
     fence_barrier_init();
   }
@@ -144,6 +149,7 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
     }
   };
   int buf = 0, slot = 0, parity = 0;
+  bool lost = false;
   int base = static_cast<int>(blockIdx.x) * kStageRows;
   if (threadIdx.x == 0)
     for (int k = 0; k < kLnStages; ++k) request(base + k * step, k);
@@ -151,9 +157,9 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
   for (; base < rows; base += step, buf ^= 1) {   // the same trips for every thread of the block
     uint4 xv[kLnRows], dv[kLnRows];
     float mu[kLnRows], rs[kLnRows];
-    // bounded; a copy that never arrives turns the rows into NaN instead of hanging
-    bool here = mbar_try_wait(smem_u32(&full[slot]), parity);
-    for (int tries = 0; !here && tries < (1 << 22); ++tries) here = mbar_try_wait(smem_u32(&full[slot]), parity);
+    // the limit is looked up only by threads that have to wait, behind the copy they wait for (looked up at the start: 0.8 us)
+    const bool here = mbar_try_wait(smem_u32(&full[slot]), parity) ||
+                      mbar_wait(smem_u32(&full[slot]), parity, &abort_word, fail_fast_limit(status, wait_limit_ns));
 #pragma unroll
     for (int u = 0; u < kLnRows; ++u) {
       const int r = u * kG + grp;
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
         xv[u] = *reinterpret_cast<const uint4*>(at);
         dv[u] = *reinterpret_cast<const uint4*>(at + half);
       }
-      mu[u] = here ? mn[u] : __int_as_float(0x7fc00000);
+      mu[u] = mn[u];
       rs[u] = rn[u];
     }
     stats(base + step);
@@ -200,7 +206,12 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
         for (int u = 0; u < kLnRows; ++u) red[buf][grp][u][wr] = make_float2(s1[u], s2[u]);
       }
     }
+    if (!here) lost_at = base;
     __syncthreads();   // row sums are there and the stage has been read; `red`'s other half is written after the next one
+    // a thread that gave up its wait takes the whole block out of the loop: every thread sees the same pass number here, even if
+    // one that is already in the next pass has written that pass's (a barrier with a reduction in it took 0.5 us of 28 more)
+    lost = *const_cast<volatile int*>(&lost_at) <= base;
+    if (lost) break;
     if (threadIdx.x == 0) request(base + kLnStages * step, slot);
     if (++slot == kLnStages) { slot = 0; parity ^= 1; }
     if constexpr (kW > 1) {
@@ -230,6 +241,21 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
       }
       reinterpret_cast<uint4*>(dx)[static_cast<size_t>(row) * vecs + v] = make_uint4(o[0], o[1], o[2], o[3]);
     }
+  }
+  if (lost) {
+    if (threadIdx.x == 0) report_status(status, CCF_ERR_MBAR_TIMEOUT, 0x50);
+    for (; base < rows; base += step) {
+      for (int u = 0; u < kLnRows; ++u) {
+        const int row = base + u * kG + grp;
+        if (row < rows && col_on)   // 0x7fff: NaN in both element types
+          reinterpret_cast<uint4*>(dx)[static_cast<size_t>(row) * vecs + v] = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) pg[i] = pb[i] = __int_as_float(0x7fc00000);
+    // give copies still in flight time to land before the shared memory goes away
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 50000ull) __nanosleep(1000);
   }
   // the block's row groups add up, then one partial row of dgamma and of dbeta per block
   if constexpr (kG > 1) {
@@ -321,9 +347,10 @@ int ccf_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* 
 int ccf_layernorm_bwd_parts(int rows, int d) { return rows < 1 || d < 8 ? 0 : ccf::ln_bwd_blocks(rows, d); }
 
 // dx [rows, d], dgamma [d] and dbeta [d] (element type; dbeta may be null) are written. `part`: scratch of
-// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats, 16-byte aligned.
+// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats, 16-byte aligned. A wait that exceeds the limit goes to `status`.
 int ccf_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
-                      float* part, void* dgamma, void* dbeta, int rows, int d, int fp16, void* stream) {
+                      float* part, void* dgamma, void* dbeta, int rows, int d, int fp16, int* status,
+                      unsigned long long wait_limit_ns, void* stream) {
   using namespace ccf;
   if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -341,7 +368,7 @@ int ccf_layernorm_bwd(const void* x, const void* dy, const void* gamma, const fl
     if (err != cudaSuccess) return -static_cast<int>(err);
     set = true;
   }
-  kern<<<blocks, 256, smem, st>>>(x, dy, gamma, mean, rstd, dx, part, rows, d, fp16);
+  kern<<<blocks, 256, smem, st>>>(x, dy, gamma, mean, rstd, dx, part, rows, d, fp16, status, wait_limit_ns);
   layernorm_bwd_finish_kernel<<<dim3((d + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, st>>>(part, blocks, d, dgamma, dbeta, fp16);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e);

@@ -9,7 +9,8 @@
 //   ccf_selftest [rows_per_group=1000] [groups=4] [k=512] [n=1024] [iters=10]
 //
 // rows_per_group need not be a multiple of the tile height: the ragged last tile of every group is part of the check.
-// Exit status 0 = all variants within tolerance and no status word set.
+// Exit status 0 = all variants within tolerance, no status word set, and the kernels' barrier wait (sm100.cuh: mbar_wait) gives up
+// a wait for an arrival that does not come within its limit.
 #include <cublas_v2.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -21,6 +22,7 @@
 #include <vector>
 
 #include "gemm_args.h"
+#include "sm100.cuh"
 
 extern "C" int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream);
 
@@ -34,6 +36,25 @@ extern "C" int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream);
   } while (0)
 
 static float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
+
+// every thread waits for an arrival that nobody makes: out = {threads that gave up, abort word, nanoseconds}
+__global__ void bounded_wait_kernel(unsigned long long limit_ns, unsigned long long* out) {
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int abort_word;
+  if (threadIdx.x == 0) {
+    abort_word = 0;
+    ccf::mbar_init(ccf::smem_u32(&bar), 1);
+    ccf::fence_barrier_init();
+  }
+  __syncthreads();
+  const uint64_t t0 = ccf::globaltimer_ns();
+  const int gave_up = __syncthreads_count(!ccf::mbar_wait(ccf::smem_u32(&bar), 0, &abort_word, limit_ns));
+  if (threadIdx.x == 0) {
+    out[0] = gave_up;
+    out[1] = abort_word;
+    out[2] = ccf::globaltimer_ns() - t0;
+  }
+}
 
 static unsigned lcg(unsigned& s) { return s = s * 1664525u + 1013904223u; }
 static float unit(unsigned& s) { return (static_cast<int>(lcg(s) >> 8) & 0xffff) / 32768.f - 1.f; }
@@ -113,6 +134,16 @@ int main(int argc, char** argv) {
     for (int r = 7; r < rows_per; r += 97) sample.push_back(g * padded + r);
   }
   int failures = 0;
+  {
+    unsigned long long *dout, w[3];
+    CK(cudaMalloc(&dout, sizeof(w)));
+    bounded_wait_kernel<<<1, 256>>>(2000000ull, dout);
+    CK(cudaMemcpy(w, dout, sizeof(w), cudaMemcpyDeviceToHost));
+    const bool ok = w[0] == 256 && w[1] == 1 && w[2] >= 2000000ull && w[2] < 1000000000ull;
+    printf("bounded wait: %llu of 256 threads gave up after %llu ns: %s\n", w[0], w[2], ok ? "ok" : "FAILED");
+    if (!ok) ++failures;
+    cudaFree(dout);
+  }
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));

@@ -210,7 +210,7 @@ def _declare(lib):
         "ccf_layernorm_max_d": ([], i),
         "ccf_layernorm_fwd": ([p, p, p, p, p, p, i, i, C.c_float, i, p], i),
         "ccf_layernorm_bwd_parts": ([i, i], i),
-        "ccf_layernorm_bwd": ([p, p, p, p, p, p, p, p, p, i, i, i, p], i),
+        "ccf_layernorm_bwd": ([p, p, p, p, p, p, p, p, p, i, i, i, p, ull, p], i),
         "ccf_symm_alloc": ([ull, C.POINTER(p)], i),
         "ccf_symm_free": ([p], i),
         "ccf_symm_handle_bytes": ([], i),

@@ -3,7 +3,7 @@
 ``LayerNorm`` is a drop-in ``nn.LayerNorm`` (same parameters, same state-dict keys); inputs the kernels do not cover
 (CPU, fp32, a normalised dimension above 2048 or not a multiple of 8, no affine parameters) take the torch path. The
 models' transformer blocks normalise a ``[tokens, d_model]`` matrix twice each; forward and backward are one pass over
-that matrix here, with the weight / bias gradients reduced in the same backward kernel.
+that matrix here; the backward kernel leaves partial weight / bias gradients, which a second small kernel adds.
 """
 from __future__ import annotations
 
@@ -12,6 +12,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import native as N
+from . import gemm as G
 
 MAX_D = 2048
 
@@ -48,7 +49,8 @@ class _LayerNormFn(torch.autograd.Function):
         db = torch.empty_like(w) if ctx.has_bias else None
         N.check(lib.ccf_layernorm_bwd(x2.data_ptr(), dy2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                       dx.data_ptr(), part.data_ptr(), dg.data_ptr(), N.ptr(db), rows, d,
-                                      int(x2.dtype == torch.float16), N.stream_ptr()), "ccf_layernorm_bwd")
+                                      int(x2.dtype == torch.float16), G.Workspace.get(x2.device).status.data_ptr(),
+                                      G.DEFAULT_WAIT_NS, N.stream_ptr()), "ccf_layernorm_bwd")
         N.count(2)
         return dx.view(ctx.shape), dg, db, None
 
