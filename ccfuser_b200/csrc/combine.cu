@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
         const int e = __ldg(a.idx + s0 + j);
         const bool routed = e >= 0 && e < a.e;
         const float g = routed ? w[j] * (dw[j] - dot) : 0.f;
-        if (v == 0) a.g[s0 + j] = a.round_g ? unpack2(pack2(g, 0.f, fp16), fp16).x : g;
+        if (v == 0) a.g[s0 + j] = g;
         if (routed) add_piece(acc, __ldg(wg + static_cast<size_t>(e) * vecs + v), g, fp16);
       }
     }

@@ -24,7 +24,6 @@ struct CcfReduceArgs {
   const void* wg;            // [e, d]
   float* g;
   int tokens, top_k, d, e, fp16;
-  int round_g;               // 1: g is written rounded to the element type (y still takes it in fp32)
 };
 
 extern "C" int ccf_reduce(const CcfReduceArgs* a, void* stream);

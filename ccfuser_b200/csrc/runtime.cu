@@ -171,9 +171,6 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
     r.dw = G->dgate;
     r.wg = G->router_w;
     r.g = G->slot_grad;
-    // from 4096 tokens on the router as a node of its own forms dWg from gradients rounded to the operand type: same here,
-    // so that both forms of a call give the same gradients
-    r.round_g = tokens >= 4096;
     r.e = L->e_total;
   }
   return ccf_reduce(&r, stream);

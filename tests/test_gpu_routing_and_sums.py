@@ -287,3 +287,28 @@ def test_few_token_layer_uses_the_bound_and_matches_the_oracle(t, e, k, act):
     assert rel(layer.experts.htoh4.weight.grad, params["htoh4.weight"].grad) < 1.5e-2
     assert rel(layer.experts.h4toh.weight.grad, params["h4toh.weight"].grad) < 1.5e-2
     layer.release()
+
+
+@pytest.mark.parametrize("act,dtype,k", [("gelu", torch.bfloat16, 2), ("swiglu", torch.float16, 3)])
+def test_router_gradients_do_not_depend_on_the_number_of_tokens(act, dtype, k):
+    """4095 tokens, and 4096 of which the last has a zero gradient: the logits' gradients are summed in fp32 at any size, so the
+    router's gradients are the same bits. (The two-node form rounds them to the element type from 4096 tokens on.)"""
+    from ccfuser_b200 import MoEConfig, MoELayer
+    torch.manual_seed(k)
+    t, d = 4096, 256
+    cfg = MoEConfig(d_model=d, d_ffn=512, num_experts=8, top_k=k, activation=act, dtype=dtype, backend="fused", max_tokens=t)
+    layer = MoELayer(cfg, device="cuda")
+    x = torch.randn(t, d, device="cuda", dtype=dtype)
+    gy = torch.randn(t, d, device="cuda", dtype=dtype)
+    gy[-1] = 0
+    got = []
+    for n in (t - 1, t):
+        xn = x[:n].clone().requires_grad_()
+        for p in layer.parameters():
+            p.grad = None
+        layer(xn).backward(gy[:n])
+        got.append((xn.grad[:t - 1], *(p.grad for p in layer.gate.parameters())))
+    layer.check_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    layer.release()
