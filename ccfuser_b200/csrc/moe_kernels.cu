@@ -232,21 +232,23 @@ __global__ void combine_wait_kernel(const int* done, int* cum, const int* sent_r
 // bias gradients: out[g, n] = sum over the rows of group g of x[r, n]. Block = 128 columns (16 lanes x 16 bytes) x 16
 // row lanes, four rows in flight per thread: the kernel streams the matrix once and has to keep enough loads in
 // flight to do so at the memory rate. With few groups and columns one block per (column block, group) leaves most of the
-// chip idle (4 groups x 4096 columns: 128 blocks that each walk 4096 rows), so up to 8 blocks of a cluster share the rows
-// and the cluster's first block adds their partial sums, read over distributed shared memory in a fixed order: no atomics,
-// no workspace, the same result every time.
+// chip idle (4 groups x 4096 columns: 128 blocks that each walk 4096 rows, 49 us, in clusters of four 24), so up to 8 blocks of
+// a cluster share the rows (combine.h: how many) and the cluster's first block adds their partial sums, read over distributed
+// shared memory in a fixed order: no atomics, no workspace, the same result every time.
 // ---------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) colsum_grouped_kernel(const void* x, long long ld, int n, const int* group_base,
                                                              const int* group_rows, void* out, int fp16) {
   __shared__ float red[16][128];
   __shared__ float part[128];
   const int g = blockIdx.y;
-  const int split = blockIdx.z, splits = gridDim.z;   // the cluster spans the z dimension of the grid
+  const int nr = group_rows[g];
+  const int split = blockIdx.z, splits = splits_with_work(nr, gridDim.z);   // the cluster spans the z dimension of the grid
+  if (split >= splits) return;
   const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
   const int col = blockIdx.x * 128 + cx * 8;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col < n) {
-    const int r0 = group_base[g], nr = group_rows[g];
+    const int r0 = group_base[g];
     const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + static_cast<size_t>(r0) * ld + col;
     for (int r = split * 64 + ry; r < nr; r += 64 * splits) {
       uint4 v[4];
@@ -483,17 +485,12 @@ int ccf_combine_reduce(const void* comb, const int* slot_row, void* y, int T, in
   return ccf_reduce(&a, stream);
 }
 
-// `rows_hint`: expected rows per group, or 0 when the caller does not know
-int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
-                            void* out, int fp16, int rows_hint, void* stream) {
+int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                       void* out, int fp16, void* stream) {
   if (n % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;   // 16-byte loads
   const int blocks = (n + 127) / 128 * groups;
   if (groups < 1 || blocks < 1) return -2;
-  // Rows are shared by a cluster while the launch has fewer than four blocks per SM (below that the loads in flight do not
-  // cover the memory latency) and every block keeps at least four passes of 64 rows: 16 groups of 188 rows took 10.5 us
-  // unshared and 15.1 us in clusters of 2 and 8, 4 groups of 4096 rows 103 us and 43 us (both for 4 d + d columns).
-  int splits = 1;
-  while (splits < 8 && blocks * splits < 4 * 148 && (rows_hint <= 0 || rows_hint >= 2 * splits * 256)) splits *= 2;
+  const int splits = ccf::group_splits(blocks);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((n + 127) / 128, groups, splits);
   cfg.blockDim = dim3(256);
@@ -503,11 +500,6 @@ int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, cons
   cfg.numAttrs = splits > 1 ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, ccf::colsum_grouped_kernel, x, ld, n, group_base, group_rows, out, fp16);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
-}
-
-int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
-                       void* out, int fp16, void* stream) {
-  return ccf_colsum_grouped_hint(x, ld, n, groups, group_base, group_rows, out, fp16, 0, stream);
 }
 
 int ccf_sgd_step(void* p, const void* g, long long n, float lr, float wd, int fp16, void* stream) {

@@ -312,3 +312,52 @@ def test_router_gradients_do_not_depend_on_the_number_of_tokens(act, dtype, k):
     for a, b in zip(*got):
         assert torch.equal(a, b)
     layer.release()
+
+
+_EDGES = [0, 1, 127, 128, 255, 256, 257, 511, 512, 1023, 1024, 1025]
+
+
+@pytest.mark.parametrize("copies,n", [(1, 256), (1, 1000), (2, 1536), (4, 1536), (8, 1024)])   # 24 to 768 blocks
+def test_column_sums_at_the_edges_of_the_sharing_rule(copies, n):
+    """Launches of every cluster size (and of none) whose groups keep all, some or one of the blocks; tolerance as above."""
+    from ccfuser_b200 import native as N
+    rows = _EDGES * copies
+    pad = [(r + 127) // 128 * 128 for r in rows]
+    base = [sum(pad[:i]) for i in range(len(rows))]
+    x = torch.randn(sum(pad), n, device="cuda").bfloat16()
+    gb, gr = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (base, rows))
+    out = torch.empty(len(rows), n, dtype=torch.bfloat16, device="cuda")
+    N.check(N.load().ccf_colsum_grouped(x.data_ptr(), n, n, len(rows), gb.data_ptr(), gr.data_ptr(), out.data_ptr(), 0,
+                                        N.stream_ptr()), "ccf_colsum_grouped")
+    ref = torch.stack([x[b:b + r].double().sum(0) for b, r in zip(base, rows)])
+    mag = torch.stack([x[b:b + r].double().abs().sum(0) for b, r in zip(base, rows)])
+    assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * 2.0 ** -16 + 1e-7).all()
+
+
+@pytest.mark.parametrize("copies,d,k,fp16", [(1, 256, 1, False), (1, 1000, 3, True), (4, 1536, 2, False), (8, 1024, 2, True)])
+def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, fp16):
+    """dWg and db from slot lists of every length against fp64: fp32 products and sums, one rounding."""
+    from ccfuser_b200 import native as N
+    dt = torch.float16 if fp16 else torch.bfloat16
+    counts = _EDGES * copies
+    e, slots = len(counts), (sum(counts) + k - 1) // k * k
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    order = torch.randperm(slots, device="cuda", generator=gen)[:sum(counts)]
+    x = torch.randn(slots // k, d, device="cuda", generator=gen).to(dt)
+    g = torch.randn(slots, device="cuda", generator=gen)
+    start = [sum(counts[:i]) for i in range(e)]
+    raw = torch.zeros(N.MAX_GROUPS + slots, dtype=torch.int32, device="cuda")
+    raw[:e] = torch.tensor(start, dtype=torch.int32)
+    raw[N.MAX_GROUPS:N.MAX_GROUPS + order.numel()] = order.int()
+    cnt = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    dw, db = torch.full((e, d), 7.0, dtype=dt, device="cuda"), torch.full((e,), 7.0, dtype=dt, device="cuda")
+    N.check(N.load().ccf_router_dw(raw.data_ptr(), cnt.data_ptr(), g.data_ptr(), x.data_ptr(), dw.data_ptr(), db.data_ptr(), d, e, k,
+                                   int(fp16), N.stream_ptr()), "ccf_router_dw")
+    ulp = 2.0 ** (-11 if fp16 else -8)
+    for i, (s, c) in enumerate(zip(start, counts)):
+        ids = order[s:s + c]
+        gs, xs = g[ids].double(), x[ids // k].double()
+        ref, mag = gs @ xs, gs.abs() @ xs.abs()
+        # the sums of the largest lists stay far below fp16's 65504; 6e-8 is its smallest number
+        assert ((dw[i].double() - ref).abs() <= ref.abs() * ulp + mag * 2.0 ** -16 + 1e-7).all(), i
+        assert (db[i].double() - gs.sum()).abs() <= gs.sum().abs() * ulp + gs.abs().sum() * 2.0 ** -16 + 1e-7, i
