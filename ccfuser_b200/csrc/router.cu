@@ -222,8 +222,6 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (mbar_wait(smem_u32(&ctrl->acc_full), 0, abort_word, limit)) {
       tc_fence_after();
       if (a.splits == 1) {
-        // running top-8 in registers, best first; a candidate enters only if it is strictly greater than the current
-        // last entry and bubbles up past strictly smaller ones, so equal logits keep the lower expert id first
         float tv[kList];
         int ti[kList];
 #pragma unroll
@@ -413,6 +411,40 @@ __global__ void __launch_bounds__(256) router_bwd_dw_kernel(const int* __restric
   }
 }
 
+// What the current device needs to know before the first launch: the kernels' shared-memory limit, and how many clusters of 2, 4
+// and 8 CTAs it holds at once when every CTA fills an SM. The number of SMs does not tell: a cluster has to fit into one GPC
+// (measured: 74, 33 and 15 of 148 SMs).
+struct RouterDevice {
+  bool ready;
+  int clusters[9];   // by cluster size
+};
+
+static int router_device(const RouterDevice** out) {
+  static RouterDevice devices[64] = {};   // the attribute belongs to the (function, device) pair
+  int dev = 0;
+  cudaGetDevice(&dev);
+  RouterDevice& r = devices[dev & 63];
+  *out = &r;
+  if (r.ready) return 0;
+  constexpr int kMaxSmem = 227 * 1024;
+  cudaError_t err = cudaFuncSetAttribute(router_topk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(router_topk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(router_topk_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  for (int splits = 2; splits <= 8 && err == cudaSuccess; splits *= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, splits);
+    cfg.blockDim = dim3(kRtThreads);
+    cfg.dynamicSmemBytes = kMaxSmem;
+    cudaLaunchAttribute attr[1] = {cluster_attribute(1, splits, 1)};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    err = cudaOccupancyMaxActiveClusters(&r.clusters[splits], router_topk_kernel<2>, &cfg);
+  }
+  if (err != cudaSuccess) return -static_cast<int>(err);
+  r.ready = true;
+  return 0;
+}
+
 // the epilogue's selection rule on host memory
 template <int kList>
 static void select_rows(const float* logits, int tokens, int e, int k, int* idx, float* w) {
@@ -462,10 +494,14 @@ int ccf_router_topk(const void* x, const void* wg, const void* bias, int tokens,
   const int stage_bytes = kRtABytes + a.n_pad * 128;
   const int kblocks = (d + BK - 1) / BK;
   const int tiles = (tokens + BM - 1) / BM;
-  // Share a row tile among as many CTAs as still fit the chip in one wave (a CTA fills an SM's shared memory); each keeps at
-  // least two k-blocks, and none is left without any.
+  const RouterDevice* device_info;
+  int rc;
+  if ((rc = router_device(&device_info))) return rc;
+  // Share a row tile among as many CTAs as still fit the chip in one wave of clusters; each keeps at least two k-blocks, and none
+  // is left without any. At the ends of the ranges, us with 8 / 4, 4 / 2 and 2 / 1 CTAs per tile: 15 tiles of 4096 columns 10.3 / 12.1,
+  // 16 tiles 17.3 / 12.1; 33 tiles of 2048 columns 13.5 / 15.5, 34 tiles 23.4 / 15.5; 74 tiles 17.1 / 19.1.
   a.splits = 8;
-  while (a.splits > 1 && (tiles * a.splits > 148 || kblocks < 2 * a.splits ||
+  while (a.splits > 1 && (tiles > device_info->clusters[a.splits] || kblocks < 2 * a.splits ||
                           (a.splits - 1) * ((kblocks + a.splits - 1) / a.splits) >= kblocks))
     a.splits /= 2;
   const int per_split = (kblocks + a.splits - 1) / a.splits;
@@ -481,19 +517,10 @@ int ccf_router_topk(const void* x, const void* wg, const void* bias, int tokens,
   a.ctrl_off = body_bytes;
   const int smem_bytes = 1024 + body_bytes + static_cast<int>(sizeof(RouterCtrl));
   CUtensorMap tmx, tmw;
-  int rc;
   if ((rc = make_tmap(&tmx, x, tokens, d, 64, BM, fp16))) return rc;
   if ((rc = make_tmap(&tmw, wg, e, d, 64, a.n_pad, fp16))) return rc;
   const int list = k <= 2 ? 0 : k <= 4 ? 1 : 2;
   auto kern = list == 0 ? router_topk_kernel<2> : list == 1 ? router_topk_kernel<4> : router_topk_kernel<8>;
-  static bool configured[64][3] = {};   // per device: the attribute belongs to the (function, device) pair
-  int cur = 0;
-  cudaGetDevice(&cur);
-  if (!configured[cur & 63][list]) {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (err != cudaSuccess) return -static_cast<int>(err);
-    configured[cur & 63][list] = true;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, a.splits);
   cfg.blockDim = dim3(kRtThreads);

@@ -361,3 +361,9 @@ def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, f
         # the sums of the largest lists stay far below fp16's 65504; 6e-8 is its smallest number
         assert ((dw[i].double() - ref).abs() <= ref.abs() * ulp + mag * 2.0 ** -16 + 1e-7).all(), i
         assert (db[i].double() - gs.sum()).abs() <= gs.sum().abs() * ulp + gs.abs().sum() * 2.0 ** -16 + 1e-7, i
+
+
+@pytest.mark.parametrize("tiles", [14, 15, 16, 17, 32, 33, 34, 38, 74, 75])
+def test_router_where_the_cluster_size_changes(tiles):
+    """Token counts on both sides of each step of the rule (clusters of eight, four, two, none)."""
+    test_router_splits(128 * tiles - 5, 2048, 64, 2, torch.bfloat16, True)
