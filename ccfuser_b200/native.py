@@ -310,18 +310,26 @@ def check(rc: int, what: str):
         raise RuntimeError(f"{what} failed with code {rc} ({'; '.join(parts)})")
 
 
-_has_gpu = None   # whether this machine has a GPU: asked once (torch.cuda.is_available reads the environment on every call)
+_gpu_seen = False   # asked until the answer is yes (torch.cuda.is_available reads the environment on every call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def current_raw_stream(device_index: int) -> int:
+    """Handle of a device's current stream. Every launcher asks for it: torch.cuda.current_stream(), the form every torch has,
+    builds a Stream object, about 3 us per launch."""
+    if _raw_stream is not None:
+        return _raw_stream(device_index)
+    return torch.cuda.current_stream(device_index).cuda_stream
 
 
 def stream_ptr() -> int:
-    """Handle of the current stream of the current device (0 without a GPU: host-side dry runs). Every launcher asks for it,
-    so it goes to the raw handle: torch.cuda.current_stream() builds a Stream object, about 3 us per launch."""
-    global _has_gpu
-    if _has_gpu is None:
-        _has_gpu = torch.cuda.is_available()
-    if not _has_gpu:
-        return 0
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """Handle of the current stream of the current device (0 without a GPU: host-side dry runs)."""
+    global _gpu_seen
+    if not _gpu_seen:
+        _gpu_seen = torch.cuda.is_available()
+        if not _gpu_seen:
+            return 0
+    return current_raw_stream(torch.cuda.current_device())
 
 
 def ptr(t) -> int:

@@ -48,7 +48,7 @@ class Workspace:
         on another stream means the two could run concurrently and corrupt each other's tile counters: that raises."""
         if not self._on_gpu:
             return
-        raw = torch._C._cuda_getCurrentRawStream(self._device_index)
+        raw = N.current_raw_stream(self._device_index)
         if self._last_stream is not None and raw == self._last_raw:
             return                                # the stream of the previous call
         cur = torch.cuda.current_stream(self.sched.device)

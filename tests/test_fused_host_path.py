@@ -217,6 +217,20 @@ def test_canary_guards_detect_an_overrun(monkeypatch):
         layer.check_status()
 
 
+def test_stream_handle_is_looked_up_per_call(monkeypatch):
+    """The answer "no GPU" is not kept, and a torch without the raw-handle query is asked for its Stream object."""
+    monkeypatch.setattr(N, "_gpu_seen", False)
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: False)
+    assert N.stream_ptr() == 0
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(N, "_raw_stream", lambda i: 100 + i)
+    assert N.stream_ptr() == 103
+    monkeypatch.setattr(N, "_raw_stream", None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda i: type("S", (), {"cuda_stream": 200 + i}))
+    assert N.stream_ptr() == 203 and N.current_raw_stream(1) == 201
+
+
 def test_device_barrier_arguments():
     cfg, layer = _layer("gelu")
     cc = layer._fused_impl().ctx
