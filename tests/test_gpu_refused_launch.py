@@ -61,3 +61,23 @@ def test_call_after_a_refused_launch(act, tokens, where, sgd):
         assert torch.equal(a, b)
     layer.check_status()
     layer.release()
+
+
+def test_call_after_a_backward_pass_that_has_no_kernel():
+    """d_model 64 runs forward only: its backward pass is refused at the weight gradient, after the dispatch of the gradients."""
+    from ccfuser_b200 import MoEConfig, MoELayer
+    torch.manual_seed(3)
+    cfg = MoEConfig(d_model=64, d_ffn=128, num_experts=8, top_k=2, dtype=torch.bfloat16, backend="fused", max_tokens=2000)
+    layer = MoELayer(cfg, device="cuda")
+    x, x2 = (torch.randn(2000, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    with torch.no_grad():
+        want = layer(x2)
+    y = layer(x)
+    with pytest.raises(RuntimeError):
+        y.backward(torch.randn_like(x))
+    torch.cuda.synchronize()
+    assert not layer._fused_impl().ctx.tile_flags.any()
+    with torch.no_grad():
+        assert torch.equal(layer(x2), want)
+    layer.check_status()
+    layer.release()

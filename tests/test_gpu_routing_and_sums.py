@@ -367,3 +367,184 @@ def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, f
 def test_router_where_the_cluster_size_changes(tiles):
     """Token counts on both sides of each step of the rule (clusters of eight, four, two, none)."""
     test_router_splits(128 * tiles - 5, 2048, 64, 2, torch.bfloat16, True)
+
+
+@pytest.mark.parametrize("world,rank,slots,e,cap", [(2, 0, 100, 8, 20), (2, 1, 1025, 64, 1 << 20), (8, 3, 20000, 64, 300),
+                                                   (8, 7, 65536, 256, 1 << 20)])
+@pytest.mark.parametrize("device_epoch", [False, True])
+def test_route_plan_exchanges_counts_as_the_separate_kernels_do(world, rank, slots, e, cap, device_epoch):
+    """One rank's view of a group: the peers' counts and flags are in its table before the launch, so nothing waits; its own
+    counts have to appear in every rank's table under the call's epoch. All outputs against ccf_route_ordered + ccf_plan and
+    the layout against its definition, with a receive buffer that some rows do not fit."""
+    from ccfuser_b200 import native as N
+    lib = N.load()
+    gen = torch.Generator(device="cuda").manual_seed(slots + rank)
+    expert = torch.randint(-1, e + 1, (slots,), dtype=torch.int32, device="cuda", generator=gen)
+    others = torch.randint(0, 300, (world, e), dtype=torch.int32, device="cuda", generator=gen)
+    i32, epoch, e_loc, nb = dict(dtype=torch.int32, device="cuda"), 5, e // world, (slots + 1023) // 1024
+    max_rows = 128 * (2 * e_loc + 1)
+    res = []
+    for one in (False, True):
+        t = {"pos": torch.zeros(slots, **i32), "raw": torch.zeros(e, **i32), "kept": torch.zeros(e, **i32),
+             "order_off": torch.zeros(e + 1, **i32), "sorted_slot": torch.full((slots,), -1, **i32),
+             "slot_row": torch.zeros(slots, **i32)}
+        out = {k: torch.full((n,), -7, **i32) for k, n in (("dst_base", e), ("group_base", e_loc), ("group_rows", e_loc),
+                                                          ("local_begin", e_loc), ("local_rows", e_loc), ("sent_rows", 8))}
+        out["table_copy"] = torch.full((world, e), -7, **i32)
+        tables, flags = torch.full((world, world, e), -7, **i32), torch.zeros(world, 8, **i32)   # what each rank would hold
+        tables[rank] = others
+        flags[rank, :world] = epoch
+        flags[rank, rank] = 0
+        status, counter = torch.zeros(2, **i32), torch.full((1,), epoch - 1, **i32)
+        p = N.PlanArgs()
+        p.count_kept = t["kept"].data_ptr()
+        for r in range(world):
+            p.peer_table[r], p.peer_flag[r] = tables[r].data_ptr(), flags[r].data_ptr()
+        for k, v in out.items():
+            setattr(p, k, v.data_ptr())
+        p.status, p.wait_limit_ns = status.data_ptr(), 1_000_000_000
+        p.world, p.my_rank, p.e_total, p.e_loc, p.epoch, p.max_rows = world, rank, e, e_loc, (0 if device_epoch else epoch), max_rows
+        if one:
+            N.check(lib.ccf_route_plan(expert.data_ptr(), slots, e, cap, t["pos"].data_ptr(), t["raw"].data_ptr(),
+                                       t["kept"].data_ptr(), t["order_off"].data_ptr(), t["sorted_slot"].data_ptr(),
+                                       t["slot_row"].data_ptr(), rank * e_loc, None, C.byref(p),
+                                       counter.data_ptr() if device_epoch else None, N.stream_ptr()), "ccf_route_plan")
+        else:
+            bh, bo, ticket = torch.zeros(nb * e, **i32), torch.zeros(nb * e, **i32), torch.zeros(1, **i32)
+            N.check(lib.ccf_route_ordered(expert.data_ptr(), slots, e, cap, t["pos"].data_ptr(), bh.data_ptr(), bo.data_ptr(),
+                                          t["raw"].data_ptr(), t["kept"].data_ptr(), ticket.data_ptr(),
+                                          t["order_off"].data_ptr(), t["sorted_slot"].data_ptr(), t["slot_row"].data_ptr(),
+                                          rank * e_loc, N.stream_ptr()), "ccf_route_ordered")
+            N.check(lib.ccf_plan_dev_epoch(C.byref(p), counter.data_ptr(), N.stream_ptr()) if device_epoch
+                    else lib.ccf_plan(C.byref(p), N.stream_ptr()), "ccf_plan")
+        torch.cuda.synchronize()
+        assert int(counter) == (epoch if device_epoch else epoch - 1)
+        assert (flags[:, rank] == epoch).all() and (tables[:, rank] == t["kept"]).all()
+        res.append({**t, **out, "status": status})
+    for k in res[0]:
+        assert torch.equal(res[0][k], res[1][k]), k
+    table = others.cpu().long()
+    table[rank] = res[1]["kept"].cpu()
+    assert torch.equal(res[1]["table_copy"].cpu().long(), table)
+    mine = table[:rank].sum(0)                                       # rows of earlier sources come first
+    for o in range(world):
+        padded = (table.sum(0)[o * e_loc:(o + 1) * e_loc] + 127) // 128 * 128
+        base = torch.cumsum(padded, 0) - padded
+        first = base + mine[o * e_loc:(o + 1) * e_loc]
+        assert torch.equal(res[1]["dst_base"].cpu().long()[o * e_loc:(o + 1) * e_loc], first)
+        assert int(res[1]["sent_rows"][o]) == int(torch.minimum(table[rank, o * e_loc:(o + 1) * e_loc], (max_rows - first).clamp(min=0)).sum())
+        if o == rank:
+            assert torch.equal(res[1]["group_base"].cpu().long(), base)
+
+
+@pytest.mark.parametrize("slots", [64, 65536])
+def test_route_plan_without_a_peer_ends_with_a_status(slots):
+    """A peer whose counts never come: the wait of the cluster's first CTA runs out, the others leave with it, no row is planned."""
+    from ccfuser_b200 import native as N
+    lib, e, i32 = N.load(), 16, dict(dtype=torch.int32, device="cuda")
+    expert = torch.arange(slots, device="cuda", dtype=torch.int32) % e
+    pos, row, srt = (torch.zeros(slots, **i32) for _ in range(3))
+    raw, kept, off = torch.zeros(e, **i32), torch.zeros(e, **i32), torch.zeros(e + 1, **i32)
+    out = {k: torch.full((e,), -7, **i32) for k in ("dst_base", "group_base", "group_rows", "local_begin", "local_rows", "sent_rows")}
+    tables, flags, status = torch.zeros(2, 2, e, **i32), torch.zeros(2, 8, **i32), torch.zeros(2, **i32)
+    p = N.PlanArgs()
+    for r in range(2):
+        p.peer_table[r], p.peer_flag[r] = tables[r].data_ptr(), flags[r].data_ptr()
+    for k, v in out.items():
+        setattr(p, k, v.data_ptr())
+    p.status, p.wait_limit_ns = status.data_ptr(), 20_000_000
+    p.world, p.my_rank, p.e_total, p.e_loc, p.epoch, p.max_rows = 2, 0, e, e // 2, 1, 1 << 20
+    N.check(lib.ccf_route_plan(expert.data_ptr(), slots, e, 1 << 20, pos.data_ptr(), raw.data_ptr(), kept.data_ptr(), off.data_ptr(),
+                               srt.data_ptr(), row.data_ptr(), 0, None, C.byref(p), None, N.stream_ptr()), "ccf_route_plan")
+    torch.cuda.synchronize()
+    assert int(status[0]) & 0xff == 2                   # CCF_ERR_FLAG_TIMEOUT
+    assert (out["group_rows"][:e // 2] == 0).all() and (out["sent_rows"][:2] == 0).all() and (out["dst_base"] == 0).all()
+    assert (kept == slots // e).all() and torch.equal(pos, torch.arange(slots, device="cuda", dtype=torch.int32) // e)
+
+
+@pytest.mark.parametrize("a_rows,bn,rows", [(32, 256, [1, 32, 0, 31, 7]), (64, 256, [64, 33, 1, 0])])
+@pytest.mark.parametrize("k", [64, 1024])
+def test_row_bound_with_mn_major_weights(a_rows, bn, rows, k):
+    """The small pipeline geometries with the operand majors of the input-gradient GEMMs (weights read [reduction, columns])."""
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops import gemm as G
+    torch.manual_seed(k + len(rows))
+    base, acc = [], 0
+    for r in rows:
+        base.append(acc)
+        acc += (r + 127) // 128 * 128
+    n, groups = 384, len(rows)
+    x = torch.full((max(acc, 128) + 128, k), float("nan"), device="cuda", dtype=torch.bfloat16)
+    for b, r in zip(base, rows):
+        x[b:b + r] = torch.randn(r, k, device="cuda").bfloat16()
+    w = (torch.randn(groups * k, n, device="cuda") * 0.1).bfloat16()
+    out = torch.full((x.shape[0], n), 7.0, dtype=torch.bfloat16, device="cuda")
+    ws = G.launch(a0=x, b0=w, a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=n, k=k,
+                  group_base=torch.tensor(base, dtype=torch.int32, device="cuda"),
+                  group_rows=torch.tensor(rows, dtype=torch.int32, device="cuda"), num_groups=groups, b_group_rows=k, out0=out,
+                  two_cta=False, bn=bn, a_rows=a_rows)
+    ws.check("row bound")
+    for i, (b, r) in enumerate(zip(base, rows)):
+        ref = x[b:b + r].double() @ w[i * k:(i + 1) * k].double()
+        assert ((out[b:b + r].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all(), i
+        assert (out[b + r:b + (r + 127) // 128 * 128] == 7.0).all()
+
+
+def _layer_against_oracle(t, d, f, e, k, act, router, tol):
+    """Output and every gradient of a layer call against the fp32 oracle on the same routing decisions, with the gate weights
+    differentiable through the oracle's router."""
+    from ccfuser_b200 import MoEConfig, MoELayer
+    from ccfuser_b200.ops.reference import dense_moe_oracle
+    torch.manual_seed(t * e + k)
+    cfg = MoEConfig(d_model=d, d_ffn=f, num_experts=e, top_k=k, activation=act, dtype=torch.bfloat16, backend="fused",
+                    max_tokens=t, router_bias=router != "no bias")
+    layer = MoELayer(cfg, device="cuda")
+    with torch.no_grad():
+        for n, p in layer.named_parameters():
+            if n.endswith("bias"):
+                p.add_(torch.randn_like(p) * 0.1)
+    if router == "frozen weight":
+        layer.gate.gate.weight.requires_grad_(False)
+    x = torch.randn(t, d, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    fm = layer._fused_impl()
+    one = fm.one_node(x) is not None
+    y = layer(x)
+    gy = torch.randn_like(y)
+    y.backward(gy)
+    layer.check_status()
+    with torch.no_grad():
+        idx, _ = fm.route(x.detach())
+    params = {n.replace("experts.", "").replace("gate.gate.", "gate."): p.detach().float().requires_grad_() for n, p in layer.named_parameters()}
+    xf = x.detach().float().requires_grad_()
+    logits = torch.nn.functional.linear(xf, params["gate.weight"], params.get("gate.bias"))
+    score = torch.softmax(torch.gather(logits, 1, idx.long()), -1)
+    (ref,) = dense_moe_oracle([xf], params, top_k=k, capacity=None, activation=act, routing=[(idx, score)])
+    ref.backward(gy.float())
+    pairs = {"y": (y.detach(), ref.detach()), "x": (x.grad, xf.grad)}
+    for n, p in layer.named_parameters():
+        if p.requires_grad:
+            pairs[n] = (p.grad, params[n.replace("experts.", "").replace("gate.gate.", "gate.")].grad)
+        else:
+            assert p.grad is None
+    layer.release()
+    # with one slot per token the gate weight is the constant 1: its router gradients are zero on both sides
+    floor = 1e-6 * float(ref.detach().norm())
+    bad = {n: err for n, (a, b) in pairs.items() if not (err := float((a.float() - b).norm()) / max(float(b.norm()), floor)) < tol}
+    assert not bad, bad
+    return one
+
+
+@pytest.mark.parametrize("t,e,k,act,router", [(1, 16, 2, "gelu", "bias"), (16, 16, 2, "swiglu", "no bias"), (8, 4, 4, "relu", "bias"),
+                                             (32, 4, 2, "swiglu", "bias"), (21, 64, 3, "gelu", "frozen weight"),
+                                             (60, 8, 1, "swiglu", "bias"), (33, 64, 2, "gelu", "no bias")])
+def test_few_token_layer_gradients_match_the_oracle(t, e, k, act, router):
+    """Calls whose rows per expert are bounded by 32, by 64 and not at all. Every stored intermediate (pre-activation, activation,
+    gate-scaled output, their gradients) is rounded to 8 significant bits, a relative error of at most 2^-8 each and about six on
+    the longest path; the router's gradients are differences of two of those."""
+    assert _layer_against_oracle(t, 256, 512, e, k, act, router, 6 * 2.0 ** -8)
+
+
+@pytest.mark.parametrize("t,k", [(32768, 2), (32769, 2)])
+def test_layer_around_the_slots_of_the_one_kernel_routing(t, k):
+    """65536 slots run as one node, 65538 with the separate routing kernels and two nodes; same tolerance as above."""
+    assert _layer_against_oracle(t, 128, 256, 8, k, "gelu", "bias", 6 * 2.0 ** -8) == (t * k <= 65536)
