@@ -13,7 +13,8 @@ namespace ccf {
 
 constexpr int kMaxK = 8;
 constexpr int kReduceThreads = 256;
-constexpr int kReducePieces = 2;   // 16-byte pieces of the result per thread
+// 16-byte pieces of the result per thread: with one slot per token a single row read would not cover the memory latency
+__host__ __device__ constexpr int reduce_pieces(int k) { return k == 1 ? 2 : 1; }
 
 __device__ __forceinline__ void add_piece(float (&acc)[8], const uint4& x, float scale, int fp16) {
   const uint32_t w[4] = {x.x, x.y, x.z, x.w};
@@ -25,11 +26,13 @@ __device__ __forceinline__ void add_piece(float (&acc)[8], const uint4& x, float
   }
 }
 
-// y[t, :] = sum_j keep(t, j) * comb[t * k + j, :] in fp32, one rounding. Bound by reading k rows and writing one per token;
-// a block takes whole tokens (512 pieces of 16 bytes) and kK is a template argument so that all rows of a token are
-// requested before the first is used. With kRouter the same pass adds the router's share of the input gradient,
-// sum_j g_j Wg[idx_j, :] (Wg is small and stays in L2), which as a kernel of its own wrote and re-read a [T, d] matrix:
-// 16384 x 4096, top-2: 166 us for both, from 94 + 58 + 66 us (reduce, router dx, addition of the two gradients).
+// y[t, :] = sum_j keep(t, j) * comb[t * k + j, :] in fp32, one rounding. Bound by reading k rows and writing one per token. kK is
+// the number of slots per token (0: more than eight, eight at a time), so that all rows of a piece are requested before the first
+// is used, and none besides. 8192 x 4096, us with 1 / 2 / 3 / 4 / 8 slots: 30 / 41 / 76 / 79 / 99 with whole tokens per block and one
+// form for three to eight slots, now 23 / 36 / 42 / 49 / 91; one token of 8192 columns, two slots: 3.2, now 1.9. With kRouter the
+// same pass adds the router's share of the input gradient, sum_j g_j Wg[idx_j, :] (Wg is small and stays in L2), which as a kernel
+// of its own wrote and re-read a [T, d] matrix: 16384 x 4096, top-2: 91 us, from 81 + 42 + 59 us (reduce, router dx, addition of
+// the two gradients).
 template <int kK, bool kRouter>
 __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __grid_constant__ CcfReduceArgs a) {
   const int vecs = a.d >> 3, K = kK > 0 ? kK : a.top_k, fp16 = a.fp16;
@@ -42,29 +45,39 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
     }
     for (int i = threadIdx.x; i < a.zero_count; i += kReduceThreads) a.zero_words[i] = 0;
   }
-  const int per_block = max(1, kReduceThreads * kReducePieces / vecs);   // tokens of this block
-  const int t0 = static_cast<int>(blockIdx.x) * per_block;
-  const int items = min(per_block, a.tokens - t0) * vecs;
   const uint4* comb = reinterpret_cast<const uint4*>(a.comb);
   const uint4* wg = reinterpret_cast<const uint4*>(a.wg);
-#pragma unroll kReducePieces
-  for (int i = threadIdx.x; i < items; i += kReduceThreads) {
-    const int lt = i / vecs, v = i - lt * vecs, t = t0 + lt;
+  constexpr int kP = reduce_pieces(kK), kSpan = kReduceThreads * kP, kN = kK > 0 ? kK : kMaxK;
+  // pieces kSpan * block + thread (+ 256, ...) of [tokens, vecs], without a product that may not fit 32 bits: `vecs` blocks are
+  // kSpan tokens
+  const int i0 = static_cast<int>(blockIdx.x % vecs) * kSpan + threadIdx.x, tb = static_cast<int>(blockIdx.x / vecs) * kSpan;
+  uint4 x[kP][kN];
+  bool on[kP][kN];
+  auto fetch = [&](int p, int j0) {
+    const int i = i0 + p * kReduceThreads, t = tb + i / vecs, v = i % vecs;
+    const size_t s0 = static_cast<size_t>(t) * K + j0;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+      on[p][j] = t < a.tokens && j0 + j < K && __ldg(a.slot_row + s0 + j) >= 0;
+      x[p][j] = make_uint4(0u, 0u, 0u, 0u);
+      if (on[p][j]) x[p][j] = comb[(s0 + j) * vecs + v];
+    }
+  };
+  if constexpr (kK > 0) {
+#pragma unroll
+    for (int p = 0; p < kP; ++p) fetch(p, 0);
+  }
+#pragma unroll
+  for (int p = 0; p < kP; ++p) {
+    const int i = i0 + p * kReduceThreads, t = tb + i / vecs, v = i % vecs;
+    if (t >= a.tokens) break;
     const size_t s0 = static_cast<size_t>(t) * K;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    constexpr int kN = kK > 0 ? kK : kMaxK;
-    bool on[kN];
     for (int j0 = 0; j0 < K; j0 += kN) {   // once, except for more than kMaxK slots per token
-      uint4 x[kN];
-#pragma unroll
-      for (int j = 0; j < kN; ++j) {
-        on[j] = j0 + j < K && __ldg(a.slot_row + s0 + j0 + j) >= 0;
-        x[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (on[j]) x[j] = comb[(s0 + j0 + j) * vecs + v];
-      }
+      if constexpr (kK == 0) fetch(p, j0);
 #pragma unroll
       for (int j = 0; j < kN; ++j)
-        if (on[j]) add_piece(acc, x[j], 1.f, fp16);
+        if (on[p][j]) add_piece(acc, x[p][j], 1.f, fp16);
     }
     if constexpr (kRouter) {
       float w[kN], dw[kN];
@@ -72,7 +85,7 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
 #pragma unroll
       for (int j = 0; j < kN; ++j) {
         w[j] = j < K ? __ldg(a.w + s0 + j) : 0.f;
-        dw[j] = on[j] ? a.dw[s0 + j] : 0.f;
+        dw[j] = on[p][j] ? a.dw[s0 + j] : 0.f;
         dot = fmaf(w[j], dw[j], dot);
       }
 #pragma unroll
@@ -183,15 +196,19 @@ int ccf_reduce(const CcfReduceArgs* a, void* stream) {
   if (a->d < 8 || a->d % 8 != 0 || a->top_k < 0) return -2;
   if (a->wg != nullptr && (a->top_k > kMaxK || a->top_k < 1)) return -2;
   if (a->tokens == 0 && a->done == nullptr) return 0;
-  const int vecs = a->d >> 3;
-  const int per_block = kReduceThreads * kReducePieces / vecs > 1 ? kReduceThreads * kReducePieces / vecs : 1;
-  int blocks = (a->tokens + per_block - 1) / per_block;
+  const int span = kReduceThreads * reduce_pieces(a->top_k);
+  long long blocks = (static_cast<long long>(a->tokens) * (a->d >> 3) + span - 1) / span;
+  if (blocks > 0x7fffffffLL) return -2;
   if (blocks < 1) blocks = 1;    // a call without tokens still consumes its completion count
-  auto kern = a->wg != nullptr ? (a->top_k == 1 ? combine_reduce_kernel<1, true> : a->top_k == 2 ? combine_reduce_kernel<2, true>
-                                                                                         : combine_reduce_kernel<0, true>)
-                               : (a->top_k == 1 ? combine_reduce_kernel<1, false> : a->top_k == 2 ? combine_reduce_kernel<2, false>
-                                                                                          : combine_reduce_kernel<0, false>);
-  kern<<<blocks, kReduceThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
+  using Kernel = void (*)(CcfReduceArgs);
+  static const Kernel plain[kMaxK + 1] = {combine_reduce_kernel<0, false>, combine_reduce_kernel<1, false>, combine_reduce_kernel<2, false>,
+                                          combine_reduce_kernel<3, false>, combine_reduce_kernel<4, false>, combine_reduce_kernel<5, false>,
+                                          combine_reduce_kernel<6, false>, combine_reduce_kernel<7, false>, combine_reduce_kernel<8, false>};
+  static const Kernel router[kMaxK + 1] = {nullptr, combine_reduce_kernel<1, true>, combine_reduce_kernel<2, true>,
+                                           combine_reduce_kernel<3, true>, combine_reduce_kernel<4, true>, combine_reduce_kernel<5, true>,
+                                           combine_reduce_kernel<6, true>, combine_reduce_kernel<7, true>, combine_reduce_kernel<8, true>};
+  const Kernel kern = a->wg != nullptr ? router[a->top_k] : plain[a->top_k > kMaxK ? 0 : a->top_k];
+  kern<<<static_cast<unsigned>(blocks), kReduceThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }

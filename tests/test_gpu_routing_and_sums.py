@@ -548,3 +548,21 @@ def test_few_token_layer_gradients_match_the_oracle(t, e, k, act, router):
 def test_layer_around_the_slots_of_the_one_kernel_routing(t, k):
     """65536 slots run as one node, 65538 with the separate routing kernels and two nodes; same tolerance as above."""
     assert _layer_against_oracle(t, 128, 256, 8, k, "gelu", "bias", 6 * 2.0 ** -8) == (t * k <= 65536)
+
+
+@pytest.mark.parametrize("k", range(0, 10))
+@pytest.mark.parametrize("tokens,d", [(1, 8), (300, 72), (513, 2056), (3, 8192)])
+def test_combine_reduce_at_every_slot_count(k, tokens, d):
+    """Each number of slots per token has its own kernel; blocks end inside tokens, tokens inside blocks. Tolerance as in
+    test_combine_reduce."""
+    from ccfuser_b200 import native as N
+    torch.manual_seed(k + tokens)
+    comb = torch.randn(tokens * k + 1, d, device="cuda").bfloat16()[:tokens * k]
+    row = torch.randint(-1, 5, (tokens * k + 1,), dtype=torch.int32, device="cuda")[:tokens * k]
+    comb[row < 0] = float("nan")
+    guard = torch.full((tokens + 1, d), 7.0, dtype=torch.bfloat16, device="cuda")
+    N.check(N.load().ccf_combine_reduce(comb.data_ptr(), row.data_ptr(), guard.data_ptr(), tokens, k, d, 0, N.stream_ptr()),
+            "ccf_combine_reduce")
+    ref = torch.where((row >= 0).unsqueeze(1), comb.double(), torch.zeros((), dtype=torch.float64, device="cuda")).view(tokens, k, d).sum(1)
+    assert ((guard[:tokens].double() - ref).abs() <= ref.abs() * 2.0 ** -8 * 1.01 + 1e-6).all()
+    assert (guard[tokens] == 7.0).all()
