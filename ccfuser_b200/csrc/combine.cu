@@ -121,11 +121,11 @@ __global__ void __launch_bounds__(256) router_dw_kernel(const int* __restrict__ 
   __shared__ float part[128];
   __shared__ float partg;
   const int e = blockIdx.y, nr = count_raw[e];
+  const int* list = raw_order + CCF_MAX_GROUPS + __ldg(raw_order + e);   // both reads on their way before either is needed
   const int split = blockIdx.z, splits = splits_with_work(nr, gridDim.z);
   if (split >= splits) return;
   const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
   const int col = blockIdx.x * 128 + cx * 8;
-  const int* list = raw_order + CCF_MAX_GROUPS + raw_order[e];
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   float sum_g = 0.f;
   const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + col;
@@ -213,11 +213,11 @@ int ccf_reduce(const CcfReduceArgs* a, void* stream) {
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }
 
-int ccf_router_dw(const int* raw_order, const int* count_raw, const float* g, const void* x, void* dwg, void* db, int d, int e,
-                  int top_k, int fp16, void* stream) {
+int ccf_router_dw(const int* raw_order, const int* count_raw, const float* g, const void* x, void* dwg, void* db, int slots, int d,
+                  int e, int top_k, int fp16, void* stream) {
   using namespace ccf;
   if (d < 8 || d % 8 != 0 || e < 1 || e > CCF_MAX_GROUPS || top_k < 1 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;
-  const int splits = group_splits((d + 127) / 128 * e);
+  const int splits = group_splits((d + 127) / 128 * e, slots / e);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((d + 127) / 128, e, splits);
   cfg.blockDim = dim3(256);

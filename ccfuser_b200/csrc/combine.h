@@ -9,17 +9,19 @@ namespace ccf {
 // Cluster size of a launch with `blocks` blocks per split: as many as keep the launch resident at once (five blocks of these kernels
 // fit on an SM; clusters of four and eight no longer pack from 704 blocks on). Column sums, us with 1024 rows per group at
 // 1 / 2 / 4 / 8 blocks per group: 32 blocks 13.4 / 8.7 / 6.5 / 5.6; 128 blocks 14.3 / 10.4 / 9.0 / 11.7; with 1 and 2 368 blocks
-// 18.9 / 17.5, 384 blocks 19.2 / 24.1; with 2 and 4 160 blocks 11.1 / 10.1, 176 blocks 11.4 / 14.2.
-inline int group_splits(int blocks) {
+// 18.9 / 17.5, 384 blocks 19.2 / 24.1; with 2 and 4 160 blocks 11.1 / 10.1, 176 blocks 11.4 / 14.2. `rows`: expected rows per group,
+// 0 = not known; blocks that will hardly find work are not launched (0.5 to 0.8 us for a launch of 96 to 128 blocks).
+constexpr int kRowsPerSplit = 128;
+inline int group_splits(int blocks, int rows) {
   int splits = 1;
-  while (splits < 8 && 2 * splits * blocks <= (splits == 1 ? 5 * 148 : 640)) splits *= 2;
+  while (splits < 8 && 2 * splits * blocks <= (splits == 1 ? 5 * 148 : 640) && (rows <= 0 || rows >= 2 * splits * kRowsPerSplit)) splits *= 2;
   return splits;
 }
 // Of those, the ones that have work: every block keeps at least two passes of 64 rows. The count is read on the device, group by
 // group; the other blocks leave at once (a cluster barrier waits for blocks that have not left). 128 blocks, 188 rows: 4.6 us
 // with one block per group, 4.9 with two, 4.8 with four; 256 rows: 5.3 / 5.1 / 5.1; 512 rows: 8.4 / 6.9 / 6.4.
 __device__ __forceinline__ int splits_with_work(int rows, int splits) {
-  while (splits > 1 && rows < 128 * splits) splits >>= 1;
+  while (splits > 1 && rows < kRowsPerSplit * splits) splits >>= 1;
   return splits;
 }
 
@@ -54,4 +56,4 @@ extern "C" int ccf_reduce(const CcfReduceArgs* a, void* stream);
 // dWg[e, :] = sum over the slots routed to e (dropped ones too) of g * x[token, :], db[e] = sum of those g. `raw_order` is
 // the list that the routing kernel wrote ([CCF_MAX_GROUPS] starts, then slots by expert), count_raw [e] its lengths.
 extern "C" int ccf_router_dw(const int* raw_order, const int* count_raw, const float* g, const void* x, void* dwg, void* db,
-                             int d, int e, int top_k, int fp16, void* stream);
+                             int slots, int d, int e, int top_k, int fp16, void* stream);

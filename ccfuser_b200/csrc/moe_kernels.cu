@@ -241,14 +241,13 @@ __global__ void __launch_bounds__(256) colsum_grouped_kernel(const void* x, long
   __shared__ float red[16][128];
   __shared__ float part[128];
   const int g = blockIdx.y;
-  const int nr = group_rows[g];
+  const int nr = __ldg(group_rows + g), r0 = __ldg(group_base + g);   // both reads on their way before either is needed
   const int split = blockIdx.z, splits = splits_with_work(nr, gridDim.z);   // the cluster spans the z dimension of the grid
   if (split >= splits) return;
   const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
   const int col = blockIdx.x * 128 + cx * 8;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col < n) {
-    const int r0 = group_base[g];
     const uint16_t* base = reinterpret_cast<const uint16_t*>(x) + static_cast<size_t>(r0) * ld + col;
     for (int r = split * 64 + ry; r < nr; r += 64 * splits) {
       uint4 v[4];
@@ -485,12 +484,13 @@ int ccf_combine_reduce(const void* comb, const int* slot_row, void* y, int T, in
   return ccf_reduce(&a, stream);
 }
 
-int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
-                       void* out, int fp16, void* stream) {
+// `rows_hint`: expected rows per group, or 0 when the caller does not know
+int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                            void* out, int fp16, int rows_hint, void* stream) {
   if (n % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;   // 16-byte loads
   const int blocks = (n + 127) / 128 * groups;
   if (groups < 1 || blocks < 1) return -2;
-  const int splits = ccf::group_splits(blocks);
+  const int splits = ccf::group_splits(blocks, rows_hint);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((n + 127) / 128, groups, splits);
   cfg.blockDim = dim3(256);
@@ -500,6 +500,11 @@ int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int
   cfg.numAttrs = splits > 1 ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, ccf::colsum_grouped_kernel, x, ld, n, group_base, group_rows, out, fp16);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
+}
+
+int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                       void* out, int fp16, void* stream) {
+  return ccf_colsum_grouped_hint(x, ld, n, groups, group_base, group_rows, out, fp16, 0, stream);
 }
 
 int ccf_sgd_step(void* p, const void* g, long long n, float lr, float wd, int fp16, void* stream) {

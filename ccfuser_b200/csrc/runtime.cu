@@ -19,8 +19,8 @@ int ccf_plan(const CcfPlanArgs* a, void* stream);
 int ccf_plan_dev_epoch(const CcfPlanArgs* a, int* epoch_counter, void* stream);
 int ccf_combine_wait(const int* done, int* cum, const int* sent_rows, int n_tiles, int world,
                      unsigned long long limit_ns, int* status, void* stream);
-int ccf_colsum_grouped(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows, void* out,
-                       int fp16, void* stream);
+int ccf_colsum_grouped_hint(const void* x, long long ld, int n, int groups, const int* group_base, const int* group_rows,
+                            void* out, int fp16, int rows_hint, void* stream);
 }
 
 namespace {
@@ -305,6 +305,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   // decides: there the one-CTA kernel is faster than CTA pairs.
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
   const int wgrad_two_cta = rows_per_expert > 512 ? L->two_cta : 0;
+  const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
   const int row_two_cta = rows_per_expert > L->small_rows ? L->two_cta : 0;
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
   // GEMM. w2 may be at any group size (dgrad-2 above it is its last reader). w1 / wg only on a single rank: dgrad-1 reads
@@ -354,7 +355,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     if ((rc = issue(g, dry, stream))) return rc;
   }
   if (G->db2 != nullptr && dry == nullptr) {
-    if ((rc = ccf_colsum_grouped(L->grecv, d, d, e_loc, L->group_base, L->group_rows, G->db2, L->fp16, stream))) return rc;
+    if ((rc = ccf_colsum_grouped_hint(L->grecv, d, d, e_loc, L->group_base, L->group_rows, G->db2, L->fp16, rows_hint, stream))) return rc;
   }
   // 4. wgrad-1: dW1[e] = dh^T x_e  [f, d]  (SwiGLU: gate projection from dh, up projection from dh2)
   auto wgrad1 = [&](const void* a0, void* out) {
@@ -402,23 +403,23 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     if ((rc = wgrad1(G->dh2, sgd ? const_cast<void*>(L->w1) : G->dw1))) return rc;
     if (dry == nullptr) {
       if (G->db1 != nullptr &&
-          (rc = ccf_colsum_grouped(G->dh2, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, stream)))
+          (rc = ccf_colsum_grouped_hint(G->dh2, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, rows_hint, stream)))
         return rc;
       if (G->dbg != nullptr &&
-          (rc = ccf_colsum_grouped(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->dbg, L->fp16, stream)))
+          (rc = ccf_colsum_grouped_hint(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->dbg, L->fp16, rows_hint, stream)))
         return rc;
     }
   } else {
     if ((rc = wgrad1(G->dh, sgd ? const_cast<void*>(L->w1) : G->dw1))) return rc;
     if (dry == nullptr && G->db1 != nullptr &&
-        (rc = ccf_colsum_grouped(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, stream)))
+        (rc = ccf_colsum_grouped_hint(G->dh, f, f, e_loc, L->group_base, L->group_rows, G->db1, L->fp16, rows_hint, stream)))
       return rc;
   }
   if (!sgd && (rc = dgrad1())) return rc;
   if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, 256, G, idx, gate_w, dry, stream))) return rc;
   if (G->router_dw != nullptr && dry == nullptr)
-    rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, d, L->e_total, L->top_k, L->fp16,
-                       stream);
+    rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d,
+                       L->e_total, L->top_k, L->fp16, stream);
   return rc;
 }
 

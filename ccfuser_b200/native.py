@@ -194,7 +194,7 @@ def _declare(lib):
         "ccf_route": ([p, i, i, i, p, p, p, p, p, p, p], i),
         "ccf_route_ordered": ([p, i, i, i, p, p, p, p, p, p, p, p, p, i, p], i),
         "ccf_route_plan": ([p, i, i, i, p, p, p, p, p, p, i, p, C.POINTER(PlanArgs), p, p], i),
-        "ccf_router_dw": ([p, p, p, p, p, p, i, i, i, i, p], i),
+        "ccf_router_dw": ([p, p, p, p, p, p, i, i, i, i, i, p], i),
         "ccf_layer_forward": ([C.POINTER(Layer), p, p, p, p, i, i, i, i, p, p, i, p], i),
         "ccf_layer_backward": ([C.POINTER(Layer), p, p, p, C.POINTER(LayerGrads), i, i, p, p, i, p], i),
         "ccf_flag_barrier": ([C.POINTER(BarrierArgs), p], i),

@@ -334,9 +334,11 @@ def test_column_sums_at_the_edges_of_the_sharing_rule(copies, n):
     assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * 2.0 ** -16 + 1e-7).all()
 
 
-@pytest.mark.parametrize("copies,d,k,fp16", [(1, 256, 1, False), (1, 1000, 3, True), (4, 1536, 2, False), (8, 1024, 2, True)])
-def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, fp16):
-    """dWg and db from slot lists of every length against fp64: fp32 products and sums, one rounding."""
+@pytest.mark.parametrize("copies,d,k,fp16,hint", [(1, 256, 1, False, 4096), (1, 256, 2, False, 300), (1, 1000, 3, True, 4096),
+                                                  (4, 1536, 2, False, 4096), (8, 1024, 2, True, 4096), (1, 256, 1, False, 1)])
+def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, fp16, hint):
+    """dWg and db from slot lists of every length (``hint``: the length the launch expects) against fp64: fp32 products and
+    sums, one rounding."""
     from ccfuser_b200 import native as N
     dt = torch.float16 if fp16 else torch.bfloat16
     counts = _EDGES * copies
@@ -351,8 +353,8 @@ def test_router_weight_gradient_at_the_edges_of_the_sharing_rule(copies, d, k, f
     raw[N.MAX_GROUPS:N.MAX_GROUPS + order.numel()] = order.int()
     cnt = torch.tensor(counts, dtype=torch.int32, device="cuda")
     dw, db = torch.full((e, d), 7.0, dtype=dt, device="cuda"), torch.full((e,), 7.0, dtype=dt, device="cuda")
-    N.check(N.load().ccf_router_dw(raw.data_ptr(), cnt.data_ptr(), g.data_ptr(), x.data_ptr(), dw.data_ptr(), db.data_ptr(), d, e, k,
-                                   int(fp16), N.stream_ptr()), "ccf_router_dw")
+    N.check(N.load().ccf_router_dw(raw.data_ptr(), cnt.data_ptr(), g.data_ptr(), x.data_ptr(), dw.data_ptr(), db.data_ptr(), hint * e, d,
+                                   e, k, int(fp16), N.stream_ptr()), "ccf_router_dw")
     ulp = 2.0 ** (-11 if fp16 else -8)
     for i, (s, c) in enumerate(zip(start, counts)):
         ids = order[s:s + c]
