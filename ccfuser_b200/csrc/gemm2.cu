@@ -20,8 +20,9 @@ namespace ccf {
 // A stage holds two k-blocks. Every hand-back of a stage (tcgen05.commit) costs the tensor pipe about 64 clocks per barrier it
 // arrives on, whatever the memory system does: with one k-block per stage and one commit per CTA of the pair a k-block took
 // 640 clocks instead of 512, also when every load hit the same lines. One multicast commit per two k-blocks is a quarter of that.
-// 32768 x 4096 x 14336, TFLOP/s (GELU forward / second projection): 1310 / 1359 before, 1361 / 1429 with the multicast commit
-// alone, 1416 / 1512 with two k-blocks per stage alone. Under the power cap the gain is smaller.
+// 32768 x 4096 x 14336, TFLOP/s (GELU forward / second projection): 1270 / 1340 before, 1412 / 1512 with both (on another box
+// 1310 / 1359 before, 1361 / 1429 with the multicast commit alone, 1416 / 1512 with two k-blocks per stage alone). Under the
+// power cap the gain is smaller.
 constexpr int k2Stages = 3;
 constexpr int k2Sub = 2;                       // k-blocks per stage
 constexpr int k2ABytes = BM * BK * 2;          // this CTA's 128 rows of A

@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(kLnThreads) layernorm_fwd_kernel(const void* _
 // rate takes. The row sums meet in shared memory with one barrier per stage, which also frees the stage, and each block
 // leaves its partial dgamma / dbeta in `part` ([blocks, 2, d] fp32), which layernorm_bwd_finish_kernel adds in block order:
 // no atomics, no zeroed buffers, no conversion passes. A copy that does not arrive within the limit ends the block: time-out
-// in the status word, no further requests, NaN in the rows it leaves undone and in its partial sums. 8192 x 2048 bf16: 39 + 7 us, where a dx kernel, a parameter kernel,
-// two fills and two conversions took 37 + 16 + 6 us and four launches more.
+// in the status word, no further requests, NaN in the rows it leaves undone and in its partial sums. 8192 x 2048 bf16:
+// 39 + 7 us, where a dx kernel, a parameter kernel, two fills and two conversions took 37 + 16 + 6 us and four launches more.
 constexpr int kLnRows = 2;       // rows per group and stage
 constexpr int kLnStages = 6;
 template <int kW>

@@ -1,8 +1,10 @@
-// Native runtime of one fused MoE layer (see runtime.h): ccf_layer_forward / ccf_layer_backward issue, in order and on
-// one stream, exactly the launches that ops/fused.py issues call by call from Python: routing, count exchange + plan,
-// dispatch fused with GEMM-1, GEMM-2 fused with combine, wait + reduce; and for backward the dy dispatch fused with
-// dgrad-2, both weight-gradient GEMMs, the bias-gradient column sums and dgrad-1 fused with combine.
-// tests/test_native_runtime.py compares the GEMM launch blocks built here with the ones the Python path builds.
+// Native runtime of one fused MoE layer (see runtime.h): ccf_layer_forward / ccf_layer_backward issue the launches of a pass in
+// order and on one stream: routing, count exchange + plan, dispatch fused with GEMM-1, GEMM-2 fused with combine, wait +
+// reduce; and for backward the dy dispatch fused with dgrad-2, both weight-gradient GEMMs, the bias-gradient column sums,
+// dgrad-1 fused with combine, wait + reduce and, where the call included the router, its gradients. The GEMM launches are
+// those that ops/fused.py issues call by call from Python (tests/test_native_runtime.py compares the launch blocks); around
+// them that path keeps the kernels apart that are one here: routing and plan, completion wait, clearing of the arrival
+// counters and reduce.
 #include <cuda_runtime.h>
 #include <string.h>
 

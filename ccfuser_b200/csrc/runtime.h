@@ -75,7 +75,8 @@ struct CcfLayer {
 
 // Per-call tensors of the backward pass (all allocated by the caller; null where the layer has no such parameter).
 struct CcfLayerGrads {
-  float* dgate;     // [tokens * top_k], zero on entry (dropped slots keep 0)
+  float* dgate;     // [tokens * top_k]; slots that are not dispatched are not written: zero on entry where the caller returns it,
+                    // any content where router_w is set (the reduction takes those slots as zero)
   void* dh;         // [max_rows, f] scratch: gradient of the (gate) pre-activation
   void* dh2;        // [max_rows, f] scratch, SwiGLU: gradient of the up pre-activation
   void* dw1;
