@@ -25,6 +25,7 @@ class Workspace:
     def __init__(self, device):
         self.sched = torch.zeros(8, dtype=torch.int32, device=device)
         self.status = torch.zeros(2, dtype=torch.int32, device=device)  # [first hard error, overflow count]
+        self.status_addr = self.status.data_ptr()
         self._last_stream, self._last_raw = None, None
         self._on_gpu = self.sched.device.type == "cuda"
         self._device_index = self.sched.device.index if self._on_gpu else -1
@@ -40,6 +41,12 @@ class Workspace:
         if ws is None:
             ws = cls._by_device[key] = Workspace(device)
         return ws
+
+    @classmethod
+    def status_of(cls, tensor) -> int:
+        """Address of the status word of a CUDA tensor's device."""
+        ws = cls._by_device.get(tensor.get_device())
+        return (ws if ws is not None else cls.get(tensor.device)).status_addr
 
     def enter(self):
         """Called by every launcher with the stream it is about to launch on. The kernels of one device share this

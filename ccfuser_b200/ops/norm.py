@@ -49,8 +49,8 @@ class _LayerNormFn(torch.autograd.Function):
         db = torch.empty_like(w) if ctx.has_bias else None
         N.check(lib.ccf_layernorm_bwd(x2.data_ptr(), dy2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                       dx.data_ptr(), part.data_ptr(), dg.data_ptr(), N.ptr(db), rows, d,
-                                      int(x2.dtype == torch.float16), G.Workspace.get(x2.device).status.data_ptr(),
-                                      G.DEFAULT_WAIT_NS, N.stream_ptr()), "ccf_layernorm_bwd")
+                                      int(x2.dtype == torch.float16), G.Workspace.status_of(x2), G.DEFAULT_WAIT_NS,
+                                      N.stream_ptr()), "ccf_layernorm_bwd")
         N.count(2)
         return dx.view(ctx.shape), dg, db, None
 
