@@ -157,9 +157,8 @@ __global__ void __launch_bounds__(256, 2) layernorm_bwd_kernel(const void* __res
   for (; base < rows; base += step, buf ^= 1) {   // the same trips for every thread of the block
     uint4 xv[kLnRows], dv[kLnRows];
     float mu[kLnRows], rs[kLnRows];
-    // the limit is looked up only by threads that have to wait, behind the copy they wait for (looked up at the start: 0.8 us)
-    const bool here = mbar_try_wait(smem_u32(&full[slot]), parity) ||
-                      mbar_wait(smem_u32(&full[slot]), parity, &abort_word, fail_fast_limit(status, wait_limit_ns));
+    // the full limit whatever is on record: these copies depend on no peer, so a lost one is no reason to give them up sooner
+    const bool here = mbar_wait(smem_u32(&full[slot]), parity, &abort_word, wait_limit_ns);
 #pragma unroll
     for (int u = 0; u < kLnRows; ++u) {
       const int r = u * kG + grp;
