@@ -4,8 +4,8 @@
 // (histogram, plan, positions) every call paid three launches and three chains of dependent global reads in front of the
 // first GEMM: 15.4 us at 32 slots, 20-24 us at 16384, now 4.6 and 8-10 us. One cluster of up to eight CTAs (co-scheduled by
 // definition, so its barrier cannot wait for a CTA that has no SM) holds all slots of a call in registers: counts per warp in
-// shared memory, counts per CTA exchanged over distributed shared memory, positions written once. Calls with more than CCF_ROUTE_CLUSTER_SLOTS slots use the three kernels
-// of moe_kernels.cu, whose grid is not limited.
+// shared memory, counts per CTA exchanged over distributed shared memory, positions written once. Calls with
+// more than CCF_ROUTE_CLUSTER_SLOTS slots use the three kernels of moe_kernels.cu, whose grid is not limited.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -292,8 +292,9 @@ class FusedMoE:
     def one_node(self, x: torch.Tensor):
         """The router's linear layer if router and experts of this call run as one autograd node (route_and_run), else None.
         They do where the one-kernel router applies, no auxiliary loss asks for the logits, and the call's slots fit the
-        one-kernel routing, which lists them by expert for the router's weight gradient. Then the input gradient through the gate weights is added in the slot
-        reduction that ends the backward pass, instead of in a kernel of its own and an addition of two [T, d] matrices."""
+        one-kernel routing, which lists them by expert for the router's weight gradient. Then the input
+        gradient through the gate weights is added in the slot reduction that ends the backward pass, instead of in a
+        kernel of its own and an addition of two [T, d] matrices."""
         cfg, gate, t = self.cfg, self.layer.gate, x.shape[0]
         lin = getattr(gate, "gate", None)
         if not (self.native_runtime and self.fused_router and isinstance(lin, torch.nn.Linear)
