@@ -261,7 +261,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
           ok = false;
           break;
         }
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t fullb = smem_u32(&ctrl->full[stage]);
           const uint32_t sa = smem_base + stage * stage_bytes;
           const uint32_t sb = sa + a_bytes;
@@ -303,6 +303,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
     const uint32_t idesc = make_idesc(BM, bn_run, args.fp16, kAMajor, kBMajor);
+    const uint64_t desc_a = operand_desc(smem_base, kAMajor), desc_b = operand_desc(smem_base + a_bytes, kBMajor);
     int stage = 0, phase = 0, ss = 0, sphase = 0, as = 0, aphase = 0, seq = -1;
     bool ok = true;
     while (ok) {
@@ -332,18 +333,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           if (kb == 0) trace_ev(args, seq, 4);
-          const uint32_t sa = smem_base + stage * stage_bytes;
-          const uint32_t sb = sa + a_bytes;
+          const uint32_t at = static_cast<uint32_t>(stage) * stage_bytes;
 #pragma unroll
-          for (int k = 0; k < BK / UK; ++k) {
-            const uint64_t da = (kAMajor == MAJ_K) ? make_smem_desc(sa + k * 32, 16, 1024)
-                                                   : make_smem_desc(sa + k * 2048, 8192, 1024);
-            const uint64_t db = (kBMajor == MAJ_K) ? make_smem_desc(sb + k * 32, 16, 1024)
-                                                   : make_smem_desc(sb + k * 2048, 8192, 1024);
-            umma_f16(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UK; ++k)
+            umma_f16(d_tmem, desc_at(desc_a, at + k * desc_step(kAMajor)), desc_at(desc_b, at + k * desc_step(kBMajor)), idesc,
+                     (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit(smem_u32(&ctrl->empty[stage]));
           if (kb == ti.kblocks - 1) {
             umma_commit(smem_u32(&ctrl->acc_full[as]));

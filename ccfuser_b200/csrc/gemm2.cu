@@ -17,12 +17,13 @@
 
 namespace ccf {
 
-// A stage holds two k-blocks. Every hand-back of a stage (tcgen05.commit) costs the tensor pipe about 64 clocks per barrier it
-// arrives on, whatever the memory system does: with one k-block per stage and one commit per CTA of the pair a k-block took
-// 640 clocks instead of 512, also when every load hit the same lines. One multicast commit per two k-blocks is a quarter of that.
-// 32768 x 4096 x 14336, TFLOP/s (GELU forward / second projection): 1270 / 1340 before, 1412 / 1512 with both (on another box
-// 1310 / 1359 before, 1361 / 1429 with the multicast commit alone, 1416 / 1512 with two k-blocks per stage alone). Under the
-// power cap the gain is smaller.
+// A stage holds two k-blocks and is handed back by one multicast commit: each wait, commit and MMA is a turn of the issuing thread,
+// and per k-block those turns have to stay below the 512 clocks that its four MMAs run. With one k-block per stage, two commits and
+// MMAs issued behind `lane == 0` (138 clocks each) a k-block took 640 clocks, whatever the memory system did. 32768 x 4096 x 14336,
+// TFLOP/s (GELU forward / second projection): 1270 / 1340 then, 1412 / 1512 with two k-blocks per stage and one commit. With the
+// MMAs issued behind elect_one the main loop runs at 97 to 100 % of the tensor pipe (GELU forward 35.3 k -> 33.4 k clocks per tile
+// of 32.8 k, with GELU' in the epilogue 37.9 k -> 33.9 k), and what is left between it and the nominal rate is the clock: these
+// launches run into the power limit. 16384 tokens, 4096 x 14336 SwiGLU, forward and backward: 31.5 -> 30.5 ms.
 constexpr int k2Stages = 3;
 constexpr int k2Sub = 2;                       // k-blocks per stage
 constexpr int k2ABytes = BM * BK * 2;          // this CTA's 128 rows of A
@@ -355,7 +356,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
           ok = false;
           break;
         }
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t full_leader = map_to_cta(smem_u32(&ctrl->full[stage]), 0);
           const int n_sub = min(k2Sub, ti.kblocks - kb0);
           if (cta == 0) mbar_arrive_expect_tx(smem_u32(&ctrl->full[stage]), static_cast<uint32_t>(n_sub) * 2 * k2SubBytes);
@@ -400,6 +401,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     // ======================= MMA issuer (leader CTA only) =======================
     if (cta == 0) {
       const uint32_t idesc = make_idesc(PM, BN, args.fp16, kAMajor, kBMajor);
+      const uint64_t desc_a = operand_desc(smem_base, kAMajor), desc_b = operand_desc(smem_base + k2ABytes, kBMajor);
       int stage = 0, phase = 0, as = 0, aphase = 0, seq = 0;
       bool ok = true;
       for (int t = pair; t < total_tiles && ok; t += n_pairs, ++seq) {
@@ -419,20 +421,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             if (kb0 == 0) trace_ev(args, seq, 4);
             const int n_sub = min(k2Sub, ti.kblocks - kb0);
             for (int u = 0; u < n_sub; ++u) {
-              const uint32_t sa = smem_base + stage * k2StageBytes + u * k2SubBytes;
-              const uint32_t sb = sa + k2ABytes;
+              const uint32_t at = static_cast<uint32_t>(stage * k2StageBytes + u * k2SubBytes);
 #pragma unroll
-              for (int k = 0; k < BK / UK; ++k) {
-                const uint64_t da = (kAMajor == MAJ_K) ? make_smem_desc(sa + k * 32, 16, 1024)
-                                                       : make_smem_desc(sa + k * 2048, 8192, 1024);
-                const uint64_t db = (kBMajor == MAJ_K) ? make_smem_desc(sb + k * 32, 16, 1024)
-                                                       : make_smem_desc(sb + k * 2048, 8192, 1024);
-                umma_f16_pair(d_tmem, da, db, idesc, (kb0 > 0 || u > 0 || k > 0) ? 1u : 0u);
-              }
+              for (int k = 0; k < BK / UK; ++k)
+                umma_f16_pair(d_tmem, desc_at(desc_a, at + k * desc_step(kAMajor)), desc_at(desc_b, at + k * desc_step(kBMajor)),
+                              idesc, (kb0 > 0 || u > 0 || k > 0) ? 1u : 0u);
             }
             umma_commit_pair(smem_u32(&ctrl->empty[stage]));   // hand the stage back to both producers
             if (kb0 + k2Sub >= ti.kblocks) {

@@ -25,6 +25,14 @@ constexpr int kEpiStageBytes = 2048;  // per epilogue warp: 32 rows x 64 bytes, 
 // swizzle (defined in gemm.cu). Returns 0 or a negative error code.
 int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows, int fp16);
 
+// Descriptor of an operand in a pipeline stage as the MMA reads it: its base, the step of one 16-deep MMA, and any other place in
+// shared memory (only the 14 address bits differ, in units of 16 bytes; shared memory ends below 2^18).
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr, int major) {
+  return major == MAJ_K ? make_smem_desc(smem_addr, 16, 1024) : make_smem_desc(smem_addr, 8192, 1024);
+}
+__device__ __forceinline__ constexpr uint32_t desc_step(int major) { return major == MAJ_K ? 32 : 2048; }
+__device__ __forceinline__ uint64_t desc_at(uint64_t base, uint32_t bytes) { return base + (bytes >> 4); }
+
 struct Tile {
   int g;           // group (expert)
   int row0;        // row-grouped: first A/C row; k-grouped: first output row inside the group (m0)

@@ -181,7 +181,7 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         report_status(a.status, CCF_ERR_MBAR_TIMEOUT, 0x40);
         break;
       }
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t fullb = smem_u32(&ctrl->full[stage]);
         const uint32_t sa = smem_base + stage * stage_bytes;
         mbar_arrive_expect_tx(fullb, static_cast<uint32_t>(stage_bytes));
@@ -201,7 +201,7 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         break;
       }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t sa = smem_base + stage * stage_bytes;
         const uint32_t sb = sa + kRtABytes;
 #pragma unroll

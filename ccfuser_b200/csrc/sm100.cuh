@@ -26,6 +26,22 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
+// True in one lane of a converged warp, the same one every time. TMA and tcgen05 instructions take their operands from uniform
+// registers; behind this predicate the compiler knows that one lane runs and issues them back to back. Behind `lane == 0` it
+// does not, and a tcgen05.mma took 138 clocks to issue whatever its size, where a 128 x 256 x 16 one takes 128 to run (an isolated
+// loop of either, one CTA per SM; with this predicate the loop runs at 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // host: launch attribute of a cluster
 inline cudaLaunchAttribute cluster_attribute(unsigned x, unsigned y, unsigned z) {
   cudaLaunchAttribute a;
