@@ -51,6 +51,7 @@ CcfGemmLaunch base_launch(const CcfLayer* L) {
   g.args.kseg = 1;
   g.args.fp16 = L->fp16;
   g.args.world = 1;
+  g.args.count_rows = 1;
   g.args.total_index = -1;
   g.args.comm_warps = L->comm_warps;
   g.device = L->device;
@@ -120,6 +121,7 @@ void set_combine(CcfGemmLaunch& g, const CcfLayer* L, void* const* peer_comb, co
   }
   g.args.world = L->world;
   g.args.send_finish = 1;
+  g.args.count_rows = L->world > 1;
   g.args.max_slots = L->max_slots;
 }
 
@@ -157,7 +159,7 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
     r.done = L->done;
     r.cum = L->done_cum;
     r.sent_rows = L->sent_rows;
-    r.n_tiles = combine_units(L->d_model, bn);
+    r.n_tiles = 0;   // the rows of a single rank are not counted
     r.status = L->status;
     r.wait_limit_ns = L->wait_limit_ns;
     r.zero_words = L->tile_flags;

@@ -51,7 +51,7 @@ class GemmArgs(C.Structure):
         ("wait_limit_ns", C.c_ulonglong), ("ld_out", C.c_longlong),
         ("n", C.c_int), ("k", C.c_int), ("num_groups", C.c_int), ("m_per_group", C.c_int), ("kseg", C.c_int),
         ("b_group_rows", C.c_int), ("act", C.c_int), ("fp16", C.c_int), ("out_fp32", C.c_int), ("world", C.c_int),
-        ("send_finish", C.c_int), ("n_comm_ctas", C.c_int), ("max_slots", C.c_int), ("trace_tiles", C.c_int),
+        ("send_finish", C.c_int), ("count_rows", C.c_int), ("n_comm_ctas", C.c_int), ("max_slots", C.c_int), ("trace_tiles", C.c_int),
         ("total_index", C.c_int), ("sgd_lr", C.c_float), ("comm_warps", C.c_int), ("sgd_wd", C.c_float), ("bn", C.c_int), ("a_rows", C.c_int),
         ("disp", DispatchArgs),
     ]

@@ -508,11 +508,13 @@ class FusedMoE:
         ctx = self.ctx
         done = [p + 4 * self.rank for p in ctx.peer("done")]
         return dict(row_src=ctx.row_src, row_gate=row_gate, peer_comb=peer_comb, peer_done=done, world=self.world,
-                    send_finish=1, max_slots=self.max_slots)
+                    send_finish=1, count_rows=int(self.world > 1), max_slots=self.max_slots)
 
     def _wait_and_reduce(self, comb: torch.Tensor, tokens: int, n_tiles: int, out: torch.Tensor):
         lib, ctx, cfg = N.load(), self.ctx, self.cfg
         st = N.stream_ptr()
+        if self.world == 1:
+            n_tiles = 0     # its rows are not counted (_combine_kw)
         N.check(lib.ccf_combine_wait(ctx.done.data_ptr(), ctx.done_cum.data_ptr(), self.sent_rows.data_ptr(), n_tiles,
                                      self.world, ctx.wait_ns, ctx.ws.status.data_ptr(), st), "ccf_combine_wait")
         N.check(lib.ccf_combine_reduce(comb.data_ptr(), self.slot_row.data_ptr(), out.data_ptr(), tokens, cfg.top_k,

@@ -145,7 +145,7 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
            a1=None, b1=None, kgroup=False, m_per_group=0, kseg=1, b_group_rows=0,
            out0=None, out1=None, out2=None, bias0=None, bias1=None, aux0=None, aux1=None, ld_out=None,
            act=N.ACT_NONE, out_fp32=False, tile_flags=None, local_begin=None, local_rows=None, row_src=None, row_gate=None,
-           peer_comb=None, peer_done=None, world=1, send_finish=0, max_slots=0,
+           peer_comb=None, peer_done=None, world=1, send_finish=0, count_rows=1, max_slots=0,
            dispatch: Optional[N.DispatchArgs] = None, n_comm_ctas=0, total_index=-1, two_cta=None, wait_ns=DEFAULT_WAIT_NS, grid=0, trace=None,
            workspace: Optional[Workspace] = None, comm_warps: Optional[int] = None, sgd=None, bn: int = 0, a_rows: int = 0):
     """Fill a CcfGemmLaunch and launch on the current stream. a0/b0 are 2-D contiguous views."""
@@ -176,6 +176,7 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     g.n, g.k, g.num_groups, g.m_per_group, g.kseg = int(n), int(k), int(num_groups), int(m_per_group), int(kseg)
     g.b_group_rows, g.act, g.fp16, g.out_fp32 = int(b_group_rows), int(act), _is_fp16(a0), int(bool(out_fp32))
     g.world, g.send_finish, g.n_comm_ctas, g.max_slots = int(world), int(send_finish), int(n_comm_ctas), int(max_slots)
+    g.count_rows = int(count_rows)
     g.total_index = int(total_index)
     g.comm_warps = int(COMM_WARPS_DEFAULT if comm_warps is None else comm_warps)
     g.bn, g.a_rows = int(bn), int(a_rows)
