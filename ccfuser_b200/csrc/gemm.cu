@@ -381,28 +381,33 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                           ti.rows_valid, q, half, lane);
       }
       const bool have_acc = ti.kblocks > 0;
-      if (have_acc) {
-        if (!mbar_wait(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
-          report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 7);
-          break;
-        }
-        tc_fence_after();
-      }
-      if (warp == 2 && lane == 0) trace_ev(args, seq, 6);
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * BN;
       const uint32_t stage = smem_base + kPipeBytes + (warp - 2) * kEpiStageBytes;
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + ti.row0;
       else row_base = ti.row0;
-      const CombineDest cd = epilogue_tile<kEpi, kFp16>(args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane);
+      const CombineDest cd = epilogue_tile<kEpi, kFp16>(
+          args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane,
+          [&] {
+            if (have_acc) {
+              if (!mbar_wait(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
+                report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 7);
+                return false;
+              }
+              tc_fence_after();
+            }
+            if (warp == 2 && lane == 0) trace_ev(args, seq, 6);
+            return true;
+          },
+          [&] {
+            if (!have_acc) return;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctrl->acc_empty[as]));
+          });
+      if (!cd.here) break;
       if (warp == 2 && lane == 0) trace_ev(args, seq, 7);
-      if (have_acc) {
-        // all TMEM reads of this accumulator stage are complete: hand it back to the MMA warp
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&ctrl->acc_empty[as]));
-        if (++as == 2) { as = 0; aphase ^= 1; }
-      }
+      if (have_acc && ++as == 2) { as = 0; aphase ^= 1; }
       if constexpr (kEpi == CCF_EPI_COMBINE) combine_signal(args, cd, lane);
       (void)cd;
     }

@@ -83,9 +83,11 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   }
   return true;
 }
-// arrive on a barrier given by its shared::cluster address (own CTA or the peer)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrive on a barrier given by its shared::cluster address (own CTA or the peer). Relaxed: what it reports is that this warp's TMEM
+// loads are in registers (tcgen05.wait::ld), no memory is handed over. With release semantics the arrival, and the warp with it,
+// waited some 4000 clocks for the tile's global stores to be performed, once per tile and warp.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load into this CTA's shared memory, completion bytes counted on a barrier of the pair (shared::cluster address)
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
@@ -153,7 +155,7 @@ __host__ __device__ __forceinline__ void tile_in_group(int t, int mt, int nt, in
 }
 
 template <bool kKGroup, int kEpi>
-__host__ __device__ __forceinline__ PairTile decode_pair_tile(int t, const CcfGemmArgs& a, const Ctrl2* c) {
+__host__ __device__ __forceinline__ PairTile decode_pair_tile(int t, const CcfGemmArgs& a, const Ctrl2* c, int& hint) {
   PairTile ti;
   constexpr int bn_out = (kEpi == CCF_EPI_SWIGLU) ? BN / 2 : BN;
   if constexpr (!kKGroup) {
@@ -163,11 +165,10 @@ __host__ __device__ __forceinline__ PairTile decode_pair_tile(int t, const CcfGe
     const bool phase_a = t < c->tiles_a;
     const int* pre = phase_a ? c->mta_prefix : c->mt_prefix;
     const int tt = phase_a ? t : t - c->tiles_a;
-    int lo = 0, hi = a.num_groups;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (nt * pre[mid] <= tt) lo = mid; else hi = mid;
-    }
+    // the group of the last tile or one soon after it: a role's tiles only go up, but for the change of phase
+    int lo = nt * pre[hint] <= tt ? hint : 0;
+    while (lo + 1 < a.num_groups && nt * pre[lo + 1] <= tt) ++lo;
+    hint = lo;
     ti.g = lo;
     const int mt_g = pre[lo + 1] - pre[lo];
     int i, j;
@@ -340,10 +341,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
 
   if (warp == 0) {
     // ======================= TMA producer (both CTAs) =======================
-    int stage = 0, phase = 0, seq = 0;
+    int stage = 0, phase = 0, seq = 0, hint = 0;
     bool all_in = false, ok = true;
     for (int t = pair; t < total_tiles && ok; t += n_pairs, ++seq) {
-      const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl);
+      const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl, hint);
       const int my_rows = kKGroup ? BM : max(0, min(BM, ti.rows_pair - static_cast<int>(cta) * BM));
       const int my_row0 = ti.row0 + static_cast<int>(cta) * BM;
       if (lane == 0) trace_ev(args, seq, 0);
@@ -420,10 +421,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     if (cta == 0) {
       const uint32_t idesc = make_idesc(PM, BN, args.fp16, kAMajor, kBMajor);
       const uint64_t desc_a = operand_desc(smem_base, kAMajor), desc_b = operand_desc(smem_base + k2ABytes, kBMajor);
-      int stage = 0, phase = 0, as = 0, aphase = 0, seq = 0;
+      int stage = 0, phase = 0, as = 0, aphase = 0, seq = 0, hint = 0;
       bool ok = true;
       for (int t = pair; t < total_tiles && ok; t += n_pairs, ++seq) {
-        const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl);
+        const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl, hint);
         if (ti.kblocks == 0) continue;
         if (!mbar_wait_cluster(smem_u32(&ctrl->acc_empty[as]), aphase ^ 1, abort_word, limit)) {
           report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x24);
@@ -471,9 +472,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     const int half = (warp - 2) >> 2;
     dispatch_role<kEpi>(args, false);
     if (warp == 2 && lane == 0 && args.trace != nullptr && !args.comm_warps) trace_ev(args, args.trace_tiles - 1, 1);
-    int as = 0, aphase = 0, seq = 0;
+    int as = 0, aphase = 0, seq = 0, hint = 0;
     for (int t = pair; t < total_tiles; t += n_pairs, ++seq) {
-      const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl);
+      const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl, hint);
       if constexpr (kEpi == CCF_EPI_STORE) {
         // SGD in the epilogue: ask L2 for the weights under this tile while its accumulator is still being filled
         if (args.sgd_lr != 0.f && !args.out_fp32)
@@ -481,14 +482,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
                           ti.n0, kKGroup ? BM : max(0, min(BM, ti.rows_pair - static_cast<int>(cta) * BM)), q, half, lane);
       }
       const bool have_acc = ti.kblocks > 0;
-      if (have_acc) {
-        if (!mbar_wait_cluster(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
-          report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x27);
-          break;
-        }
-        tc_fence_after();
-      }
-      if (warp == 2 && lane == 0) trace_ev(args, seq, 6);
       const int my_rows = kKGroup ? BM : max(0, min(BM, ti.rows_pair - static_cast<int>(cta) * BM));
       const int rows_store = my_rows > 0 ? BM : 0;   // an empty second half may belong to the next group: never written
       Tile tt;
@@ -503,14 +496,28 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + tt.row0;
       else row_base = tt.row0;
-      const CombineDest cd = epilogue_tile<kEpi, kFp16>(args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane);
+      const CombineDest cd = epilogue_tile<kEpi, kFp16>(
+          args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane,
+          [&] {
+            if (have_acc) {
+              if (!mbar_wait_cluster(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
+                report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x27);
+                return false;
+              }
+              tc_fence_after();
+            }
+            if (warp == 2 && lane == 0) trace_ev(args, seq, 6);
+            return true;
+          },
+          [&] {
+            if (!have_acc) return;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctrl->acc_empty[as]), 0));
+          });
+      if (!cd.here) break;
       if (warp == 2 && lane == 0) trace_ev(args, seq, 7);
-      if (have_acc) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctrl->acc_empty[as]), 0));
-        if (++as == 2) { as = 0; aphase ^= 1; }
-      }
+      if (have_acc && ++as == 2) { as = 0; aphase ^= 1; }
       if constexpr (kEpi == CCF_EPI_COMBINE) combine_signal(args, cd, lane);
       (void)cd;
     }
@@ -627,12 +634,12 @@ extern "C" int ccf_debug_pair_tile_order(const int* group_base, const int* group
   a.k = k;
   a.kseg = 1;
   Ctrl2* c = new Ctrl2;
-  int total;
+  int total, hint = 0;
   if (swiglu) {
     pair_tile_tables_host<CCF_EPI_SWIGLU>(a, c);
     total = c->total_tiles;
     for (int t = 0; t < total && t < cap; ++t) {
-      const PairTile ti = decode_pair_tile<false, CCF_EPI_SWIGLU>(t, a, c);
+      const PairTile ti = decode_pair_tile<false, CCF_EPI_SWIGLU>(t, a, c, hint);
       const int rec[5] = {ti.g, ti.row0, ti.n0, ti.rows_pair, t < c->tiles_a ? 0 : 1};
       memcpy(out + 5 * t, rec, sizeof(rec));
     }
@@ -640,7 +647,7 @@ extern "C" int ccf_debug_pair_tile_order(const int* group_base, const int* group
     pair_tile_tables_host<CCF_EPI_STORE>(a, c);
     total = c->total_tiles;
     for (int t = 0; t < total && t < cap; ++t) {
-      const PairTile ti = decode_pair_tile<false, CCF_EPI_STORE>(t, a, c);
+      const PairTile ti = decode_pair_tile<false, CCF_EPI_STORE>(t, a, c, hint);
       const int rec[5] = {ti.g, ti.row0, ti.n0, ti.rows_pair, t < c->tiles_a ? 0 : 1};
       memcpy(out + 5 * t, rec, sizeof(rec));
     }

@@ -232,11 +232,15 @@ __device__ __forceinline__ void trace_ev(const CcfGemmArgs& a, int seq, int ev) 
 //   row_base     first output row of this CTA's 128 accumulator rows (group offset included for k-grouped mode)
 //   rows_valid   rows of this CTA's part that hold data
 //   rows_store   rows of this CTA's part that may be written at all (rows in [rows_valid, rows_store) get zeros)
-// Returns where the row went (COMBINE) so that the caller can report completion after releasing the accumulator.
+//   acquire      waits for the accumulator (false: given up); what the first chunk needs from global memory is requested before
+//   release      hands the accumulator back to the MMA warp; called once the warp's last part of it is in registers, with that part's
+//                arithmetic and stores still to come
+// Returns where the row went (COMBINE) so that the caller can report completion; `here` false if the accumulator never came.
 // ---------------------------------------------------------------------------------------------------
 struct CombineDest {
   int rank;
   bool ok;
+  bool here;
 };
 
 // In-place SGD epilogue (STORE with sgd_lr != 0): the weights under the tile are read before they are rewritten. One
@@ -268,26 +272,14 @@ __device__ __forceinline__ void sgd_fetch_lin(unsigned long long base, unsigned 
     if (row < rows_ok) v[i] = *reinterpret_cast<const uint4*>(base + row * stride + piece * 16);
   }
 }
-__device__ __forceinline__ void staged_load64_lin(uint32_t stage, int lane, uint32_t (&w)[16], unsigned long long base,
-                                                  unsigned long long stride, int rows_ok) {
+// the same for matrices that the launch only reads
+__device__ __forceinline__ void fetch_lin(unsigned long long base, unsigned long long stride, int rows_ok, int lane, uint4 (&v)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = 8 * i + (lane >> 2), piece = lane & 3;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < rows_ok) v = __ldg(reinterpret_cast<const uint4*>(base + row * stride + piece * 16));
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + stage_off(row, piece)), "r"(v.x), "r"(v.y),
-                 "r"(v.z), "r"(v.w)
-                 : "memory");
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows_ok) v[i] = __ldg(reinterpret_cast<const uint4*>(base + row * stride + piece * 16));
   }
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3])
-                 : "r"(stage + stage_off(lane, j))
-                 : "memory");
-  }
-  __syncwarp();
 }
 __device__ __forceinline__ void staged_store64_lin(uint32_t stage, int lane, const uint32_t (&w)[16], unsigned long long base,
                                                    unsigned long long stride, int rows_ok) {
@@ -310,8 +302,8 @@ __device__ __forceinline__ void staged_store64_lin(uint32_t stage, int lane, con
   }
   __syncwarp();
 }
-// the chunk fetched by sgd_fetch, transposed through the warp's staging area into one row per lane
-__device__ __forceinline__ void sgd_unstage(uint32_t stage, int lane, const uint4 (&v)[4], uint32_t (&w)[16]) {
+// a chunk fetched by sgd_fetch_lin or fetch_lin, transposed through the warp's staging area into one row per lane
+__device__ __forceinline__ void unstage(uint32_t stage, int lane, const uint4 (&v)[4], uint32_t (&w)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = 8 * i + (lane >> 2), piece = lane & 3;
@@ -332,11 +324,15 @@ __device__ __forceinline__ void sgd_unstage(uint32_t stage, int lane, const uint
 
 // kFp16 is a template argument: as a run-time value every conversion of an element pair computed both types' results and
 // selected one, about a third of an epilogue's instructions.
-template <int kEpi, int kFp16>
+template <int kEpi, int kFp16, typename Acquire, typename Release>
 __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, const Tile& ti, long long row_base,
                                                      int rows_valid, int rows_store, bool have_acc, uint32_t t_row,
-                                                     uint32_t stage, int q, int half, int lane) {
+                                                     uint32_t stage, int q, int half, int lane, Acquire acquire, Release release) {
   constexpr int fp16 = kFp16;
+  CombineDest cd;
+  cd.rank = 0;
+  cd.ok = false;
+  cd.here = false;
   const int r_in_tile = q * 32 + lane;
   const bool valid = r_in_tile < rows_valid;
   const long long orow = row_base + r_in_tile;
@@ -365,6 +361,9 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
   // of every group) most warps are of that kind and only held the others' issue slots. Outputs that a weight-gradient
   // reduction may read get their zeros.
   if (q * 32 >= rows_valid) {
+    if (!acquire()) return cd;
+    cd.here = true;
+    release();
     if constexpr (kEpi != CCF_EPI_STORE && kEpi != CCF_EPI_COMBINE) {
       const uint32_t zero[16] = {};
       const int ok = min(32, max(0, rows_store - q * 32));
@@ -381,13 +380,8 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         if constexpr (kEpi == CCF_EPI_SWIGLU) put(args.out2);
       }
     }
-    CombineDest none;
-    none.rank = 0;
-    none.ok = false;
-    return none;
+    return cd;
   }
-  uint32_t racc[32];  // one buffer: the next chunk is requested right after this one is copied out to f[]
-  if (have_acc) tmem_ld32(t_row + chunk0 * 32, racc);
   constexpr bool kBias0Prefetch = (kEpi == CCF_EPI_STORE || kEpi == CCF_EPI_BIAS_ACT || kEpi == CCF_EPI_COMBINE);
   uint4 bcur[4], bnext[4];
   const bool has_b0 = kBias0Prefetch && args.bias0 != nullptr;
@@ -403,6 +397,19 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
   auto lin_of = [&](const void* p) { return addr2(p, row_base + q * 32, args.ld_out, 0); };
   const unsigned long long lin_base = lin_of(args.out0);
   if (sgd) sgd_fetch_lin(lin_base + (ti.n0 + chunk0 * 32) * 2ull, lin_stride, ti.n0 + chunk0 * 32 < args.n ? lin_rows : 0, lane, bnext);
+  // DACT, DSWIGLU: the saved pre-activations, one chunk ahead like the bias: loaded where they are used, each chunk of a tile
+  // waited for one more trip to memory (4 experts x 4096 rows, 1024 -> 4096, GELU': 151 us a launch, 144 so)
+  uint4 unext[4];
+  auto fetch_aux = [&](int c) {
+    const int n = ti.n0 + c * 32, ok = n < args.n ? lin_rows : 0;
+    if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux0) + n * 2ull, lin_stride, ok, lane, bnext);
+    if constexpr (kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux1) + n * 2ull, lin_stride, ok, lane, unext);
+  };
+  fetch_aux(chunk0);
+  if (!acquire()) return cd;
+  cd.here = true;
+  uint32_t racc[32];  // one buffer: the next chunk is requested right after this one is copied out to f[]
+  if (have_acc) tmem_ld32(t_row + chunk0 * 32, racc);
   // not unrolled: the body is large and every launch pays for fetching the kernel's code once per SM
 #pragma unroll 1
   for (int c = 0; c < n_chunks; ++c) {
@@ -422,6 +429,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
       if constexpr (kEpi != CCF_EPI_SWIGLU) {
         // next chunk's TMEM load overlaps this chunk's math and stores
         if (c + 1 < n_chunks) tmem_ld32(t_row + (cg + 1) * 32, racc);
+        else release();
       }
     } else {
 #pragma unroll
@@ -435,6 +443,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         tmem_ld_wait();
         acc_to_float(racc, u);
         if (c + 1 < n_chunks) tmem_ld32(t_row + (cg + 1) * 32, racc);
+        else release();
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) u[i] = 0.f;
@@ -480,7 +489,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         } else if (sgd) {
           // the accumulator is a weight gradient and out0 the weights themselves: plain SGD applied here saves writing
           // the gradient, and the optimizer's pass that would read it and the weights again
-          sgd_unstage(stage, lane, bcur, w);
+          unstage(stage, lane, bcur, w);
           const float lr = args.sgd_lr, wd = args.sgd_wd;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -516,7 +525,8 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         // peer stores over NVLink (or local when c_rank is this rank), 64 contiguous bytes per row
         staged_store64(stage, lane, w, c_ok ? addr2(args.peer_comb[c_rank], c_slot, args.ld_out, n) : 0ull);
       } else if constexpr (kEpi == CCF_EPI_DACT) {
-        staged_load64_lin(stage, lane, w, lin_of(args.aux0) + n * 2ull, lin_stride, lin_rows);
+        unstage(stage, lane, bcur, w);
+        if (c + 1 < n_chunks) fetch_aux(cg + 1);
         {
           float pz[32];
           unpack32(w, pz, fp16);
@@ -530,8 +540,9 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
       } else if constexpr (kEpi == CCF_EPI_DSWIGLU) {
         uint32_t wu[16];
-        staged_load64_lin(stage, lane, w, lin_of(args.aux0) + n * 2ull, lin_stride, lin_rows);
-        staged_load64_lin(stage, lane, wu, lin_of(args.aux1) + n * 2ull, lin_stride, lin_rows);
+        unstage(stage, lane, bcur, w);
+        unstage(stage, lane, unext, wu);
+        if (c + 1 < n_chunks) fetch_aux(cg + 1);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const float2 gp = unpack2(w[j], fp16), up = unpack2(wu[j], fp16);
@@ -552,7 +563,6 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
       }
     }
   }
-  CombineDest cd;
   cd.rank = c_rank;
   cd.ok = c_ok;
   return cd;
