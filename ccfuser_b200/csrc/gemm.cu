@@ -579,21 +579,23 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     const bool bwd = L->epi == CCF_EPI_DACT || L->epi == CCF_EPI_DSWIGLU;
     if (!(fwd && a.disp.backward == 0) && !(bwd && a.disp.backward == 1)) return -9;
   }
-  CUtensorMap tm[4];
+  CUtensorMap tm[6];
   const int fp16 = a.fp16;
-  const bool pair = L->two_cta != 0;
+  const bool swap = L->few_rows != 0;
+  if (swap && (L->kgroup || L->a_major != MAJ_K || a.out_fp32 || a.sgd_lr != 0.f || a.bn != 0 || a.a_rows != 0)) return -12;
+  const bool pair = L->two_cta != 0 && !swap;
   if (a.a_rows != 0 && a.a_rows != BM) {
     // the row bound exists in the one-CTA kernel for row-grouped launches with a K-major A operand
     if ((a.a_rows != 32 && a.a_rows != 64) || pair || L->kgroup || L->a_major != MAJ_K) return -11;
   }
-  const int a_box_rows = (L->a_major == MAJ_K) ? (a.a_rows > 0 ? a.a_rows : BM) : BK;
+  const int a_box_rows = swap ? swap_box_rows(false) : (L->a_major == MAJ_K) ? (a.a_rows > 0 ? a.a_rows : BM) : BK;
   if (pair && L->kgroup && (a.m_per_group % (2 * BM) != 0)) return -8;
   if (a.bn != 0 && a.bn != BN) {
     // the narrow tile exists in the one-CTA kernel for row-grouped launches with a K-major B operand
     if (a.bn != 128 || pair || L->kgroup || L->b_major != MAJ_K || L->epi == CCF_EPI_SWIGLU) return -10;
   }
   int b_box_rows = (L->b_major == MAJ_K) ? (a.bn == 128 ? 128 : BN) : BK;
-  if (L->epi == CCF_EPI_SWIGLU || (pair && L->b_major == MAJ_K)) b_box_rows = BN / 2;  // a pair member loads half of B
+  if (L->epi == CCF_EPI_SWIGLU || ((pair || swap) && L->b_major == MAJ_K)) b_box_rows = BN / 2;  // a pair member loads half of B
   int rc;
   if ((rc = make_tmap(&tm[0], L->a0, L->a_rows, L->a_cols, 64, a_box_rows, fp16))) return rc;
   if ((rc = make_tmap(&tm[1], L->a1 ? L->a1 : L->a0, L->a_rows, L->a_cols, 64, a_box_rows, fp16))) return rc;
@@ -605,6 +607,11 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     grid = sms;
+  }
+  if (swap) {
+    if ((rc = make_tmap(&tm[4], L->a0, L->a_rows, L->a_cols, 64, swap_box_rows(true), fp16))) return rc;
+    if ((rc = make_tmap(&tm[5], L->a1 ? L->a1 : L->a0, L->a_rows, L->a_cols, 64, swap_box_rows(true), fp16))) return rc;
+    return launch_swap_by_key(L->b_major, L->epi, tm, a, grid, stream);
   }
   const int key = (L->a_major << 12) | (L->b_major << 8) | (L->epi << 4) | (L->kgroup ? 1 : 0);
   if (pair) return launch_pair_by_key(key, tm, a, grid, stream);

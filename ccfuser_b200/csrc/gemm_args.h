@@ -81,6 +81,8 @@ struct CcfGemmArgs {
   int* peer_done[CCF_MAX_RANKS];    // COMBINE: this rank's completion counter on every rank
   int* sched;               // {tile counter, finished CTAs, spare, spare}; zero before the first launch
   int* status;              // error word (first error wins)
+  float* split_ws;          // swapped kernel: parts of sums shared by several CTA pairs, CCF_SPLIT_WS_FLOATS (null = sums are not shared)
+  int* split_cnt;           // their arrival counters, CCF_SPLIT_COUNTERS, zero before and after every launch
   long long* trace;         // optional [grid, trace_tiles, 8] clock stamps per tile and role (null = off)
   unsigned long long wait_limit_ns;
   long long ld_out;         // leading dimension (elements) of out0/out1/out2/aux0/aux1
@@ -111,6 +113,12 @@ struct CcfGemmArgs {
   CcfDispatchArgs disp;
 };
 
+// Workspace of sums that several CTA pairs share (gemm_swap.cu): two slots per pair, each of up to 32 shares (2 parts of a tile x
+// 2 CTAs x 8 warps) of 3072 floats or 16 of 4096; arrival counters for the shares of two waves of tiles.
+#define CCF_SPLIT_PAIRS 74
+#define CCF_SPLIT_WS_FLOATS (2ll * CCF_SPLIT_PAIRS * 32 * 3072)
+#define CCF_SPLIT_COUNTERS (2 * CCF_SPLIT_PAIRS * 32)
+
 // One launch of the grouped GEMM as the host entry point ccf_gemm_launch takes it: the kernel arguments plus the 2-D
 // views of the operands, from which the tensor maps are encoded.
 struct CcfGemmLaunch {
@@ -127,7 +135,7 @@ struct CcfGemmLaunch {
   int grid;                  // 0 = one CTA per SM
   int device;                // CUDA device of the operands; made current for the calling thread (-1 = leave)
   int two_cta;               // 1 = 256x256 tiles on CTA pairs (tcgen05 cta_group::2), 0 = 128x256 tiles per CTA
-  int pad0;
+  int few_rows;              // 1: the kernel for few rows per group (gemm_swap.cu; row-grouped, K-major rows)
 };
 
 // Arguments of the count exchange + planning kernel (ccf_plan).

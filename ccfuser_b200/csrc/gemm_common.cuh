@@ -106,6 +106,26 @@ __device__ __forceinline__ void act_grad32(float (&f)[32], const float (&pz)[32]
   }
 }
 
+// SwiGLU backward for two elements: a = gradient of silu(g) * u; g and u come packed in wg / wu and leave as their gradients
+__device__ __forceinline__ void dswiglu2(float a0, float a1, uint32_t& wg, uint32_t& wu, int fp16) {
+  const float2 gp = unpack2(wg, fp16), up = unpack2(wu, fp16);
+  const f32x2 a = pk2(a0, a1), g = pk2(gp.x, gp.y), u = pk2(up.x, up.y);
+  const float s0 = fast_rcp(1.f + __expf(-gp.x)), s1 = fast_rcp(1.f + __expf(-gp.y));
+  const f32x2 sg = pk2(s0, s1);
+  const f32x2 dg = mul2(mul2(a, u), mul2(sg, fma2(g, pk2(1.f - s0, 1.f - s1), bc2(1.f))));
+  const f32x2 du = mul2(mul2(a, g), sg);
+  float d0, d1;
+  upk2(dg, d0, d1);
+  wg = pack2(d0, d1, fp16);
+  upk2(du, d0, d1);
+  wu = pack2(d0, d1, fp16);
+}
+
+__device__ __forceinline__ float load_elem(const void* p, size_t i, int fp16) {
+  if (fp16) return __half2float(reinterpret_cast<const __half*>(p)[i]);
+  return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
+}
+
 // 32 consecutive 2-byte elements -> floats (64 bytes, 16-byte aligned)
 __device__ __forceinline__ void load32(const void* p, float (&f)[32], int fp16) {
   const uint4* q = reinterpret_cast<const uint4*>(p);
@@ -545,18 +565,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         if (c + 1 < n_chunks) fetch_aux(cg + 1);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float2 gp = unpack2(w[j], fp16), up = unpack2(wu[j], fp16);
-          const f32x2 a = valid ? pk2(f[2 * j], f[2 * j + 1]) : 0ull;
-          const f32x2 g = pk2(gp.x, gp.y), u = pk2(up.x, up.y);
-          const float s0 = fast_rcp(1.f + __expf(-gp.x)), s1 = fast_rcp(1.f + __expf(-gp.y));
-          const f32x2 sg = pk2(s0, s1);
-          const f32x2 dg = mul2(mul2(a, u), mul2(sg, fma2(g, pk2(1.f - s0, 1.f - s1), bc2(1.f))));
-          const f32x2 du = mul2(mul2(a, g), sg);
-          float d0, d1;
-          upk2(dg, d0, d1);
-          w[j] = pack2(d0, d1, fp16);
-          upk2(du, d0, d1);
-          wu[j] = pack2(d0, d1, fp16);
+          dswiglu2(valid ? f[2 * j] : 0.f, valid ? f[2 * j + 1] : 0.f, w[j], wu[j], fp16);
         }
         staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
         staged_store64_lin(stage, lane, wu, lin_of(args.out1) + n * 2ull, lin_stride, lin_rows_store);
@@ -604,5 +613,8 @@ __device__ __forceinline__ void dispatch_role(const CcfGemmArgs& args, bool comm
 
 // two-CTA kernels (gemm2.cu), selected by the same key as the one-CTA ones
 int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
+// few rows per group: weights on the M side (gemm_swap.cu)
+int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
+int swap_box_rows(bool big);
 
 }  // namespace ccf

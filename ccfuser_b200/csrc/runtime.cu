@@ -35,8 +35,19 @@ struct Dry {
   int n;
 };
 
-// completion-counter increments per row of a COMBINE GEMM with n columns (two epilogue warps per 256-column tile)
-int combine_units(int n, int bn) { return 2 * ((n + bn - 1) / bn); }
+// completion-counter increments per row of a COMBINE GEMM with n columns: two epilogue warps per 256-column tile report it, in the
+// swapped kernel one per 32 columns
+int combine_units(int n, bool swap) { return swap ? n / 32 : 2 * ((n + 255) / 256); }
+
+// Row-grouped launches of a call that expects at most small_rows rows per expert run on the swapped kernel. CCFUSER_TWO_CTA=0
+// keeps them on 128-row tiles (one-CTA kernel) for comparison.
+bool few_rows(const CcfLayer* L, long long rows_per_expert) { return rows_per_expert <= L->small_rows && L->two_cta; }
+void set_swap(CcfGemmLaunch& g, const CcfLayer* L, bool swap) {
+  g.few_rows = swap;
+  if (!swap) return;
+  g.args.split_ws = L->split_ws;
+  g.args.split_cnt = L->split_cnt;
+}
 
 // fields every launch of this layer shares
 CcfGemmLaunch base_launch(const CcfLayer* L) {
@@ -125,10 +136,6 @@ void set_combine(CcfGemmLaunch& g, const CcfLayer* L, void* const* peer_comb, co
   g.args.max_slots = L->max_slots;
 }
 
-// Bound on the rows of any expert of a single-rank call (its capacity, at most all slots of the call; other ranks may bring
-// any number of rows), rounded up to a pipeline geometry of the one-CTA kernel: 32, 64, or 0 for no bound.
-int row_bound(int capacity, int world) { return world != 1 || capacity > 64 ? 0 : capacity > 32 ? 64 : 32; }
-
 int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
   // the pair kernel needs 256-row output tiles in k-grouped mode
   if (g.kgroup && g.args.m_per_group % 256 != 0) g.two_cta = 0;
@@ -143,7 +150,7 @@ int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
 
 // Wait for the owners and sum the k slots of each token. With G (backward) and a router in the call, the sum also carries
 // the gradient through the gate weights.
-int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, int bn, const CcfLayerGrads* G, const int* idx,
+int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, bool swap, const CcfLayerGrads* G, const int* idx,
                     const float* gate_w, Dry* dry, void* stream) {
   if (dry != nullptr) return 0;
   CcfReduceArgs r;
@@ -165,7 +172,7 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
     r.zero_words = L->tile_flags;
     r.zero_count = L->max_rows / 128 + 1;
   } else {
-    const int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model, bn), L->world,
+    const int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model, swap), L->world,
                                     L->wait_limit_ns, L->status, stream);
     if (rc) return rc;
   }
@@ -205,17 +212,8 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
                  int save_pre, int epoch, void* stream, Dry* dry) {
   const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
   int rc = 0;
-  // An expert that receives about one 256-row pair tile's worth of rows fills most second tiles with padding: such
-  // calls run on 128-row tiles (one-CTA kernel).
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
-  const int row_two_cta = rows_per_expert > L->small_rows ? L->two_cta : 0;
-  // GEMM-2 on the one-CTA kernel with so few tiles that most SMs would idle: 128-column tiles (twice as many)
-  int gemm2_bn = 256;
-  if (row_two_cta == 0) {
-    const long long tiles = static_cast<long long>(e_loc) * ((rows_per_expert + 127) / 128 > 0 ? (rows_per_expert + 127) / 128 : 1) *
-                            ((d + 255) / 256);
-    if (tiles < 148) gemm2_bn = 128;
-  }
+  const bool swap = few_rows(L, rows_per_expert);
   if (dry == nullptr) {
     if (L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
     // 1. positions, kept counts, destination order of this rank's slots; count exchange with all ranks + row layout
@@ -274,8 +272,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
       g.args.act = L->act;
     }
     set_dispatch(g, L, x, idx, gate_w, tokens, capacity, 0, nullptr);
-    g.two_cta = row_two_cta;
-    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
+    set_swap(g, L, swap);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -291,13 +288,11 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     g.args.bias0 = L->b2;
     g.args.ld_out = d;
     set_combine(g, L, L->peer_comb, L->row_gate);
-    g.two_cta = row_two_cta;
-    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
-    g.args.bn = gemm2_bn;
+    set_swap(g, L, swap);
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
-  return wait_and_reduce(L, L->comb, y, tokens, gemm2_bn, nullptr, nullptr, nullptr, dry, stream);
+  return wait_and_reduce(L, L->comb, y, tokens, swap, nullptr, nullptr, nullptr, dry, stream);
 }
 
 int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G, int tokens,
@@ -310,7 +305,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
   const int wgrad_two_cta = rows_per_expert > 512 ? L->two_cta : 0;
   const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
-  const int row_two_cta = rows_per_expert > L->small_rows ? L->two_cta : 0;
+  const bool swap = few_rows(L, rows_per_expert);
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
   // GEMM. w2 may be at any group size (dgrad-2 above it is its last reader). w1 / wg only on a single rank: dgrad-1 reads
   // them and, with peers, has to stay the last owner-side kernel of the pass.
@@ -337,8 +332,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       g.args.act = L->act;
     }
     set_dispatch(g, L, dy, idx, gate_w, tokens, capacity, 1, G->dgate);
-    g.two_cta = row_two_cta;
-    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
+    set_swap(g, L, swap);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -397,8 +391,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       set_b(g, L->w1, static_cast<long long>(e_loc) * f, d, kMajMN);
     }
     set_combine(g, L, L->peer_gcomb, nullptr);
-    g.two_cta = row_two_cta;
-    g.args.a_rows = row_two_cta ? 0 : row_bound(capacity, L->world);
+    set_swap(g, L, swap);
     return issue(g, dry, stream);
   };
   if (sgd && (rc = dgrad1())) return rc;
@@ -420,7 +413,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       return rc;
   }
   if (!sgd && (rc = dgrad1())) return rc;
-  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, 256, G, idx, gate_w, dry, stream))) return rc;
+  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, swap, G, idx, gate_w, dry, stream))) return rc;
   if (G->router_dw != nullptr && dry == nullptr)
     rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d,
                        L->e_total, L->top_k, L->fp16, stream);

@@ -48,6 +48,8 @@ struct CcfLayer {
   int* sched;       // scheduler words of the device's workspace (8 ints)
   int* status;      // status words of the device's workspace (2 ints)
   int* epoch_dev;   // device-side call epoch (used when a call passes epoch < 0)
+  float* split_ws;  // the device's workspace for sums shared by CTA pairs, and its counters (gemm_args.h)
+  int* split_cnt;
   // the same buffers on every rank of the group, as mapped into this process
   void* peer_xrecv[CCF_MAX_RANKS];
   void* peer_comb[CCF_MAX_RANKS];
@@ -70,7 +72,7 @@ struct CcfLayer {
   int device;       // CUDA device (-1: leave the calling thread's device alone)
   int pad0;
   int comm_warps;   // 1: dedicated dispatch warps carry the row push, 0: the epilogue warps do
-  int small_rows;   // calls that expect at most this many rows per expert use the one-CTA kernel (128-row tiles)
+  int small_rows;   // calls that expect at most this many rows per expert use the kernel for few rows (gemm_swap.cu)
 };
 
 // Per-call tensors of the backward pass (all allocated by the caller; null where the layer has no such parameter).

@@ -285,18 +285,27 @@ __device__ __forceinline__ int ld_acquire_sys(const int* addr) {
   asm volatile("ld.acquire.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ int ld_acquire_gpu(const int* addr) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ int ld_relaxed_sys(const int* addr) {
   int v;
   asm volatile("ld.relaxed.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
 }
 
-// Spin until *addr >= target (bounded). Returns false on timeout.
+// Spin until *addr has reached target (bounded); the completion counters wrap around, so it is their distance that counts.
+// Returns false on timeout.
+__device__ __forceinline__ bool flag_reached(const int* addr, int target) {
+  return static_cast<int>(static_cast<unsigned>(ld_acquire_sys(addr)) - static_cast<unsigned>(target)) >= 0;
+}
 __device__ __forceinline__ bool wait_flag_ge(const int* addr, int target, uint64_t limit_ns) {
-  if (ld_acquire_sys(addr) >= target) return true;
+  if (flag_reached(addr, target)) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
-  while (ld_acquire_sys(addr) < target) {
+  while (!flag_reached(addr, target)) {
     if ((++spins & 31u) == 0u) {
       if (globaltimer_ns() - t0 > limit_ns) return false;
       __nanosleep(64);

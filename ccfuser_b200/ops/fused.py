@@ -91,6 +91,7 @@ class CommContext:
         self.epoch_dev = torch.zeros(1, dtype=torch.int32, device=device)
         self.device_epoch = bool(env_flag("DEVICE_EPOCH", 0))
         self.ws = G.Workspace.get(device)
+        self.ws.split()         # allocated with the other buffers, not inside a first call that may be captured
         self.users = 0          # fused layers currently attached (FusedMoE.__init__ / close)
         # scratch of the routing kernels
         s_max = max_slots
@@ -271,9 +272,7 @@ class FusedMoE:
         self._desc = None
         self._desc_key = None
         self.sgd = None         # (lr, weight decay): expert weights are updated by the weight-gradient GEMMs (fuse_sgd)
-        self._call_bn = 256
-        self._call_rows = 0
-        self._call_two_cta = None   # kernel choice of the current call's row-grouped launches (_row_two_cta)
+        self._call_few_rows = False     # kernel choice of the current call's row-grouped launches (_few_rows)
         self._owed = None       # weak reference to the autograd node whose backward still needs this layer's buffers
 
     # ------------------------------------------------------------------------------------------
@@ -394,6 +393,7 @@ class FusedMoE:
                      "ticket", "epoch_dev"):
             setattr(L, name, getattr(cc, name).data_ptr())
         L.sched, L.status = cc.ws.sched.data_ptr(), cc.ws.status.data_ptr()
+        L.split_ws, L.split_cnt = cc.ws.split()
         peers = {"peer_xrecv": self.buf.peer_ptrs(self.off_xrecv), "peer_comb": self.buf.peer_ptrs(self.off_comb),
                  "peer_grecv": cc.peer("grecv"), "peer_gcomb": cc.peer("gcomb"), "peer_row_src": cc.peer("row_src"),
                  "peer_row_gate": cc.peer("row_gate"), "peer_tile_flags": cc.peer("tile_flags"),
@@ -486,23 +486,11 @@ class FusedMoE:
         a.total_index = self.max_rows // TILE  # last element of tile_flags: all rows arrived on that rank
         return a
 
-    def _row_two_cta(self, tokens: int):
-        """Kernel choice of the row-grouped launches of a call with ``tokens`` tokens per rank: None (the default, CTA
-        pairs) or False (one-CTA kernel, 128-row tiles) when an expert expects at most ``CCFUSER_SMALL_ROWS`` rows."""
+    def _few_rows(self, tokens: int) -> bool:
+        """Kernel choice of the row-grouped launches of a call with ``tokens`` tokens per rank: weights on the M side
+        (csrc/gemm_swap.cu) when an expert expects at most ``CCFUSER_SMALL_ROWS`` rows."""
         rows = tokens * self.cfg.top_k * self.world // max(1, self.cfg.num_experts)
-        return None if rows > G.SMALL_ROWS_DEFAULT else False
-
-    def _row_bound(self, tokens: int) -> int:
-        """Row bound of the row-grouped launches of a call with ``tokens`` tokens per rank (ops/gemm.py: row_bound)."""
-        if G.TWO_CTA_DEFAULT and self._row_two_cta(tokens) is None:
-            return 0
-        return G.row_bound(self.cfg.capacity(tokens), self.world)
-
-    def _gemm2_bn(self, tokens: int) -> int:
-        """Tile width of the forward GEMM-2 + combine launch of a call with ``tokens`` tokens per rank (ops/gemm.py:
-        narrow_tiles); the source-side wait counts its completion units with the same width."""
-        rows = tokens * self.cfg.top_k * self.world // max(1, self.cfg.num_experts)
-        return G.narrow_tiles(rows, self.cfg.experts_per_rank, self.cfg.d_model, self._row_two_cta(tokens) is False)
+        return rows <= G.SMALL_ROWS_DEFAULT and bool(G.TWO_CTA_DEFAULT)
 
     def _combine_kw(self, peer_comb, row_gate):
         ctx = self.ctx
@@ -563,9 +551,8 @@ class FusedMoE:
         common = dict(group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, tile_flags=cc.tile_flags,
                       dispatch=disp, n_comm_ctas=cc.n_comm, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace,
                       total_index=self.max_rows // TILE, local_begin=self.local_begin, local_rows=self.local_rows,
-                      two_cta=self._row_two_cta(t), a_rows=self._row_bound(t))
-        self._call_two_cta, self._call_rows = common["two_cta"], common["a_rows"]
-        self._call_bn = self._gemm2_bn(t)
+                      few_rows=self._few_rows(t))
+        self._call_few_rows = common["few_rows"]
         if cfg.activation == "swiglu":
             G.launch(a0=self.xrecv, b0=w1.view(e_loc * f, d), b1=wg.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_K,
                      epi=N.EPI_SWIGLU, n=f, k=d, b_group_rows=f, out0=self.h_act, out1=self.h_pre if save_pre else None,
@@ -582,13 +569,12 @@ class FusedMoE:
         d, f, e_loc = cfg.d_model, cfg.d_ffn, cfg.experts_per_rank
         G.launch(a0=self.h_act, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_COMBINE, n=d, k=f,
                  group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, b_group_rows=d, bias0=b2,
-                 ld_out=d, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace, two_cta=self._call_two_cta, bn=self._call_bn,
-                 a_rows=self._call_rows,
+                 ld_out=d, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace, few_rows=self._call_few_rows,
                  **self._combine_kw(self.buf.peer_ptrs(self.off_comb), cc.row_gate))
 
     def stage_reduce(self, tokens: int, out: torch.Tensor):
         """Wait until every owner has delivered this rank's rows, then sum the k slots of each token."""
-        self._wait_and_reduce(self.comb, tokens, G.combine_units(self.cfg.d_model, self._call_bn), out)
+        self._wait_and_reduce(self.comb, tokens, G.combine_units(self.cfg.d_model, self._call_few_rows), out)
 
 
 class GraphedForward:
@@ -800,17 +786,17 @@ class _FusedMoEFn(torch.autograd.Function):
                       workspace=cc.ws)
         dh = torch.empty(fm.max_rows, f, dtype=cfg.dtype, device=dy.device)
         dh2 = torch.empty_like(dh) if swiglu else None
-        rt, ar = fm._row_two_cta(t), fm._row_bound(t)
+        few = fm._few_rows(t)
         if swiglu:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DSWIGLU, n=f, k=d,
                      b_group_rows=d, out0=dh, out1=dh2, aux0=fm.h_pre, aux1=fm.h_pre2, tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, two_cta=rt, a_rows=ar, **common)
+                     local_rows=fm.local_rows, few_rows=few, **common)
         else:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DACT, n=f, k=d,
                      b_group_rows=d, out0=dh, aux0=fm.h_pre, act=N.ACT_CODE[cfg.activation], tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, two_cta=rt, a_rows=ar, **common)
+                     local_rows=fm.local_rows, few_rows=few, **common)
         cc.tile_flags.zero_()
         # 3. wgrad-2: dW2[e] = (g dy)^T h_act   [d, f]
         # With few rows per expert the reduction is only a handful of k-blocks and the per-tile latency chain decides:
@@ -834,11 +820,11 @@ class _FusedMoEFn(torch.autograd.Function):
             ck = fm._combine_kw(cc.peer("gcomb"), None)
             if swiglu:
                 G.launch(a0=dh, a1=dh2, b0=wg.view(e_loc * f, d), b1=w1.view(e_loc * f, d), a_major=N.MAJ_K,
-                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d, two_cta=rt, a_rows=ar,
+                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d, few_rows=few,
                          **common, **ck)
             else:
                 G.launch(a0=dh, b0=w1.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f,
-                         b_group_rows=f, ld_out=d, two_cta=rt, a_rows=ar, **common, **ck)
+                         b_group_rows=f, ld_out=d, few_rows=few, **common, **ck)
 
         if sgd is not None:
             dgrad1()            # reads w1 / wg before the weight-gradient GEMMs below overwrite them
@@ -860,7 +846,7 @@ class _FusedMoEFn(torch.autograd.Function):
         if sgd is None:
             dgrad1()
         dx = torch.empty(t, d, dtype=dy.dtype, device=dy.device)
-        fm._wait_and_reduce(cc.gcomb, t, G.combine_units(d), dx)
+        fm._wait_and_reduce(cc.gcomb, t, G.combine_units(d, few), dx)
         if fm.check_every_call:
             cc.check_status("fused MoE backward")
         return dx, dgate.view(t, cfg.top_k), None, dw1, db1, dwg, dbg, dw2, db2, None

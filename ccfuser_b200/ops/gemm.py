@@ -27,6 +27,7 @@ class Workspace:
         self.status = torch.zeros(2, dtype=torch.int32, device=device)  # [first hard error, overflow count]
         self.status_addr = self.status.data_ptr()
         self._last_stream, self._last_raw = None, None
+        self._split = None
         self._on_gpu = self.sched.device.type == "cuda"
         self._device_index = self.sched.device.index if self._on_gpu else -1
 
@@ -47,6 +48,14 @@ class Workspace:
         """Address of the status word of a CUDA tensor's device."""
         ws = cls._by_device.get(tensor.get_device())
         return (ws if ws is not None else cls.get(tensor.device)).status_addr
+
+    def split(self):
+        """Addresses of the workspace for sums that CTA pairs share (58 MB) and of its arrival counters."""
+        if self._split is None:
+            dev = self.sched.device
+            self._split = (torch.empty(N.SPLIT_WS_FLOATS, dtype=torch.float32, device=dev),
+                           torch.zeros(N.SPLIT_COUNTERS, dtype=torch.int32, device=dev))
+        return self._split[0].data_ptr(), self._split[1].data_ptr()
 
     def enter(self):
         """Called by every launcher with the stream it is about to launch on. The kernels of one device share this
@@ -97,7 +106,9 @@ _MBAR_SITES = {1: "tile scheduler slot (producer)", 2: "free pipeline stage (pro
                4: "free accumulator (MMA warp)", 5: "operands of a stage (MMA warp)", 6: "tile index (epilogue)",
                7: "finished accumulator (epilogue)", 0x22: "free pipeline stage (producer, CTA-pair kernel)",
                0x24: "free accumulator (MMA warp, CTA-pair kernel)", 0x25: "operands of a stage (MMA warp, CTA-pair kernel)",
-               0x27: "finished accumulator (epilogue, CTA-pair kernel)", 0x40: "free pipeline stage (router producer)",
+               0x27: "finished accumulator (epilogue, CTA-pair kernel)", 0x32: "free pipeline stage (producer, swapped kernel)",
+               0x34: "free accumulator (MMA warp, swapped kernel)", 0x35: "operands of a stage (MMA warp, swapped kernel)",
+               0x37: "finished accumulator (epilogue, swapped kernel)", 0x40: "free pipeline stage (router producer)",
                0x41: "operands of a stage (router MMA warp)", 0x42: "finished accumulator (router epilogue)"}
 
 
@@ -128,8 +139,8 @@ TWO_CTA_DEFAULT = bool(int(__import__('os').environ.get('CCFUSER_TWO_CTA', '1'))
 # 1: the two dedicated dispatch warps of every CTA push the rows (next to the MMA and epilogue warps); 0: the epilogue
 # warps push them before their first tile
 COMM_WARPS_DEFAULT = int(__import__('os').environ.get('CCFUSER_COMM_WARPS', '1'))
-# calls that expect at most this many rows per expert run on the one-CTA kernel's 128-row tiles: around one 256-row pair
-# tile per expert most second pair tiles would be padding
+# the row-grouped launches of calls that expect at most this many rows per expert run on the kernel with the weights on the M
+# side (csrc/gemm_swap.cu), whose tiles are as wide as an expert has rows; with CCFUSER_TWO_CTA=0 on 128-row tiles
 SMALL_ROWS_DEFAULT = int(__import__('os').environ.get('CCFUSER_SMALL_ROWS', '320'))
 
 
@@ -147,7 +158,8 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
            act=N.ACT_NONE, out_fp32=False, tile_flags=None, local_begin=None, local_rows=None, row_src=None, row_gate=None,
            peer_comb=None, peer_done=None, world=1, send_finish=0, count_rows=1, max_slots=0,
            dispatch: Optional[N.DispatchArgs] = None, n_comm_ctas=0, total_index=-1, two_cta=None, wait_ns=DEFAULT_WAIT_NS, grid=0, trace=None,
-           workspace: Optional[Workspace] = None, comm_warps: Optional[int] = None, sgd=None, bn: int = 0, a_rows: int = 0):
+           workspace: Optional[Workspace] = None, comm_warps: Optional[int] = None, sgd=None, bn: int = 0, a_rows: int = 0,
+           few_rows: bool = False):
     """Fill a CcfGemmLaunch and launch on the current stream. a0/b0 are 2-D contiguous views."""
     lib = N.load()
     ws = workspace or Workspace.get(a0.device)
@@ -180,6 +192,9 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     g.total_index = int(total_index)
     g.comm_warps = int(COMM_WARPS_DEFAULT if comm_warps is None else comm_warps)
     g.bn, g.a_rows = int(bn), int(a_rows)
+    L.few_rows = int(bool(few_rows))
+    if few_rows:            # weights on the M side, for few rows per group (csrc/gemm_swap.cu)
+        g.split_ws, g.split_cnt = ws.split()
     if sgd is not None:     # (lr, weight decay): EPI_STORE updates out0 in place instead of storing the product
         g.sgd_lr, g.sgd_wd = float(sgd[0]), float(sgd[1])
     if dispatch is not None:
@@ -203,25 +218,11 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     return ws
 
 
-def combine_units(n: int, bn: int = 256) -> int:
-    """Completion-counter increments per output row of a COMBINE GEMM with n columns and bn-column tiles: every tile
-    is stored by two epilogue warps per row quarter (one per half of its columns), and each of them reports its rows."""
-    return 2 * ((n + bn - 1) // bn)
-
-
-def narrow_tiles(rows_per_expert: int, experts: int, n: int, one_cta: bool) -> int:
-    """Tile width of a row-grouped, K-major-B launch on the one-CTA kernel: 128 when 256-column tiles would leave most of
-    the 148 SMs without a tile (a handful of experts with a few hundred rows: the latency-bound serving shapes)."""
-    if not one_cta:
-        return 256
-    tiles = experts * max(1, (rows_per_expert + 127) // 128) * ((n + 255) // 256)
-    return 128 if tiles < 148 else 256
-
-
-def row_bound(capacity: int, world: int) -> int:
-    """Bound on the rows of any expert of a single-rank call (its capacity, at most all slots of the call; other ranks may
-    bring any number of rows), rounded up to a pipeline geometry of the one-CTA kernel: 32, 64, or 0 for no bound."""
-    return 0 if world != 1 or capacity > 64 else 64 if capacity > 32 else 32
+def combine_units(n: int, few_rows: bool = False) -> int:
+    """Completion-counter increments per output row of a COMBINE GEMM with n columns: every 256-column tile is stored by two
+    epilogue warps per row quarter (one per half of its columns), and each of them reports its rows; in the swapped kernel
+    a warp stores 32 columns of a row."""
+    return n // 32 if few_rows else 2 * ((n + 255) // 256)
 
 
 def single_group(rows: int, device):
