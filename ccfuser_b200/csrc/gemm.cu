@@ -581,9 +581,12 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
   }
   CUtensorMap tm[6];
   const int fp16 = a.fp16;
-  const bool swap = L->few_rows != 0;
-  if (swap && (L->kgroup || L->a_major != MAJ_K || a.out_fp32 || a.sgd_lr != 0.f || a.bn != 0 || a.a_rows != 0)) return -12;
-  const bool pair = L->two_cta != 0 && !swap;
+  const bool swap = L->few_rows && !L->kgroup, wgrad = L->few_rows && L->kgroup;
+  if (wgrad && (L->a_major != MAJ_MN || L->b_major != MAJ_MN || L->epi != CCF_EPI_STORE || a.out_fp32 || a.bias0 != nullptr ||
+                a.ld_out != a.n || a.m_per_group % (2 * BM) != 0))
+    return -13;
+  if (swap && (L->a_major != MAJ_K || a.out_fp32 || a.sgd_lr != 0.f || a.bn != 0 || a.a_rows != 0)) return -12;
+  const bool pair = L->two_cta != 0 && !L->few_rows;
   if (a.a_rows != 0 && a.a_rows != BM) {
     // the row bound exists in the one-CTA kernel for row-grouped launches with a K-major A operand
     if ((a.a_rows != 32 && a.a_rows != 64) || pair || L->kgroup || L->a_major != MAJ_K) return -11;
@@ -607,6 +610,10 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     grid = sms;
+  }
+  if (wgrad) {
+    if ((rc = make_tmap(&tm[4], a.out0, static_cast<long long>(a.num_groups) * a.m_per_group, a.n, 64, BM, fp16))) return rc;
+    return launch_wgrad(tm, a, grid, stream);
   }
   if (swap) {
     if ((rc = make_tmap(&tm[4], L->a0, L->a_rows, L->a_cols, 64, swap_box_rows(true), fp16))) return rc;

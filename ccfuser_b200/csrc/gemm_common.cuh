@@ -616,5 +616,7 @@ int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int
 // few rows per group: weights on the M side (gemm_swap.cu)
 int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
 int swap_box_rows(bool big);
+// weight gradients of few rows per group (gemm_wgrad.cu)
+int launch_wgrad(const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
 
 }  // namespace ccf

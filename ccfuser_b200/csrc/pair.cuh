@@ -1,4 +1,4 @@
-// Cluster and cta_group::2 primitives of the kernels that run on CTA pairs (gemm2.cu, gemm_swap.cu).
+// Cluster and cta_group::2 primitives of the kernels that run on CTA pairs (gemm2.cu, gemm_swap.cu, gemm_wgrad.cu).
 #pragma once
 #include "gemm_common.cuh"
 

@@ -108,7 +108,10 @@ _MBAR_SITES = {1: "tile scheduler slot (producer)", 2: "free pipeline stage (pro
                0x24: "free accumulator (MMA warp, CTA-pair kernel)", 0x25: "operands of a stage (MMA warp, CTA-pair kernel)",
                0x27: "finished accumulator (epilogue, CTA-pair kernel)", 0x32: "free pipeline stage (producer, swapped kernel)",
                0x34: "free accumulator (MMA warp, swapped kernel)", 0x35: "operands of a stage (MMA warp, swapped kernel)",
-               0x37: "finished accumulator (epilogue, swapped kernel)", 0x40: "free pipeline stage (router producer)",
+               0x37: "finished accumulator (epilogue, swapped kernel)", 0x60: "free pipeline stage (producer, few-row weight gradient)",
+               0x61: "free accumulator (MMA warp, few-row weight gradient)", 0x62: "operands of a stage (MMA warp, few-row weight gradient)",
+               0x63: "free chunk (weight producer, few-row weight gradient)", 0x64: "finished chunk (store warp, few-row weight gradient)",
+               0x65: "finished accumulator (epilogue, few-row weight gradient)", 0x66: "chunk (epilogue, few-row weight gradient)", 0x40: "free pipeline stage (router producer)",
                0x41: "operands of a stage (router MMA warp)", 0x42: "finished accumulator (router epilogue)"}
 
 
@@ -192,8 +195,10 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     g.total_index = int(total_index)
     g.comm_warps = int(COMM_WARPS_DEFAULT if comm_warps is None else comm_warps)
     g.bn, g.a_rows = int(bn), int(a_rows)
-    L.few_rows = int(bool(few_rows))
-    if few_rows:            # weights on the M side, for few rows per group (csrc/gemm_swap.cu)
+    # the kernels for few rows per group: weights on the M side (csrc/gemm_swap.cu); k-grouped, where output rows come in 256s,
+    # csrc/gemm_wgrad.cu
+    L.few_rows = int(bool(few_rows) and not (kgroup and m_per_group % 256 != 0))
+    if few_rows and not kgroup:
         g.split_ws, g.split_cnt = ws.split()
     if sgd is not None:     # (lr, weight decay): EPI_STORE updates out0 in place instead of storing the product
         g.sgd_lr, g.sgd_wd = float(sgd[0]), float(sgd[1])
