@@ -16,6 +16,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libccfuser_b200.so")
+TORCH_PATH = os.path.join(LIB_DIR, "_ccf_torch.so")    # autograd functions in C++ (csrc/torch_norm.cpp)
+TORCH_SOURCE = os.path.join(CSRC, "torch_norm.cpp")
 SOURCES = ["gemm.cu", "gemm2.cu", "gemm_swap.cu", "gemm_wgrad.cu", "moe_kernels.cu", "route.cu", "combine.cu", "router.cu", "runtime.cu", "no_alloc.cu", "norm.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
@@ -33,7 +35,9 @@ def sources():
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(TORCH_PATH):
+        return True
+    if os.path.getmtime(TORCH_SOURCE) > os.path.getmtime(TORCH_PATH):
         return True
     t = os.path.getmtime(LIB_PATH)
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
@@ -62,7 +66,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
     tmp = LIB_PATH + ".tmp"
     subprocess.check_call([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", tmp, *objs, "-lcudart"])
     os.replace(tmp, LIB_PATH)
+    if force or not os.path.exists(TORCH_PATH) or os.path.getmtime(TORCH_SOURCE) > os.path.getmtime(TORCH_PATH):
+        build_torch_module()
     return LIB_PATH
+
+
+def build_torch_module() -> str:
+    """``lib/_ccf_torch.so``: a Python module against the installed torch, linked to the CUDA library beside it."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), sysconfig.get_paths()["include"]]
+    tmp = TORCH_PATH + ".tmp"
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           *("-I" + i for i in inc), TORCH_SOURCE, "-o", tmp, "-L", LIB_DIR, "-lccfuser_b200", "-Wl,-rpath,$ORIGIN",
+                           "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+                           "-ltorch_python"])
+    os.replace(tmp, TORCH_PATH)
+    return TORCH_PATH
 
 
 def build_selftest() -> str:

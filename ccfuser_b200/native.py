@@ -129,15 +129,39 @@ class LayerGrads(C.Structure):
 
 _lib = None
 _lock = threading.Lock()
-LAUNCHES = [0]   # kernels of this library launched by this process (bench.py reports the count)
+class _Launches(list):
+    """[0]: kernels of this library launched by this process (bench.py reports the count), those of the torch module included."""
+
+    def __getitem__(self, i):
+        return super().__getitem__(i) + (_torch_module.launches() if _torch_module is not None else 0)
+
+
+LAUNCHES = _Launches([0])
+_torch_module = None
 
 
 def count(n: int = 1):
-    LAUNCHES[0] += n
+    LAUNCHES[0] = list.__getitem__(LAUNCHES, 0) + n
 
 
 def lib_path() -> str:
     return os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libccfuser_b200.so")
+
+
+def torch_module():
+    """The autograd functions in C++ (csrc/torch_norm.cpp)."""
+    global _torch_module
+    if _torch_module is None:
+        load()      # builds both where the sources are newer
+        import importlib.util
+        path = os.path.join(os.path.dirname(lib_path()), "_ccf_torch.so")
+        with _lock:
+            if _torch_module is None:
+                spec = importlib.util.spec_from_file_location("_ccf_torch", path)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                _torch_module = module
+    return _torch_module
 
 
 def load(build_if_missing: bool = True):
