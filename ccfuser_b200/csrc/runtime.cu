@@ -137,8 +137,8 @@ void set_combine(CcfGemmLaunch& g, const CcfLayer* L, void* const* peer_comb, co
 }
 
 int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
-  // the pair kernel needs 256-row output tiles in k-grouped mode
-  if (g.kgroup && g.args.m_per_group % 256 != 0) g.two_cta = 0;
+  // the kernels on CTA pairs need 256-row output tiles in k-grouped mode
+  if (g.kgroup && g.args.m_per_group % 256 != 0) g.two_cta = g.few_rows = 0;
   if (g.args.ld_out == 0) g.args.ld_out = g.args.n;
   if (dry != nullptr) {
     if (dry->n < dry->cap) dry->out[dry->n] = g;
@@ -300,10 +300,11 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
   int rc = 0;
   if (dry == nullptr && L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
-  // With few rows per expert the weight-gradient reduction is only a handful of k-blocks and the per-tile latency chain
-  // decides: there the one-CTA kernel is faster than CTA pairs.
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
-  const int wgrad_two_cta = rows_per_expert > 512 ? L->two_cta : 0;
+  // With few rows per expert the weight-gradient reduction is only a handful of k-blocks, and moving the result decides.
+  // In-place launches, 2048 x 8192: 811 us against 1214 on the pair kernel at 64 x 256 rows, 309 against 355 at 16 x 512,
+  // 553 against 467 at 16 x 1024.
+  const int wgrad_few = rows_per_expert <= 512 && L->two_cta;
   const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
   const bool swap = few_rows(L, rows_per_expert);
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
@@ -349,7 +350,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     g.args.sgd_lr = sgd2 ? G->sgd_lr : 0.f;
     g.args.sgd_wd = sgd2 ? G->sgd_wd : 0.f;
     g.args.ld_out = f;
-    g.two_cta = wgrad_two_cta;
+    g.few_rows = wgrad_few;
     if ((rc = issue(g, dry, stream))) return rc;
   }
   if (G->db2 != nullptr && dry == nullptr) {
@@ -368,7 +369,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     g.args.sgd_lr = sgd ? G->sgd_lr : 0.f;
     g.args.sgd_wd = sgd ? G->sgd_wd : 0.f;
     g.args.ld_out = d;
-    g.two_cta = wgrad_two_cta;
+    g.few_rows = wgrad_few;
     return issue(g, dry, stream);
   };
   // 5. dgrad-1 + combine: dx rows go back to the ranks the tokens came from. Issued after the weight gradients (its
