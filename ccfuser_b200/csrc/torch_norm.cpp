@@ -1,6 +1,6 @@
 // LayerNorm as an autograd function in C++: what ops/norm.py did around the kernels of norm.cu, without the Python of an
 // autograd.Function on either side. One forward and backward of 8192 x 2048 took 127 us of host time from Python for kernels that
-// run 85 us. The kernels and their launchers stay in libccfuser_b200.so, which this module is linked against.
+// run 85 us when cold; one such pass among others 173 us before and 86 now. The kernels and their launchers stay in libccfuser_b200.so, which this module is linked against.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -32,7 +32,7 @@ at::Tensor rows_of(const at::Tensor& t, int64_t rows, int64_t d) { return t.resh
 
 struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
-                            double eps, int64_t status, int64_t wait_ns) {
+                            const at::Tensor& status, double eps, int64_t wait_ns) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t d = x.size(-1), rows = x.numel() / d;
     const at::Tensor x2 = rows_of(x, rows, d), w = weight.contiguous();
@@ -64,7 +64,7 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
     const at::Tensor part = at::empty({ccf_layernorm_bwd_parts(static_cast<int>(rows), static_cast<int>(d)), 2, d}, x2.options().dtype(at::kFloat));
     check(ccf_layernorm_bwd(x2.data_ptr(), dy.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
                             part.data_ptr<float>(), dg.data_ptr(), has_bias ? db.data_ptr() : nullptr, static_cast<int>(rows),
-                            static_cast<int>(d), x2.scalar_type() == at::kHalf, reinterpret_cast<int*>(ctx->saved_data["status"].toInt()),
+                            static_cast<int>(d), x2.scalar_type() == at::kHalf, ctx->saved_data["status"].toTensor().data_ptr<int>(),
                             static_cast<unsigned long long>(ctx->saved_data["wait_ns"].toInt()),
                             c10::cuda::getCurrentCUDAStream().stream()),
           "ccf_layernorm_bwd");
@@ -78,8 +78,8 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
 PYBIND11_MODULE(_ccf_torch, m) {
   m.def(
       "layer_norm",
-      [](const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias, double eps, int64_t status, int64_t wait_ns) {
-        return LayerNormFn::apply(x, weight, bias, eps, status, wait_ns);
+      [](const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias, const at::Tensor& status, double eps,
+         int64_t wait_ns) { return LayerNormFn::apply(x, weight, bias, status, eps, wait_ns);
       },
       py::call_guard<py::gil_scoped_release>());
   m.def("launches", [] { return g_launches.load(); });

@@ -129,6 +129,8 @@ class LayerGrads(C.Structure):
 
 _lib = None
 _lock = threading.Lock()
+
+
 class _Launches(list):
     """[0]: kernels of this library launched by this process (bench.py reports the count), those of the torch module included."""
 

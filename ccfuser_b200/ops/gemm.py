@@ -44,10 +44,15 @@ class Workspace:
         return ws
 
     @classmethod
+    def of(cls, tensor) -> "Workspace":
+        """The workspace of a CUDA tensor's device."""
+        ws = cls._by_device.get(tensor.get_device())
+        return ws if ws is not None else cls.get(tensor.device)
+
+    @classmethod
     def status_of(cls, tensor) -> int:
         """Address of the status word of a CUDA tensor's device."""
-        ws = cls._by_device.get(tensor.get_device())
-        return (ws if ws is not None else cls.get(tensor.device)).status_addr
+        return cls.of(tensor).status_addr
 
     def split(self):
         """Addresses of the workspace for sums that CTA pairs share (58 MB) and of its arrival counters."""

@@ -27,7 +27,7 @@ def supported(x: torch.Tensor, normalized_shape, weight) -> bool:
 def layer_norm(x, normalized_shape, weight, bias, eps=1e-5):
     """``F.layer_norm`` that runs on the library's kernels where they apply."""
     if supported(x, tuple(normalized_shape), weight) and (bias is None or bias.dtype == x.dtype):
-        return N.torch_module().layer_norm(x, weight, bias, eps, G.Workspace.status_of(x), G.DEFAULT_WAIT_NS)
+        return N.torch_module().layer_norm(x, weight, bias, G.Workspace.of(x).status, eps, G.DEFAULT_WAIT_NS)
     return F.layer_norm(x, normalized_shape, weight, bias, eps)
 
 

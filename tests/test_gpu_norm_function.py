@@ -1,0 +1,70 @@
+"""LayerNorm's autograd function (csrc/torch_norm.cpp): what autograd asks of a function, and the forward kernel's walk over rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# bf16 results of sums in fp32: half a unit in the last place of the largest value, 2^-9, and as much for the rounded inputs' products
+TOL = 2.0 ** -8
+
+
+def _ref(x, w, b, gy, eps=1e-5):
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    bd = None if b is None else b.detach().double().requires_grad_(True)
+    y = torch.nn.functional.layer_norm(xd, (x.shape[-1],), wd, bd, eps)
+    y.backward(gy.double())
+    return y, xd.grad, wd.grad, None if b is None else bd.grad
+
+
+def _close(a, r):
+    assert a.shape == r.shape
+    assert float((a.double() - r).abs().max() / r.abs().max().clamp_min(1e-6)) < TOL
+
+
+# one row, one block, one row more than the grid's warps take at once (2 blocks of 8 rows on each of 148 SMs), several rows per warp
+@pytest.mark.parametrize("rows", [1, 8, 2369, 2368 * 3 + 5])
+@pytest.mark.parametrize("d", [8, 264, 768, 2048])
+def test_rows_per_warp(rows, d):
+    from ccfuser_b200.ops.norm import layer_norm
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + d)
+    x = torch.randn(rows, d, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = (1 + 0.2 * torch.randn(d, generator=g, device="cuda")).bfloat16().requires_grad_(True)
+    b = (0.1 * torch.randn(d, generator=g, device="cuda")).bfloat16().requires_grad_(True)
+    gy = torch.randn(rows, d, generator=g, device="cuda").bfloat16()
+    y = layer_norm(x, (d,), w, b)
+    y.backward(gy)
+    ry, rx, rw, rb = _ref(x, w, b, gy)
+    _close(y, ry)
+    _close(x.grad, rx)
+    _close(w.grad, rw)
+    _close(b.grad, rb)
+
+
+def test_strided_inputs_saved_tensor_hooks_and_frozen_weights():
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops.norm import layer_norm
+    torch.manual_seed(5)
+    base = torch.randn(4, 50, 96, device="cuda").bfloat16()
+    x = base.transpose(0, 1)[:, :, ::2].detach().requires_grad_(True)        # no stride of a contiguous tensor
+    w = torch.randn(48, device="cuda").bfloat16()                            # needs no gradient
+    gy = torch.randn(48, 50, 4, device="cuda").bfloat16().permute(1, 2, 0)
+    packed = []
+    before = N.LAUNCHES[0]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t.shape), t.cpu())[1], lambda t: t.cuda()):
+        y = layer_norm(x, (48,), w, None)
+    y.backward(gy)
+    assert len(packed) == 4 and N.LAUNCHES[0] - before == 3
+    assert w.grad is None
+    ry, rx, _, _ = _ref(x, w, None, gy)
+    _close(y, ry)
+    _close(x.grad, rx)
+
+
+def test_transforms_are_refused():
+    from ccfuser_b200.ops.norm import layer_norm
+    x, w = torch.randn(4, 3, 64, device="cuda").bfloat16(), torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda t: layer_norm(t, (64,), w, None))(x)
+    import torch.autograd.forward_ad as fwd
+    with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        layer_norm(fwd.make_dual(x, torch.ones_like(x)), (64,), w, None)
