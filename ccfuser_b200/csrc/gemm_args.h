@@ -81,8 +81,6 @@ struct CcfGemmArgs {
   int* peer_done[CCF_MAX_RANKS];    // COMBINE: this rank's completion counter on every rank
   int* sched;               // {tile counter, finished CTAs, spare, spare}; zero before the first launch
   int* status;              // error word (first error wins)
-  float* split_ws;          // swapped kernel: parts of sums shared by several CTA pairs, CCF_SPLIT_WS_FLOATS (null = sums are not shared)
-  int* split_cnt;           // their arrival counters, CCF_SPLIT_COUNTERS, zero before and after every launch
   long long* trace;         // optional [grid, trace_tiles, 8] clock stamps per tile and role (null = off)
   unsigned long long wait_limit_ns;
   long long ld_out;         // leading dimension (elements) of out0/out1/out2/aux0/aux1
@@ -112,12 +110,6 @@ struct CcfGemmArgs {
                             // bound). The pipeline then keeps only so many rows of A per stage and holds more stages
   CcfDispatchArgs disp;
 };
-
-// Workspace of sums that several CTA pairs share (gemm_swap.cu): two slots per pair, each of up to 32 shares (2 parts of a tile x
-// 2 CTAs x 8 warps) of 3072 floats or 16 of 4096; arrival counters for the shares of two waves of tiles.
-#define CCF_SPLIT_PAIRS 74
-#define CCF_SPLIT_WS_FLOATS (2ll * CCF_SPLIT_PAIRS * 32 * 3072)
-#define CCF_SPLIT_COUNTERS (2 * CCF_SPLIT_PAIRS * 32)
 
 // One launch of the grouped GEMM as the host entry point ccf_gemm_launch takes it: the kernel arguments plus the 2-D
 // views of the operands, from which the tensor maps are encoded.

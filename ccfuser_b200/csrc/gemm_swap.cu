@@ -11,9 +11,12 @@
 //   parts       a tile of more columns than an accumulator holds is two parts that share every stage of weights
 //   accumulators  ring of 2 x 256 or, when some group has more than 256 rows, 3 x 160 TMEM columns: with two parts per tile the
 //               next tile's first part has a free accumulator while the last tile's parts are stored
-//   split       when the tiles do not fill the last wave of CTA pairs, the pairs share the last tiles' k-blocks evenly. Parts of a
-//               sum go through an fp32 workspace; whoever delivers the last one adds them in order and runs the epilogue. Nobody
-//               waits for anybody, and the result does not depend on who came last.
+//   tiles       pair p takes tiles p, p + pairs, ...: every sum runs over k in order on one pair, as in gemm2.cu, so that a row's result
+//               does not depend on what is routed beside it. A version in which the pairs shared the k-blocks of the last tiles through
+//               an fp32 workspace gave that up, and cost more than the even split saved: of 1032 launches measured (512 x 2048 to
+//               4096 x 14336, 4 to 64 experts, 8 to 320 rows each) it was slower in 308 and more than 4 % faster in 33; 8 experts of
+//               256 rows, 4096 x 14336: 255 us without against 300 with it for the second projection, 470 against 628 for its
+//               input gradient; 4 experts of 8 rows, 4096 x 1024, SwiGLU, input gradient: 73 against 48.
 //
 // The epilogue reads the accumulator in fragments of 8 features x 8 rows and transposes them by stmatrix into the warp's staging
 // area, from where rows leave as 64-byte segments like those of the other kernels. Arrival gating, dispatch role, combine with
@@ -39,9 +42,8 @@ constexpr int kSwMaxBufs = 3;
 
 // What an epilogue warp has in hand, kept in shared memory: as registers it pushed the epilogue's own values out to local memory.
 struct SwapWork {
-  int t, pos, end;                                   // SwapSegments
+  int t;                                             // next tile
   int g, row0, tokens, zero_rows, n0, parts, np;     // SwapTile
-  int tile, tile_start, first, sharers;              // of a segment of a shared tile
 };
 
 struct __align__(16) CtrlS {
@@ -76,18 +78,6 @@ __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[32]) 
   tmem_ld_16x256b_x4(taddr, r);
   tmem_ld_16x256b_x4(taddr + (16u << 16), r + 16);
 }
-__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const float* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]), "f"(r[10]), "f"(r[11]),
-      "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const float (&r)[32]) {
-  tmem_st_16x256b_x4(taddr, r);
-  tmem_st_16x256b_x4(taddr + (16u << 16), r + 16);
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // word m = 8 h + 2 j + s holds rows (8 j + 2 (l % 4), + 1) of feature 8 p + l / 4, p = 2 h + s
 __device__ __forceinline__ constexpr int frag_piece(int m) { return 2 * (m >> 3) + (m & 1); }
 
@@ -185,25 +175,20 @@ __device__ __forceinline__ SwapTile decode_swap_tile(int t, const CtrlS* c, int 
   return ti;
 }
 
-// The next piece of an epilogue warp's work; out of line, the registers it needs are not the epilogue's.
-__device__ __noinline__ bool swap_next(const CtrlS* ctrl, SwapWork* w, int pair, int n_pairs, int num_groups) {
-  const SwapShape& s = ctrl->shape;
-  SwapSegments it(s, w->t, w->pos, w->end, n_pairs);
-  SwapSegment sg;
+// The next tile of an epilogue warp; out of line, the registers it needs are not the epilogue's.
+__device__ __noinline__ bool swap_next(const CtrlS* ctrl, SwapWork* w, int n_pairs, int num_groups) {
+  const int t = w->t;
   __syncwarp();
-  if (!it.next(sg)) return false;
-  const SwapTile ti = decode_swap_tile(sg.tile, ctrl, num_groups);
-  int first = pair, sharers = 1;
-  if (sg.kb0 != 0 || sg.kb1 != s.kblocks) it.contributors(sg, pair, first, sharers);
-  if ((threadIdx.x & 31) == 0)
-    *w = SwapWork{it.t, it.pos, it.end, ti.g, ti.row0, ti.tokens, ti.zero_rows, ti.n0, ti.parts, ti.np, sg.tile, sg.kb0 == 0, first, sharers};
+  if (t >= ctrl->shape.total_tiles) return false;
+  const SwapTile ti = decode_swap_tile(t, ctrl, num_groups);
+  if ((threadIdx.x & 31) == 0) *w = SwapWork{t + n_pairs, ti.g, ti.row0, ti.tokens, ti.zero_rows, ti.n0, ti.parts, ti.np};
   __syncwarp();
   return true;
 }
 
 // Tile tables of one launch, filled by one warp of every CTA at start-up
 template <int kEpi>
-__device__ __forceinline__ void swap_tables_warp(const CcfGemmArgs& args, CtrlS* ctrl, int n_pairs, int lane) {
+__device__ __forceinline__ void swap_tables_warp(const CcfGemmArgs& args, CtrlS* ctrl, int lane) {
   constexpr bool kWide = kEpi == CCF_EPI_SWIGLU;
   int max_rows = 0, total_rows = 0;
   for (int g0 = 0; g0 < args.num_groups; g0 += 32) {
@@ -241,7 +226,7 @@ __device__ __forceinline__ void swap_tables_warp(const CcfGemmArgs& args, CtrlS*
   max_half = __reduce_max_sync(0xffffffffu, max_half);
   if (lane == 0) {
     ctrl->mt_prefix[args.num_groups] = acc;
-    ctrl->shape = swap_shape(args, acc, total_rows, max_half, width, kWide, n_pairs, kSwPipeBytes, kSwMaxStages);
+    ctrl->shape = swap_shape(args, acc, total_rows, max_half, width, kWide, kSwPipeBytes, kSwMaxStages);
   }
 }
 
@@ -256,68 +241,7 @@ struct SwapPart {
   int first;   // this warp's first chunk
 };
 
-// A tile whose k-blocks several pairs share, one warp's share of one part: deliver this segment's sum, unless all others are there
-// already. Whoever is last adds them to its accumulator in the order of the pairs, wherever in that order its own comes, and
-// returns true: the accumulator then holds the whole sum. Out of line: the epilogue keeps its registers.
-template <bool kWide>
-__device__ __noinline__ bool swap_share(float* share, int* counter, int first_pair, int n, int index, int n_acc, uint32_t t_col,
-                                        uint32_t up_col, int c0, int lane, int slot_floats, bool tile_start) {
-  constexpr int kChunkFloats = kWide ? 2048 : 1024;
-  int seen = 0;
-  if (lane == 0) seen = ld_acquire_gpu(counter);
-  seen = __shfl_sync(0xffffffffu, seen, 0);
-  if (seen != n - 1) {
-    float* ws = share + (2ll * (first_pair + index) + (tile_start ? 1 : 0)) * slot_floats;
-    for (int c = c0; c < n_acc; c += 2) {
-      for (int a = 0; a < (kWide ? 2 : 1); ++a) {
-        uint32_t r[32];
-        tmem_ld_frag((a ? up_col : t_col) + 32 * c, r);
-        tmem_ld_wait();
-        float4* o = reinterpret_cast<float4*>(ws + (c >> 1) * kChunkFloats + a * 1024) + lane;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          __stcg(o + 32 * i, make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
-                                         __uint_as_float(r[4 * i + 3])));
-      }
-    }
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) seen = atomicAdd(counter, 1);
-    seen = __shfl_sync(0xffffffffu, seen, 0);
-    if (seen != n - 1) return false;
-  }
-  __threadfence();
-  if (lane == 0) *counter = 0;
-  for (int c = c0; c < n_acc; c += 2) {
-    for (int a = 0; a < (kWide ? 2 : 1); ++a) {
-      const uint32_t col = (a ? up_col : t_col) + 32 * c;
-      uint32_t r[32];
-      float f[32];
-      tmem_ld_frag(col, r);
-      tmem_ld_wait();
-      // f = p_0 + p_1 + ...; contributor k's segment starts inside the tile unless it is the first
-      for (int k = 0; k < n; ++k) {
-        const float4* o = reinterpret_cast<const float4*>(share + (2ll * (first_pair + k) + (k == 0 ? 1 : 0)) * slot_floats +
-                                                          (c >> 1) * kChunkFloats + a * 1024) + lane;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 v = k == index ? make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
-                                                    __uint_as_float(r[4 * i + 3]))
-                                      : __ldcg(o + 32 * i);
-          f[4 * i] = k == 0 ? v.x : f[4 * i] + v.x;
-          f[4 * i + 1] = k == 0 ? v.y : f[4 * i + 1] + v.y;
-          f[4 * i + 2] = k == 0 ? v.z : f[4 * i + 2] + v.z;
-          f[4 * i + 3] = k == 0 ? v.w : f[4 * i + 3] + v.w;
-        }
-      }
-      tmem_st_frag(col, f);
-    }
-  }
-  tmem_st_wait();
-  return true;
-}
-
-// `acquire` waits for the accumulator and says whether it is this warp's to finish; bias and saved inputs are requested before.
+// `acquire` waits for the accumulator (false: given up); bias and saved inputs are requested before.
 // `release` hands it back; called once this warp's last chunk of it is in registers.
 template <int kEpi, int kFp16, typename Acquire, typename Release>
 __device__ __forceinline__ void swap_epilogue(const CcfGemmArgs& args, const SwapPart& pt, uint32_t t_col, uint32_t up_col,
@@ -532,7 +456,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
-  if (warp == 2) swap_tables_warp<kEpi>(args, ctrl, n_pairs, lane);
+  if (warp == 2) swap_tables_warp<kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
@@ -549,8 +473,6 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
     // ======================= TMA producer (both CTAs) =======================
     int stage = 0, phase = 0, seq = 0;
     bool ok = true, all_in = false;
-    SwapSegments it(sh, pair, n_pairs);
-    SwapSegment sg;
     const int nh = static_cast<int>(cta) * BM;
     const uint32_t bar_own0 = smem_u32(&ctrl->full[0]), full_leader0 = map_to_cta(bar_own0, 0), empty0 = smem_u32(&ctrl->empty[0]);
     auto load_weights = [&](const CUtensorMap* mw, int w_row, int n_col, int kk, uint32_t sw, uint32_t bar) {
@@ -566,23 +488,22 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         tma_load_2d_pair(sw + 8192, mw, bar, n_col + 64, w_row + kk);
       }
     };
-    while (ok && it.next(sg)) {
-      const SwapTile ti = decode_swap_tile(sg.tile, ctrl, args.num_groups);
+    for (int t = pair; t < sh.total_tiles && ok; t += n_pairs, ++seq) {
+      const SwapTile ti = decode_swap_tile(t, ctrl, args.num_groups);
       if (lane == 0) trace_ev(args, seq, 0);
       const int half = ti.np >> 1, boxes = (half + kSwBox - 1) / kSwBox;
       const uint32_t bytes = 2 * (kW + static_cast<uint32_t>(ti.parts * boxes * (kSwBox * 128)));   // of both CTAs
       const int n_col = ti.n0 + nh, w_row = ti.g * args.b_group_rows + (kWMajor == MAJ_K ? n_col : 0);
       const int x_row = ti.row0 + static_cast<int>(cta) * half;
-      const int seg0 = sg.kb0 >= kb_per_seg ? 1 : 0;   // at most two segments
       // The first stages' weights are requested before the rows are waited for: they depend on nothing.
       int pre = 0;
       if (seq == 0) {
-        pre = min(stages, sg.kb1 - sg.kb0);
+        pre = min(stages, sh.kblocks);
         if (elect_one()) {
           for (int i = 0; i < pre; ++i) {
-            const int kb = sg.kb0 + i, seg = kb >= kb_per_seg ? 1 : 0;
+            const int seg = i >= kb_per_seg ? 1 : 0;   // at most two segments
             if (cta == 0) mbar_arrive_expect_tx(smem_u32(&ctrl->full[i]), bytes);
-            load_weights(seg ? &tmW1 : &tmW0, w_row, n_col, (kb - seg * kb_per_seg) * BK, smem_base + i * stage_bytes,
+            load_weights(seg ? &tmW1 : &tmW0, w_row, n_col, (i - seg * kb_per_seg) * BK, smem_base + i * stage_bytes,
                          map_to_cta(smem_u32(&ctrl->full[i]), 0));
           }
         }
@@ -607,9 +528,9 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         fence_proxy_async();   // generic-proxy peer stores -> async-proxy (TMA) reads
       }
       if (lane == 0) trace_ev(args, seq, 1);
-      const CUtensorMap *mw = seg0 ? &tmW1 : &tmW0, *mx = seg0 ? &tmX1 : &tmX0, *mxb = seg0 ? &tmXb1 : &tmXb0;
-      int kk = (sg.kb0 - seg0 * kb_per_seg) * BK;
-      for (int kb = sg.kb0; kb < sg.kb1; ++kb, kk += BK) {
+      const CUtensorMap *mw = &tmW0, *mx = &tmX0, *mxb = &tmXb0;
+      int kk = 0;
+      for (int kb = 0; kb < sh.kblocks; ++kb, kk += BK) {
         if (kb == kb_per_seg) {
           mw = &tmW1;
           mx = &tmX1;
@@ -640,7 +561,6 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (lane == 0) trace_ev(args, seq, 2);
-      ++seq;
     }
   } else if (warp == 1) {
     // ======================= MMA issuer (leader CTA only) =======================
@@ -649,10 +569,8 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
       const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
       int stage = 0, phase = 0, buf = 0, bphase = 0, seq = 0;
       bool ok = true;
-      SwapSegments it(sh, pair, n_pairs);
-      SwapSegment sg;
-      while (ok && it.next(sg)) {
-        const SwapTile ti = decode_swap_tile(sg.tile, ctrl, args.num_groups);
+      for (int t = pair; t < sh.total_tiles && ok; t += n_pairs, ++seq) {
+        const SwapTile ti = decode_swap_tile(t, ctrl, args.num_groups);
         const uint32_t idesc = make_idesc(PM, ti.np, args.fp16, kWMajor, MAJ_K);
         const uint32_t part_bytes = static_cast<uint32_t>((((ti.np >> 1) + kSwBox - 1) / kSwBox) * kSwBox) * 128;
         if (lane == 0) trace_ev(args, seq, 3);
@@ -665,7 +583,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
             ok = false;
           }
         }
-        for (int kb = sg.kb0; kb < sg.kb1 && ok; ++kb) {
+        for (int kb = 0; kb < sh.kblocks && ok; ++kb) {
           if (!mbar_wait_cluster(full0 + 8 * stage, phase, abort_word, limit)) {
             report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x35);
             ok = false;
@@ -673,9 +591,9 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
           }
           tc_fence_after();
           if (elect_one()) {
-            if (kb == sg.kb0) trace_ev(args, seq, 4);
+            if (kb == 0) trace_ev(args, seq, 4);
             const uint32_t at = static_cast<uint32_t>(stage) * stage_bytes;
-            const uint32_t acc = kb > sg.kb0 ? 1u : 0u;
+            const uint32_t acc = kb > 0 ? 1u : 0u;
 #pragma unroll
             for (int a = 0; a < (kWide ? 2 : 1); ++a) {
 #pragma unroll
@@ -690,7 +608,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
                               k > 0 ? 1u : acc);
             }
             umma_commit_pair(empty0 + 8 * stage);   // hand the stage back to both producers
-            if (kb == sg.kb1 - 1) {
+            if (kb == sh.kblocks - 1) {
               umma_commit_pair(smem_u32(&ctrl->acc_full[buf]));
               if (ti.parts > 1) umma_commit_pair(smem_u32(&ctrl->acc_full[b1]));
               trace_ev(args, seq, 5);
@@ -701,7 +619,6 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         }
         buf += ti.parts;
         if (buf >= sh.bufs) { buf -= sh.bufs; bphase ^= 1; }
-        ++seq;
       }
     }
   } else if (warp >= 2 + kEpiWarps) {
@@ -720,16 +637,9 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
     // outputs that a reduction over rows reads get zeros up to the next multiple of its 64-row step
     const bool zeros = kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU || ((kEpi == CCF_EPI_BIAS_ACT || kWide) && args.out1 != nullptr);
     SwapWork* const w = &ctrl->work[warp - 2];
-    {
-      const SwapSegments it(sh, pair, n_pairs);
-      if (lane == 0) {
-        w->t = it.t;
-        w->pos = it.pos;
-        w->end = it.end;
-      }
-      __syncwarp();
-    }
-    while (ok && swap_next(ctrl, w, pair, n_pairs, args.num_groups)) {
+    if (lane == 0) w->t = pair;
+    __syncwarp();
+    while (ok && swap_next(ctrl, w, n_pairs, args.num_groups)) {
       for (int p = 0; p < w->parts; ++p) {
         const int fbase = w->n0 + static_cast<int>(cta) * BM + q * 32, np = w->np;
         // two warps share a part's chunks; with an odd number they take turns in having one more
@@ -748,15 +658,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
           }
           tc_fence_after();
           if (p == 0 && warp == 2 && lane == 0) trace_ev(args, seq, 6);
-          bool finish = fbase < args.n;
-          if (finish && w->sharers > 1) {
-            const int share = (p * 2 + static_cast<int>(cta)) * kEpiWarps + warp - 2;
-            finish = swap_share<kWide>(args.split_ws + share * sh.share_floats, args.split_cnt + (w->tile - sh.dp_tiles) * (4 * kEpiWarps) + share,
-                                       w->first, w->sharers, pair - w->first, chunks, col, col + (sh.buf_cols >> 1), c0, lane,
-                                       (sh.width == 160 ? 4 : 2) * kEpiWarps * sh.share_floats, w->tile_start != 0);
-          }
-          if (!finish) release();
-          return finish;
+          return true;
         };
         if (fbase < args.n) {
           SwapPart pt;
@@ -767,8 +669,8 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
           pt.valid = min(np, w->tokens - p * np);
           pt.end = pt.valid + (zeros && p == w->parts - 1 ? w->zero_rows : 0);
           swap_epilogue<kEpi, kFp16>(args, pt, col, col + (sh.buf_cols >> 1), stage, fbase, lane, acquire, release);
-        } else {
-          acquire();
+        } else if (acquire()) {
+          release();
         }
         if (!ok) break;
         if (++buf == sh.bufs) { buf = 0; bphase ^= 1; }
@@ -802,10 +704,6 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
           for (int s = 0; s < args.world; ++s) red_release_sys_add(args.peer_done[s], 1);
         }
       }
-      // a launch that was given up may have left parts of sums uncounted
-      const int code = args.status != nullptr ? *reinterpret_cast<volatile int*>(args.status) & 0xff : 0;
-      if (args.split_cnt != nullptr && (code == CCF_ERR_MBAR_TIMEOUT || code == CCF_ERR_FLAG_TIMEOUT))
-        for (int i = 0; i < CCF_SPLIT_COUNTERS; ++i) args.split_cnt[i] = 0;
       args.sched[0] = 0;
       args.sched[1] = 0;
       args.sched[2] = 0;
@@ -861,20 +759,19 @@ int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGem
 
 }  // namespace ccf
 
-// The work of a launch of the swapped kernel, computed on the host with the kernel's own functions: for every CTA pair its segments
-// in order, out[9 i ...] = {pair, tile, first k-block, one past the last, first sharer, sharers, rows per stage of the launch, stages,
-// shared tiles begin at}. Host arrays in, nothing touches a device. Returns the number of segments (only the first `cap` are written).
+// The tiles of a launch of the swapped kernel, computed on the host with the kernel's own functions: for every CTA pair its tiles in
+// order, out[9 i ...] = {pair, tile, first k-block, one past the last, first pair that works on the tile, number of such pairs, rows
+// per stage of the launch, stages, number of tiles}. Host arrays in, nothing touches a device. Returns the number of records
+// (only the first `cap` are written).
 extern "C" int ccf_debug_swap_segments(const int* group_rows, int num_groups, int n, int k, int kseg, int wide, int n_pairs, int* out,
                                        int cap) {
   using namespace ccf;
   if (num_groups < 1 || num_groups > CCF_MAX_GROUPS) return -2;
-  static float ws;
   CcfGemmArgs a;
   memset(&a, 0, sizeof(a));
   a.n = n;
   a.k = k;
   a.kseg = kseg;
-  a.split_ws = &ws;
   int max_rows = 0, total = 0, tiles = 0, half = 0;
   for (int g = 0; g < num_groups; ++g) {
     max_rows = group_rows[g] > max_rows ? group_rows[g] : max_rows;
@@ -888,18 +785,12 @@ extern "C" int ccf_debug_swap_segments(const int* group_rows, int num_groups, in
     half = h > half ? h : half;
     tiles += mt;
   }
-  const SwapShape s = swap_shape(a, tiles, total, half, width, wide != 0, n_pairs, kSwPipeBytes, kSwMaxStages);
+  const SwapShape s = swap_shape(a, tiles, total, half, width, wide != 0, kSwPipeBytes, kSwMaxStages);
   int i = 0;
-  for (int p = 0; p < n_pairs; ++p) {
-    SwapSegments it(s, p, n_pairs);
-    SwapSegment g;
-    while (it.next(g)) {
-      int first = p, sharers = 1;
-      if (g.kb0 != 0 || g.kb1 != s.kblocks) it.contributors(g, p, first, sharers);
-      const int rec[9] = {p, g.tile, g.kb0, g.kb1, first, sharers, half, s.stages, s.dp_tiles};
+  for (int p = 0; p < n_pairs; ++p)
+    for (int t = p; t < s.total_tiles; t += n_pairs, ++i) {
+      const int rec[9] = {p, t, 0, s.kblocks, p, 1, half, s.stages, s.total_tiles};
       if (i < cap) memcpy(out + 9 * i, rec, sizeof(rec));
-      ++i;
     }
-  }
   return i;
 }

@@ -42,12 +42,6 @@ int combine_units(int n, bool swap) { return swap ? n / 32 : 2 * ((n + 255) / 25
 // Row-grouped launches of a call that expects at most small_rows rows per expert run on the swapped kernel. CCFUSER_TWO_CTA=0
 // keeps them on 128-row tiles (one-CTA kernel) for comparison.
 bool few_rows(const CcfLayer* L, long long rows_per_expert) { return rows_per_expert <= L->small_rows && L->two_cta; }
-void set_swap(CcfGemmLaunch& g, const CcfLayer* L, bool swap) {
-  g.few_rows = swap;
-  if (!swap) return;
-  g.args.split_ws = L->split_ws;
-  g.args.split_cnt = L->split_cnt;
-}
 
 // fields every launch of this layer shares
 CcfGemmLaunch base_launch(const CcfLayer* L) {
@@ -272,7 +266,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
       g.args.act = L->act;
     }
     set_dispatch(g, L, x, idx, gate_w, tokens, capacity, 0, nullptr);
-    set_swap(g, L, swap);
+    g.few_rows = swap;
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -288,7 +282,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     g.args.bias0 = L->b2;
     g.args.ld_out = d;
     set_combine(g, L, L->peer_comb, L->row_gate);
-    set_swap(g, L, swap);
+    g.few_rows = swap;
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
@@ -333,7 +327,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       g.args.act = L->act;
     }
     set_dispatch(g, L, dy, idx, gate_w, tokens, capacity, 1, G->dgate);
-    set_swap(g, L, swap);
+    g.few_rows = swap;
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -392,7 +386,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       set_b(g, L->w1, static_cast<long long>(e_loc) * f, d, kMajMN);
     }
     set_combine(g, L, L->peer_gcomb, nullptr);
-    set_swap(g, L, swap);
+    g.few_rows = swap;
     return issue(g, dry, stream);
   };
   if (sgd && (rc = dgrad1())) return rc;

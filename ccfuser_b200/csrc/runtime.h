@@ -48,8 +48,6 @@ struct CcfLayer {
   int* sched;       // scheduler words of the device's workspace (8 ints)
   int* status;      // status words of the device's workspace (2 ints)
   int* epoch_dev;   // device-side call epoch (used when a call passes epoch < 0)
-  float* split_ws;  // the device's workspace for sums shared by CTA pairs, and its counters (gemm_args.h)
-  int* split_cnt;
   // the same buffers on every rank of the group, as mapped into this process
   void* peer_xrecv[CCF_MAX_RANKS];
   void* peer_comb[CCF_MAX_RANKS];

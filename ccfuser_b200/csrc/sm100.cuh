@@ -285,11 +285,6 @@ __device__ __forceinline__ int ld_acquire_sys(const int* addr) {
   asm volatile("ld.acquire.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ int ld_acquire_gpu(const int* addr) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
-  return v;
-}
 __device__ __forceinline__ int ld_relaxed_sys(const int* addr) {
   int v;
   asm volatile("ld.relaxed.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");

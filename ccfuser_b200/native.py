@@ -14,7 +14,6 @@ import torch
 
 MAX_RANKS = 8
 MAX_GROUPS = 256
-SPLIT_WS_FLOATS, SPLIT_COUNTERS = 2 * 74 * 32 * 3072, 2 * 74 * 32   # csrc/gemm_args.h: workspace of shared sums
 ROUTE_CLUSTER_SLOTS = 65536   # csrc/route.h: slots that the one-kernel routing + plan holds
 
 EPI_STORE, EPI_BIAS_ACT, EPI_SWIGLU, EPI_COMBINE, EPI_DACT, EPI_DSWIGLU = range(6)
@@ -48,7 +47,7 @@ class GemmArgs(C.Structure):
         ("out0", _vp), ("out1", _vp), ("out2", _vp), ("bias0", _vp), ("bias1", _vp), ("aux0", _vp), ("aux1", _vp),
         ("row_src", _vp), ("row_gate", _vp),
         ("peer_comb", _vp * MAX_RANKS), ("peer_done", _vp * MAX_RANKS),
-        ("sched", _vp), ("status", _vp), ("split_ws", _vp), ("split_cnt", _vp), ("trace", _vp),
+        ("sched", _vp), ("status", _vp), ("trace", _vp),
         ("wait_limit_ns", C.c_ulonglong), ("ld_out", C.c_longlong),
         ("n", C.c_int), ("k", C.c_int), ("num_groups", C.c_int), ("m_per_group", C.c_int), ("kseg", C.c_int),
         ("b_group_rows", C.c_int), ("act", C.c_int), ("fp16", C.c_int), ("out_fp32", C.c_int), ("world", C.c_int),
@@ -107,7 +106,7 @@ class Layer(C.Structure):
         ("group_rows", _vp), ("sent_rows", _vp), ("table_copy", _vp), ("raw_order", _vp),
         ("grecv", _vp), ("gcomb", _vp), ("row_src", _vp), ("row_gate", _vp), ("tile_flags", _vp), ("done", _vp),
         ("done_cum", _vp), ("block_hist", _vp), ("block_off", _vp), ("ticket", _vp), ("sched", _vp), ("status", _vp),
-        ("epoch_dev", _vp), ("split_ws", _vp), ("split_cnt", _vp),
+        ("epoch_dev", _vp),
         ("peer_xrecv", _vp * MAX_RANKS), ("peer_comb", _vp * MAX_RANKS), ("peer_grecv", _vp * MAX_RANKS),
         ("peer_gcomb", _vp * MAX_RANKS), ("peer_row_src", _vp * MAX_RANKS), ("peer_row_gate", _vp * MAX_RANKS),
         ("peer_tile_flags", _vp * MAX_RANKS), ("peer_cnt_table", _vp * MAX_RANKS), ("peer_cnt_flag", _vp * MAX_RANKS),

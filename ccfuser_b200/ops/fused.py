@@ -91,7 +91,6 @@ class CommContext:
         self.epoch_dev = torch.zeros(1, dtype=torch.int32, device=device)
         self.device_epoch = bool(env_flag("DEVICE_EPOCH", 0))
         self.ws = G.Workspace.get(device)
-        self.ws.split()         # allocated with the other buffers, not inside a first call that may be captured
         self.users = 0          # fused layers currently attached (FusedMoE.__init__ / close)
         # scratch of the routing kernels
         s_max = max_slots
@@ -393,7 +392,6 @@ class FusedMoE:
                      "ticket", "epoch_dev"):
             setattr(L, name, getattr(cc, name).data_ptr())
         L.sched, L.status = cc.ws.sched.data_ptr(), cc.ws.status.data_ptr()
-        L.split_ws, L.split_cnt = cc.ws.split()
         peers = {"peer_xrecv": self.buf.peer_ptrs(self.off_xrecv), "peer_comb": self.buf.peer_ptrs(self.off_comb),
                  "peer_grecv": cc.peer("grecv"), "peer_gcomb": cc.peer("gcomb"), "peer_row_src": cc.peer("row_src"),
                  "peer_row_gate": cc.peer("row_gate"), "peer_tile_flags": cc.peer("tile_flags"),

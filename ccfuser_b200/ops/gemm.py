@@ -27,7 +27,6 @@ class Workspace:
         self.status = torch.zeros(2, dtype=torch.int32, device=device)  # [first hard error, overflow count]
         self.status_addr = self.status.data_ptr()
         self._last_stream, self._last_raw = None, None
-        self._split = None
         self._on_gpu = self.sched.device.type == "cuda"
         self._device_index = self.sched.device.index if self._on_gpu else -1
 
@@ -53,14 +52,6 @@ class Workspace:
     def status_of(cls, tensor) -> int:
         """Address of the status word of a CUDA tensor's device."""
         return cls.of(tensor).status_addr
-
-    def split(self):
-        """Addresses of the workspace for sums that CTA pairs share (58 MB) and of its arrival counters."""
-        if self._split is None:
-            dev = self.sched.device
-            self._split = (torch.empty(N.SPLIT_WS_FLOATS, dtype=torch.float32, device=dev),
-                           torch.zeros(N.SPLIT_COUNTERS, dtype=torch.int32, device=dev))
-        return self._split[0].data_ptr(), self._split[1].data_ptr()
 
     def enter(self):
         """Called by every launcher with the stream it is about to launch on. The kernels of one device share this
@@ -203,8 +194,6 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     # the kernels for few rows per group: weights on the M side (csrc/gemm_swap.cu); k-grouped, where output rows come in 256s,
     # csrc/gemm_wgrad.cu
     L.few_rows = int(bool(few_rows) and not (kgroup and m_per_group % 256 != 0))
-    if few_rows and not kgroup:
-        g.split_ws, g.split_cnt = ws.split()
     if sgd is not None:     # (lr, weight decay): EPI_STORE updates out0 in place instead of storing the product
         g.sgd_lr, g.sgd_wd = float(sgd[0]), float(sgd[1])
     if dispatch is not None:
