@@ -35,9 +35,8 @@ struct Dry {
   int n;
 };
 
-// completion-counter increments per row of a COMBINE GEMM with n columns: two epilogue warps per 256-column tile report it, in the
-// swapped kernel one per 32 columns
-int combine_units(int n, bool swap) { return swap ? n / 32 : 2 * ((n + 255) / 256); }
+// completion-counter increments per row of a COMBINE GEMM with n columns: one per 32 columns, whatever kernel stores them
+int combine_units(int n) { return n / 32; }
 
 // Row-grouped launches of a call that expects at most small_rows rows per expert run on the swapped kernel. CCFUSER_TWO_CTA=0
 // keeps them on 128-row tiles (one-CTA kernel) for comparison.
@@ -144,7 +143,7 @@ int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
 
 // Wait for the owners and sum the k slots of each token. With G (backward) and a router in the call, the sum also carries
 // the gradient through the gate weights.
-int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, bool swap, const CcfLayerGrads* G, const int* idx,
+int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, const CcfLayerGrads* G, const int* idx,
                     const float* gate_w, Dry* dry, void* stream) {
   if (dry != nullptr) return 0;
   CcfReduceArgs r;
@@ -166,7 +165,7 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
     r.zero_words = L->tile_flags;
     r.zero_count = L->max_rows / 128 + 1;
   } else {
-    const int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model, swap), L->world,
+    const int rc = ccf_combine_wait(L->done, L->done_cum, L->sent_rows, combine_units(L->d_model), L->world,
                                     L->wait_limit_ns, L->status, stream);
     if (rc) return rc;
   }
@@ -286,7 +285,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
-  return wait_and_reduce(L, L->comb, y, tokens, swap, nullptr, nullptr, nullptr, dry, stream);
+  return wait_and_reduce(L, L->comb, y, tokens, nullptr, nullptr, nullptr, dry, stream);
 }
 
 int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G, int tokens,
@@ -408,7 +407,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       return rc;
   }
   if (!sgd && (rc = dgrad1())) return rc;
-  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, swap, G, idx, gate_w, dry, stream))) return rc;
+  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, G, idx, gate_w, dry, stream))) return rc;
   if (G->router_dw != nullptr && dry == nullptr)
     rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d,
                        L->e_total, L->top_k, L->fp16, stream);

@@ -572,7 +572,7 @@ class FusedMoE:
 
     def stage_reduce(self, tokens: int, out: torch.Tensor):
         """Wait until every owner has delivered this rank's rows, then sum the k slots of each token."""
-        self._wait_and_reduce(self.comb, tokens, G.combine_units(self.cfg.d_model, self._call_few_rows), out)
+        self._wait_and_reduce(self.comb, tokens, G.combine_units(self.cfg.d_model), out)
 
 
 class GraphedForward:
@@ -845,7 +845,7 @@ class _FusedMoEFn(torch.autograd.Function):
         if sgd is None:
             dgrad1()
         dx = torch.empty(t, d, dtype=dy.dtype, device=dy.device)
-        fm._wait_and_reduce(cc.gcomb, t, G.combine_units(d, few), dx)
+        fm._wait_and_reduce(cc.gcomb, t, G.combine_units(d), dx)
         if fm.check_every_call:
             cc.check_status("fused MoE backward")
         return dx, dgate.view(t, cfg.top_k), None, dw1, db1, dwg, dbg, dw2, db2, None

@@ -218,10 +218,10 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
 
 
 def combine_units(n: int, few_rows: bool = False) -> int:
-    """Completion-counter increments per output row of a COMBINE GEMM with n columns: every 256-column tile is stored by two
-    epilogue warps per row quarter (one per half of its columns), and each of them reports its rows; in the swapped kernel
-    a warp stores 32 columns of a row."""
-    return n // 32 if few_rows else 2 * ((n + 255) // 256)
+    """Completion-counter increments per output row of a COMBINE GEMM with n columns: one per 32 columns. The same in every
+    kernel (``few_rows`` changes nothing), because the rank that stores a row and the rank that waits for it choose their
+    kernels separately."""
+    return n // 32
 
 
 def single_group(rows: int, device):
