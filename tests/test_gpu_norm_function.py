@@ -68,3 +68,29 @@ def test_transforms_are_refused():
     import torch.autograd.forward_ad as fwd
     with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
         layer_norm(fwd.make_dual(x, torch.ones_like(x)), (64,), w, None)
+
+
+@pytest.mark.parametrize("bias", [True, False])
+def test_a_traced_graph_replays_the_kernels(bias):
+    """torch.jit.trace records the operation, not only the allocation of its output: on another input the graph gives what the module
+    gives, forward and backward, to the bit."""
+    from ccfuser_b200.ops.norm import LayerNorm
+    torch.manual_seed(11)
+    norm = LayerNorm(768, bias=bias, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        for p in norm.parameters():
+            p.normal_()
+    x, x2, gy = (torch.randn(5, 31, 768, device="cuda").bfloat16() for _ in range(3))
+    traced = torch.jit.trace(norm, (x,), check_trace=False)
+
+    def run(f):
+        v = x2.clone().requires_grad_(True)
+        norm.zero_grad()
+        # what an allocation finds is not an earlier result
+        junk = [torch.full_like(x, 3.0) for _ in range(8)]
+        del junk
+        y = f(v)
+        y.backward(gy)
+        return [y.detach(), v.grad] + [p.grad.clone() for p in norm.parameters()]
+    for a, b in zip(run(traced), run(norm)):
+        assert torch.equal(a, b)
