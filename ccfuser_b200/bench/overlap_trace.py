@@ -46,7 +46,6 @@ def analyze(trace: torch.Tensor, kblocks: int, leaders_only: bool = True) -> Dic
 
 def main():
     from .. import MoEConfig, MoELayer
-    from ..ops import gemm as G
     from .kernel_bench import synthetic_routing
     d, f = int(os.environ.get("D", 2048)), int(os.environ.get("F", 8192))
     tokens, e_loc, act = int(os.environ.get("TOKENS", 16384)), int(os.environ.get("E_LOC", 8)), os.environ.get("ACT", "gelu")
@@ -75,7 +74,7 @@ def main():
     fwd(t1)
     torch.cuda.synchronize()
     t = t1.cpu().double()
-    pair = fm._call_few_rows or bool(G.TWO_CTA_DEFAULT)
+    pair = fm._call_pair
     lead = t[0::2] if pair else t     # in the CTA-pair kernel the leader CTAs record the MMA events
     start, disp = lead[:, nt - 1, 0], lead[:, nt - 1, 1]
     first_ops, first_commit, first_epi = lead[:, 0, 4], lead[:, 0, 5], lead[:, 0, 7]

@@ -38,9 +38,35 @@ struct Dry {
 // completion-counter increments per row of a COMBINE GEMM with n columns: one per 32 columns, whatever kernel stores them
 int combine_units(int n) { return n / 32; }
 
-// Row-grouped launches of a call that expects at most small_rows rows per expert run on the swapped kernel. CCFUSER_TWO_CTA=0
-// keeps them on 128-row tiles (one-CTA kernel) for comparison.
-bool few_rows(const CcfLayer* L, long long rows_per_expert) { return rows_per_expert <= L->small_rows && L->two_cta; }
+// Kernel of a row-grouped launch (row_kernel below)
+struct RowKernel {
+  int few_rows, two_cta, a_rows, bn;
+};
+
+// Bound on the rows of any expert of a single-rank call (its capacity, at most all slots of the call; other ranks may bring
+// any number of rows), rounded up to a pipeline geometry of the one-CTA kernel: 32, 64, or 0 for no bound.
+int row_bound(int capacity, int world) { return world != 1 || capacity > 64 ? 0 : capacity > 32 ? 64 : 32; }
+
+// The kernel of a row-grouped launch of a call that expects `rows` rows for each of `experts` experts of this rank:
+// at most small_rows: weights on the M side (gemm_swap.cu); more: CTA pairs (gemm2.cu). Without CTA pairs (CCFUSER_TWO_CTA=0) the
+// one-CTA kernel, with the pipeline that the capacity allows, and with 128-column tiles for a second projection whose 256-column
+// tiles would leave most of the 148 SMs without one. Every rank of a group may come to another choice: what it counts for
+// the others does not depend on the kernel (combine_units).
+RowKernel row_kernel(int epi, int b_major, long long rows, int experts, int n, int capacity, int world, int small_rows, int two_cta) {
+  if (rows <= small_rows && two_cta) return {1, 0, 0, 0};
+  if (two_cta) return {0, 1, 0, 0};
+  const long long tiles = experts * (rows > 128 ? (rows + 127) / 128 : 1) * ((n + 255) / 256);
+  return {0, 0, row_bound(capacity, world), epi == CCF_EPI_COMBINE && b_major == kMajK && tiles < 148 ? 128 : 0};
+}
+
+void set_row_kernel(CcfGemmLaunch& g, const CcfLayer* L, int tokens, int capacity) {
+  const long long rows = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
+  const RowKernel r = row_kernel(g.epi, g.b_major, rows, L->e_loc, g.args.n, capacity, L->world, L->small_rows, L->two_cta);
+  g.few_rows = r.few_rows;
+  g.two_cta = r.two_cta;
+  g.args.a_rows = r.a_rows;
+  g.args.bn = r.bn;
+}
 
 // fields every launch of this layer shares
 CcfGemmLaunch base_launch(const CcfLayer* L) {
@@ -205,8 +231,6 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
                  int save_pre, int epoch, void* stream, Dry* dry) {
   const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
   int rc = 0;
-  const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
-  const bool swap = few_rows(L, rows_per_expert);
   if (dry == nullptr) {
     if (L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
     // 1. positions, kept counts, destination order of this rank's slots; count exchange with all ranks + row layout
@@ -265,7 +289,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
       g.args.act = L->act;
     }
     set_dispatch(g, L, x, idx, gate_w, tokens, capacity, 0, nullptr);
-    g.few_rows = swap;
+    set_row_kernel(g, L, tokens, capacity);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -281,7 +305,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     g.args.bias0 = L->b2;
     g.args.ld_out = d;
     set_combine(g, L, L->peer_comb, L->row_gate);
-    g.few_rows = swap;
+    set_row_kernel(g, L, tokens, capacity);
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
@@ -299,7 +323,6 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   // 553 against 467 at 16 x 1024.
   const int wgrad_few = rows_per_expert <= 512 && L->two_cta;
   const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
-  const bool swap = few_rows(L, rows_per_expert);
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
   // GEMM. w2 may be at any group size (dgrad-2 above it is its last reader). w1 / wg only on a single rank: dgrad-1 reads
   // them and, with peers, has to stay the last owner-side kernel of the pass.
@@ -326,7 +349,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       g.args.act = L->act;
     }
     set_dispatch(g, L, dy, idx, gate_w, tokens, capacity, 1, G->dgate);
-    g.few_rows = swap;
+    set_row_kernel(g, L, tokens, capacity);
     if ((rc = issue(g, dry, stream))) return rc;
     if ((rc = zero_tile_flags(L, dry, stream))) return rc;
   }
@@ -385,7 +408,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       set_b(g, L->w1, static_cast<long long>(e_loc) * f, d, kMajMN);
     }
     set_combine(g, L, L->peer_gcomb, nullptr);
-    g.few_rows = swap;
+    set_row_kernel(g, L, tokens, capacity);
     return issue(g, dry, stream);
   };
   if (sgd && (rc = dgrad1())) return rc;
@@ -417,6 +440,16 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
 }  // namespace
 
 extern "C" {
+
+// The rule of row_kernel for a caller that issues the launches itself: out = {few_rows, two_cta, a_rows, bn}
+int ccf_row_kernel(int epi, int b_major, int rows, int experts, int n, int capacity, int world, int small_rows, int two_cta, int* out) {
+  const RowKernel r = row_kernel(epi, b_major, rows, experts, n, capacity, world, small_rows, two_cta);
+  out[0] = r.few_rows;
+  out[1] = r.two_cta;
+  out[2] = r.a_rows;
+  out[3] = r.bn;
+  return 0;
+}
 
 int ccf_sizeof_layer() { return static_cast<int>(sizeof(CcfLayer)); }
 int ccf_sizeof_layer_grads() { return static_cast<int>(sizeof(CcfLayerGrads)); }

@@ -70,7 +70,7 @@ struct CcfLayer {
   int device;       // CUDA device (-1: leave the calling thread's device alone)
   int pad0;
   int comm_warps;   // 1: dedicated dispatch warps carry the row push, 0: the epilogue warps do
-  int small_rows;   // calls that expect at most this many rows per expert use the kernel for few rows (gemm_swap.cu)
+  int small_rows;   // calls that expect at most this many rows per expert use a kernel for few rows (row_kernel in runtime.cu)
 };
 
 // Per-call tensors of the backward pass (all allocated by the caller; null where the layer has no such parameter).

@@ -224,6 +224,7 @@ def _declare(lib):
         "ccf_router_dw": ([p, p, p, p, p, p, i, i, i, i, i, p], i),
         "ccf_layer_forward": ([C.POINTER(Layer), p, p, p, p, i, i, i, i, p, p, i, p], i),
         "ccf_layer_backward": ([C.POINTER(Layer), p, p, p, C.POINTER(LayerGrads), i, i, p, p, i, p], i),
+        "ccf_row_kernel": ([i, i, i, i, i, i, i, i, i, p], i),
         "ccf_flag_barrier": ([C.POINTER(BarrierArgs), p], i),
         "ccf_plan": ([C.POINTER(PlanArgs), p], i),
         "ccf_plan_dev_epoch": ([C.POINTER(PlanArgs), p, p], i),
@@ -270,10 +271,10 @@ class _DeclaredOnly:
 class LaunchRecorder:
     """Stands in for the library and records every launcher call instead of running it, so the host side of the fused
     path (which launches, in which order, with which argument blocks) can be tested on a machine without a GPU.
-    Size queries and error strings go to the real library; everything else returns 0. Structures passed with
+    Size queries, error strings and the choice of kernels go to the real library; everything else returns 0. Structures passed with
     ``ctypes.byref`` are stored as their raw bytes (``GemmLaunch.from_buffer_copy`` turns them back into fields)."""
 
-    _PASS_THROUGH = ("ccf_sizeof_", "ccf_error_string", "ccf_gemm_smem_bytes", "ccf_symm_handle_bytes")
+    _PASS_THROUGH = ("ccf_sizeof_", "ccf_error_string", "ccf_gemm_smem_bytes", "ccf_symm_handle_bytes", "ccf_row_kernel")
 
     def __init__(self, real):
         self._real = real

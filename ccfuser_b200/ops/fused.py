@@ -271,7 +271,8 @@ class FusedMoE:
         self._desc = None
         self._desc_key = None
         self.sgd = None         # (lr, weight decay): expert weights are updated by the weight-gradient GEMMs (fuse_sgd)
-        self._call_few_rows = False     # kernel choice of the current call's row-grouped launches (_few_rows)
+        self._call_tokens = 0           # tokens of the current call (stage_dispatch_gemm1)
+        self._call_pair = False         # whether its first GEMM ran on CTA pairs
         self._owed = None       # weak reference to the autograd node whose backward still needs this layer's buffers
 
     # ------------------------------------------------------------------------------------------
@@ -484,11 +485,11 @@ class FusedMoE:
         a.total_index = self.max_rows // TILE  # last element of tile_flags: all rows arrived on that rank
         return a
 
-    def _few_rows(self, tokens: int) -> bool:
-        """Kernel choice of the row-grouped launches of a call with ``tokens`` tokens per rank: weights on the M side
-        (csrc/gemm_swap.cu) when an expert expects at most ``CCFUSER_SMALL_ROWS`` rows."""
-        rows = tokens * self.cfg.top_k * self.world // max(1, self.cfg.num_experts)
-        return rows <= G.SMALL_ROWS_DEFAULT and bool(G.TWO_CTA_DEFAULT)
+    def _row_kernel(self, tokens: int, epi: int, b_major: int, n: int) -> dict:
+        """Kernel choice of a row-grouped launch of a call with ``tokens`` tokens on this rank (ops/gemm.py: row_kernel)."""
+        cfg = self.cfg
+        rows = tokens * cfg.top_k * self.world // max(1, cfg.num_experts)
+        return G.row_kernel(epi, b_major, rows, cfg.experts_per_rank, n, cfg.capacity(tokens), self.world)
 
     def _combine_kw(self, peer_comb, row_gate):
         ctx = self.ctx
@@ -549,8 +550,8 @@ class FusedMoE:
         common = dict(group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, tile_flags=cc.tile_flags,
                       dispatch=disp, n_comm_ctas=cc.n_comm, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace,
                       total_index=self.max_rows // TILE, local_begin=self.local_begin, local_rows=self.local_rows,
-                      few_rows=self._few_rows(t))
-        self._call_few_rows = common["few_rows"]
+                      **self._row_kernel(t, N.EPI_SWIGLU if cfg.activation == "swiglu" else N.EPI_BIAS_ACT, N.MAJ_K, f))
+        self._call_tokens, self._call_pair = t, common["few_rows"] or common["two_cta"]
         if cfg.activation == "swiglu":
             G.launch(a0=self.xrecv, b0=w1.view(e_loc * f, d), b1=wg.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_K,
                      epi=N.EPI_SWIGLU, n=f, k=d, b_group_rows=f, out0=self.h_act, out1=self.h_pre if save_pre else None,
@@ -567,7 +568,8 @@ class FusedMoE:
         d, f, e_loc = cfg.d_model, cfg.d_ffn, cfg.experts_per_rank
         G.launch(a0=self.h_act, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_COMBINE, n=d, k=f,
                  group_base=self.group_base, group_rows=self.group_rows, num_groups=e_loc, b_group_rows=d, bias0=b2,
-                 ld_out=d, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace, few_rows=self._call_few_rows,
+                 ld_out=d, wait_ns=cc.wait_ns, workspace=cc.ws, trace=trace,
+                 **self._row_kernel(self._call_tokens, N.EPI_COMBINE, N.MAJ_K, d),
                  **self._combine_kw(self.buf.peer_ptrs(self.off_comb), cc.row_gate))
 
     def stage_reduce(self, tokens: int, out: torch.Tensor):
@@ -784,17 +786,17 @@ class _FusedMoEFn(torch.autograd.Function):
                       workspace=cc.ws)
         dh = torch.empty(fm.max_rows, f, dtype=cfg.dtype, device=dy.device)
         dh2 = torch.empty_like(dh) if swiglu else None
-        few = fm._few_rows(t)
+        rk = fm._row_kernel(t, N.EPI_DSWIGLU if swiglu else N.EPI_DACT, N.MAJ_MN, f)
         if swiglu:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DSWIGLU, n=f, k=d,
                      b_group_rows=d, out0=dh, out1=dh2, aux0=fm.h_pre, aux1=fm.h_pre2, tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, few_rows=few, **common)
+                     local_rows=fm.local_rows, **rk, **common)
         else:
             G.launch(a0=cc.grecv, b0=w2.view(e_loc * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DACT, n=f, k=d,
                      b_group_rows=d, out0=dh, aux0=fm.h_pre, act=N.ACT_CODE[cfg.activation], tile_flags=cc.tile_flags,
                      dispatch=disp, n_comm_ctas=cc.n_comm, total_index=fm.max_rows // TILE, local_begin=fm.local_begin,
-                     local_rows=fm.local_rows, few_rows=few, **common)
+                     local_rows=fm.local_rows, **rk, **common)
         cc.tile_flags.zero_()
         # 3. wgrad-2: dW2[e] = (g dy)^T h_act   [d, f]
         # With few rows per expert the reduction is only a handful of k-blocks, and moving the result decides.
@@ -816,14 +818,14 @@ class _FusedMoEFn(torch.autograd.Function):
         db2 = colsum(cc.grecv, d) if has_b2 else None
         # 5 (defined here, issued below). dgrad-1 + combine: dx rows go back to the ranks the tokens came from
         def dgrad1():
-            ck = fm._combine_kw(cc.peer("gcomb"), None)
+            ck = dict(fm._combine_kw(cc.peer("gcomb"), None), **fm._row_kernel(t, N.EPI_COMBINE, N.MAJ_MN, d))
             if swiglu:
                 G.launch(a0=dh, a1=dh2, b0=wg.view(e_loc * f, d), b1=w1.view(e_loc * f, d), a_major=N.MAJ_K,
-                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d, few_rows=few,
+                         b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f, kseg=2, b_group_rows=f, ld_out=d,
                          **common, **ck)
             else:
                 G.launch(a0=dh, b0=w1.view(e_loc * f, d), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_COMBINE, n=d, k=f,
-                         b_group_rows=f, ld_out=d, few_rows=few, **common, **ck)
+                         b_group_rows=f, ld_out=d, **common, **ck)
 
         if sgd is not None:
             dgrad1()            # reads w1 / wg before the weight-gradient GEMMs below overwrite them

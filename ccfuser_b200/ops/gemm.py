@@ -138,8 +138,8 @@ TWO_CTA_DEFAULT = bool(int(__import__('os').environ.get('CCFUSER_TWO_CTA', '1'))
 # 1: the two dedicated dispatch warps of every CTA push the rows (next to the MMA and epilogue warps); 0: the epilogue
 # warps push them before their first tile
 COMM_WARPS_DEFAULT = int(__import__('os').environ.get('CCFUSER_COMM_WARPS', '1'))
-# the row-grouped launches of calls that expect at most this many rows per expert run on the kernel with the weights on the M
-# side (csrc/gemm_swap.cu), whose tiles are as wide as an expert has rows; with CCFUSER_TWO_CTA=0 on 128-row tiles
+# the row-grouped launches of calls that expect at most this many rows per expert run on a kernel for few rows (row_kernel in
+# csrc/runtime.cu)
 SMALL_ROWS_DEFAULT = int(__import__('os').environ.get('CCFUSER_SMALL_ROWS', '320'))
 
 
@@ -215,6 +215,14 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     N.check(lib.ccf_gemm_launch(C.byref(L), N.stream_ptr()), "ccf_gemm_launch")
     N.count(1)
     return ws
+
+
+def row_kernel(epi: int, b_major: int, rows: int, experts: int, n: int, capacity: int, world: int) -> dict:
+    """Arguments of ``launch`` that choose the kernel of a row-grouped launch, by the rule of csrc/runtime.cu (row_kernel): ``rows``
+    rows expected for each of this rank's ``experts`` experts, ``capacity`` rows at most from one rank."""
+    out = (C.c_int * 4)()
+    N.load().ccf_row_kernel(epi, b_major, rows, experts, n, capacity, world, SMALL_ROWS_DEFAULT, int(TWO_CTA_DEFAULT), C.addressof(out))
+    return dict(few_rows=bool(out[0]), two_cta=bool(out[1]), a_rows=out[2], bn=out[3])
 
 
 def combine_units(n: int, few_rows: bool = False) -> int:
