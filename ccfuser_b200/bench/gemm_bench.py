@@ -159,13 +159,12 @@ def main():
         report("dgrad2_plain_store", 2 * r * d * f, gemm(
             a0=y, b0=w2.view(e * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, k=d,
             group_base=gb, group_rows=gr, num_groups=e, b_group_rows=d, out0=h), kblocks=(d + 63) // 64)
-    # few rows per expert (many experts on one GPU): the one-CTA kernel, as the layer chooses there
-    wgrad_few = rows_per <= 512    # the layer's rule
+    # weight gradients on the kernel that the layer chooses for this number of rows
     if "wgrad" in cases:
         dw = torch.empty(e, d, f, device=dev, dtype=torch.bfloat16)
         report("wgrad2", 2 * r * d * f, gemm(
             a0=y, b0=h, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, kgroup=True, m_per_group=d,
-            group_base=gb, group_rows=gr, num_groups=e, out0=dw, ld_out=f, few_rows=wgrad_few), kblocks=(rows_per + 63) // 64)
+            group_base=gb, group_rows=gr, num_groups=e, out0=dw, ld_out=f, few_rows=G.wgrad_few(rows_per, False)), kblocks=(rows_per + 63) // 64)
         del dw
     if "wgrad_sgd" in cases:
         # the same product with the SGD step in its epilogue: w2 is read and rewritten in place, no gradient is stored
@@ -173,7 +172,7 @@ def main():
         h.normal_()
         report("wgrad2_sgd_in_place", 2 * r * d * f, gemm(
             a0=y, b0=h, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, kgroup=True, m_per_group=d,
-            group_base=gb, group_rows=gr, num_groups=e, out0=w2, ld_out=f, few_rows=wgrad_few, sgd=(1e-6, 0.0)),
+            group_base=gb, group_rows=gr, num_groups=e, out0=w2, ld_out=f, few_rows=G.wgrad_few(rows_per, True), sgd=(1e-6, 0.0)),
             kblocks=(rows_per + 63) // 64)
     sampler.stop()
     if args.out:

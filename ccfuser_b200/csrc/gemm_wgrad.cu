@@ -12,8 +12,8 @@
 //
 // Measured, one-CTA / pair / this kernel, cold operands, us: 64 groups of 256 rows, 2048 x 8192: 697 / 670 / 635 plain and 1258 / 1214 /
 // 811 in place (4.3 GB read and written: 5.3 TB/s); 64 x 128 rows: 764 / 709 / 423 and 1167 / 1161 / 836; 16 x 192 rows, 768 x 3072:
-// 45 / 44 / 34 and 68 / 67 / 39; 16 x 512 rows, 2048 x 8192: 277 / 239 / 246 and 340 / 355 / 309. From some 600 rows on the main loop
-// decides and the pair kernel's deeper ring wins: 16 x 1024 rows 478 / 417 / 512 and 562 / 467 / 553.
+// 45 / 44 / 34 and 68 / 67 / 39; 16 x 512 rows, 2048 x 8192: 277 / 239 / 246 and 340 / 355 / 309. With more rows the main loop
+// decides and the pair kernel's deeper ring wins: 16 x 1024 rows 478 / 417 / 512 and 562 / 467 / 553 (wgrad_few in runtime.cu).
 //
 // Everything else is as in gemm2.cu: CTA pairs, MN-major operands, two accumulators. All waits are bounded; no TMA load uses cluster
 // multicast.

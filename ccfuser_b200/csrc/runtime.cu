@@ -68,6 +68,15 @@ void set_row_kernel(CcfGemmLaunch& g, const CcfLayer* L, int tokens, int capacit
   g.args.bn = r.bn;
 }
 
+// Whether a weight-gradient launch of a call that expects `rows` rows per expert runs on gemm_wgrad.cu, which moves its result by TMA,
+// or on the pair kernel: with few rows the reduction is only a handful of k-blocks, and moving the weights decides. In place the
+// weights are read as well as written, and the line lies higher. gemm_wgrad.cu against pair kernel, cold, us:
+//   plain     64 x 256 rows, 2048 x 8192: 646 / 702, 64 x 384: 873 / 823; 64 x 256, 1024 x 4096: 177 / 178, 64 x 512: 288 / 233.
+//             Whole training passes, 300 rows: 64 experts of 2048 x 8192 4957 / 5139, of 1024 x 4096 1350 / 1350; 400 rows: 6086 / 6145
+//             and 1774 / 1678; 16 experts of 1024 x 4096, 400 rows: 517 / 501
+//   in place  64 x 256 rows, 2048 x 8192: 811 / 1214, 16 x 512: 309 / 355, 16 x 1024: 553 / 467
+bool wgrad_few(long long rows, bool in_place, int two_cta) { return two_cta && rows <= (in_place ? 512 : 384); }
+
 // fields every launch of this layer shares
 CcfGemmLaunch base_launch(const CcfLayer* L) {
   CcfGemmLaunch g;
@@ -318,10 +327,6 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   int rc = 0;
   if (dry == nullptr && L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
-  // With few rows per expert the weight-gradient reduction is only a handful of k-blocks, and moving the result decides.
-  // In-place launches, 2048 x 8192: 811 us against 1214 on the pair kernel at 64 x 256 rows, 309 against 355 at 16 x 512,
-  // 553 against 467 at 16 x 1024.
-  const int wgrad_few = rows_per_expert <= 512 && L->two_cta;
   const int rows_hint = static_cast<int>(rows_per_expert > 0 ? rows_per_expert : 1);
   // In-place SGD (sgd_lr != 0), matrix by matrix: a weight whose gradient pointer is null is updated by its weight-gradient
   // GEMM. w2 may be at any group size (dgrad-2 above it is its last reader). w1 / wg only on a single rank: dgrad-1 reads
@@ -366,7 +371,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     g.args.sgd_lr = sgd2 ? G->sgd_lr : 0.f;
     g.args.sgd_wd = sgd2 ? G->sgd_wd : 0.f;
     g.args.ld_out = f;
-    g.few_rows = wgrad_few;
+    g.few_rows = wgrad_few(rows_per_expert, g.args.sgd_lr != 0.f, L->two_cta);
     if ((rc = issue(g, dry, stream))) return rc;
   }
   if (G->db2 != nullptr && dry == nullptr) {
@@ -385,7 +390,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     g.args.sgd_lr = sgd ? G->sgd_lr : 0.f;
     g.args.sgd_wd = sgd ? G->sgd_wd : 0.f;
     g.args.ld_out = d;
-    g.few_rows = wgrad_few;
+    g.few_rows = wgrad_few(rows_per_expert, g.args.sgd_lr != 0.f, L->two_cta);
     return issue(g, dry, stream);
   };
   // 5. dgrad-1 + combine: dx rows go back to the ranks the tokens came from. Issued after the weight gradients (its
@@ -450,6 +455,8 @@ int ccf_row_kernel(int epi, int b_major, int rows, int experts, int n, int capac
   out[3] = r.bn;
   return 0;
 }
+
+int ccf_wgrad_few(int rows, int in_place, int two_cta) { return wgrad_few(rows, in_place != 0, two_cta); }
 
 int ccf_sizeof_layer() { return static_cast<int>(sizeof(CcfLayer)); }
 int ccf_sizeof_layer_grads() { return static_cast<int>(sizeof(CcfLayerGrads)); }

@@ -225,6 +225,7 @@ def _declare(lib):
         "ccf_layer_forward": ([C.POINTER(Layer), p, p, p, p, i, i, i, i, p, p, i, p], i),
         "ccf_layer_backward": ([C.POINTER(Layer), p, p, p, C.POINTER(LayerGrads), i, i, p, p, i, p], i),
         "ccf_row_kernel": ([i, i, i, i, i, i, i, i, i, p], i),
+        "ccf_wgrad_few": ([i, i, i], i),
         "ccf_flag_barrier": ([C.POINTER(BarrierArgs), p], i),
         "ccf_plan": ([C.POINTER(PlanArgs), p], i),
         "ccf_plan_dev_epoch": ([C.POINTER(PlanArgs), p, p], i),
@@ -274,7 +275,8 @@ class LaunchRecorder:
     Size queries, error strings and the choice of kernels go to the real library; everything else returns 0. Structures passed with
     ``ctypes.byref`` are stored as their raw bytes (``GemmLaunch.from_buffer_copy`` turns them back into fields)."""
 
-    _PASS_THROUGH = ("ccf_sizeof_", "ccf_error_string", "ccf_gemm_smem_bytes", "ccf_symm_handle_bytes", "ccf_row_kernel")
+    _PASS_THROUGH = ("ccf_sizeof_", "ccf_error_string", "ccf_gemm_smem_bytes", "ccf_symm_handle_bytes", "ccf_row_kernel",
+                     "ccf_wgrad_few")
 
     def __init__(self, real):
         self._real = real

@@ -799,13 +799,11 @@ class _FusedMoEFn(torch.autograd.Function):
                      local_rows=fm.local_rows, **rk, **common)
         cc.tile_flags.zero_()
         # 3. wgrad-2: dW2[e] = (g dy)^T h_act   [d, f]
-        # With few rows per expert the reduction is only a handful of k-blocks, and moving the result decides.
-        # In-place launches, 2048 x 8192: 811 us against 1214 on the pair kernel at 64 x 256 rows, 309 against 355 at 16 x 512,
-        # 553 against 467 at 16 x 1024.
-        wgrad_few = (t * cfg.top_k * fm.world) // max(1, cfg.num_experts) <= 512 and bool(G.TWO_CTA_DEFAULT)
+        rows = t * cfg.top_k * fm.world // max(1, cfg.num_experts)
         dw2 = torch.empty_like(w2) if sgd2 is None else None
         G.launch(a0=cc.grecv, b0=fm.h_act, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, kgroup=True,
-                 m_per_group=d, out0=dw2 if sgd2 is None else w2, ld_out=f, few_rows=wgrad_few, sgd=sgd2, **common)
+                 m_per_group=d, out0=dw2 if sgd2 is None else w2, ld_out=f, few_rows=G.wgrad_few(rows, sgd2 is not None),
+                 sgd=sgd2, **common)
         has_b1, has_bg, has_b2 = ctx.has_bias
 
         def colsum(src, n):
@@ -833,7 +831,7 @@ class _FusedMoEFn(torch.autograd.Function):
         dw1 = torch.empty_like(w1) if sgd is None else None
         dwg = dbg = None
         wkw = dict(b0=fm.xrecv, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=d, kgroup=True, m_per_group=f, ld_out=d,
-                   few_rows=wgrad_few, sgd=sgd, **common)
+                   few_rows=G.wgrad_few(rows, sgd is not None), sgd=sgd, **common)
         if swiglu:
             # dh = d(gate pre-activation), dh2 = d(up pre-activation)
             dwg = torch.empty_like(wg) if sgd is None else None

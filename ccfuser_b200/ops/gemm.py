@@ -225,6 +225,11 @@ def row_kernel(epi: int, b_major: int, rows: int, experts: int, n: int, capacity
     return dict(few_rows=bool(out[0]), two_cta=bool(out[1]), a_rows=out[2], bn=out[3])
 
 
+def wgrad_few(rows: int, in_place: bool) -> bool:
+    """``few_rows`` of a weight-gradient launch of a call that expects ``rows`` rows per expert (csrc/runtime.cu: wgrad_few)."""
+    return bool(N.load().ccf_wgrad_few(rows, int(in_place), int(TWO_CTA_DEFAULT)))
+
+
 def combine_units(n: int, few_rows: bool = False) -> int:
     """Completion-counter increments per output row of a COMBINE GEMM with n columns: one per 32 columns. The same in every
     kernel (``few_rows`` changes nothing), because the rank that stores a row and the rank that waits for it choose their

@@ -57,3 +57,14 @@ def test_one_cta_kernel_keeps_its_row_bound_and_narrow_tiles(native, monkeypatch
     assert kernel(got["gemm1"]) == (0, 0, 64, 0) and kernel(got["gemm2"]) == (0, 0, 64, 128)
     got = launches(3000, d=1024, experts=32, native=native)     # no bound, 256 tiles
     assert kernel(got["gemm1"]) == kernel(got["gemm2"]) == (0, 0, 0, 0)
+
+
+@pytest.mark.parametrize("native", [False, True])
+def test_weight_gradients_change_kernels_at_the_measured_rows(native):
+    """Plain ones run on gemm_wgrad.cu up to 384 expected rows per expert, in-place ones up to 512, then on CTA pairs."""
+    def few(rows, sgd):
+        got = launches(rows * 8, d=256, f=512, sgd=sgd, native=native)
+        assert all(got[k].two_cta == 1 for k in ("wgrad1", "wgrad2"))
+        return [got[k].few_rows for k in ("wgrad1", "wgrad2")]
+    assert few(384, False) == [1, 1] and few(385, False) == [0, 0]
+    assert few(512, True) == [1, 1] and few(513, True) == [0, 0]
