@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "dispatch.cuh"   // pack2 / unpack2
+#include "norm.h"
 #include "sm100.cuh"
 
 namespace ccf {

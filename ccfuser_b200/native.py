@@ -139,6 +139,7 @@ class _Launches(list):
 
 LAUNCHES = _Launches([0])
 _torch_module = None
+_torch_module_tried = False
 
 
 def count(n: int = 1):
@@ -149,19 +150,47 @@ def lib_path() -> str:
     return os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libccfuser_b200.so")
 
 
+def _build_locked(needed, make):
+    """``make()`` if ``needed()``. Several ranks of one job may arrive here together: one builds, the others wait for the lock."""
+    if not needed():
+        return
+    import fcntl
+    os.makedirs(os.path.dirname(lib_path()), exist_ok=True)
+    with open(lib_path() + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if needed():
+                make()
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
 def torch_module():
-    """The autograd functions in C++ (csrc/torch_norm.cpp)."""
-    global _torch_module
-    if _torch_module is None:
-        load()      # builds both where the sources are newer
-        import importlib.util
-        path = os.path.join(os.path.dirname(lib_path()), "_ccf_torch.so")
-        with _lock:
-            if _torch_module is None:
-                spec = importlib.util.spec_from_file_location("_ccf_torch", path)
+    """The autograd functions in C++ (csrc/torch_norm.cpp), or None where this torch has no module and none can be built: the
+    kernels do not need it (ops/norm.py has the function in Python). Tried once; says so once."""
+    global _torch_module, _torch_module_tried
+    if _torch_module is not None or _torch_module_tried:
+        return _torch_module
+    load()
+    with _lock:
+        if not _torch_module_tried:
+            from . import build as _build
+            import importlib.util
+            try:
+                try:
+                    _build_locked(_build.needs_torch_module, _build.build_torch_module)
+                except Exception:
+                    if not os.path.exists(_build.torch_path()):
+                        raise
+                spec = importlib.util.spec_from_file_location("_ccf_torch", _build.torch_path())
                 module = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(module)
                 _torch_module = module
+            except Exception as e:  # noqa: BLE001
+                import warnings
+                warnings.warn(f"ccfuser_b200: {_build.torch_path()} could not be built or loaded ({e}); LayerNorm's autograd "
+                              "function runs in Python, on the same kernels")
+            _torch_module_tried = True
     return _torch_module
 
 
@@ -177,17 +206,7 @@ def load(build_if_missing: bool = True):
         if build_if_missing:
             from . import build as _build
             try:
-                if _build.needs_build():
-                    # several ranks of one job may arrive here together: one builds, the others wait for the lock
-                    import fcntl
-                    os.makedirs(os.path.dirname(path), exist_ok=True)
-                    with open(path + ".lock", "w") as lock:
-                        fcntl.flock(lock, fcntl.LOCK_EX)
-                        try:
-                            if _build.needs_build():
-                                _build.build()
-                        finally:
-                            fcntl.flock(lock, fcntl.LOCK_UN)
+                _build_locked(_build.needs_build, _build.build_library)
             except Exception:
                 if not os.path.exists(path):
                     raise

@@ -4,8 +4,8 @@
 (CPU, fp32, a normalised dimension above 2048 or not a multiple of 8, no affine parameters) take the torch path. The
 models' transformer blocks normalise a ``[tokens, d_model]`` matrix twice each; forward and backward are one pass over
 that matrix here; the backward kernel leaves partial weight / bias gradients, which a second small kernel adds. The autograd
-function around them is C++ (csrc/torch_norm.cpp); while ``torch.jit.trace`` records a graph it is the Python one below, which the
-tracer keeps as an operation of its own.
+function around them is C++ (csrc/torch_norm.cpp). It is the Python one below while ``torch.jit.trace`` records a graph, which
+keeps that one as an operation of its own, and where the C++ module is missing and cannot be built.
 """
 from __future__ import annotations
 
@@ -65,9 +65,10 @@ def supported(x: torch.Tensor, normalized_shape, weight) -> bool:
 def layer_norm(x, normalized_shape, weight, bias, eps=1e-5):
     """``F.layer_norm`` that runs on the library's kernels where they apply."""
     if supported(x, tuple(normalized_shape), weight) and (bias is None or bias.dtype == x.dtype):
-        if torch.jit.is_tracing():
+        module = N.torch_module()
+        if module is None or torch.jit.is_tracing():
             return _LayerNormFn.apply(x, weight, bias, eps)
-        return N.torch_module().layer_norm(x, weight, bias, G.Workspace.of(x).status, eps, G.DEFAULT_WAIT_NS)
+        return module.layer_norm(x, weight, bias, G.Workspace.of(x).status, eps, G.DEFAULT_WAIT_NS)
     return F.layer_norm(x, normalized_shape, weight, bias, eps)
 
 

@@ -94,3 +94,24 @@ def test_a_traced_graph_replays_the_kernels(bias):
         return [y.detach(), v.grad] + [p.grad.clone() for p in norm.parameters()]
     for a, b in zip(run(traced), run(norm)):
         assert torch.equal(a, b)
+
+
+def test_without_the_module_the_kernels_run_from_python(monkeypatch):
+    from ccfuser_b200 import native as N
+    from ccfuser_b200.ops.norm import LayerNorm
+    torch.manual_seed(13)
+    norm = LayerNorm(264, device="cuda", dtype=torch.float16)
+    x, gy = (torch.randn(37, 264, device="cuda").half() for _ in range(2))
+
+    def run():
+        v = x.clone().requires_grad_(True)
+        norm.zero_grad()
+        before = N.LAUNCHES[0]
+        norm(v).backward(gy)
+        assert N.LAUNCHES[0] - before == 3
+        return [v.grad] + [p.grad.clone() for p in norm.parameters()]
+    want = run()
+    monkeypatch.setattr(N, "_torch_module", None)
+    monkeypatch.setattr(N, "_torch_module_tried", True)
+    for a, b in zip(run(), want):
+        assert torch.equal(a, b)
