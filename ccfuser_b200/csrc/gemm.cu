@@ -578,6 +578,7 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     const bool fwd = L->epi == CCF_EPI_BIAS_ACT || L->epi == CCF_EPI_SWIGLU;
     const bool bwd = L->epi == CCF_EPI_DACT || L->epi == CCF_EPI_DSWIGLU;
     if (!(fwd && a.disp.backward == 0) && !(bwd && a.disp.backward == 1)) return -9;
+    if (reinterpret_cast<uintptr_t>(a.disp.x) & 15) return -14;   // the role moves 16 bytes at a time
   }
   CUtensorMap tm[6];
   const int fp16 = a.fp16;

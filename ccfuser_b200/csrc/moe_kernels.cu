@@ -451,7 +451,7 @@ int ccf_plan_dev_epoch(const ccf::PlanArgs* a, int* epoch_counter, void* stream)
 }
 
 int ccf_dispatch(const CcfDispatchArgs* a, int* status, int* done_ctas, int grid, void* stream) {
-  if (a->d % 8 != 0) return -2;
+  if (a->d % 8 != 0 || (reinterpret_cast<uintptr_t>(a->x) & 15)) return -2;
   if (grid <= 0) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

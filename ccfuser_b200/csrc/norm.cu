@@ -336,6 +336,12 @@ static int ln_bwd_blocks(int rows, int d) {
   return blocks < 2 * 148 ? blocks : 2 * 148;
 }
 
+// The kernels move 16 bytes at a time.
+template <typename... T>
+static bool aligned16(const T*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0;
+}
+
 template <int kV>
 static int launch_ln_fwd(const void* x, const void* gamma, const void* beta, void* out, float* mean, float* rstd, int rows, int d,
                          float eps, int fp16, cudaStream_t st) {
@@ -353,11 +359,12 @@ extern "C" {
 int ccf_layernorm_max_d() { return 2048; }
 
 // y = (x - mean) * rstd * gamma + beta over the last dimension of x [rows, d] (2-byte elements, gamma / beta of the same
-// type, beta may be null); mean and rstd [rows] fp32 are written for the backward pass. d % 8 == 0, d <= 2048.
+// type, beta may be null); mean and rstd [rows] fp32 are written for the backward pass. d % 8 == 0, d <= 2048, x, y, gamma and
+// beta on 16-byte boundaries.
 int ccf_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows,
                       int d, float eps, int fp16, void* stream) {
   using namespace ccf;
-  if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048) return -2;
+  if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048 || !aligned16(x, gamma, beta, y)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (d <= 512) return launch_ln_fwd<2>(x, gamma, beta, y, mean, rstd, rows, d, eps, fp16, st);
   if (d <= 1024) return launch_ln_fwd<4>(x, gamma, beta, y, mean, rstd, rows, d, eps, fp16, st);
@@ -368,12 +375,12 @@ int ccf_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* 
 int ccf_layernorm_bwd_parts(int rows, int d) { return rows < 1 || d < 8 ? 0 : ccf::ln_bwd_blocks(rows, d); }
 
 // dx [rows, d], dgamma [d] and dbeta [d] (element type; dbeta may be null) are written. `part`: scratch of
-// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats, 16-byte aligned. A wait that exceeds the limit goes to `status`.
+// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats; it, x, dy, gamma and dx on 16-byte boundaries. A wait that exceeds the limit goes to `status`.
 int ccf_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
                       float* part, void* dgamma, void* dbeta, int rows, int d, int fp16, int* status,
                       unsigned long long wait_limit_ns, void* stream) {
   using namespace ccf;
-  if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048) return -2;
+  if (rows < 1 || d < 8 || d % 8 != 0 || d > 2048 || !aligned16(x, dy, gamma, dx, part)) return -2;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int blocks = ln_bwd_blocks(rows, d);
   const int w = (d + 255) / 256, kw = w <= 1 ? 1 : w <= 2 ? 2 : w <= 4 ? 4 : 8;

@@ -22,16 +22,20 @@ std::atomic<long long> g_launches{0};
 
 void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed with code ", rc); }
 
-// rows of the last dimension, contiguous
-at::Tensor rows_of(const at::Tensor& t, int64_t rows, int64_t d) { return t.reshape({rows, d}).contiguous(); }
+// as the kernels read it: contiguous and on a 16-byte boundary (a view may begin anywhere)
+at::Tensor packed(const at::Tensor& t) {
+  const at::Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
+}
+at::Tensor rows_of(const at::Tensor& t, int64_t rows, int64_t d) { return packed(t.reshape({rows, d})); }
 
 struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias,
                             const at::Tensor& status, double eps, int64_t wait_ns) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t d = x.size(-1), rows = x.numel() / d;
-    const at::Tensor x2 = rows_of(x, rows, d), w = weight.contiguous();
-    const at::Tensor b = bias.has_value() ? bias->contiguous() : at::Tensor();
+    const at::Tensor x2 = rows_of(x, rows, d), w = packed(weight);
+    const at::Tensor b = bias.has_value() ? packed(*bias) : at::Tensor();
     const at::Tensor y = at::empty_like(x2);
     const auto f32 = x2.options().dtype(at::kFloat);
     const at::Tensor mean = at::empty({rows}, f32), rstd = at::empty({rows}, f32);

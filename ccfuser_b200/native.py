@@ -333,14 +333,17 @@ class record_launches:
 
 
 # Argument checks of the host launchers return small negative numbers before any CUDA call is made; failures of CUDA
-# calls come back as minus the cudaError_t value. The two ranges overlap for -2 ... -9, so a message names both readings.
+# calls come back as minus the cudaError_t value. The two ranges overlap for -2 ... -14, so a message names both readings.
 ARG_ERRORS = {-2: "argument out of range", -3: "n must be a multiple of 32", -4: "k-grouped GEMM needs m_per_group % 128 == 0",
               -5: "k must be a multiple of 8", -6: "no kernel for this combination of operand majors and epilogue",
               -7: "cudaSetDevice failed", -8: "the CTA-pair kernel needs m_per_group % 256 == 0 in k-grouped mode",
               -9: "the dispatch role exists only in the kernels that read the receive buffer (forward: bias+activation / "
                   "SwiGLU epilogues with backward=0, backward: activation-derivative epilogues with backward=1)",
               -10: "128-column tiles exist in the one-CTA kernel for row-grouped launches with a K-major B operand only",
-              -11: "the row bound (32 or 64) exists in the one-CTA kernel for row-grouped launches with a K-major A operand only"}
+              -11: "the row bound (32 or 64) exists in the one-CTA kernel for row-grouped launches with a K-major A operand only",
+              -12: "the kernel for few rows takes a K-major A operand, 16-bit outputs, no row bound, no narrow tile and no in-place update",
+              -13: "the weight-gradient kernel for few rows takes MN-major operands, 16-bit outputs of n columns, no bias, m_per_group % 256 == 0",
+              -14: "the rows to be dispatched must begin on a 16-byte boundary"}
 
 
 def check(rc: int, what: str):

@@ -723,7 +723,7 @@ class _FusedLayerFn(torch.autograd.Function):
         dgate = torch.empty(gate_w.numel(), dtype=torch.float32, device=dy.device)
         drw = torch.empty_like(rw) if (need_rw or need_rb) else None
         drb = torch.empty(rw.shape[0], dtype=rw.dtype, device=dy.device) if need_rb else None
-        dx, grads = _native_backward(fm, dy.contiguous(), idx, gate_w, dgate, w1, wg, w2, ctx.has_bias, (rw, x, drw, drb))
+        dx, grads = _native_backward(fm, G.packed(dy), idx, gate_w, dgate, w1, wg, w2, ctx.has_bias, (rw, x, drw, drb))
         return (dx, drw if need_rw else None, drb) + grads + (None,)
 
 
@@ -769,7 +769,7 @@ class _FusedMoEFn(torch.autograd.Function):
         st = N.stream_ptr()
         t, d, f, e_loc = ctx.tokens, cfg.d_model, cfg.d_ffn, cfg.experts_per_rank
         fp16 = int(cfg.dtype == torch.float16)
-        dy = dy.contiguous()
+        dy = G.packed(dy)
         dgate = torch.zeros(t * cfg.top_k, dtype=torch.float32, device=dy.device)  # dropped slots keep 0
         swiglu = cfg.activation == "swiglu"
         # fuse_sgd: the weight-gradient GEMMs update the weights in place (single-rank layers); no weight gradient is

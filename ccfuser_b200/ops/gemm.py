@@ -151,6 +151,12 @@ def _is_fp16(t: torch.Tensor) -> int:
     raise TypeError(f"grouped GEMM operands must be bf16 or fp16, got {t.dtype}")
 
 
+def packed(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels read it: contiguous and on a 16-byte boundary (a view may begin anywhere)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num_groups,
            a1=None, b1=None, kgroup=False, m_per_group=0, kseg=1, b_group_rows=0,
            out0=None, out1=None, out2=None, bias0=None, bias1=None, aux0=None, aux1=None, ld_out=None,

@@ -27,8 +27,8 @@ class _LayerNormFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, eps):
         lib = N.load()
         d = x.shape[-1]
-        x2, w = x.reshape(-1, d).contiguous(), weight.contiguous()
-        b = None if bias is None else bias.contiguous()
+        x2, w = G.packed(x.reshape(-1, d)), G.packed(weight)
+        b = None if bias is None else G.packed(bias)
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         mean, rstd = (torch.empty(rows, dtype=torch.float32, device=x.device) for _ in range(2))
@@ -45,7 +45,7 @@ class _LayerNormFn(torch.autograd.Function):
         lib = N.load()
         x2, w, mean, rstd = ctx.saved_tensors
         rows, d = x2.shape
-        dy2, dx, dg = dy.reshape(rows, d).contiguous(), torch.empty_like(x2), torch.empty_like(w)
+        dy2, dx, dg = G.packed(dy.reshape(rows, d)), torch.empty_like(x2), torch.empty_like(w)
         db = torch.empty_like(w) if ctx.has_bias else None
         part = torch.empty(lib.ccf_layernorm_bwd_parts(rows, d), 2, d, dtype=torch.float32, device=x2.device)
         N.check(lib.ccf_layernorm_bwd(x2.data_ptr(), dy2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
