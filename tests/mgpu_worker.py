@@ -31,7 +31,7 @@ def gather(t, world):
     return out
 
 
-def run_case(rank, world, act, cf, tokens, e_loc, d, f, iters=3):
+def run_case(rank, world, act, cf, tokens, e_loc, d, f, odd_ranks=None, iters=3):
     torch.manual_seed(7)
     e = e_loc * world
     cfg = MoEConfig(d_model=d, d_ffn=f, num_experts=e, top_k=2, capacity_factor=cf, activation=act,
@@ -58,7 +58,9 @@ def run_case(rank, world, act, cf, tokens, e_loc, d, f, iters=3):
     for it in range(iters):
         gx = torch.Generator(device="cuda").manual_seed(100 * it + rank)
         # uneven token counts across ranks exercise ragged segments
-        t_r = tokens - 37 * rank - 5 * it
+        t_r = max(1, tokens - 37 * rank - 5 * it)
+        if odd_ranks is not None and (rank + it) % 2:
+            t_r = odd_ranks + it
         x = (torch.randn(t_r, d, device="cuda", generator=gx) * 0.5).bfloat16().requires_grad_(True)
         idx, w = topk_softmax(layer.gate.logits(x.detach()), 2)
         w = w.detach().requires_grad_(True)
@@ -102,10 +104,14 @@ def run_case(rank, world, act, cf, tokens, e_loc, d, f, iters=3):
 
 def main():
     rank, local_rank, world = init_distributed()
-    cases = [("gelu", 1.25, 1024, 4, 256, 512), ("swiglu", None, 700, 2, 256, 384), ("relu", 1.0, 2048, 8, 512, 1024)]
+    cases = [("gelu", 1.25, 1024, 4, 256, 512, None), ("swiglu", None, 700, 2, 256, 384, None), ("relu", 1.0, 2048, 8, 512, 1024, None),
+             # every launch on the kernels for few rows: 30 to 250 rows per expert
+             ("gelu", None, 500, 4, 256, 512, None), ("swiglu", 2.0, 90, 4, 256, 384, None),
+             # ranks whose calls lie on both sides of the kernels' limits, each in turn: 600 and a handful of expected rows
+             ("gelu", None, 1200, 4, 320, 512, 12), ("swiglu", None, 1200, 4, 256, 384, 1)]
     worst = 0.0
-    for act, cf, tokens, e_loc, d, f in cases:
-        worst = max(worst, run_case(rank, world, act, cf, tokens, e_loc, d, f))
+    for act, cf, tokens, e_loc, d, f, odd_ranks in cases:
+        worst = max(worst, run_case(rank, world, act, cf, tokens, e_loc, d, f, odd_ranks))
         dist.barrier()
     t = torch.tensor([worst], device="cuda")
     dist.all_reduce(t, op=dist.ReduceOp.MAX)
