@@ -95,8 +95,8 @@ struct CcfGemmArgs {
   int out_fp32;             // EPI_STORE: write fp32
   int world;                // COMBINE: number of ranks
   int send_finish;          // COMBINE: the last CTA adds 1 to every rank's completion counter
-  int count_rows;           // COMBINE: stored rows are added, 1 per 32 columns, to the completion counter of the rank they went to. 0 on a single rank:
-                            // its reduction follows on the stream, and the last CTA's 1 says that every row is there
+  int count_rows;           // COMBINE: stored rows are added, 1 per 32 columns, to the completion counter of the rank they went to. 0 on
+                            // a single rank: its reduction follows on the stream, and the last CTA's 1 says that every row is there
   int n_comm_ctas;          // CTAs that run the dispatch role before taking GEMM tiles (0 = none)
   int max_slots;            // COMBINE: rows of a combine buffer (bounds check)
   int trace_tiles;          // tiles per CTA recorded in `trace`

@@ -85,8 +85,8 @@ __device__ __forceinline__ constexpr int frag_piece(int m) { return 2 * (m >> 3)
 __device__ __forceinline__ void frag_to_stage(uint32_t stage, int lane, const uint32_t (&w)[16]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(stage + stage_off(8 * j + (lane & 7), lane >> 3)),
-                 "r"(w[2 * j]), "r"(w[2 * j + 1]), "r"(w[8 + 2 * j]), "r"(w[9 + 2 * j])
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(stage + stage_off(8 * j + (lane & 7), lane >> 3)), "r"(w[2 * j]), "r"(w[2 * j + 1]), "r"(w[8 + 2 * j]), "r"(w[9 + 2 * j])
                  : "memory");
   __syncwarp();
 }
@@ -134,8 +134,8 @@ __device__ __forceinline__ void frag_fetch(const char* from, unsigned long long 
 __device__ __forceinline__ void fetched_to_frag(uint32_t stage, int lane, const uint4 (&v)[4], uint32_t (&w)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + stage_off(8 * i + (lane >> 2), lane & 3)), "r"(v[i].x), "r"(v[i].y),
-                 "r"(v[i].z), "r"(v[i].w)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + stage_off(8 * i + (lane >> 2), lane & 3)), "r"(v[i].x),
+                 "r"(v[i].y), "r"(v[i].z), "r"(v[i].w)
                  : "memory");
   __syncwarp();
   stage_to_frag(stage, lane, w);
@@ -252,7 +252,9 @@ __device__ __forceinline__ void swap_epilogue(const CcfGemmArgs& args, const Swa
   const unsigned long long step = static_cast<unsigned long long>(args.ld_out) * 16ull;   // bytes of eight rows
   // this lane's place in row l / 4 of the part, bytes
   const long long at0 = ((pt.row0 + (lane >> 2)) * args.ld_out + fbase + (lane & 3) * 8) * 2;
-  auto at = [&](const void* p, int c) { return const_cast<char*>(reinterpret_cast<const char*>(p)) + (at0 + 4ll * c * static_cast<long long>(step)); };
+  auto at = [&](const void* p, int c) {
+    return const_cast<char*>(reinterpret_cast<const char*>(p)) + (at0 + 4ll * c * static_cast<long long>(step));
+  };
   float b0[4] = {0, 0, 0, 0}, b1[4] = {0, 0, 0, 0};
   {
     const size_t off = static_cast<size_t>(pt.g) * args.n + fbase + (lane >> 2);
@@ -348,7 +350,8 @@ __device__ __forceinline__ void swap_epilogue(const CcfGemmArgs& args, const Swa
       if (args.row_gate != nullptr) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float g0 = __shfl_sync(0xffffffffu, gate, 8 * j + 2 * (lane & 3)), g1 = __shfl_sync(0xffffffffu, gate, 8 * j + 2 * (lane & 3) + 1);
+          const float g0 = __shfl_sync(0xffffffffu, gate, 8 * j + 2 * (lane & 3));
+          const float g1 = __shfl_sync(0xffffffffu, gate, 8 * j + 2 * (lane & 3) + 1);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const int m = 8 * (k >> 1) + 2 * j + (k & 1);
@@ -598,14 +601,14 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
             for (int a = 0; a < (kWide ? 2 : 1); ++a) {
 #pragma unroll
               for (int k = 0; k < BK / UK; ++k)
-                umma_f16_pair(d0 + a * 128, desc_at(desc_w, at + a * kSwWBytes + k * desc_step(kWMajor)), desc_at(desc_x, at + k * desc_step(MAJ_K)),
-                              idesc, k > 0 ? 1u : acc);
+                umma_f16_pair(d0 + a * 128, desc_at(desc_w, at + a * kSwWBytes + k * desc_step(kWMajor)),
+                              desc_at(desc_x, at + k * desc_step(MAJ_K)), idesc, k > 0 ? 1u : acc);
             }
             if (!kWide && ti.parts > 1) {
 #pragma unroll
               for (int k = 0; k < BK / UK; ++k)
-                umma_f16_pair(d1, desc_at(desc_w, at + k * desc_step(kWMajor)), desc_at(desc_x, at + part_bytes + k * desc_step(MAJ_K)), idesc,
-                              k > 0 ? 1u : acc);
+                umma_f16_pair(d1, desc_at(desc_w, at + k * desc_step(kWMajor)),
+                              desc_at(desc_x, at + part_bytes + k * desc_step(MAJ_K)), idesc, k > 0 ? 1u : acc);
             }
             umma_commit_pair(empty0 + 8 * stage);   // hand the stage back to both producers
             if (kb == sh.kblocks - 1) {

@@ -86,8 +86,8 @@ struct ChunkPos {
 
 template <int kFp16, bool kSgd>
 __global__ void __launch_bounds__(kWgThreads, 1)
-grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                     const __grid_constant__ CcfGemmArgs args) {
+grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CcfGemmArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   CtrlW* ctrl = reinterpret_cast<CtrlW*>(smem + kWgStages * kWgStageBytes + kWgChunks * kWgChunkBytes);

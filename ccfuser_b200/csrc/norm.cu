@@ -23,16 +23,15 @@ constexpr int kLnWarps = kLnThreads / 32;
 template <int kV>
 constexpr int kLnBlocks = kV >= 8 ? 2 : kV >= 4 ? 3 : 4;
 
-// kV = 16-byte pieces of a row per lane (row length <= 256 * kV elements). Bound by reading x and writing y once. The grid is one wave, each
-// warp walks rows `warps` apart and requests its next row before it works on the current one: with a block per eight rows the launch ran its
-// waves one after the other, each of them a load, two reductions and a store. gamma and beta stay in shared memory. Cold, in a graph, before
-// and now, us: 16384 x 2048 38.4 and 29.0 (4.6 TB/s), 8192 x 2048 20.5 and 17.7, 2048 x 2048 9.2 and 7.3, 8192 x 768 9.9 and 8.4,
-// 16 x 2048 5.9 and 3.7, 4100 x 264 (one wave either way) 3.7 and 3.9.
+// kV = 16-byte pieces of a row per lane (row length <= 256 * kV elements). Bound by reading x and writing y once. The grid is one
+// wave, each warp walks rows `warps` apart and requests its next row before it works on the current one: with a block per eight
+// rows the launch ran its waves one after the other, each of them a load, two reductions and a store. gamma and beta stay in
+// shared memory. Cold, in a graph, before and now, us: 16384 x 2048 38.4 and 29.0 (4.6 TB/s), 8192 x 2048 20.5 and 17.7,
+// 2048 x 2048 9.2 and 7.3, 8192 x 768 9.9 and 8.4, 16 x 2048 5.9 and 3.7, 4100 x 264 (one wave either way) 3.7 and 3.9.
 template <int kV>
-__global__ void __launch_bounds__(kLnThreads, kLnBlocks<kV>) layernorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ gamma,
-                                                                      const void* __restrict__ beta, void* __restrict__ y,
-                                                                      float* __restrict__ mean_out, float* __restrict__ rstd_out,
-                                                                      int rows, int d, float eps, int fp16) {
+__global__ void __launch_bounds__(kLnThreads, kLnBlocks<kV>)
+layernorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ gamma, const void* __restrict__ beta, void* __restrict__ y,
+                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int d, float eps, int fp16) {
   __shared__ uint4 gs[32 * kV], bs[32 * kV];
   const int lane = threadIdx.x & 31, vecs = d >> 3;
   const uint32_t warps = gridDim.x * kLnWarps, n_rows = static_cast<uint32_t>(rows);
@@ -345,7 +344,10 @@ static bool aligned16(const T*... p) {
 template <int kV>
 static int launch_ln_fwd(const void* x, const void* gamma, const void* beta, void* out, float* mean, float* rstd, int rows, int d,
                          float eps, int fp16, cudaStream_t st) {
-  const int need = (rows + kLnWarps - 1) / kLnWarps, wave = kLnBlocks<kV> * 148, blocks = need < wave ? need : wave;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int need = (rows + kLnWarps - 1) / kLnWarps, wave = kLnBlocks<kV> * (sms > 0 ? sms : 1), blocks = need < wave ? need : wave;
   layernorm_fwd_kernel<kV><<<blocks, kLnThreads, 0, st>>>(x, gamma, beta, out, mean, rstd, rows, d, eps, fp16);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
@@ -375,7 +377,8 @@ int ccf_layernorm_fwd(const void* x, const void* gamma, const void* beta, void* 
 int ccf_layernorm_bwd_parts(int rows, int d) { return rows < 1 || d < 8 ? 0 : ccf::ln_bwd_blocks(rows, d); }
 
 // dx [rows, d], dgamma [d] and dbeta [d] (element type; dbeta may be null) are written. `part`: scratch of
-// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats; it, x, dy, gamma and dx on 16-byte boundaries. A wait that exceeds the limit goes to `status`.
+// ccf_layernorm_bwd_parts(rows, d) x 2 x d floats; it, x, dy, gamma and dx on 16-byte boundaries. A wait that exceeds the
+// limit goes to `status`.
 int ccf_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
                       float* part, void* dgamma, void* dbeta, int rows, int d, int fp16, int* status,
                       unsigned long long wait_limit_ns, void* stream) {

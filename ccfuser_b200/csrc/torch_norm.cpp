@@ -60,7 +60,8 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const at::Tensor dy = rows_of(grads[0], rows, d), dx = at::empty_like(x2), dg = at::empty_like(w);
     const at::Tensor db = has_bias ? at::empty_like(w) : at::Tensor();
-    const at::Tensor part = at::empty({ccf_layernorm_bwd_parts(static_cast<int>(rows), static_cast<int>(d)), 2, d}, x2.options().dtype(at::kFloat));
+    const int parts = ccf_layernorm_bwd_parts(static_cast<int>(rows), static_cast<int>(d));
+    const at::Tensor part = at::empty({parts, 2, d}, x2.options().dtype(at::kFloat));
     check(ccf_layernorm_bwd(x2.data_ptr(), dy.data_ptr(), w.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(),
                             part.data_ptr<float>(), dg.data_ptr(), has_bias ? db.data_ptr() : nullptr, static_cast<int>(rows),
                             static_cast<int>(d), x2.scalar_type() == at::kHalf, ctx->saved_data["status"].toTensor().data_ptr<int>(),
@@ -78,8 +79,7 @@ PYBIND11_MODULE(_ccf_torch, m) {
   m.def(
       "layer_norm",
       [](const at::Tensor& x, const at::Tensor& weight, const std::optional<at::Tensor>& bias, const at::Tensor& status, double eps,
-         int64_t wait_ns) { return LayerNormFn::apply(x, weight, bias, status, eps, wait_ns);
-      },
+         int64_t wait_ns) { return LayerNormFn::apply(x, weight, bias, status, eps, wait_ns); },
       py::call_guard<py::gil_scoped_release>());
   m.def("launches", [] { return g_launches.load(); });
 }

@@ -342,7 +342,8 @@ ARG_ERRORS = {-2: "argument out of range", -3: "n must be a multiple of 32", -4:
               -10: "128-column tiles exist in the one-CTA kernel for row-grouped launches with a K-major B operand only",
               -11: "the row bound (32 or 64) exists in the one-CTA kernel for row-grouped launches with a K-major A operand only",
               -12: "the kernel for few rows takes a K-major A operand, 16-bit outputs, no row bound, no narrow tile and no in-place update",
-              -13: "the weight-gradient kernel for few rows takes MN-major operands, 16-bit outputs of n columns, no bias, m_per_group % 256 == 0",
+              -13: "the weight-gradient kernel for few rows takes MN-major operands, 16-bit outputs of n columns, no bias and "
+                   "m_per_group % 256 == 0",
               -14: "the rows to be dispatched must begin on a 16-byte boundary"}
 
 

@@ -227,7 +227,8 @@ def row_kernel(epi: int, b_major: int, rows: int, experts: int, n: int, capacity
     """Arguments of ``launch`` that choose the kernel of a row-grouped launch, by the rule of csrc/runtime.cu (row_kernel): ``rows``
     rows expected for each of this rank's ``experts`` experts, ``capacity`` rows at most from one rank."""
     out = (C.c_int * 4)()
-    N.load().ccf_row_kernel(epi, b_major, rows, experts, n, capacity, world, SMALL_ROWS_DEFAULT, int(TWO_CTA_DEFAULT), C.addressof(out))
+    N.load().ccf_row_kernel(epi, b_major, rows, experts, n, capacity, world, SMALL_ROWS_DEFAULT, int(TWO_CTA_DEFAULT),
+                            C.addressof(out))
     return dict(few_rows=bool(out[0]), two_cta=bool(out[1]), a_rows=out[2], bn=out[3])
 
 
