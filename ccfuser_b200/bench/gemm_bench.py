@@ -68,7 +68,7 @@ def time_fn(fn, iters=10, warmup=3, flush_mb=256, back_to_back=0):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--cases", default="square,fwd1,fwd2,dgrad,dgrad_plain,wgrad,cublas",
-                    help="comma-separated; also fwd1_parts and wgrad_sgd")
+                    help="comma-separated; also fwd1_parts, fwd2_combine and wgrad_sgd")
     ap.add_argument("--rows", type=int, default=4096 * 8)
     ap.add_argument("--experts", type=int, default=8)
     ap.add_argument("--d", type=int, default=4096)
@@ -120,6 +120,10 @@ def main():
     def gemm(**kw):
         return lambda trace=None: G.launch(trace=trace, **kw)
 
+    def row_kernel(epi, b_major, n):
+        # the kernel that a layer without a capacity chooses for this number of rows
+        return G.row_kernel(epi, b_major, rows_per, e, n, r, 1)
+
     cases = args.cases.split(",")
     if "square" in cases:
         m = 8192
@@ -136,7 +140,8 @@ def main():
     if "fwd1" in cases:
         report("fwd1_gelu", 2 * r * d * f, gemm(
             a0=x, b0=w1.view(e * f, d), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_BIAS_ACT, n=f, k=d,
-            group_base=gb, group_rows=gr, num_groups=e, b_group_rows=f, out0=h, out1=pre, act=N.ACT_GELU), kblocks=(d + 63) // 64)
+            group_base=gb, group_rows=gr, num_groups=e, b_group_rows=f, out0=h, out1=pre, act=N.ACT_GELU,
+            **row_kernel(N.EPI_BIAS_ACT, N.MAJ_K, f)), kblocks=(d + 63) // 64)
     # the same GEMM with parts of its epilogue taken away: which part costs the main loop its efficiency
     if "fwd1_parts" in cases:
         common = dict(a0=x, b0=w1.view(e * f, d), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_BIAS_ACT, n=f, k=d,
@@ -147,6 +152,14 @@ def main():
         report("fwd1_two_outputs_relu", 2 * r * d * f, gemm(act=N.ACT_RELU, out1=pre, **common), kblocks=(d + 63) // 64)
     w2 = torch.randn(e, d, f, device=dev, dtype=torch.bfloat16) * 0.02
     y = torch.empty(r, d, device=dev, dtype=torch.bfloat16)
+    if "fwd2_combine" in cases:
+        # the second projection as the layer launches it: rows scattered into the combine buffer (here in place)
+        slots = torch.arange(r, dtype=torch.int32, device=dev)
+        done = torch.zeros(8, dtype=torch.int32, device=dev)
+        report("fwd2_combine", 2 * r * d * f, gemm(
+            a0=h, b0=w2.view(e * d, f), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_COMBINE, n=d, k=f, group_base=gb, group_rows=gr,
+            num_groups=e, b_group_rows=d, row_src=slots, peer_comb=[y.data_ptr()], peer_done=[done.data_ptr()], send_finish=1,
+            count_rows=0, max_slots=r, ld_out=d, **row_kernel(N.EPI_COMBINE, N.MAJ_K, d)), kblocks=(f + 63) // 64)
     if "fwd2" in cases:
         report("fwd2_store", 2 * r * d * f, gemm(
             a0=h, b0=w2.view(e * d, f), a_major=N.MAJ_K, b_major=N.MAJ_K, epi=N.EPI_STORE, n=d, k=f,
@@ -154,7 +167,8 @@ def main():
     if "dgrad" in cases:
         report("dgrad2_dact", 2 * r * d * f, gemm(
             a0=y, b0=w2.view(e * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_DACT, n=f, k=d,
-            group_base=gb, group_rows=gr, num_groups=e, b_group_rows=d, out0=h, aux0=pre, act=N.ACT_GELU), kblocks=(d + 63) // 64)
+            group_base=gb, group_rows=gr, num_groups=e, b_group_rows=d, out0=h, aux0=pre, act=N.ACT_GELU,
+            **row_kernel(N.EPI_DACT, N.MAJ_MN, f)), kblocks=(d + 63) // 64)
     if "dgrad_plain" in cases:
         report("dgrad2_plain_store", 2 * r * d * f, gemm(
             a0=y, b0=w2.view(e * d, f), a_major=N.MAJ_K, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, k=d,
@@ -164,7 +178,8 @@ def main():
         dw = torch.empty(e, d, f, device=dev, dtype=torch.bfloat16)
         report("wgrad2", 2 * r * d * f, gemm(
             a0=y, b0=h, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, kgroup=True, m_per_group=d,
-            group_base=gb, group_rows=gr, num_groups=e, out0=dw, ld_out=f, few_rows=G.wgrad_few(rows_per, False)), kblocks=(rows_per + 63) // 64)
+            group_base=gb, group_rows=gr, num_groups=e, out0=dw, ld_out=f, few_rows=G.wgrad_few(rows_per, False)),
+            kblocks=(rows_per + 63) // 64)
         del dw
     if "wgrad_sgd" in cases:
         # the same product with the SGD step in its epilogue: w2 is read and rewritten in place, no gradient is stored
@@ -172,8 +187,8 @@ def main():
         h.normal_()
         report("wgrad2_sgd_in_place", 2 * r * d * f, gemm(
             a0=y, b0=h, a_major=N.MAJ_MN, b_major=N.MAJ_MN, epi=N.EPI_STORE, n=f, kgroup=True, m_per_group=d,
-            group_base=gb, group_rows=gr, num_groups=e, out0=w2, ld_out=f, few_rows=G.wgrad_few(rows_per, True), sgd=(1e-6, 0.0)),
-            kblocks=(rows_per + 63) // 64)
+            group_base=gb, group_rows=gr, num_groups=e, out0=w2, ld_out=f, few_rows=G.wgrad_few(rows_per, True),
+            sgd=(1e-6, 0.0)), kblocks=(rows_per + 63) // 64)
     sampler.stop()
     if args.out:
         os.makedirs(os.path.dirname(args.out) or ".", exist_ok=True)
