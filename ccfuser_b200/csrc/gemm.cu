@@ -38,7 +38,8 @@ namespace ccf {
 // the stages smaller and their number larger: a launch that streams weights for a handful of rows is limited by the weight
 // bytes it has in flight, and with 128-column tiles four fixed stages hold 64 KB of them per SM where nine 20 KB stages hold
 // 144 (GEMM-2 of 16 tokens, 16 experts, 1024 x 4096: 43 -> 39 us). Without the bound more stages only hurt: six 32 KB
-// stages for 128-column tiles took 236 us where four take 195 (128 tokens, 8 experts, 4096 x 14336).
+// stages for 128-column tiles took 236 us where four take 195 (128 tokens, 8 experts, 4096 x 14336). The layer's launches come here
+// with CCFUSER_TWO_CTA=0 only; with CTA pairs gemm_swap.cu has them (row_kernel in runtime.cu).
 constexpr int kABytes = BM * BK * 2;
 constexpr int kBBytes = BN * BK * 2;
 constexpr int kPipeBytes = 4 * (kABytes + kBBytes);

@@ -105,7 +105,7 @@ struct CcfGemmArgs {
   int comm_warps;           // 1: the CTA's two dedicated warps run the dispatch role; 0: its epilogue warps do, before their first tile
   float sgd_wd;             // weight decay of that update
   int bn;                   // one-CTA kernel, row-grouped, K-major B: output tile width, 256 (or 0) / 128. The narrow tile doubles
-                            // the number of tiles of a launch that would otherwise leave most SMs idle
+                            // the number of tiles of a launch that would otherwise leave most SMs idle (CCFUSER_TWO_CTA=0)
   int a_rows;               // one-CTA kernel, row-grouped, K-major A: no tile has more than this many rows (32 or 64; 0 / 128 = no
                             // bound). The pipeline then keeps only so many rows of A per stage and holds more stages
   CcfDispatchArgs disp;
