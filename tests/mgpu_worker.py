@@ -108,7 +108,7 @@ def main():
              # every launch on the kernels for few rows: 30 to 250 rows per expert
              ("gelu", None, 500, 4, 256, 512, None), ("swiglu", 2.0, 90, 4, 256, 384, None),
              # ranks whose calls lie on both sides of the kernels' limits, each in turn: 600 and a handful of expected rows
-             ("gelu", None, 1200, 4, 320, 512, 12), ("swiglu", None, 1200, 4, 256, 384, 1)]
+             ("gelu", None, 1200, 4, 384, 512, 12), ("swiglu", None, 1200, 4, 256, 384, 1)]
     worst = 0.0
     for act, cf, tokens, e_loc, d, f, odd_ranks in cases:
         worst = max(worst, run_case(rank, world, act, cf, tokens, e_loc, d, f, odd_ranks))
