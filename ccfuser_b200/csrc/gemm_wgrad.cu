@@ -10,10 +10,10 @@
 //   the epilogue warps update them where they lie (one row per lane; 16-byte accesses of eight lanes fall into different banks), a
 //   store warp writes them back, and a chunk whose store has been read is loaded again. Without weights the chunks are output buffers.
 //
-// Measured, one-CTA / pair / this kernel, cold operands, us: 64 groups of 256 rows, 2048 x 8192: 697 / 670 / 635 plain and 1258 / 1214 /
-// 811 in place (4.3 GB read and written: 5.3 TB/s); 64 x 128 rows: 764 / 709 / 423 and 1167 / 1161 / 836; 16 x 192 rows, 768 x 3072:
-// 45 / 44 / 34 and 68 / 67 / 39; 16 x 512 rows, 2048 x 8192: 277 / 239 / 246 and 340 / 355 / 309. With more rows the main loop
-// decides and the pair kernel's deeper ring wins: 16 x 1024 rows 478 / 417 / 512 and 562 / 467 / 553 (wgrad_few in runtime.cu).
+// Measured, pair kernel / this one, operands of several layers in turn, us (plain and in place): 16 x 256 rows, 768 x 3072: 31 / 25 and 51 / 37; 64 x 256,
+// 1024 x 4096: 186 / 147 and 346 / 219; 64 x 256, 2048 x 8192: 842 / 611 and 1343 / 834 (4.3 GB read and written: 5.1 TB/s);
+// 16 x 512, 2048 x 8192: 255 / 240 and 375 / 283. With more rows the main loop decides, and the pair kernel's deeper ring wins:
+// 16 x 1024 rows 411 / 447 and 478 / 496 (wgrad_few in runtime.cu).
 //
 // Everything else is as in gemm2.cu: CTA pairs, MN-major operands, two accumulators. All waits are bounded; no TMA load uses cluster
 // multicast.
@@ -26,9 +26,13 @@
 
 namespace ccf {
 
-constexpr int kWgStages = 3;                         // k-blocks of operands
+// Four k-blocks of operands beside five chunks. With three and seven a stage's round trip from L2 did not fit behind the other two, and
+// a k-block took 800 clocks instead of 600 (64 x 256 rows, 1024 x 4096, plain: 172 -> 156 us). With four chunks updates in place wait for
+// their weights (64 x 256 rows, 2048 x 8192: 812 -> 866 us); five stages and four chunks are no faster than this.
+constexpr int kWgStages = 4;                         // k-blocks of operands
 constexpr int kWgStageBytes = 2 * BM * BK * 2;       // this CTA's 128 rows of A^T and its half of B
-constexpr int kWgChunks = 7;
+constexpr int kWgChunks = 5;
+static_assert(kWgChunks >= 4, "ChunkPos moves by up to a tile's four chunks and wraps once");
 constexpr int kWgChunkBytes = BM * 64 * 2;
 constexpr int kWgThreads = 384;                      // warps 0 operands, 1 MMA, 2 weights, 3 stores, 4..11 epilogue
 
@@ -58,15 +62,28 @@ template <int kPending>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kPending) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1) : "memory");
+}
+
 struct WgTile {
   int g, m0, n0, kblocks, krow0, chunks;   // chunks: 64-column chunks inside the matrix
 };
+// Stored: along the shorter side of the result first, so that the pairs of a wave share the fewest panels (64 x 384 rows, 2048 x 8192:
+// 885 -> 785 us). In place: columns first, so that a wave reads and writes whole rows of the weights (64 x 512 rows: 1127 against 1276).
+template <bool kSgd>
 __device__ __forceinline__ WgTile decode_wg_tile(int t, const CcfGemmArgs& a, const CtrlW* c, int mt, int nt) {
   WgTile ti;
   ti.g = t / (mt * nt);
   const int local = t - ti.g * (mt * nt);
-  // columns first: the pairs of a wave then cover whole rows of the weights
-  const int i = local / nt, j = local - i * nt;
+  int i, j;
+  if (!kSgd && mt < nt) {
+    j = local / mt;
+    i = local - j * mt;
+  } else {
+    i = local / nt;
+    j = local - i * nt;
+  }
   ti.m0 = i * PM;
   ti.n0 = j * BN;
   ti.kblocks = (c->rows[ti.g] + BK - 1) / BK;
@@ -141,9 +158,29 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     bool ok = true;
     const uint32_t full0 = smem_u32(&ctrl->full[0]), leader0 = map_to_cta(full0, 0), empty0 = smem_u32(&ctrl->empty[0]);
     for (int t = pair; t < total && ok; t += n_pairs, ++seq) {
-      const WgTile ti = decode_wg_tile(t, args, ctrl, mt, nt);
+      const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
       const int m = ti.m0 + static_cast<int>(cta) * BM, n = ti.n0 + static_cast<int>(cta) * (BN / 2);
       if (lane == 0) trace_ev(args, seq, 0);
+      // The operands of this pair's next tile are asked of L2 a tile ahead: four stages do not cover a trip to DRAM, and all pairs of a
+      // wave meet a group's rows for the first time together (64 x 256 rows, 1024 x 4096: 156 -> 145 us). The pairs that share a panel
+      // take its k-blocks in turns. In place the weights decide, and it gives nothing.
+      if constexpr (!kSgd) {
+        if (t + n_pairs < total) {
+          const WgTile nx = decode_wg_tile<kSgd>(t + n_pairs, args, ctrl, mt, nt);
+          const int pm = nx.m0 + static_cast<int>(cta) * BM, pn = nx.n0 + static_cast<int>(cta) * (BN / 2);
+          if (elect_one()) {
+            for (int kb = nx.n0 / BN; kb < nx.kblocks; kb += nt) {
+              tma_prefetch_2d(&tmA, pm, nx.krow0 + kb * BK);
+              tma_prefetch_2d(&tmA, pm + 64, nx.krow0 + kb * BK);
+            }
+            for (int kb = nx.m0 / PM; kb < nx.kblocks; kb += mt) {
+              tma_prefetch_2d(&tmB, pn, nx.krow0 + kb * BK);
+              tma_prefetch_2d(&tmB, pn + 64, nx.krow0 + kb * BK);
+            }
+          }
+          __syncwarp();
+        }
+      }
       for (int kb = 0; kb < ti.kblocks; ++kb) {
         if (!mbar_wait_cluster(empty0 + 8 * stage, phase ^ 1, abort_word, limit)) {
           report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x60);
@@ -172,7 +209,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       int stage = 0, phase = 0, as = 0, aphase = 0, seq = 0;
       bool ok = true;
       for (int t = pair; t < total && ok; t += n_pairs, ++seq) {
-        const WgTile ti = decode_wg_tile(t, args, ctrl, mt, nt);
+        const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
         if (ti.kblocks == 0) continue;   // empty group: the epilogue takes zeros
         if (!mbar_wait_cluster(smem_u32(&ctrl->acc_empty[as]), aphase ^ 1, abort_word, limit)) {
           report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x61);
@@ -213,7 +250,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       ChunkPos pos;
       bool ok = true;
       for (int t = pair; t < total && ok; t += n_pairs) {
-        const WgTile ti = decode_wg_tile(t, args, ctrl, mt, nt);
+        const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
         const int row = ti.g * args.m_per_group + ti.m0 + static_cast<int>(cta) * BM;
         for (int c = 0; c < ti.chunks; ++c, pos.advance(1)) {
           if (!mbar_wait(smem_u32(&ctrl->free_[pos.slot]), pos.phase ^ 1, abort_word, limit)) {
@@ -236,7 +273,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       bool ok = true;
       int pending = 0;   // stores that may still be reading their chunk
       for (int t = pair; t < total && ok; t += n_pairs) {
-        const WgTile ti = decode_wg_tile(t, args, ctrl, mt, nt);
+        const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
         const int row = ti.g * args.m_per_group + ti.m0 + static_cast<int>(cta) * BM;
         for (int c = 0; c < ti.chunks; ++c, pos.advance(1)) {
           if (!mbar_wait(smem_u32(&ctrl->done[pos.slot]), pos.phase, abort_word, limit)) {
@@ -267,7 +304,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // this lane's row of a chunk: 16-byte piece p lies at p ^ (row mod 8)
     const uint32_t row_at = static_cast<uint32_t>((q * 32 + lane) * 128), swz = static_cast<uint32_t>(lane & 7) << 4;
     for (int t = pair; t < total && ok; t += n_pairs, ++seq) {
-      const WgTile ti = decode_wg_tile(t, args, ctrl, mt, nt);
+      const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
       const bool have_acc = ti.kblocks > 0;
       if (have_acc) {
         if (!mbar_wait_cluster(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {

@@ -70,11 +70,12 @@ void set_row_kernel(CcfGemmLaunch& g, const CcfLayer* L, int tokens, int capacit
 
 // Whether a weight-gradient launch of a call that expects `rows` rows per expert runs on gemm_wgrad.cu, which moves its result by TMA,
 // or on the pair kernel: with few rows the reduction is only a handful of k-blocks, and moving the weights decides. In place the
-// weights are read as well as written, and the line lies higher. gemm_wgrad.cu against pair kernel, cold, us:
-//   plain     64 x 256 rows, 2048 x 8192: 646 / 702, 64 x 384: 873 / 823; 64 x 256, 1024 x 4096: 177 / 178, 64 x 512: 288 / 233.
-//             Whole training passes, 300 rows: 64 experts of 2048 x 8192 4957 / 5139, of 1024 x 4096 1350 / 1350; 400 rows: 6086 / 6145
-//             and 1774 / 1678; 16 experts of 1024 x 4096, 400 rows: 517 / 501
-//   in place  64 x 256 rows, 2048 x 8192: 811 / 1214, 16 x 512: 309 / 355, 16 x 1024: 553 / 467
+// weights are read as well as written, and the line lies higher. Both lie on the safe side since gemm_wgrad.cu holds four stages:
+// gemm_wgrad.cu over pair kernel, time, both in alternation:
+//   plain     1024 x 4096, 64 experts: 0.94 at 512 rows, 0.94 at 640, 1.01 at 768; 2048 x 8192, 16: 0.93, 0.95, 1.00, and 1.05 at 1024;
+//             768 x 3072, 16: 0.92, 0.95, 1.02, 1.05; 4096 x 14336, 8: 0.93, 0.92, 0.99
+//   in place  1024 x 4096, 64 experts: 0.83 at 512 rows, 0.94 at 640, 0.99 at 768; 2048 x 8192, 16: 0.79, 0.90, 0.94, and 1.03 at 1024;
+//             4096 x 14336, 8: 0.79, 0.91, 0.97
 bool wgrad_few(long long rows, bool in_place, int two_cta) { return two_cta && rows <= (in_place ? 512 : 384); }
 
 // fields every launch of this layer shares
