@@ -359,6 +359,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
   } else {
     // ======================= epilogue (warps 2..9) =======================
     const int q = warp & 3;               // TMEM lane quarter this warp may read
+    const CUtensorMap* const no_maps[3] = {nullptr, nullptr, nullptr};
     const int half = (warp - 2) >> 2;     // which half of the tile's columns this warp handles
     dispatch_role<kEpi>(args, false);
     if (warp == 2 && lane == 0 && args.trace != nullptr && !args.comm_warps) trace_ev(args, args.trace_tiles - 1, 1);
@@ -387,8 +388,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + ti.row0;
       else row_base = ti.row0;
-      const CombineDest cd = epilogue_tile<kEpi, kFp16>(
-          args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane,
+      const CombineDest cd = epilogue_tile<kEpi, kFp16, false>(
+          args, ti, row_base, ti.rows_valid, BM, have_acc, t_row, stage, q, half, lane, no_maps,
           [&] {
             if (have_acc) {
               if (!mbar_wait(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
@@ -474,9 +475,10 @@ struct TmapKey {
   const void* base;
   long long rows, cols;
   int box_cols, box_rows, fp16;
+  long long ld;
   bool operator==(const TmapKey& o) const {
     return base == o.base && rows == o.rows && cols == o.cols && box_cols == o.box_cols && box_rows == o.box_rows &&
-           fp16 == o.fp16;
+           fp16 == o.fp16 && ld == o.ld;
   }
 };
 struct TmapEntry {
@@ -497,8 +499,9 @@ size_t tmap_hash(const TmapKey& k) {
 }  // namespace
 
 int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows,
-                     int fp16) {
-  const TmapKey key = {base, rows, cols, box_cols, box_rows, fp16};
+                     int fp16, long long ld) {
+  if (ld == 0) ld = cols;
+  const TmapKey key = {base, rows, cols, box_cols, box_rows, fp16, ld};
   const size_t slot = tmap_hash(key);
   {
     std::lock_guard<std::mutex> lock(g_tmap_mutex);
@@ -511,12 +514,12 @@ int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, 
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return -1;
   cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstr[1] = {static_cast<cuuint64_t>(cols) * 2};
+  cuuint64_t gstr[1] = {static_cast<cuuint64_t>(ld) * 2};
   cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                   const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return -static_cast<int>(r) - 1000;
   {
@@ -581,7 +584,7 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     if (!(fwd && a.disp.backward == 0) && !(bwd && a.disp.backward == 1)) return -9;
     if (reinterpret_cast<uintptr_t>(a.disp.x) & 15) return -14;   // the role moves 16 bytes at a time
   }
-  CUtensorMap tm[6];
+  CUtensorMap tm[7];
   const int fp16 = a.fp16;
   const bool swap = L->few_rows && !L->kgroup, wgrad = L->few_rows && L->kgroup;
   if (wgrad && (L->a_major != MAJ_MN || L->b_major != MAJ_MN || L->epi != CCF_EPI_STORE || a.out_fp32 || a.bias0 != nullptr ||
@@ -623,7 +626,18 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     return launch_swap_by_key(L->b_major, L->epi, tm, a, grid, stream);
   }
   const int key = (L->a_major << 12) | (L->b_major << 8) | (L->epi << 4) | (L->kgroup ? 1 : 0);
-  if (pair) return launch_pair_by_key(key, tm, a, grid, stream);
+  if (pair) {
+    // tm[4..6]: the outputs that leave by bulk tensor stores, in boxes of 32 x 32
+    void* const outs[3] = {a.out0, a.out1, a.out2};
+    const bool tma_out = L->epi != CCF_EPI_COMBINE && !(L->epi == CCF_EPI_STORE && (!L->kgroup || a.out_fp32 || a.sgd_lr != 0.f));
+    const long long out_rows = L->kgroup ? static_cast<long long>(a.num_groups) * a.m_per_group : L->a_rows;
+    for (int i = 0; i < 3; ++i) {
+      const void* p = tma_out && outs[i] != nullptr ? outs[i] : nullptr;
+      if (p == nullptr) tm[4 + i] = tm[0];
+      else if ((rc = make_tmap(&tm[4 + i], p, out_rows, a.n, 32, 32, fp16, a.ld_out))) return rc;
+    }
+    return launch_pair_by_key(key, tm, a, grid, stream);
+  }
   switch (key) {
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_STORE << 4):
       return launch_variant<MAJ_K, MAJ_K, CCF_EPI_STORE, false>(tm, a, grid, stream);

@@ -211,11 +211,13 @@ static void pair_tile_tables_host(const CcfGemmArgs& args, Ctrl2* ctrl) {
   pair_tile_totals<false, kEpi>(args, ctrl, acc_a, acc_b, rows);
 }
 
-template <int kAMajor, int kBMajor, int kEpi, bool kKGroup, int kFp16>
+template <int kAMajor, int kBMajor, int kEpi, bool kKGroup, int kFp16, bool kSgd>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                          const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
-                         const __grid_constant__ CcfGemmArgs args) {
+                         const __grid_constant__ CUtensorMap tmC0, const __grid_constant__ CUtensorMap tmC1,
+                         const __grid_constant__ CUtensorMap tmC2, const __grid_constant__ CcfGemmArgs args) {
+  constexpr bool kTma = kEpi != CCF_EPI_COMBINE && (kEpi != CCF_EPI_STORE || (kKGroup && !kSgd));
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Ctrl2* ctrl = reinterpret_cast<Ctrl2*>(smem + k2Stages * k2StageBytes + kEpiWarps * kEpiStageBytes);
@@ -399,6 +401,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     const int half = (warp - 2) >> 2;
     dispatch_role<kEpi>(args, false);
     if (warp == 2 && lane == 0 && args.trace != nullptr && !args.comm_warps) trace_ev(args, args.trace_tiles - 1, 1);
+    const CUtensorMap* const out_map[3] = {&tmC0, &tmC1, &tmC2};
     int as = 0, aphase = 0, seq = 0, hint = 0;
     for (int t = pair; t < total_tiles; t += n_pairs, ++seq) {
       const PairTile ti = decode_pair_tile<kKGroup, kEpi>(t, args, ctrl, hint);
@@ -423,8 +426,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       long long row_base;
       if constexpr (kKGroup) row_base = static_cast<long long>(ti.g) * args.m_per_group + tt.row0;
       else row_base = tt.row0;
-      const CombineDest cd = epilogue_tile<kEpi, kFp16>(
-          args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane,
+      const CombineDest cd = epilogue_tile<kEpi, kFp16, kTma>(
+          args, tt, row_base, my_rows, rows_store, have_acc, t_row, stage, q, half, lane, out_map,
           [&] {
             if (have_acc) {
               if (!mbar_wait_cluster(smem_u32(&ctrl->acc_full[as]), aphase, abort_word, limit)) {
@@ -447,6 +450,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       if (have_acc && ++as == 2) { as = 0; aphase ^= 1; }
       if constexpr (kEpi == CCF_EPI_COMBINE) combine_signal(args, cd, lane);
       (void)cd;
+    }
+    if constexpr (kTma) {
+      if (elect_one()) bulk_wait_all();
+      __syncwarp();
     }
   }
 
@@ -481,9 +488,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
   }
 }
 
-template <int A, int B, int E, bool KG, int FP16>
+template <int A, int B, int E, bool KG, int FP16, bool SGD>
 static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
-  auto kern = grouped_gemm_pair_kernel<A, B, E, KG, FP16>;
+  auto kern = grouped_gemm_pair_kernel<A, B, E, KG, FP16, SGD>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
   int dev = 0;
@@ -501,14 +508,19 @@ static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args
   cudaLaunchAttribute attr[1] = {cluster_attribute(2, 1, 1)};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], args);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], tm[6], args);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 template <int A, int B, int E, bool KG>
 static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
-  return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1>(tm, args, grid, stream)
-                   : launch_pair_variant_of<A, B, E, KG, 0>(tm, args, grid, stream);
+  if constexpr (E == CCF_EPI_STORE && KG) {   // in place or in fp32 the result leaves by plain stores
+    if (args.sgd_lr != 0.f || args.out_fp32)
+      return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, true>(tm, args, grid, stream)
+                       : launch_pair_variant_of<A, B, E, KG, 0, true>(tm, args, grid, stream);
+  }
+  return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, false>(tm, args, grid, stream)
+                   : launch_pair_variant_of<A, B, E, KG, 0, false>(tm, args, grid, stream);
 }
 
 // Called by ccf_gemm_launch (gemm.cu) when the two-CTA kernel is requested. `key` encodes (A-major, B-major, epilogue,

@@ -23,7 +23,7 @@ constexpr int kEpiStageBytes = 2048;  // per epilogue warp: 32 rows x 64 bytes, 
 
 // Host: tensor map of a 2-D row-major view [rows, cols] of 2-byte elements with box {box_cols, box_rows} and 128-byte
 // swizzle (defined in gemm.cu). Returns 0 or a negative error code.
-int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows, int fp16);
+int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows, int fp16, long long ld = 0);
 
 // Descriptor of an operand in a pipeline stage as the MMA reads it: its base, the step of one 16-deep MMA, and any other place in
 // shared memory (only the 14 address bits differ, in units of 16 bytes; shared memory ends below 2^18).
@@ -45,44 +45,56 @@ struct Tile {
 // ---------------------------------------------------------------------------------------------------
 // epilogue math
 // ---------------------------------------------------------------------------------------------------
-// erf as an odd polynomial: erf(z) ~= z * P(z^2) on |z| <= 3 (degree 8 in z^2, fitted minimax-style; |error| <= 2.6e-5
-// in fp32 Horner form, erf(3) = 1 - 2.2e-5 beyond the clamp), far below bf16 / fp16 resolution. No MUFU operation and
-// no branch: libm's erff and the exp/rcp-based forms kept the SFU pipe busy for ~4 k cycles per 128x256 tile.
+// The normal distribution function, 1/2 + x Q(x^2), saturated to [0, 1]: Q is a degree-8 polynomial in x^2 (erf(z) ~= z P(z^2) on
+// |z| <= 3, fitted minimax-style, with z = x / sqrt 2 folded into the coefficients; |error| <= 1.3e-5 in fp32 Horner form), x^2 held at
+// its end of the range, 18. Beyond it x Q(18) passes 1/2 and the saturation gives 0 and 1 themselves. No MUFU operation and no branch:
+// libm's erff and the exp/rcp-based forms kept the SFU pipe busy for ~4 k cycles per 128x256 tile.
 // Two elements at a time (packed fp32 multiply-adds): the epilogue warps are bound by the instructions they issue, and the
-// polynomial is most of an activation epilogue's.
-__device__ __forceinline__ f32x2 erf_poly2(f32x2 z) {
-  float z0, z1;
-  upk2(z, z0, z1);
-  z = pk2(fminf(fmaxf(z0, -3.f), 3.f), fminf(fmaxf(z1, -3.f), 3.f));
-  const f32x2 u = mul2(z, z);
-  f32x2 p = bc2(4.074189994e-08f);
-  p = fma2(p, u, bc2(-1.944814854e-06f));
-  p = fma2(p, u, bc2(4.106040073e-05f));
-  p = fma2(p, u, bc2(-5.110358431e-04f));
-  p = fma2(p, u, bc2(4.235422620e-03f));
-  p = fma2(p, u, bc2(-2.510284860e-02f));
-  p = fma2(p, u, bc2(1.110793178e-01f));
-  p = fma2(p, u, bc2(-3.753148649e-01f));
-  p = fma2(p, u, bc2(1.128268424e+00f));
-  return mul2(p, z);
+// polynomial is most of an activation epilogue's. Squares held from above and a sum that saturates take 14 instructions per pair and
+// activation where a clamped argument took 17, and 19 where 27 for the derivative.
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float y;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+__device__ __forceinline__ f32x2 normal_cdf2(float x0, float x1, f32x2 square) {
+  float u0, u1;
+  upk2(square, u0, u1);
+  const f32x2 u = pk2(fminf(u0, 18.f), fminf(u1, 18.f));
+  f32x2 p = bc2(5.626733150e-11f);
+  p = fma2(p, u, bc2(-5.371842857e-09f));
+  p = fma2(p, u, bc2(2.268288109e-07f));
+  p = fma2(p, u, bc2(-5.646201720e-06f));
+  p = fma2(p, u, bc2(9.359050174e-05f));
+  p = fma2(p, u, bc2(-1.109399655e-03f));
+  p = fma2(p, u, bc2(9.818117358e-03f));
+  p = fma2(p, u, bc2(-6.634692151e-02f));
+  p = fma2(p, u, bc2(3.989031268e-01f));
+  upk2(p, u0, u1);
+  return pk2(fma_sat(x0, u0, 0.5f), fma_sat(x1, u1, 0.5f));
 }
 __device__ __forceinline__ float fast_rcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));  // branch-free, 1 ulp: keeps the element loops interleavable
   return y;
 }
-__device__ __forceinline__ void gelu2(float& x0, float& x1) {
-  const f32x2 x = pk2(x0, x1), hx = mul2(x, bc2(0.5f));
-  upk2(fma2(hx, erf_poly2(mul2(x, bc2(0.70710678118654752f))), hx), x0, x1);
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
-// f *= gelu'(x)
-__device__ __forceinline__ void gelu_grad2(float& f0, float& f1, float x0, float x1) {
+__device__ __forceinline__ void gelu2(float& x0, float& x1) {
   const f32x2 x = pk2(x0, x1);
-  const f32x2 cdf = fma2(bc2(0.5f), erf_poly2(mul2(x, bc2(0.70710678118654752f))), bc2(0.5f));
+  upk2(mul2(x, normal_cdf2(x0, x1, mul2(x, x))), x0, x1);
+}
+// f *= gelu'(x) = cdf(x) + x pdf(x)
+__device__ __forceinline__ void gelu_grad2(float& f0, float& f1, float x0, float x1) {
+  const f32x2 x = pk2(x0, x1), square = mul2(x, x);
+  const f32x2 cdf = normal_cdf2(x0, x1, square);
   float e0, e1;
-  upk2(mul2(mul2(bc2(-0.5f), x), x), e0, e1);
-  const f32x2 pdf = mul2(bc2(0.3989422804014327f), pk2(__expf(e0), __expf(e1)));
-  upk2(mul2(pk2(f0, f1), fma2(x, pdf, cdf)), f0, f1);
+  upk2(mul2(square, bc2(-0.72134752044448170f)), e0, e1);   // -x^2 / 2 as a power of two
+  const f32x2 density = pk2(fast_exp2(e0), fast_exp2(e1));
+  upk2(mul2(pk2(f0, f1), fma2(mul2(x, bc2(0.3989422804014327f)), density, cdf)), f0, f1);
 }
 // The activation switch sits outside the element loop: with a branch per element the compiler cannot
 // interleave the 32 independent dependency chains and the epilogue ran ~200 clocks per element.
@@ -222,6 +234,51 @@ __device__ __forceinline__ void staged_store64(uint32_t stage, int lane, const u
   __syncwarp();
 }
 
+// Bulk tensor stores. The staging area is laid out as the 64-byte swizzle has it, so that a staged chunk can leave as one box of 32
+// columns x 32 rows: the CTA-pair kernel stores its activations, their gradients and weight gradients so. Read back and stored by the
+// warp itself a chunk took eight more shared- and global-memory instructions and two turns through the staging area in the warp's own
+// chain. Saved pre-activations come straight into their row's lane: the second quarter of a sector is an L1 hit. 4 groups of 4096 rows,
+// 1024 x 4096, clocks per launch, with the shorter normal_cdf2 and the accumulator read when it is due (32 registers fewer):
+// GELU 193 k -> 167 k, GELU' 228 k -> 176 k (of 120 k that the MMAs take).
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t smem_src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(m)),
+               "r"(smem_src), "r"(c0), "r"(c1)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kPending) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void staged_store_tma(uint32_t stage, int lane, const uint32_t (&w)[16], const CUtensorMap* m, int col, int row) {
+  if (elect_one()) bulk_wait_read<0>();   // the store before this one has read the staging area
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + stage_off(lane, j)), "r"(w[4 * j]), "r"(w[4 * j + 1]),
+                 "r"(w[4 * j + 2]), "r"(w[4 * j + 3])
+                 : "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (elect_one()) {
+    tma_store_2d(m, stage, col, row);
+    bulk_commit();
+  }
+  __syncwarp();
+}
+// one lane's 64 bytes of a row that the launch only reads
+__device__ __forceinline__ void fetch_row64(unsigned long long p, bool ok, uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (ok) v = __ldg(reinterpret_cast<const uint4*>(p) + i);
+    w[4 * i] = v.x;
+    w[4 * i + 1] = v.y;
+    w[4 * i + 2] = v.z;
+    w[4 * i + 3] = v.w;
+  }
+}
+
 __device__ __forceinline__ void pack32(const float (&f)[32], uint32_t (&w)[16], int fp16) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) w[i] = pack2(f[2 * i], f[2 * i + 1], fp16);
@@ -252,6 +309,7 @@ __device__ __forceinline__ void trace_ev(const CcfGemmArgs& a, int seq, int ev) 
 //   row_base     first output row of this CTA's 128 accumulator rows (group offset included for k-grouped mode)
 //   rows_valid   rows of this CTA's part that hold data
 //   rows_store   rows of this CTA's part that may be written at all (rows in [rows_valid, rows_store) get zeros)
+//   out_map      kTma: tensor maps of the outputs (boxes of 32 x 32), which leave by bulk tensor stores
 //   acquire      waits for the accumulator (false: given up); what the first chunk needs from global memory is requested before
 //   release      hands the accumulator back to the MMA warp; called once the warp's last part of it is in registers, with that part's
 //                arithmetic and stores still to come
@@ -345,10 +403,11 @@ __device__ __forceinline__ void unstage(uint32_t stage, int lane, const uint4 (&
 
 // kFp16 is a template argument: as a run-time value every conversion of an element pair computed both types' results and
 // selected one, about a third of an epilogue's instructions.
-template <int kEpi, int kFp16, typename Acquire, typename Release>
+template <int kEpi, int kFp16, bool kTma, typename Acquire, typename Release>
 __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, const Tile& ti, long long row_base,
                                                      int rows_valid, int rows_store, bool have_acc, uint32_t t_row,
-                                                     uint32_t stage, int q, int half, int lane, Acquire acquire, Release release) {
+                                                     uint32_t stage, int q, int half, int lane, const CUtensorMap* const (&out_map)[3],
+                                                     Acquire acquire, Release release) {
   constexpr int fp16 = kFp16;
   CombineDest cd;
   cd.rank = 0;
@@ -392,14 +451,16 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
       for (int c = 0; c < n_chunks; ++c) {
         const int n = ti.n0 + (chunk0 + c) * 32;
         if (n >= args.n || ok == 0) break;
-        auto put = [&](void* p) {
-          if (p != nullptr)
+        auto put = [&](void* p, int i) {
+          if (p == nullptr) return;
+          if constexpr (kTma) staged_store_tma(stage, lane, zero, out_map[i], n, static_cast<int>(row_base) + q * 32);
+          else
             staged_store64_lin(stage, lane, zero, addr2(p, row_base + q * 32, args.ld_out, n),
                                static_cast<unsigned long long>(args.ld_out) * 2ull, ok);
         };
-        put(args.out0);
-        if constexpr (kEpi != CCF_EPI_DACT) put(args.out1);
-        if constexpr (kEpi == CCF_EPI_SWIGLU) put(args.out2);
+        put(args.out0, 0);
+        if constexpr (kEpi != CCF_EPI_DACT) put(args.out1, 1);
+        if constexpr (kEpi == CCF_EPI_SWIGLU) put(args.out2, 2);
       }
     }
     return cd;
@@ -418,20 +479,32 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
   const int lin_rows_store = min(32, max(0, rows_store - q * 32));
   auto lin_of = [&](const void* p) { return addr2(p, row_base + q * 32, args.ld_out, 0); };
   const unsigned long long lin_base = lin_of(args.out0);
+  // a chunk of the warp's 32 rows into output i
+  auto put = [&](const uint32_t (&w)[16], int i, void* p, int n) {
+    if constexpr (kTma) {
+      if (lin_rows_store > 0) staged_store_tma(stage, lane, w, out_map[i], n, static_cast<int>(row_base) + q * 32);
+    } else {
+      staged_store64_lin(stage, lane, w, lin_of(p) + n * 2ull, lin_stride, lin_rows_store);
+    }
+  };
   if (sgd) sgd_fetch_lin(lin_base + (ti.n0 + chunk0 * 32) * 2ull, lin_stride, ti.n0 + chunk0 * 32 < args.n ? lin_rows : 0, lane, bnext);
   // DACT, DSWIGLU: the saved pre-activations, one chunk ahead like the bias: loaded where they are used, each chunk of a tile
   // waited for one more trip to memory (4 experts x 4096 rows, 1024 -> 4096, GELU': 151 us a launch, 144 so)
   uint4 unext[4];
+  uint32_t arow[16], urow[16];   // kTma: this lane's row, no staging
   auto fetch_aux = [&](int c) {
     const int n = ti.n0 + c * 32, ok = n < args.n ? lin_rows : 0;
-    if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux0) + n * 2ull, lin_stride, ok, lane, bnext);
-    if constexpr (kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux1) + n * 2ull, lin_stride, ok, lane, unext);
+    if constexpr (kTma) {
+      if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) fetch_row64(lin_of(args.aux0) + n * 2ull + lane * lin_stride, lane < ok, arow);
+      if constexpr (kEpi == CCF_EPI_DSWIGLU) fetch_row64(lin_of(args.aux1) + n * 2ull + lane * lin_stride, lane < ok, urow);
+    } else {
+      if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux0) + n * 2ull, lin_stride, ok, lane, bnext);
+      if constexpr (kEpi == CCF_EPI_DSWIGLU) fetch_lin(lin_of(args.aux1) + n * 2ull, lin_stride, ok, lane, unext);
+    }
   };
   fetch_aux(chunk0);
   if (!acquire()) return cd;
   cd.here = true;
-  uint32_t racc[32];  // one buffer: the next chunk is requested right after this one is copied out to f[]
-  if (have_acc) tmem_ld32(t_row + chunk0 * 32, racc);
   // not unrolled: the body is large and every launch pays for fetching the kernel's code once per SM
 #pragma unroll 1
   for (int c = 0; c < n_chunks; ++c) {
@@ -446,12 +519,12 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
     if (sgd && c + 1 < n_chunks)
       sgd_fetch_lin(lin_base + (n + 32) * 2ull, lin_stride, n + 32 < args.n ? lin_rows : 0, lane, bnext);
     if (have_acc) {
+      uint32_t racc[32];
+      tmem_ld32(t_row + cg * 32, racc);
       tmem_ld_wait();
       acc_to_float(racc, f);
       if constexpr (kEpi != CCF_EPI_SWIGLU) {
-        // next chunk's TMEM load overlaps this chunk's math and stores
-        if (c + 1 < n_chunks) tmem_ld32(t_row + (cg + 1) * 32, racc);
-        else release();
+        if (c + 1 == n_chunks) release();
       }
     } else {
 #pragma unroll
@@ -461,11 +534,11 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
       // f = gate pre-activation (accumulator columns cg*32..), u = up pre-activation (+128)
       float u[32];
       if (have_acc) {
+        uint32_t racc[32];
         tmem_ld32(t_row + 128 + cg * 32, racc);
         tmem_ld_wait();
         acc_to_float(racc, u);
-        if (c + 1 < n_chunks) tmem_ld32(t_row + (cg + 1) * 32, racc);
-        else release();
+        if (c + 1 == n_chunks) release();
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) u[i] = 0.f;
@@ -489,11 +562,11 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         }
         if (args.out1) {
           pack32(f, w, fp16);
-          staged_store64_lin(stage, lane, w, lin_of(args.out1) + n * 2ull, lin_stride, lin_rows_store);
+          put(w, 1, args.out1, n);
         }
         if (args.out2) {
           pack32(u, w, fp16);
-          staged_store64_lin(stage, lane, w, lin_of(args.out2) + n * 2ull, lin_stride, lin_rows_store);
+          put(w, 2, args.out2, n);
         }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
@@ -501,7 +574,7 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
           upk2(mul2(mul2(pk2(f[i], f[i + 1]), sg), pk2(u[i], u[i + 1])), f[i], f[i + 1]);
         }
         pack32(f, w, fp16);
-        staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
+        put(w, 0, args.out0, n);
       }
     } else if (n < args.n) {  // column edge: chunks beyond the matrix are skipped
       if constexpr (kEpi == CCF_EPI_STORE) {
@@ -524,21 +597,22 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
           staged_store64_lin(stage, lane, w, lin_base + n * 2ull, lin_stride, lin_rows);
         } else {
           pack32(f, w, fp16);
-          staged_store64_lin(stage, lane, w, lin_base + n * 2ull, lin_stride, lin_rows);
+          if constexpr (kTma) staged_store_tma(stage, lane, w, out_map[0], n, static_cast<int>(row_base) + q * 32);
+          else staged_store64_lin(stage, lane, w, lin_base + n * 2ull, lin_stride, lin_rows);
         }
       } else if constexpr (kEpi == CCF_EPI_BIAS_ACT) {
         if (has_b0) add_bias_raw(f, bcur, fp16);
-        if (!valid) {
+        if (lin_rows < 32 && !valid) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) f[i] = 0.f;
         }
         if (args.out1) {
           pack32(f, w, fp16);
-          staged_store64_lin(stage, lane, w, lin_of(args.out1) + n * 2ull, lin_stride, lin_rows_store);
+          put(w, 1, args.out1, n);
         }
         act32(f, args.act);  // rows beyond the group hold zeros: act(0) = 0 for every supported activation
         pack32(f, w, fp16);
-        staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
+        put(w, 0, args.out0, n);
       } else if constexpr (kEpi == CCF_EPI_COMBINE) {
         if (has_b0) add_bias_raw(f, bcur, fp16);
 #pragma unroll
@@ -547,30 +621,42 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
         // peer stores over NVLink (or local when c_rank is this rank), 64 contiguous bytes per row
         staged_store64(stage, lane, w, c_ok ? addr2(args.peer_comb[c_rank], c_slot, args.ld_out, n) : 0ull);
       } else if constexpr (kEpi == CCF_EPI_DACT) {
-        unstage(stage, lane, bcur, w);
-        if (c + 1 < n_chunks) fetch_aux(cg + 1);
         {
           float pz[32];
-          unpack32(w, pz, fp16);
+          if constexpr (kTma) {
+            unpack32(arow, pz, fp16);
+          } else {
+            unstage(stage, lane, bcur, w);
+            unpack32(w, pz, fp16);
+          }
+          if (c + 1 < n_chunks) fetch_aux(cg + 1);
           act_grad32(f, pz, args.act);
-          if (!valid) {
+          if (lin_rows < 32 && !valid) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = 0.f;
           }
         }
         pack32(f, w, fp16);
-        staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
+        put(w, 0, args.out0, n);
       } else if constexpr (kEpi == CCF_EPI_DSWIGLU) {
         uint32_t wu[16];
-        unstage(stage, lane, bcur, w);
-        unstage(stage, lane, unext, wu);
+        if constexpr (kTma) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            w[j] = arow[j];
+            wu[j] = urow[j];
+          }
+        } else {
+          unstage(stage, lane, bcur, w);
+          unstage(stage, lane, unext, wu);
+        }
         if (c + 1 < n_chunks) fetch_aux(cg + 1);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           dswiglu2(valid ? f[2 * j] : 0.f, valid ? f[2 * j + 1] : 0.f, w[j], wu[j], fp16);
         }
-        staged_store64_lin(stage, lane, w, lin_of(args.out0) + n * 2ull, lin_stride, lin_rows_store);
-        staged_store64_lin(stage, lane, wu, lin_of(args.out1) + n * 2ull, lin_stride, lin_rows_store);
+        put(w, 0, args.out0, n);
+        put(wu, 1, args.out1, n);
       }
     }
   }
