@@ -51,6 +51,21 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int fp16) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// whether the phase of this parity has completed; never waits
+__device__ __forceinline__ bool mbar_phase_done(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // One warp works on chunks of kChunk consecutive positions of the destination order (rows of this rank's own experts
 // first, then the next owner's, ...; inside an expert in position order), claimed from a shared counter. Consecutive
 // positions land on consecutive rows of one receive buffer, so tiles fill up one after the other: the owner's GEMM can
@@ -62,8 +77,10 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int fp16) {
 // Not inlined, and one instantiation per direction: the role keeps kChunk rows' worth of pointers and data in registers
 // (the backward form twice as much), which must not be added to the register budget of the GEMM roles it shares a
 // kernel with (168 registers per thread at 320 threads).
+// `stop_bar`: a barrier in shared memory whose first phase ends the role of this warp (0: none). It finishes the chunk that it has
+// claimed and claims no other; warps without one push whatever is left.
 template <int kChunk, bool kBackward>
-__device__ __noinline__ void dispatch_rows(const CcfDispatchArgs& a, int* status) {
+__device__ __noinline__ void dispatch_rows(const CcfDispatchArgs& a, int* status, uint32_t stop_bar = 0) {
   static_assert(kChunk <= 16, "one lane per row of a chunk; rows of a chunk are held in registers");
   // Scalars used inside the copy loops are read once: `a` arrives by reference, so the compiler must assume that the
   // row stores below may alias it and would otherwise reload them after every store.
@@ -82,7 +99,8 @@ __device__ __noinline__ void dispatch_rows(const CcfDispatchArgs& a, int* status
   for (;;) {
     const int c = __shfl_sync(0xffffffffu, c_next, 0);
     if (c >= n_chunks) break;
-    if (lane == 0) c_next = atomicAdd(a.work_counter, 1);
+    const bool last = stop_bar != 0 && mbar_phase_done(stop_bar, 0);
+    if (lane == 0) c_next = last ? n_chunks : atomicAdd(a.work_counter, 1);
     const int i0 = c * kChunk;
     const int ns = min(kChunk, kept - i0);
     // lane i plans the row at position i0 + i of the destination order
@@ -158,27 +176,36 @@ __device__ __noinline__ void dispatch_rows(const CcfDispatchArgs& a, int* status
                     ? reinterpret_cast<const uint4*>(saved_comb) + static_cast<size_t>(slot[i]) * vecs
                     : nullptr;
       }
-      for (int v = lane; v < vecs; v += 32) {
-        uint4 xr[kChunk], cr[kChunk];
+      constexpr int kU = 8 / kChunk > 0 ? 8 / kChunk : 1;
+      for (int v0 = lane; v0 < vecs; v0 += 32 * kU) {
+        uint4 xr[kChunk][kU], cr[kChunk][kU];
 #pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
-          if (src[i]) xr[i] = __ldg(src[i] + v);
-          cr[i] = sv[i] ? __ldg(sv[i] + v) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < kU; ++u) {
+          const int v = v0 + 32 * u;
+#pragma unroll
+          for (int i = 0; i < kChunk; ++i) {
+            if (src[i] && v < vecs) xr[i][u] = __ldg(src[i] + v);
+            cr[i][u] = sv[i] && v < vecs ? __ldg(sv[i] + v) : make_uint4(0, 0, 0, 0);
+          }
         }
 #pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
-          if (!dst[i]) continue;
-          const uint32_t xi[4] = {xr[i].x, xr[i].y, xr[i].z, xr[i].w};
-          const uint32_t ci[4] = {cr[i].x, cr[i].y, cr[i].z, cr[i].w};
-          uint32_t o[4];
+        for (int u = 0; u < kU; ++u) {
+          const int v = v0 + 32 * u;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 xf = unpack2(xi[q], fp16);
-            const float2 cf = unpack2(ci[q], fp16);
-            dot[i] += xf.x * cf.x + xf.y * cf.y;
-            o[q] = pack2(xf.x * g[i], xf.y * g[i], fp16);
+          for (int i = 0; i < kChunk; ++i) {
+            if (!dst[i] || v >= vecs) continue;
+            const uint32_t xi[4] = {xr[i][u].x, xr[i][u].y, xr[i][u].z, xr[i][u].w};
+            const uint32_t ci[4] = {cr[i][u].x, cr[i][u].y, cr[i][u].z, cr[i][u].w};
+            uint32_t o[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float2 xf = unpack2(xi[q], fp16);
+              const float2 cf = unpack2(ci[q], fp16);
+              dot[i] += xf.x * cf.x + xf.y * cf.y;
+              o[q] = pack2(xf.x * g[i], xf.y * g[i], fp16);
+            }
+            dst[i][v] = make_uint4(o[0], o[1], o[2], o[3]);
           }
-          dst[i][v] = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
 #pragma unroll

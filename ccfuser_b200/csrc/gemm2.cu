@@ -399,7 +399,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     // ======================= epilogue (warps 2..9, both CTAs) =======================
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
-    dispatch_role<kEpi>(args, false);
+    dispatch_role<kEpi, true>(args, false, smem_u32(&ctrl->acc_full[0]));
     if (warp == 2 && lane == 0 && args.trace != nullptr && !args.comm_warps) trace_ev(args, args.trace_tiles - 1, 1);
     const CUtensorMap* const out_map[3] = {&tmC0, &tmC1, &tmC2};
     int as = 0, aphase = 0, seq = 0, hint = 0;

@@ -632,7 +632,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
     // ======================= epilogue (warps 2..9, both CTAs) =======================
     const int q = warp & 3;
     const int hw = (warp - 2) >> 2;
-    dispatch_role<kEpi>(args, false);
+    dispatch_role<kEpi>(args, false, smem_u32(&ctrl->acc_full[0]));
     if (warp == 2 && lane == 0 && args.trace != nullptr && !args.comm_warps) trace_ev(args, args.trace_tiles - 1, 1);
     int buf = 0, bphase = 0, seq = 0;
     bool ok = true;
