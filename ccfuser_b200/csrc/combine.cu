@@ -36,6 +36,7 @@ __device__ __forceinline__ void add_piece(float (&acc)[8], const uint4& x, float
 template <int kK, bool kRouter>
 __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __grid_constant__ CcfReduceArgs a) {
   const int vecs = a.d >> 3, K = kK > 0 ? kK : a.top_k, fp16 = a.fp16;
+  after_previous();
   if (blockIdx.x == 0 && a.done != nullptr) {
     if (threadIdx.x == 0) {
       const int target = *a.cum + *a.sent_rows * a.n_tiles + 1;
@@ -45,8 +46,10 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
     }
     for (int i = threadIdx.x; i < a.zero_count; i += kReduceThreads) a.zero_words[i] = 0;
   }
-  const uint4* comb = reinterpret_cast<const uint4*>(a.comb);
-  const uint4* wg = reinterpret_cast<const uint4*>(a.wg);
+  const uint4* comb = behind(reinterpret_cast<const uint4*>(a.comb));
+  const uint4* wg = behind(reinterpret_cast<const uint4*>(a.wg));
+  const int *const slot_row = behind(a.slot_row), *const idx = behind(a.idx);
+  const float* const gate_w = behind(a.w);
   constexpr int kP = reduce_pieces(kK), kSpan = kReduceThreads * kP, kN = kK > 0 ? kK : kMaxK;
   // pieces kSpan * block + thread (+ 256, ...) of [tokens, vecs], without a product that may not fit 32 bits: `vecs` blocks are
   // kSpan tokens
@@ -58,7 +61,7 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
     const size_t s0 = static_cast<size_t>(t) * K + j0;
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
-      on[p][j] = t < a.tokens && j0 + j < K && __ldg(a.slot_row + s0 + j) >= 0;
+      on[p][j] = t < a.tokens && j0 + j < K && __ldg(slot_row + s0 + j) >= 0;
       x[p][j] = make_uint4(0u, 0u, 0u, 0u);
       if (on[p][j]) x[p][j] = comb[(s0 + j) * vecs + v];
     }
@@ -84,14 +87,14 @@ __global__ void __launch_bounds__(kReduceThreads) combine_reduce_kernel(const __
       float dot = 0.f;
 #pragma unroll
       for (int j = 0; j < kN; ++j) {
-        w[j] = j < K ? __ldg(a.w + s0 + j) : 0.f;
+        w[j] = j < K ? __ldg(gate_w + s0 + j) : 0.f;
         dw[j] = on[p][j] ? a.dw[s0 + j] : 0.f;
         dot = fmaf(w[j], dw[j], dot);
       }
 #pragma unroll
       for (int j = 0; j < kN; ++j) {
         if (j >= K) continue;
-        const int e = __ldg(a.idx + s0 + j);
+        const int e = __ldg(idx + s0 + j);
         const bool routed = e >= 0 && e < a.e;
         const float g = routed ? w[j] * (dw[j] - dot) : 0.f;
         if (v == 0) a.g[s0 + j] = g;
@@ -208,8 +211,14 @@ int ccf_reduce(const CcfReduceArgs* a, void* stream) {
                                            combine_reduce_kernel<3, true>, combine_reduce_kernel<4, true>, combine_reduce_kernel<5, true>,
                                            combine_reduce_kernel<6, true>, combine_reduce_kernel<7, true>, combine_reduce_kernel<8, true>};
   const Kernel kern = a->wg != nullptr ? router[a->top_k] : plain[a->top_k > kMaxK ? 0 : a->top_k];
-  kern<<<static_cast<unsigned>(blocks), kReduceThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
-  cudaError_t err = cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(kReduceThreads);
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1] = {early_attribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = a->early;
+  cudaError_t err = cudaLaunchKernelEx(&cfg, kern, *a);
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }
 

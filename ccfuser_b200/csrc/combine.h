@@ -49,6 +49,7 @@ struct CcfReduceArgs {
   const void* wg;            // [e, d]
   float* g;
   int tokens, top_k, d, e, fp16;
+  int early;                 // 1: may be set up while the kernel in front of it still runs (sm100.cuh)
 };
 
 extern "C" int ccf_reduce(const CcfReduceArgs* a, void* stream);

@@ -618,12 +618,12 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
   }
   if (wgrad) {
     if ((rc = make_tmap(&tm[4], a.out0, static_cast<long long>(a.num_groups) * a.m_per_group, a.n, 64, BM, fp16))) return rc;
-    return launch_wgrad(tm, a, grid, stream);
+    return launch_wgrad(tm, a, grid, L->early, stream);
   }
   if (swap) {
     if ((rc = make_tmap(&tm[4], L->a0, L->a_rows, L->a_cols, 64, swap_box_rows(true), fp16))) return rc;
     if ((rc = make_tmap(&tm[5], L->a1 ? L->a1 : L->a0, L->a_rows, L->a_cols, 64, swap_box_rows(true), fp16))) return rc;
-    return launch_swap_by_key(L->b_major, L->epi, tm, a, grid, stream);
+    return launch_swap_by_key(L->b_major, L->epi, tm, a, grid, L->early, stream);
   }
   const int key = (L->a_major << 12) | (L->b_major << 8) | (L->epi << 4) | (L->kgroup ? 1 : 0);
   if (pair) {
@@ -636,7 +636,7 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
       if (p == nullptr) tm[4 + i] = tm[0];
       else if ((rc = make_tmap(&tm[4 + i], p, out_rows, a.n, 32, 32, fp16, a.ld_out))) return rc;
     }
-    return launch_pair_by_key(key, tm, a, grid, stream);
+    return launch_pair_by_key(key, tm, a, grid, L->early, stream);
   }
   switch (key) {
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_STORE << 4):

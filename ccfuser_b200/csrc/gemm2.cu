@@ -228,7 +228,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int n_pairs = static_cast<int>(gridDim.x) >> 1;
   volatile int* abort_word = &ctrl->abort_word;
-  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
 
   // ---- set-up ------------------------------------------------------------------------------------
   if (threadIdx.x == 0) {
@@ -254,6 +253,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
+  after_previous();
+  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   if (warp == 2) pair_tile_tables_warp<kKGroup, kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
@@ -489,7 +490,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
 }
 
 template <int A, int B, int E, bool KG, int FP16, bool SGD>
-static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, int early, cudaStream_t stream) {
   auto kern = grouped_gemm_pair_kernel<A, B, E, KG, FP16, SGD>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
@@ -505,46 +506,46 @@ static int launch_pair_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = k2SmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {cluster_attribute(2, 1, 1)};
+  cudaLaunchAttribute attr[2] = {cluster_attribute(2, 1, 1), early_attribute()};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], tm[6], args);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 template <int A, int B, int E, bool KG>
-static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+static int launch_pair_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, int early, cudaStream_t stream) {
   if constexpr (E == CCF_EPI_STORE && KG) {   // in place or in fp32 the result leaves by plain stores
     if (args.sgd_lr != 0.f || args.out_fp32)
-      return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, true>(tm, args, grid, stream)
-                       : launch_pair_variant_of<A, B, E, KG, 0, true>(tm, args, grid, stream);
+      return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, true>(tm, args, grid, early, stream)
+                       : launch_pair_variant_of<A, B, E, KG, 0, true>(tm, args, grid, early, stream);
   }
-  return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, false>(tm, args, grid, stream)
-                   : launch_pair_variant_of<A, B, E, KG, 0, false>(tm, args, grid, stream);
+  return args.fp16 ? launch_pair_variant_of<A, B, E, KG, 1, false>(tm, args, grid, early, stream)
+                   : launch_pair_variant_of<A, B, E, KG, 0, false>(tm, args, grid, early, stream);
 }
 
 // Called by ccf_gemm_launch (gemm.cu) when the two-CTA kernel is requested. `key` encodes (A-major, B-major, epilogue,
 // k-grouped) exactly as there. Returns -6 for a combination that has no two-CTA instantiation.
-int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream) {
+int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream) {
   switch (key) {
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_STORE << 4):
-      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_STORE, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_STORE, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_BIAS_ACT << 4):
-      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_BIAS_ACT, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_BIAS_ACT, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_SWIGLU << 4):
-      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_SWIGLU, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_SWIGLU, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_K << 8) | (CCF_EPI_COMBINE << 4):
-      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_COMBINE, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_K, CCF_EPI_COMBINE, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_MN << 8) | (CCF_EPI_STORE << 4):
-      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_STORE, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_STORE, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_MN << 8) | (CCF_EPI_DACT << 4):
-      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_DACT, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_DACT, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_MN << 8) | (CCF_EPI_DSWIGLU << 4):
-      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_DSWIGLU, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_DSWIGLU, false>(tm, a, grid, early, stream);
     case (MAJ_K << 12) | (MAJ_MN << 8) | (CCF_EPI_COMBINE << 4):
-      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_COMBINE, false>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_K, MAJ_MN, CCF_EPI_COMBINE, false>(tm, a, grid, early, stream);
     case (MAJ_MN << 12) | (MAJ_MN << 8) | (CCF_EPI_STORE << 4) | 1:
-      return launch_pair_variant<MAJ_MN, MAJ_MN, CCF_EPI_STORE, true>(tm, a, grid, stream);
+      return launch_pair_variant<MAJ_MN, MAJ_MN, CCF_EPI_STORE, true>(tm, a, grid, early, stream);
     default:
       return -6;
   }

@@ -713,11 +713,11 @@ __device__ __forceinline__ void dispatch_role(const CcfGemmArgs& args, bool comm
 }
 
 // two-CTA kernels (gemm2.cu), selected by the same key as the one-CTA ones
-int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
+int launch_pair_by_key(int key, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream);
 // few rows per group: weights on the M side (gemm_swap.cu)
-int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
+int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream);
 int swap_box_rows(bool big);
 // weight gradients of few rows per group (gemm_wgrad.cu)
-int launch_wgrad(const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream);
+int launch_wgrad(const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream);
 
 }  // namespace ccf

@@ -431,7 +431,6 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int n_pairs = static_cast<int>(gridDim.x) >> 1;
   volatile int* abort_word = &ctrl->abort_word;
-  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
 
   // ---- set-up ------------------------------------------------------------------------------------
   if (threadIdx.x == 0) {
@@ -459,6 +458,8 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
+  after_previous();
+  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   if (warp == 2) swap_tables_warp<kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
@@ -716,7 +717,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
 }
 
 template <int W, int E, int FP16>
-static int launch_swap_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+static int launch_swap_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, int early, cudaStream_t stream) {
   auto kern = grouped_gemm_swap_kernel<W, E, FP16>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
@@ -732,30 +733,30 @@ static int launch_swap_variant_of(const CUtensorMap* tm, const CcfGemmArgs& args
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSwSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {cluster_attribute(2, 1, 1)};
+  cudaLaunchAttribute attr[2] = {cluster_attribute(2, 1, 1), early_attribute()};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], args);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 template <int W, int E>
-static int launch_swap_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
-  return args.fp16 ? launch_swap_variant_of<W, E, 1>(tm, args, grid, stream) : launch_swap_variant_of<W, E, 0>(tm, args, grid, stream);
+static int launch_swap_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, int early, cudaStream_t stream) {
+  return args.fp16 ? launch_swap_variant_of<W, E, 1>(tm, args, grid, early, stream) : launch_swap_variant_of<W, E, 0>(tm, args, grid, early, stream);
 }
 
 int swap_box_rows(bool big) { return big ? kSwBig : kSwBox; }
 
 // Called by ccf_gemm_launch (gemm.cu) for row-grouped launches with `few_rows` set; returns -6 for a combination that does not exist.
 // tm[0], tm[1]: rows in boxes of 16; tm[4], tm[5]: the same in boxes of 64; tm[2], tm[3]: weights.
-int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream) {
+int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream) {
   switch ((b_major << 4) | epi) {
-    case (MAJ_K << 4) | CCF_EPI_BIAS_ACT: return launch_swap_variant<MAJ_K, CCF_EPI_BIAS_ACT>(tm, a, grid, stream);
-    case (MAJ_K << 4) | CCF_EPI_SWIGLU: return launch_swap_variant<MAJ_K, CCF_EPI_SWIGLU>(tm, a, grid, stream);
-    case (MAJ_K << 4) | CCF_EPI_COMBINE: return launch_swap_variant<MAJ_K, CCF_EPI_COMBINE>(tm, a, grid, stream);
-    case (MAJ_MN << 4) | CCF_EPI_DACT: return launch_swap_variant<MAJ_MN, CCF_EPI_DACT>(tm, a, grid, stream);
-    case (MAJ_MN << 4) | CCF_EPI_DSWIGLU: return launch_swap_variant<MAJ_MN, CCF_EPI_DSWIGLU>(tm, a, grid, stream);
-    case (MAJ_MN << 4) | CCF_EPI_COMBINE: return launch_swap_variant<MAJ_MN, CCF_EPI_COMBINE>(tm, a, grid, stream);
+    case (MAJ_K << 4) | CCF_EPI_BIAS_ACT: return launch_swap_variant<MAJ_K, CCF_EPI_BIAS_ACT>(tm, a, grid, early, stream);
+    case (MAJ_K << 4) | CCF_EPI_SWIGLU: return launch_swap_variant<MAJ_K, CCF_EPI_SWIGLU>(tm, a, grid, early, stream);
+    case (MAJ_K << 4) | CCF_EPI_COMBINE: return launch_swap_variant<MAJ_K, CCF_EPI_COMBINE>(tm, a, grid, early, stream);
+    case (MAJ_MN << 4) | CCF_EPI_DACT: return launch_swap_variant<MAJ_MN, CCF_EPI_DACT>(tm, a, grid, early, stream);
+    case (MAJ_MN << 4) | CCF_EPI_DSWIGLU: return launch_swap_variant<MAJ_MN, CCF_EPI_DSWIGLU>(tm, a, grid, early, stream);
+    case (MAJ_MN << 4) | CCF_EPI_COMBINE: return launch_swap_variant<MAJ_MN, CCF_EPI_COMBINE>(tm, a, grid, early, stream);
     default: return -6;
   }
 }

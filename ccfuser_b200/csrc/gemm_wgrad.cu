@@ -103,7 +103,6 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const uint32_t cta = cluster_ctarank();
   const int pair = static_cast<int>(blockIdx.x) >> 1, n_pairs = static_cast<int>(gridDim.x) >> 1;
   volatile int* abort_word = &ctrl->abort_word;
-  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   const int mt = args.m_per_group / PM, nt = (args.n + BN - 1) / BN, total = args.num_groups * mt * nt;
 
   if (threadIdx.x == 0) {
@@ -131,6 +130,8 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
+  after_previous();
+  const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   for (int g = static_cast<int>(threadIdx.x) - 64; g >= 0 && g < args.num_groups; g += kWgThreads - 64) {
     ctrl->rows[g] = args.group_rows[g];
     ctrl->base[g] = args.group_base[g];
@@ -384,7 +385,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 }
 
 template <int FP16, bool SGD>
-static int launch_wgrad_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, cudaStream_t stream) {
+static int launch_wgrad_variant(const CUtensorMap* tm, const CcfGemmArgs& args, int grid, int early, cudaStream_t stream) {
   auto kern = grouped_wgrad_kernel<FP16, SGD>;
   // the attribute belongs to the (function, device) pair: set it once per device this process launches on
   static bool configured[64] = {};
@@ -400,18 +401,18 @@ static int launch_wgrad_variant(const CUtensorMap* tm, const CcfGemmArgs& args, 
   cfg.blockDim = dim3(kWgThreads);
   cfg.dynamicSmemBytes = kWgSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1] = {cluster_attribute(2, 1, 1)};
+  cudaLaunchAttribute attr[2] = {cluster_attribute(2, 1, 1), early_attribute()};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tm[0], tm[2], tm[4], args);
   return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 
 // tm[0]: A, tm[2]: B, tm[4]: the result (boxes of 64 columns x 128 rows)
-int launch_wgrad(const CUtensorMap* tm, const CcfGemmArgs& a, int grid, cudaStream_t stream) {
+int launch_wgrad(const CUtensorMap* tm, const CcfGemmArgs& a, int grid, int early, cudaStream_t stream) {
   const bool sgd = a.sgd_lr != 0.f;
-  if (a.fp16) return sgd ? launch_wgrad_variant<1, true>(tm, a, grid, stream) : launch_wgrad_variant<1, false>(tm, a, grid, stream);
-  return sgd ? launch_wgrad_variant<0, true>(tm, a, grid, stream) : launch_wgrad_variant<0, false>(tm, a, grid, stream);
+  if (a.fp16) return sgd ? launch_wgrad_variant<1, true>(tm, a, grid, early, stream) : launch_wgrad_variant<1, false>(tm, a, grid, early, stream);
+  return sgd ? launch_wgrad_variant<0, true>(tm, a, grid, early, stream) : launch_wgrad_variant<0, false>(tm, a, grid, early, stream);
 }
 
 }  // namespace ccf

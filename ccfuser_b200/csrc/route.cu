@@ -52,11 +52,13 @@ __global__ void __launch_bounds__(kRouteThreads) route_plan_kernel(const __grid_
   const int E = a.e_total;
   const int s0 = (rank * kRouteWarps + warp) * kL * 32 + lane;
   int e[kL], r[kL];
+  after_previous();
+  const int* const expert = behind(a.expert);
   for (int i = lane; i < E; i += 32) wh[warp][i] = 0;
 #pragma unroll
   for (int l = 0; l < kL; ++l) {
     const int s = s0 + 32 * l;
-    e[l] = s < a.slots ? a.expert[s] : -1;
+    e[l] = s < a.slots ? expert[s] : -1;
   }
   __syncwarp();
 #pragma unroll
@@ -163,9 +165,9 @@ int ccf_route_plan(const int* expert, int S, int E, int cap, int* pos, int* coun
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kRouteThreads);
   cfg.stream = reinterpret_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1] = {cluster_attribute(ctas, 1, 1)};
+  cudaLaunchAttribute attr[2] = {cluster_attribute(ctas, 1, 1), early_attribute()};
   cfg.attrs = attr;
-  cfg.numAttrs = ctas > 1 ? 1 : 0;
+  cfg.numAttrs = 1 + (plan->world == 1 ? early_launches(S, cfg.stream) : 0);
   auto kern = per == 1 ? route_plan_kernel<1> : per == 2 ? route_plan_kernel<2> : per == 4 ? route_plan_kernel<4> : route_plan_kernel<8>;
   cudaError_t err = cudaLaunchKernelEx(&cfg, kern, a, *plan, epoch_counter);
   return err == cudaSuccess ? 0 : -static_cast<int>(err);

@@ -138,7 +138,6 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const uint32_t smem_base = smem_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_word = &ctrl->abort_word;
-  const uint64_t limit = fail_fast_limit(a.status, a.wait_limit_ns);
   const int row0 = blockIdx.x * BM;
   const int kblocks_all = (a.d + BK - 1) / BK;
   const int per_split = (kblocks_all + a.splits - 1) / a.splits;
@@ -161,11 +160,14 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tmem_alloc(smem_u32(&ctrl->tmem_base), static_cast<uint32_t>(a.tmem_cols));
     tmem_relinquish();
   }
+  after_previous();
+  const uint64_t limit = fail_fast_limit(a.status, a.wait_limit_ns);
+  const void* const bias = a.bias;
   for (int e = threadIdx.x; e < 256; e += kRtThreads) {
     float b = 0.f;
-    if (a.bias != nullptr && e < a.e)
-      b = a.fp16 ? __half2float(reinterpret_cast<const __half*>(a.bias)[e])
-                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.bias)[e]);
+    if (bias != nullptr && e < a.e)
+      b = a.fp16 ? __half2float(reinterpret_cast<const __half*>(bias)[e])
+                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[e]);
     ctrl->bias[e] = b;
   }
   tc_fence_before();

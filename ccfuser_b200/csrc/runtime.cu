@@ -11,6 +11,7 @@
 #include "combine.h"
 #include "route.h"
 #include "runtime.h"
+#include "sm100.cuh"
 
 extern "C" {
 int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream);
@@ -78,8 +79,14 @@ void set_row_kernel(CcfGemmLaunch& g, const CcfLayer* L, int tokens, int capacit
 //             4096 x 14336, 8: 0.79, 0.91, 0.97
 bool wgrad_few(long long rows, bool in_place, int two_cta) { return two_cta && rows <= (in_place ? 512 : 384); }
 
+// Whether the launches of a call may overlap with the end of the ones in front of them (sm100.cuh). A group of ranks leaves it: there a
+// clearing of counters lies between its kernels.
+int early_of(const CcfLayer* L, int tokens, const Dry* dry, void* stream) {
+  return dry == nullptr && L->world == 1 ? ccf::early_launches(static_cast<long long>(tokens) * L->top_k, reinterpret_cast<cudaStream_t>(stream)) : 0;
+}
+
 // fields every launch of this layer shares
-CcfGemmLaunch base_launch(const CcfLayer* L) {
+CcfGemmLaunch base_launch(const CcfLayer* L, int early) {
   CcfGemmLaunch g;
   memset(&g, 0, sizeof(g));
   g.args.group_base = L->group_base;
@@ -96,6 +103,7 @@ CcfGemmLaunch base_launch(const CcfLayer* L) {
   g.args.comm_warps = L->comm_warps;
   g.device = L->device;
   g.two_cta = L->two_cta;
+  g.early = early;
   return g;
 }
 
@@ -180,7 +188,7 @@ int issue(CcfGemmLaunch& g, Dry* dry, void* stream) {
 // Wait for the owners and sum the k slots of each token. With G (backward) and a router in the call, the sum also carries
 // the gradient through the gate weights.
 int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, const CcfLayerGrads* G, const int* idx,
-                    const float* gate_w, Dry* dry, void* stream) {
+                    const float* gate_w, int early, Dry* dry, void* stream) {
   if (dry != nullptr) return 0;
   CcfReduceArgs r;
   memset(&r, 0, sizeof(r));
@@ -191,6 +199,7 @@ int wait_and_reduce(const CcfLayer* L, const void* comb, void* out, int tokens, 
   r.top_k = L->top_k;
   r.d = L->d_model;
   r.fp16 = L->fp16;
+  r.early = early;
   if (L->world == 1) {
     r.done = L->done;
     r.cum = L->done_cum;
@@ -239,7 +248,7 @@ int end_of_pass(const CcfLayer* L, int rc, Dry* dry, void* stream) {
 
 int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* gate_w, void* y, int tokens, int capacity,
                  int save_pre, int epoch, void* stream, Dry* dry) {
-  const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
+  const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc, early = early_of(L, tokens, dry, stream);
   int rc = 0;
   if (dry == nullptr) {
     if (L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
@@ -280,7 +289,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
   }
   // 3. dispatch + GEMM-1 (+ bias + activation)
   {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, L->xrecv, L->max_rows, d, kMajK);
     set_b(g, L->w1, static_cast<long long>(e_loc) * f, d, kMajK);
     g.args.n = f;
@@ -305,7 +314,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
   }
   // 4. GEMM-2 + combine into the source ranks
   {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, L->h_act, L->max_rows, f, kMajK);
     set_b(g, L->w2, static_cast<long long>(e_loc) * d, f, kMajK);
     g.epi = CCF_EPI_COMBINE;
@@ -319,12 +328,12 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     if ((rc = issue(g, dry, stream))) return rc;
   }
   // 5. wait for every owner, sum the k slots of each token
-  return wait_and_reduce(L, L->comb, y, tokens, nullptr, nullptr, nullptr, dry, stream);
+  return wait_and_reduce(L, L->comb, y, tokens, nullptr, nullptr, nullptr, early, dry, stream);
 }
 
 int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float* gate_w, const CcfLayerGrads* G, int tokens,
                   int capacity, void* stream, Dry* dry) {
-  const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc;
+  const int d = L->d_model, f = L->d_ffn, e_loc = L->e_loc, early = early_of(L, tokens, dry, stream);
   int rc = 0;
   if (dry == nullptr && L->device >= 0 && cudaSetDevice(L->device) != cudaSuccess) return -7;
   const long long rows_per_expert = static_cast<long long>(tokens) * L->top_k * L->world / (L->e_total > 0 ? L->e_total : 1);
@@ -338,7 +347,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   if (sgd && L->swiglu && G->dwg != nullptr) return -2;
   // 1 + 2. push g * dy rows + dgrad-2 with the activation derivative
   {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, L->grecv, L->max_rows, d, kMajK);
     set_b(g, L->w2, static_cast<long long>(e_loc) * d, f, kMajMN);
     g.args.n = f;
@@ -361,7 +370,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   }
   // 3. wgrad-2: dW2[e] = (g dy)^T h_act  [d, f]
   {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, L->grecv, L->max_rows, d, kMajMN);
     set_b(g, L->h_act, L->max_rows, f, kMajMN);
     g.epi = CCF_EPI_STORE;
@@ -380,7 +389,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   }
   // 4. wgrad-1: dW1[e] = dh^T x_e  [f, d]  (SwiGLU: gate projection from dh, up projection from dh2)
   auto wgrad1 = [&](const void* a0, void* out) {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, a0, L->max_rows, f, kMajMN);
     set_b(g, L->xrecv, L->max_rows, d, kMajMN);
     g.epi = CCF_EPI_STORE;
@@ -398,7 +407,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
   // finish token then tells the sources that every buffer of this call is free), except when those update w1 / wg in
   // place: then it must read them first.
   auto dgrad1 = [&]() {
-    CcfGemmLaunch g = base_launch(L);
+    CcfGemmLaunch g = base_launch(L, early);
     set_a(g, G->dh, L->max_rows, f, kMajK);
     g.epi = CCF_EPI_COMBINE;
     g.args.n = d;
@@ -436,7 +445,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
       return rc;
   }
   if (!sgd && (rc = dgrad1())) return rc;
-  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, G, idx, gate_w, dry, stream))) return rc;
+  if ((rc = wait_and_reduce(L, L->gcomb, G->dx, tokens, G, idx, gate_w, early, dry, stream))) return rc;
   if (G->router_dw != nullptr && dry == nullptr)
     rc = ccf_router_dw(L->raw_order, L->count_raw, G->slot_grad, G->x, G->router_dw, G->router_db, tokens * L->top_k, d,
                        L->e_total, L->top_k, L->fp16, stream);
