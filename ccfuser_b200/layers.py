@@ -82,7 +82,8 @@ class MoELayer(nn.Module):
         output rows are zero. Stays on the device (no host synchronisation)."""
         cfg = self.config
         shape = inp.shape
-        x = inp.reshape(-1, cfg.d_model)
+        # a matrix is taken as it is: a reshape of it costs a view and a node of the backward pass, here and in _finish
+        x = inp if len(shape) == 2 and shape[1] == cfg.d_model else inp.reshape(-1, cfg.d_model)
         backend = self.backend(x)
         group = self.ep_group if cfg.ep_size > 1 else None
         if backend == "fused":
@@ -123,7 +124,7 @@ class MoELayer(nn.Module):
             y = y + y_shadow.to(y.dtype)
         if self.shared is not None:
             y = y + self.shared.expert_forward(0, x).to(y.dtype)
-        return y.reshape(shape[:-1] + (y.shape[-1],))
+        return y if y.dim() == len(shape) == 2 else y.reshape(shape[:-1] + (y.shape[-1],))
 
     # ---- placement ---------------------------------------------------------------------------
     def count_table(self) -> Optional[torch.Tensor]:

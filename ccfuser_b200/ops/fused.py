@@ -28,6 +28,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import weakref
 from typing import Dict
 
 import torch
@@ -416,6 +417,14 @@ class FusedMoE:
         self._desc, self._desc_key = L, key
         return L
 
+    def backward_desc(self, w1, wg, w2) -> N.Layer:
+        """``native_desc`` for a backward pass with these weights, which reads no bias: the one of its forward pass, unless a weight
+        lies somewhere else."""
+        key = self._desc_key
+        if key is not None and key[0] == w1.data_ptr() and key[2] == N.ptr(wg) and key[4] == w2.data_ptr():
+            return self._desc
+        return self.native_desc()
+
     # ---- one outstanding forward per layer ----------------------------------------------------------
     def claim_buffers(self, fn_ctx):
         """The saved activations of a forward pass (received rows, pre-activations, activations, routing arrays) live
@@ -423,7 +432,6 @@ class FusedMoE:
         training step, activation checkpointing's recomputation, two micro-batches before one backward) would
         overwrite them and the first backward would silently use the wrong data: raise instead. The claim ends when the
         backward runs or when the autograd graph that holds it is freed."""
-        import weakref
         owner = self._owed() if self._owed is not None else None
         if owner is not None and not getattr(owner, "ccf_backward_done", False):
             raise RuntimeError(
@@ -682,10 +690,10 @@ def _native_backward(fm: FusedMoE, dy, idx, gate_w, dgate, w1, wg, w2, has_bias,
         g.sgd_lr, g.sgd_wd = float(sgd2[0]), float(sgd2[1])
     if router is not None:
         wt, x, dwt, drb = router
-        slot_grad = torch.empty(t * cfg.top_k, dtype=torch.float32, device=dy.device)
-        g.router_w, g.x, g.slot_grad = wt.data_ptr(), x.data_ptr(), slot_grad.data_ptr()
+        # dgate has a second half for the gradients of the logits
+        g.router_w, g.x, g.slot_grad = wt.data_ptr(), x.data_ptr(), dgate.data_ptr() + 4 * t * cfg.top_k
         g.router_dw, g.router_db = N.ptr(dwt), N.ptr(drb)
-    N.check(N.load().ccf_layer_backward(C.byref(fm.native_desc()), dy.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
+    N.check(N.load().ccf_layer_backward(C.byref(fm.backward_desc(w1, wg, w2)), dy.data_ptr(), idx.data_ptr(), gate_w.data_ptr(),
                                         C.byref(g), t, cfg.capacity(t), N.stream_ptr(), None, 0, None), "ccf_layer_backward")
     # kernels: dy dispatch + dgrad-2, wgrad-2, wgrad-1 (two for SwiGLU), dgrad-1 + combine, reduce, column sums, the router's
     # weight gradient; with peers also the wait
@@ -720,7 +728,7 @@ class _FusedLayerFn(torch.autograd.Function):
         x, rw, idx, gate_w, w1, wg, w2 = ctx.saved_tensors
         need_rw, need_rb = ctx.needs_input_grad[1], ctx.has_router_bias and ctx.needs_input_grad[2]
         # the gate gradient of a dropped slot stays unwritten: the reduction takes it as zero
-        dgate = torch.empty(gate_w.numel(), dtype=torch.float32, device=dy.device)
+        dgate = torch.empty(2 * gate_w.numel(), dtype=torch.float32, device=dy.device)
         drw = torch.empty_like(rw) if (need_rw or need_rb) else None
         drb = torch.empty(rw.shape[0], dtype=rw.dtype, device=dy.device) if need_rb else None
         dx, grads = _native_backward(fm, G.packed(dy), idx, gate_w, dgate, w1, wg, w2, ctx.has_bias, (rw, x, drw, drb))

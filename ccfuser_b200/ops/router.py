@@ -30,11 +30,9 @@ def route_topk(x: torch.Tensor, wt: torch.Tensor, bias, k: int, want_logits: boo
     idx = torch.empty(t, k, dtype=torch.int32, device=x.device)
     w = torch.empty(t, k, dtype=torch.float32, device=x.device)
     logits = torch.empty(t, e, dtype=torch.float32, device=x.device) if want_logits else None
-    ws = Workspace.get(x.device)
-    dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
     N.check(N.load().ccf_router_topk(x.data_ptr(), wt.data_ptr(), N.ptr(bias), t, d, e, k, int(x.dtype == torch.float16),
-                                     idx.data_ptr(), w.data_ptr(), N.ptr(logits), ws.status.data_ptr(),
-                                     5_000_000_000, dev, N.stream_ptr()), "ccf_router_topk")
+                                     idx.data_ptr(), w.data_ptr(), N.ptr(logits), Workspace.status_of(x),
+                                     5_000_000_000, x.get_device(), N.stream_ptr()), "ccf_router_topk")
     N.count(1)
     return idx, w, logits
 

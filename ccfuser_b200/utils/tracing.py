@@ -15,15 +15,19 @@ NVTX = bool(int(os.environ.get("CCFUSER_NVTX", "0")))
 
 
 @contextlib.contextmanager
-def nvtx_range(name: str):
-    if NVTX and torch.cuda.is_available():
-        torch.cuda.nvtx.range_push(name)
-        try:
-            yield
-        finally:
-            torch.cuda.nvtx.range_pop()
-    else:
+def _nvtx_range(name: str):
+    torch.cuda.nvtx.range_push(name)
+    try:
         yield
+    finally:
+        torch.cuda.nvtx.range_pop()
+
+
+_NO_RANGE = contextlib.nullcontext()   # one for all: it holds no state, and a generator per stage costs a microsecond
+
+
+def nvtx_range(name: str):
+    return _nvtx_range(name) if NVTX and torch.cuda.is_available() else _NO_RANGE
 
 
 class StageTimer:
