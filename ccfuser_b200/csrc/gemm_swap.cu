@@ -11,7 +11,10 @@
 //   parts       a tile of more columns than an accumulator holds is two parts that share every stage of weights
 //   accumulators  ring of 2 x 256 or, when some group has more than 256 rows, 3 x 160 TMEM columns: with two parts per tile the
 //               next tile's first part has a free accumulator while the last tile's parts are stored
-//   tiles       pair p takes tiles p, p + pairs, ...: every sum runs over k in order on one pair, as in gemm2.cu, so that a row's result
+//   tiles       pair p takes tiles p, p + pairs, ...; where the last round would leave half of the pairs or more without one, its tiles
+//               come in pieces of their rows (swap_last_round). One round of few tiles gained most: second projection of 300 rows, 4
+//               experts of 1024 x 4096 (16 tiles) 42 -> 33 us, 8 experts of 768 x 3072 36 -> 29; 64 experts of 256 rows, 1024 x 4096
+//               (3.5 rounds) 154 -> 148. Every sum runs over k in order on one pair, as in gemm2.cu, so that a row's result
 //               does not depend on what is routed beside it. A version in which the pairs shared the k-blocks of the last tiles through
 //               an fp32 workspace gave that up, and cost more than the even split saved: of 1032 launches measured (512 x 2048 to
 //               4096 x 14336, 4 to 64 experts, 8 to 320 rows each) it was slower in 308 and more than 4 % faster in 33; 8 experts of
@@ -54,6 +57,7 @@ struct __align__(16) CtrlS {
   uint32_t tmem_base;
   int abort_word;
   SwapShape shape;
+  SwapRound round;
   int mt_prefix[CCF_MAX_GROUPS + 1];   // row tiles, prefix over groups
   int base[CCF_MAX_GROUPS];
   int rows[CCF_MAX_GROUPS];
@@ -152,9 +156,17 @@ struct SwapTile {
   int np;         // columns of a part, a multiple of 16
 };
 
-__device__ __forceinline__ SwapTile decode_swap_tile(int t, const CtrlS* c, int num_groups) {
+// Work item w: a whole tile or, in the last round, a piece of one (without rows where they do not suffice).
+__device__ __forceinline__ SwapTile decode_swap_item(int w, const CtrlS* c, int num_groups) {
   SwapTile ti;
   const SwapShape& s = c->shape;
+  int t = w, piece = 0, pieces = 1;
+  if (w >= c->round.whole) {
+    pieces = c->round.pieces;
+    const int u = w - c->round.whole;
+    t = c->round.whole + u / pieces;
+    piece = u % pieces;
+  }
   int lo = 0, hi = num_groups;   // largest g with f_tiles * mt_prefix[g] <= t
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -163,25 +175,40 @@ __device__ __forceinline__ SwapTile decode_swap_tile(int t, const CtrlS* c, int 
   ti.g = lo;
   const int mt = c->mt_prefix[lo + 1] - c->mt_prefix[lo];
   const int local = t - s.f_tiles * c->mt_prefix[lo];
-  const int j = local / mt, i = local - j * mt;   // the row tiles of one block of features side by side: they share its weights
   const int rows = c->rows[lo];
-  const int per = swap_round16((rows + mt - 1) / mt);
+  // the row tiles of one block of features side by side: they share its weights. Mostly there is one, and no division to wait for
+  int j = local, i = 0, per = rows;
+  if (mt > 1) {
+    j = local / mt;
+    i = local - j * mt;
+    per = swap_round16((rows + mt - 1) / mt);
+  }
   ti.row0 = c->base[lo] + i * per;
   ti.tokens = min(per, rows - i * per);
   ti.zero_rows = i == mt - 1 ? ((rows + 63) & ~63) - rows : 0;
+  if (pieces > 1) {
+    const int all = ti.tokens, of = swap_round16((all + pieces - 1) / pieces), at = min(piece * of, all);
+    ti.row0 += at;
+    ti.tokens = min(of, all - at);
+    if (ti.tokens == 0 || at + ti.tokens < all) ti.zero_rows = 0;   // they lie behind the tile's last row
+  }
   ti.n0 = j * PM;
   ti.parts = ti.tokens > s.width ? 2 : 1;
-  ti.np = swap_round16((ti.tokens + ti.parts - 1) / ti.parts);
+  ti.np = swap_round16(ti.parts > 1 ? (ti.tokens + 1) >> 1 : ti.tokens);
   return ti;
 }
 
 // The next tile of an epilogue warp; out of line, the registers it needs are not the epilogue's.
 __device__ __noinline__ bool swap_next(const CtrlS* ctrl, SwapWork* w, int n_pairs, int num_groups) {
-  const int t = w->t;
+  int t = w->t;
   __syncwarp();
-  if (t >= ctrl->shape.total_tiles) return false;
-  const SwapTile ti = decode_swap_tile(t, ctrl, num_groups);
-  if ((threadIdx.x & 31) == 0) *w = SwapWork{t + n_pairs, ti.g, ti.row0, ti.tokens, ti.zero_rows, ti.n0, ti.parts, ti.np};
+  SwapTile ti;
+  do {
+    if (t >= ctrl->round.items) return false;
+    ti = decode_swap_item(t, ctrl, num_groups);
+    t += n_pairs;
+  } while (ti.tokens <= 0);
+  if ((threadIdx.x & 31) == 0) *w = SwapWork{t, ti.g, ti.row0, ti.tokens, ti.zero_rows, ti.n0, ti.parts, ti.np};
   __syncwarp();
   return true;
 }
@@ -227,6 +254,7 @@ __device__ __forceinline__ void swap_tables_warp(const CcfGemmArgs& args, CtrlS*
   if (lane == 0) {
     ctrl->mt_prefix[args.num_groups] = acc;
     ctrl->shape = swap_shape(args, acc, total_rows, max_half, width, kWide, kSwPipeBytes, kSwMaxStages);
+    ctrl->round = swap_last_round(ctrl->shape.total_tiles, static_cast<int>(gridDim.x) >> 1, min(max_rows, cap));
   }
 }
 
@@ -469,7 +497,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
   const SwapShape& sh = ctrl->shape;
   const int stages = sh.stages;
   const uint32_t stage_bytes = sh.stage_bytes;
-  const int kb_per_seg = (args.k + BK - 1) / BK;
+  const int kb_per_seg = (args.k + BK - 1) / BK, kblocks = sh.kblocks, items = ctrl->round.items;
 
   if (threadIdx.x == 0 && args.trace != nullptr) trace_ev(args, args.trace_tiles - 1, 0);
 
@@ -492,8 +520,9 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         tma_load_2d_pair(sw + 8192, mw, bar, n_col + 64, w_row + kk);
       }
     };
-    for (int t = pair; t < sh.total_tiles && ok; t += n_pairs, ++seq) {
-      const SwapTile ti = decode_swap_tile(t, ctrl, args.num_groups);
+    for (int t = pair; t < items && ok; t += n_pairs) {
+      const SwapTile ti = decode_swap_item(t, ctrl, args.num_groups);
+      if (ti.tokens <= 0) continue;
       if (lane == 0) trace_ev(args, seq, 0);
       const int half = ti.np >> 1, boxes = (half + kSwBox - 1) / kSwBox;
       const uint32_t bytes = 2 * (kW + static_cast<uint32_t>(ti.parts * boxes * (kSwBox * 128)));   // of both CTAs
@@ -502,7 +531,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
       // The first stages' weights are requested before the rows are waited for: they depend on nothing.
       int pre = 0;
       if (seq == 0) {
-        pre = min(stages, sh.kblocks);
+        pre = min(stages, kblocks);
         if (elect_one()) {
           for (int i = 0; i < pre; ++i) {
             const int seg = i >= kb_per_seg ? 1 : 0;   // at most two segments
@@ -534,7 +563,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
       if (lane == 0) trace_ev(args, seq, 1);
       const CUtensorMap *mw = &tmW0, *mx = &tmX0, *mxb = &tmXb0;
       int kk = 0;
-      for (int kb = 0; kb < sh.kblocks; ++kb, kk += BK) {
+      for (int kb = 0; kb < kblocks; ++kb, kk += BK) {
         if (kb == kb_per_seg) {
           mw = &tmW1;
           mx = &tmX1;
@@ -565,6 +594,7 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (lane == 0) trace_ev(args, seq, 2);
+      ++seq;
     }
   } else if (warp == 1) {
     // ======================= MMA issuer (leader CTA only) =======================
@@ -573,8 +603,9 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
       const uint32_t full0 = smem_u32(&ctrl->full[0]), empty0 = smem_u32(&ctrl->empty[0]);
       int stage = 0, phase = 0, buf = 0, bphase = 0, seq = 0;
       bool ok = true;
-      for (int t = pair; t < sh.total_tiles && ok; t += n_pairs, ++seq) {
-        const SwapTile ti = decode_swap_tile(t, ctrl, args.num_groups);
+      for (int t = pair; t < items && ok; t += n_pairs) {
+        const SwapTile ti = decode_swap_item(t, ctrl, args.num_groups);
+        if (ti.tokens <= 0) continue;
         const uint32_t idesc = make_idesc(PM, ti.np, args.fp16, kWMajor, MAJ_K);
         const uint32_t part_bytes = static_cast<uint32_t>((((ti.np >> 1) + kSwBox - 1) / kSwBox) * kSwBox) * 128;
         if (lane == 0) trace_ev(args, seq, 3);
@@ -587,7 +618,8 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
             ok = false;
           }
         }
-        for (int kb = 0; kb < sh.kblocks && ok; ++kb) {
+        const bool two = !kWide && ti.parts > 1;
+        for (int kb = 0; kb < kblocks && ok; ++kb) {
           if (!mbar_wait_cluster(full0 + 8 * stage, phase, abort_word, limit)) {
             report_status(args.status, CCF_ERR_MBAR_TIMEOUT, 0x35);
             ok = false;
@@ -605,24 +637,26 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
                 umma_f16_pair(d0 + a * 128, desc_at(desc_w, at + a * kSwWBytes + k * desc_step(kWMajor)),
                               desc_at(desc_x, at + k * desc_step(MAJ_K)), idesc, k > 0 ? 1u : acc);
             }
-            if (!kWide && ti.parts > 1) {
+            if (two) {
 #pragma unroll
               for (int k = 0; k < BK / UK; ++k)
                 umma_f16_pair(d1, desc_at(desc_w, at + k * desc_step(kWMajor)),
                               desc_at(desc_x, at + part_bytes + k * desc_step(MAJ_K)), idesc, k > 0 ? 1u : acc);
             }
             umma_commit_pair(empty0 + 8 * stage);   // hand the stage back to both producers
-            if (kb == sh.kblocks - 1) {
-              umma_commit_pair(smem_u32(&ctrl->acc_full[buf]));
-              if (ti.parts > 1) umma_commit_pair(smem_u32(&ctrl->acc_full[b1]));
-              trace_ev(args, seq, 5);
-            }
           }
           __syncwarp();
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
+        if (ok && elect_one()) {
+          umma_commit_pair(smem_u32(&ctrl->acc_full[buf]));
+          if (two) umma_commit_pair(smem_u32(&ctrl->acc_full[b1]));
+          trace_ev(args, seq, 5);
+        }
+        __syncwarp();
         buf += ti.parts;
         if (buf >= sh.bufs) { buf -= sh.bufs; bphase ^= 1; }
+        ++seq;
       }
     }
   } else if (warp >= 2 + kEpiWarps) {

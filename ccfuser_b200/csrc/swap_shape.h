@@ -31,6 +31,25 @@ __host__ __device__ inline int swap_half_rows(int tokens, int width) {
   return parts * (((np >> 1) + 15) & ~15);
 }
 
+// The last round: `whole` tiles fill the rounds before it, each of the others comes in `pieces` parts of its rows, so that no pair has
+// more than one. A piece streams the tile's weights again, from L2, and its MMAs take no less than a turn of the issuing thread (377
+// clocks a k-block up to 128 rows, 512 with 256 rows), so pieces have 64 rows or more: `tile_rows` is the most that a tile holds.
+struct SwapRound {
+  int whole, pieces, items;
+};
+__host__ __device__ inline SwapRound swap_last_round(int tiles, int pairs, int tile_rows) {
+  SwapRound r = {tiles, 1, tiles};
+  if (tile_rows < 128) return r;
+  // quotients below 2^16 of integers, half a unit above a multiple at most: exact in fp32, and a few instructions
+  const int rest = tiles - pairs * static_cast<int>((static_cast<float>(tiles) + 0.5f) / static_cast<float>(pairs));
+  if (2 * rest > pairs || rest < 1) return r;
+  const int fit = static_cast<int>((static_cast<float>(pairs) + 0.5f) / static_cast<float>(rest)), most = tile_rows >> 6;
+  r.whole = tiles - rest;
+  r.pieces = fit < most ? fit : most;
+  r.items = r.whole + rest * r.pieces;
+  return r;
+}
+
 __host__ __device__ inline SwapShape swap_shape(const CcfGemmArgs& a, int row_tiles, int total_rows, int half_rows, int width, bool wide,
                                                 int pipe_bytes, int max_stages) {
   SwapShape s;
