@@ -528,9 +528,9 @@ int ccf_router_topk(const void* x, const void* wg, const void* bias, int tokens,
   cfg.blockDim = dim3(kRtThreads);
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = reinterpret_cast<cudaStream_t>(stream_v);
-  cudaLaunchAttribute attr[1] = {cluster_attribute(1, a.splits, 1)};
+  cudaLaunchAttribute attr[2] = {cluster_attribute(1, a.splits, 1), early_attribute()};
   cfg.attrs = attr;
-  cfg.numAttrs = a.splits > 1 ? 1 : 0;
+  cfg.numAttrs = 1 + early_launches(static_cast<long long>(tokens) * k, cfg.stream);
   cudaError_t err = cudaLaunchKernelEx(&cfg, kern, tmx, tmw, a);
   return err == cudaSuccess ? 0 : -static_cast<int>(err);
 }
