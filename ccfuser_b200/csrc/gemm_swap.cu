@@ -300,7 +300,22 @@ __device__ __forceinline__ void swap_epilogue(const CcfGemmArgs& args, const Swa
     if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) frag_fetch(at(args.aux0, c), step, pt.valid - 32 * c, lane, an0);
     if constexpr (kEpi == CCF_EPI_DSWIGLU) frag_fetch(at(args.aux1, c), step, pt.valid - 32 * c, lane, an1);
   };
+  // COMBINE: where row `lane` of the next chunk goes, a chunk ahead like the auxiliary inputs: read where they were used, the two stood
+  // a trip to memory in front of every chunk's shuffles
+  int dest_next = -1;
+  float gate_next = 1.f;
+  auto fetch_dest = [&](int c) {
+    if constexpr (kEpi == CCF_EPI_COMBINE) {
+      dest_next = -1;
+      if (lane < pt.valid - 32 * c) {
+        const int row = pt.row0 + 32 * c + lane;
+        dest_next = args.row_src[row];
+        if (args.row_gate != nullptr) gate_next = args.row_gate[row];
+      }
+    }
+  };
   fetch(pt.first);
+  fetch_dest(pt.first);
   if (!acquire()) return;
   if (pt.first >= n_acc || pt.first * 32 >= pt.end) release();   // no chunk of it is this warp's
   int sent = 0;   // COMBINE: lane s counts the rows stored for rank s
@@ -364,17 +379,13 @@ __device__ __forceinline__ void swap_epilogue(const CcfGemmArgs& args, const Swa
     } else if constexpr (kEpi == CCF_EPI_COMBINE) {
       add_bias(f, b0);
       // lane l: where row l of the chunk goes
-      int packed = -1;
-      float gate = 1.f;
-      if (lane < valid) {
-        const int row = pt.row0 + 32 * c + lane;
-        packed = args.row_src[row];
-        if (args.row_gate != nullptr) gate = args.row_gate[row];
-        if (packed < 0 || ((packed >> 24) & 0xff) >= args.world || (packed & 0xffffff) >= args.max_slots) {
-          report_status(args.status, CCF_ERR_BOUNDS, row & 0xffffff);
-          packed = -1;
-        }
+      int packed = dest_next;
+      const float gate = gate_next;
+      if (lane < valid && (packed < 0 || ((packed >> 24) & 0xff) >= args.world || (packed & 0xffffff) >= args.max_slots)) {
+        report_status(args.status, CCF_ERR_BOUNDS, (pt.row0 + 32 * c + lane) & 0xffffff);
+        packed = -1;
       }
+      if ((c + 2) * 32 < pt.end) fetch_dest(c + 2);
       if (args.row_gate != nullptr) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
