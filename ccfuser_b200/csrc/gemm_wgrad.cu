@@ -11,7 +11,7 @@
 //   store warp writes them back, and a chunk whose store has been read is loaded again. Without weights the chunks are output buffers.
 //
 // Measured, pair kernel / this one, operands of several layers in turn, us (plain and in place): 16 x 256 rows, 768 x 3072: 31 / 25 and 51 / 37; 64 x 256,
-// 1024 x 4096: 186 / 147 and 346 / 219; 64 x 256, 2048 x 8192: 842 / 611 and 1343 / 834 (4.3 GB read and written: 5.1 TB/s);
+// 1024 x 4096: 186 / 147 and 346 / 219; 64 x 256, 2048 x 8192: 842 / 611 and 1343 / 770 (4.3 GB read and written: 5.6 TB/s);
 // 16 x 512, 2048 x 8192: 255 / 240 and 375 / 283. With more rows the main loop decides, and the pair kernel's deeper ring wins:
 // 16 x 1024 rows 411 / 447 and 478 / 496 (wgrad_few in runtime.cu).
 //
@@ -262,7 +262,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (elect_one()) {
       ChunkPos pos, freed;
       bool ok = true;
-      int pending = 0;   // stores that may still be reading their chunk
+      [[maybe_unused]] int pending = 0;   // stores that may still be reading their chunk
       for (int t = pair; t < total && ok; t += n_pairs) {
         const WgTile ti = decode_wg_tile<kSgd>(t, args, ctrl, mt, nt);
         const int row = ti.g * args.m_per_group + ti.m0 + static_cast<int>(cta) * BM;
@@ -274,7 +274,13 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
           tma_store_2d(&tmC, ring + pos.slot * kWgChunkBytes, ti.n0 + 64 * c, row);
           bulk_commit();
-          if (++pending == 2) {   // the older one has been read by now, or nearly
+          // In place a chunk is handed back as soon as it has been read: the next weights wait for it (64 x 256 rows, 2048 x 8192: 810 ->
+          // 768 us). Without weights to load the older of two is, and the stores follow each other closer (1024 x 4096: 153 against 165).
+          if constexpr (kSgd) {
+            bulk_wait_read<0>();
+            mbar_arrive(smem_u32(&ctrl->free_[freed.slot]));
+            freed.advance(1);
+          } else if (++pending == 2) {   // the older one has been read by now, or nearly
             bulk_wait_read<1>();
             mbar_arrive(smem_u32(&ctrl->free_[freed.slot]));
             freed.advance(1);
