@@ -124,7 +124,7 @@ class MoELayer(nn.Module):
             y = y + y_shadow.to(y.dtype)
         if self.shared is not None:
             y = y + self.shared.expert_forward(0, x).to(y.dtype)
-        return y if y.dim() == len(shape) == 2 else y.reshape(shape[:-1] + (y.shape[-1],))
+        return y if len(shape) == 2 and y.shape[0] == shape[0] else y.reshape(shape[:-1] + (y.shape[-1],))
 
     # ---- placement ---------------------------------------------------------------------------
     def count_table(self) -> Optional[torch.Tensor]:
