@@ -232,3 +232,30 @@ def test_environment_report():
     assert r["library"]["path"].endswith("libccfuser_b200.so")
     if not r["cuda_available"]:
         assert any("no CUDA device" in p for p in r["problems"])
+
+
+def test_nvtx_range_decorates_a_function_with_ranges_on_and_off(monkeypatch):
+    """As a context manager and as a decorator, and it looks at the switch when the range begins, not where it was made."""
+    from ccfuser_b200.utils import tracing
+    seen = []
+    monkeypatch.setattr(tracing.torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(tracing.torch.cuda.nvtx, "range_push", lambda name: seen.append(name))
+    monkeypatch.setattr(tracing.torch.cuda.nvtx, "range_pop", lambda: seen.append("end"))
+    monkeypatch.setattr(tracing, "NVTX", False)
+
+    @tracing.nvtx_range("f")
+    def f(x):
+        return x + 1
+
+    early = tracing.nvtx_range("early")
+    assert f(1) == 2 and seen == []
+    with tracing.nvtx_range("a"), tracing.nvtx_range("a"):
+        pass
+    assert seen == []
+    monkeypatch.setattr(tracing, "NVTX", True)
+    assert f(1) == 2 and f(2) == 3 and seen == ["f", "end"] * 2
+    with early:
+        seen.append("inside")
+    with pytest.raises(ValueError), tracing.nvtx_range("b"):
+        raise ValueError
+    assert seen[4:] == ["early", "inside", "end", "b", "end"]
