@@ -630,7 +630,8 @@ int ccf_gemm_launch(const CcfGemmLaunch* L, void* stream_v) {
     // tm[4..6]: the outputs that leave by bulk tensor stores, in boxes of 32 x 32
     void* const outs[3] = {a.out0, a.out1, a.out2};
     const bool tma_out = L->epi != CCF_EPI_COMBINE && !(L->epi == CCF_EPI_STORE && (!L->kgroup || a.out_fp32 || a.sgd_lr != 0.f));
-    const long long out_rows = L->kgroup ? static_cast<long long>(a.num_groups) * a.m_per_group : L->a_rows;
+    const long long out_rows = L->kgroup ? static_cast<long long>(a.num_groups) * a.m_per_group
+                               : L->out_rows > 0 ? L->out_rows : L->a_rows;
     for (int i = 0; i < 3; ++i) {
       const void* p = tma_out && outs[i] != nullptr ? outs[i] : nullptr;
       if (p == nullptr) tm[4 + i] = tm[0];

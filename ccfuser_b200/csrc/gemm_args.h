@@ -129,6 +129,7 @@ struct CcfGemmLaunch {
   int two_cta;               // 1 = 256x256 tiles on CTA pairs (tcgen05 cta_group::2), 0 = 128x256 tiles per CTA
   int few_rows;              // 1: the kernels for few rows per group (row-grouped: gemm_swap.cu, k-grouped: gemm_wgrad.cu)
   int early;                 // 1: may be set up while the kernel in front of it still runs (kernels on CTA pairs; sm100.cuh)
+  long long out_rows;        // row-grouped launches on CTA pairs: rows that the outputs have (0: a_rows); nothing is written behind them
 };
 
 // Arguments of the count exchange + planning kernel (ccf_plan).

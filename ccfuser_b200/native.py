@@ -65,6 +65,7 @@ class GemmLaunch(C.Structure):
         ("a_rows", C.c_longlong), ("a_cols", C.c_longlong), ("b_rows", C.c_longlong), ("b_cols", C.c_longlong),
         ("a_major", C.c_int), ("b_major", C.c_int), ("epi", C.c_int), ("kgroup", C.c_int), ("grid", C.c_int),
         ("device", C.c_int), ("two_cta", C.c_int), ("few_rows", C.c_int), ("early", C.c_int),
+        ("out_rows", C.c_longlong),
     ]
 
 

@@ -209,6 +209,9 @@ def launch(*, a0, b0, a_major, b_major, epi, n, k=0, group_base, group_rows, num
     L.a0, L.a1, L.b0, L.b1 = N.ptr(a0), N.ptr(a1), N.ptr(b0), N.ptr(b1)
     L.a_rows, L.a_cols = a0.shape
     L.b_rows, L.b_cols = b0.shape
+    # the outputs may end later than the operand: whole tiles of 128 rows are written, zeros behind a group's last row
+    rows = [t.numel() // n for t in (out0, out1, out2) if t is not None]
+    L.out_rows = 0 if kgroup or not rows else min(rows)
     L.a_major, L.b_major, L.epi, L.kgroup, L.grid = int(a_major), int(b_major), int(epi), int(bool(kgroup)), int(grid)
     if a0.device.type != "cuda":
         L.device = -1
