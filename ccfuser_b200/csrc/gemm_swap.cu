@@ -146,58 +146,6 @@ __device__ __forceinline__ void fetched_to_frag(uint32_t stage, int lane, const 
 }
 
 // ---- tiles --------------------------------------------------------------------------------------------
-struct SwapTile {
-  int g;
-  int row0;       // first row (absolute)
-  int tokens;     // rows of the tile
-  int zero_rows;  // rows behind them that get zeros where a reduction over rows reads the output
-  int n0;         // first feature of the pair
-  int parts;
-  int np;         // columns of a part, a multiple of 16
-};
-
-// Work item w: a whole tile or, in the last round, a piece of one (without rows where they do not suffice).
-__device__ __forceinline__ SwapTile decode_swap_item(int w, const CtrlS* c, int num_groups) {
-  SwapTile ti;
-  const SwapShape& s = c->shape;
-  int t = w, piece = 0, pieces = 1;
-  if (w >= c->round.whole) {
-    pieces = c->round.pieces;
-    const int u = w - c->round.whole;
-    t = c->round.whole + u / pieces;
-    piece = u % pieces;
-  }
-  int lo = 0, hi = num_groups;   // largest g with f_tiles * mt_prefix[g] <= t
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (s.f_tiles * c->mt_prefix[mid] <= t) lo = mid; else hi = mid;
-  }
-  ti.g = lo;
-  const int mt = c->mt_prefix[lo + 1] - c->mt_prefix[lo];
-  const int local = t - s.f_tiles * c->mt_prefix[lo];
-  const int rows = c->rows[lo];
-  // the row tiles of one block of features side by side: they share its weights. Mostly there is one, and no division to wait for
-  int j = local, i = 0, per = rows;
-  if (mt > 1) {
-    j = local / mt;
-    i = local - j * mt;
-    per = swap_round16((rows + mt - 1) / mt);
-  }
-  ti.row0 = c->base[lo] + i * per;
-  ti.tokens = min(per, rows - i * per);
-  ti.zero_rows = i == mt - 1 ? ((rows + 63) & ~63) - rows : 0;
-  if (pieces > 1) {
-    const int all = ti.tokens, of = swap_round16((all + pieces - 1) / pieces), at = min(piece * of, all);
-    ti.row0 += at;
-    ti.tokens = min(of, all - at);
-    if (ti.tokens == 0 || at + ti.tokens < all) ti.zero_rows = 0;   // they lie behind the tile's last row
-  }
-  ti.n0 = j * PM;
-  ti.parts = ti.tokens > s.width ? 2 : 1;
-  ti.np = swap_round16(ti.parts > 1 ? (ti.tokens + 1) >> 1 : ti.tokens);
-  return ti;
-}
-
 // The next tile of an epilogue warp; out of line, the registers it needs are not the epilogue's.
 __device__ __noinline__ bool swap_next(const CtrlS* ctrl, SwapWork* w, int n_pairs, int num_groups) {
   int t = w->t;
@@ -808,38 +756,83 @@ int launch_swap_by_key(int b_major, int epi, const CUtensorMap* tm, const CcfGem
 
 }  // namespace ccf
 
-// The tiles of a launch of the swapped kernel, computed on the host with the kernel's own functions: for every CTA pair its tiles in
-// order, out[9 i ...] = {pair, tile, first k-block, one past the last, first pair that works on the tile, number of such pairs, rows
-// per stage of the launch, stages, number of tiles}. Host arrays in, nothing touches a device. Returns the number of records
-// (only the first `cap` are written).
-extern "C" int ccf_debug_swap_segments(const int* group_rows, int num_groups, int n, int k, int kseg, int wide, int n_pairs, int* out,
-                                       int cap) {
-  using namespace ccf;
+namespace ccf {
+
+// The tables of a launch, on the host
+struct SwapTables {
+  SwapShape shape;
+  SwapRound round;
+  int half;
+  int mt_prefix[CCF_MAX_GROUPS + 1], base[CCF_MAX_GROUPS], rows[CCF_MAX_GROUPS];
+};
+static int swap_tables_host(const int* group_rows, int num_groups, int n, int k, int kseg, int wide, int n_pairs, SwapTables* c) {
   if (num_groups < 1 || num_groups > CCF_MAX_GROUPS) return -2;
   CcfGemmArgs a;
   memset(&a, 0, sizeof(a));
   a.n = n;
   a.k = k;
   a.kseg = kseg;
-  int max_rows = 0, total = 0, tiles = 0, half = 0;
+  int max_rows = 0, total = 0, tiles = 0, half = 0, base = 0;
   for (int g = 0; g < num_groups; ++g) {
     max_rows = group_rows[g] > max_rows ? group_rows[g] : max_rows;
     total += group_rows[g];
   }
   const int width = swap_width(max_rows, wide != 0), rows_cap = swap_cap(max_rows, wide != 0);
   for (int g = 0; g < num_groups; ++g) {
+    c->rows[g] = group_rows[g];
+    c->base[g] = base;
+    c->mt_prefix[g] = tiles;
+    base += (group_rows[g] + 127) / 128 * 128;
     const int mt = (group_rows[g] + rows_cap - 1) / rows_cap;
     if (mt == 0) continue;
     const int h = swap_half_rows(swap_round16((group_rows[g] + mt - 1) / mt), width);
     half = h > half ? h : half;
     tiles += mt;
   }
-  const SwapShape s = swap_shape(a, tiles, total, half, width, wide != 0, kSwPipeBytes, kSwMaxStages);
+  c->mt_prefix[num_groups] = tiles;
+  c->half = half;
+  c->shape = swap_shape(a, tiles, total, half, width, wide != 0, kSwPipeBytes, kSwMaxStages);
+  c->round = swap_last_round(c->shape.total_tiles, n_pairs, swap_min(max_rows, rows_cap));
+  return 0;
+}
+
+}  // namespace ccf
+
+// The whole tiles of a launch of the swapped kernel, before those of its last round are cut (ccf_debug_swap_items), computed on the
+// host with the kernel's own functions: out[9 i ...] = {pair, tile, first k-block, one past the last, first pair that works on the tile,
+// number of such pairs, rows per stage of the launch, stages, number of tiles}. Host arrays in, nothing touches a device. Returns the
+// number of records (only the first `cap` are written).
+extern "C" int ccf_debug_swap_segments(const int* group_rows, int num_groups, int n, int k, int kseg, int wide, int n_pairs, int* out,
+                                       int cap) {
+  using namespace ccf;
+  SwapTables c;
+  if (int rc = swap_tables_host(group_rows, num_groups, n, k, kseg, wide, n_pairs, &c)) return rc;
+  const SwapShape& s = c.shape;
   int i = 0;
   for (int p = 0; p < n_pairs; ++p)
     for (int t = p; t < s.total_tiles; t += n_pairs, ++i) {
-      const int rec[9] = {p, t, 0, s.kblocks, p, 1, half, s.stages, s.total_tiles};
+      const int rec[9] = {p, t, 0, s.kblocks, p, 1, c.half, s.stages, s.total_tiles};
       if (i < cap) memcpy(out + 9 * i, rec, sizeof(rec));
+    }
+  return i;
+}
+
+// What every CTA pair of such a launch works on, in order: out[12 i ...] = {pair, item, first item of the last round if it is cut (else
+// the number of items), group, first row in the group, rows, rows behind them that get zeros, first feature, parts, columns of a part,
+// rows per stage that it takes, rows per stage that there are}. Groups lie as they do in a launch, on multiples of 128 rows.
+extern "C" int ccf_debug_swap_items(const int* group_rows, int num_groups, int n, int k, int kseg, int wide, int n_pairs, int* out, int cap) {
+  using namespace ccf;
+  SwapTables c;
+  if (int rc = swap_tables_host(group_rows, num_groups, n, k, kseg, wide, n_pairs, &c)) return rc;
+  int i = 0;
+  for (int p = 0; p < n_pairs; ++p)
+    for (int w = p; w < c.round.items; w += n_pairs) {
+      const SwapTile t = decode_swap_item(w, &c, num_groups);
+      if (t.tokens <= 0) continue;
+      const int rec[12] = {p, w, c.round.whole, t.g, t.row0 - c.base[t.g], t.tokens, t.zero_rows, t.n0, t.parts, t.np,
+                           t.parts * ((((t.np >> 1) + kSwBox - 1) / kSwBox) * kSwBox), c.half};
+      if (i < cap) memcpy(out + 12 * i, rec, sizeof(rec));
+      ++i;
     }
   return i;
 }
