@@ -561,6 +561,11 @@ extern "C" {
 int ccf_gemm_smem_bytes() { return ccf::kSmemBytes; }
 
 // sizes of the argument blocks, so the Python mirror of the structures can be checked at load time
+// Whether epilogue warps help to push rows (gemm_common.cuh), for host-side checks of the rule.
+int ccf_dispatch_help(int kept, int n_comm_ctas, int ctas, int pair_kernel) {
+  return ccf::dispatch_help(kept, n_comm_ctas, ctas, pair_kernel != 0) ? 1 : 0;
+}
+
 int ccf_sizeof_gemm_args() { return static_cast<int>(sizeof(CcfGemmArgs)); }
 int ccf_sizeof_dispatch_args() { return static_cast<int>(sizeof(CcfDispatchArgs)); }
 int ccf_sizeof_gemm_launch() { return static_cast<int>(sizeof(CcfGemmLaunch)); }

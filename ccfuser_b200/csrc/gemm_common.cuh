@@ -681,6 +681,26 @@ __device__ __forceinline__ void combine_signal(const CcfGemmArgs& args, const Co
   }
 }
 
+// Rows of a chunk: a chunk is pushed by one warp from start to end. With only a few thousand rows in all (the latency-bound serving
+// shapes) chunks of two rows spread them over more warps, and the first tile's rows are complete after microseconds instead of tens.
+__host__ __device__ constexpr int dispatch_chunk(int kept) { return kept <= 4096 ? 2 : 8; }
+
+// Whether epilogue warps help the dedicated ones of the first n_comm_ctas of `ctas` CTAs to push `kept` rows (dispatch_role). Not where it
+// costs: of one chunk per dedicated warp or less (more warps only contend for the counter), and of more than 4096 rows in the kernel for
+// few rows, where the first wave needs few of them and more rows under way at once make those late. Whole training passes replayed from
+// a graph, us without and with help, rows = slots of the call, all CTAs pushing (one chunk per warp: 592 rows):
+//   kernel for few rows   768 x 3072, 16 experts: 592 rows 189 / 187, 1024 203 / 198, 2048 226 / 217, 4096 297 / 266;
+//                         1024 x 4096, 16 experts: 256 rows 250 / 256, 592 248 / 250, 1024 263 / 261, 4096 361 / 339;
+//                         64 experts: 256 rows 702 / 711, 1024 711 / 710, 4096 764 / 750, 6144 807 / 807, 8192 840 / 843, 12288 911 / 904,
+//                         16384 1072 / 1094
+//   pair kernel           1024 x 4096, 4 experts: 4096 rows 316 / 287, 6144 407 / 396, 8192 472 /
+//                         456, 12288 650 / 618, 16384 821 / 783; 512 x 2048, 8 experts: 6144 238 / 230, 16384 401 / 360
+// With several ranks the claims are the same and nobody waits for a helper; it has not been measured there.
+__host__ __device__ constexpr bool dispatch_help(int kept, int n_comm_ctas, int ctas, bool pair_kernel) {
+  const int chunks = (kept + dispatch_chunk(kept) - 1) / dispatch_chunk(kept);
+  return kept <= 4096 ? chunks > kCommWarps * (n_comm_ctas < ctas ? n_comm_ctas : ctas) : pair_kernel;
+}
+
 // The dispatch role as the epilogue warps of a GEMM kernel run it before their first accumulator is due. Only the
 // kernels whose A operand is the receive buffer carry it: the forward ones (bias + activation, SwiGLU) push x rows, the
 // backward ones (activation derivative) push g * dy rows; every other epilogue compiles to nothing here.
@@ -689,9 +709,7 @@ __device__ __forceinline__ void combine_signal(const CcfGemmArgs& args, const Co
 // barrier of their first accumulator, help until it is complete: until then they have nothing else to do, and the first tiles wait
 // for rows that two warps per SM push at the pace of their memory latencies. Passes, before and with help: GELU' of 16384 rows,
 // 4 experts of 1024 x 4096 (pair kernel: the first wave of tiles needs a quarter of all rows) 186 -> 149 us; ReLU and ReLU' of 3001 rows,
-// 16 experts of 768 x 3072 (kernel for few rows, chunks of two) 45.5 -> 37.4 and 57 -> 45 us. Not where it costs: of up to two chunks
-// per dedicated warp (more warps only contend for the counter), and of more than 4096 rows in the kernel for few rows, where the first
-// wave needs few of them and more rows under way at once make those late (64 experts, 16384 rows, GELU' 211 -> 219 us).
+// 16 experts of 768 x 3072 (kernel for few rows, chunks of two) 45.5 -> 37.4 and 57 -> 45 us. dispatch_help says where they do.
 template <int kEpi, bool kPairKernel = false>
 __device__ __forceinline__ void dispatch_role(const CcfGemmArgs& args, bool comm_warp, uint32_t first_acc = 0) {
   const bool carries = comm_warp == (args.comm_warps != 0);
@@ -699,15 +717,12 @@ __device__ __forceinline__ void dispatch_role(const CcfGemmArgs& args, bool comm
   if (static_cast<int>(blockIdx.x) >= args.n_comm_ctas) return;
   const uint32_t stop = carries ? 0u : first_acc;
   const int kept = args.disp.order_off[args.disp.e_total];
-  if (!carries && (kept <= 4096 ? kept <= 2 * kCommWarps * static_cast<int>(gridDim.x) : !kPairKernel)) return;
-  // A chunk is pushed by one warp from start to end. With only a few thousand rows in all (the latency-bound
-  // serving shapes) chunks of two rows spread them over sixteen times as many warps, and the first tile's rows are
-  // complete after microseconds instead of tens of them.
+  if (!carries && !dispatch_help(kept, args.n_comm_ctas, static_cast<int>(gridDim.x), kPairKernel)) return;
   if constexpr (kEpi == CCF_EPI_BIAS_ACT || kEpi == CCF_EPI_SWIGLU) {
-    if (kept <= 4096) dispatch_rows<2, false>(args.disp, args.status, stop);
+    if (dispatch_chunk(kept) == 2) dispatch_rows<2, false>(args.disp, args.status, stop);
     else dispatch_rows<8, false>(args.disp, args.status, stop);
   } else if constexpr (kEpi == CCF_EPI_DACT || kEpi == CCF_EPI_DSWIGLU) {
-    if (kept <= 4096) dispatch_rows<2, true>(args.disp, args.status, stop);
+    if (dispatch_chunk(kept) == 2) dispatch_rows<2, true>(args.disp, args.status, stop);
     else dispatch_rows<8, true>(args.disp, args.status, stop);
   }
 }

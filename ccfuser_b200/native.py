@@ -232,6 +232,7 @@ def _declare(lib):
         "ccf_gemm_launch": ([C.POINTER(GemmLaunch), p], i),
         "ccf_gemm_smem_bytes": ([], i),
         "ccf_debug_pair_tile_order": ([p, p, p, p, i, i, i, i, i, p, i], i),
+        "ccf_dispatch_help": ([i, i, i, i], i),
         "ccf_debug_swap_segments": ([p, i, i, i, i, i, i, p, i], i),
         "ccf_debug_swap_items": ([p, i, i, i, i, i, i, p, i], i),
         "ccf_router_topk": ([p, p, p, i, i, i, i, i, p, p, p, p, ull, i, p], i),
