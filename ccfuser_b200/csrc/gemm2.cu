@@ -249,17 +249,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_
       prefetch_tensormap(&tmB1);
     }
   }
+  wait_for_previous();
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
-  after_previous();
   const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   if (warp == 2) pair_tile_tables_warp<kKGroup, kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
+  let_next_in();
   const uint32_t tmem_base = ctrl->tmem_base;
   const int total_tiles = ctrl->total_tiles;
 

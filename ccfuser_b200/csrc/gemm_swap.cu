@@ -441,17 +441,18 @@ grouped_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_
       prefetch_tensormap(&tmW1);
     }
   }
+  wait_for_previous();
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
-  after_previous();
   const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   if (warp == 2) swap_tables_warp<kEpi>(args, ctrl, lane);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
+  let_next_in();
   const uint32_t tmem_base = ctrl->tmem_base;
   const SwapShape& sh = ctrl->shape;
   const int stages = sh.stages;

@@ -126,11 +126,11 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     prefetch_tensormap(&tmB);
     prefetch_tensormap(&tmC);
   }
+  wait_for_previous();
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(&ctrl->tmem_base), kTmemCols);
     tmem_relinquish_pair();
   }
-  after_previous();
   const uint64_t limit = fail_fast_limit(args.status, args.wait_limit_ns);
   for (int g = static_cast<int>(threadIdx.x) - 64; g >= 0 && g < args.num_groups; g += kWgThreads - 64) {
     ctrl->rows[g] = args.group_rows[g];
@@ -140,6 +140,7 @@ grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   __syncthreads();
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
+  let_next_in();
   const uint32_t tmem_base = ctrl->tmem_base;
   if (threadIdx.x == 0 && args.trace != nullptr) trace_ev(args, args.trace_tiles - 1, 0);
 

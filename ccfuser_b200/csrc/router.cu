@@ -156,11 +156,11 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     prefetch_tensormap(&tmX);
     prefetch_tensormap(&tmW);
   }
+  wait_for_previous();
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctrl->tmem_base), static_cast<uint32_t>(a.tmem_cols));
     tmem_relinquish();
   }
-  after_previous();
   const uint64_t limit = fail_fast_limit(a.status, a.wait_limit_ns);
   const void* const bias = a.bias;
   for (int e = threadIdx.x; e < 256; e += kRtThreads) {
@@ -173,6 +173,7 @@ router_topk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  let_next_in();
   const uint32_t tmem_base = ctrl->tmem_base;
 
   if (warp == 0) {
