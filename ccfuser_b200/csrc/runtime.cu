@@ -296,6 +296,7 @@ int forward_pass(const CcfLayer* L, const void* x, const int* idx, const float* 
     g.args.k = d;
     g.args.b_group_rows = f;
     g.args.out0 = L->h_act;
+    g.out_rows = L->max_rows;
     g.args.out1 = save_pre ? L->h_pre : nullptr;
     g.args.bias0 = L->b1;
     if (L->swiglu) {
@@ -354,6 +355,7 @@ int backward_pass(const CcfLayer* L, const void* dy, const int* idx, const float
     g.args.k = d;
     g.args.b_group_rows = d;
     g.args.out0 = G->dh;
+    g.out_rows = L->max_rows;
     g.args.aux0 = L->h_pre;
     if (L->swiglu) {
       g.epi = CCF_EPI_DSWIGLU;
