@@ -466,8 +466,8 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 2-D row-major view [rows, cols] of 2-byte elements, box = {box_cols, box_rows}, 128-byte swizzle.
-// A tensor map is a pure function of (address, extents, box, type), so encoded maps are kept in a small direct-mapped
+// 2-D row-major view [rows, cols] of 2-byte elements, rows ld elements apart, box = {box_cols, box_rows}; the swizzle is the box's width.
+// A tensor map is a pure function of (address, extents, distance of rows, box, type), so encoded maps are kept in a small direct-mapped
 // cache: a layer launches the same few operands every step, and in the latency-bound regime four driver calls per
 // launch cost as much as a small kernel.
 namespace {
@@ -501,6 +501,7 @@ size_t tmap_hash(const TmapKey& k) {
 int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows,
                      int fp16, long long ld) {
   if (ld == 0) ld = cols;
+  if (box_cols != 32 && box_cols != 64) return -15;
   const TmapKey key = {base, rows, cols, box_cols, box_rows, fp16, ld};
   const size_t slot = tmap_hash(key);
   {

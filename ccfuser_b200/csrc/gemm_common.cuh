@@ -21,8 +21,9 @@ constexpr int kTmemCols = 512;
 constexpr int MAJ_K = 0, MAJ_MN = 1;
 constexpr int kEpiStageBytes = 2048;  // per epilogue warp: 32 rows x 64 bytes, XOR-swizzled
 
-// Host: tensor map of a 2-D row-major view [rows, cols] of 2-byte elements with box {box_cols, box_rows} and 128-byte
-// swizzle (defined in gemm.cu). Returns 0 or a negative error code.
+// Host: tensor map of a 2-D row-major view [rows, cols] of 2-byte elements, rows ld elements apart (0: cols), with box {box_cols,
+// box_rows} (defined in gemm.cu). A box is as wide as its swizzle: 64 columns for the operands of an MMA (128 bytes), 32 for the staging
+// areas of the epilogues (64 bytes, stage_off); no other width is taken. Returns 0 or a negative error code.
 int make_tmap(CUtensorMap* m, const void* base, long long rows, long long cols, int box_cols, int box_rows, int fp16, long long ld = 0);
 
 // Descriptor of an operand in a pipeline stage as the MMA reads it: its base, the step of one 16-deep MMA, and any other place in
@@ -207,9 +208,20 @@ __device__ __forceinline__ void acc_to_float(const uint32_t (&r)[32], float (&f)
 // bytes (full 32-byte sectors). Lane l owns row l; `row_ptr` is the global address of this lane's
 // 64-byte segment (0 = skip the row).
 // ---------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t stage_off(int row, int piece) {
+__host__ __device__ __forceinline__ constexpr uint32_t stage_off(int row, int piece) {
   return static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
 }
+// It has to be the 64-byte swizzle of a bulk tensor copy (address bits 4 and 5 exclusive-or bits 7 and 8): staged_store_tma hands the area
+// over as a box of 32 columns.
+constexpr bool stage_is_swizzled_64() {
+  for (int row = 0; row < 32; ++row)
+    for (int piece = 0; piece < 4; ++piece) {
+      const uint32_t at = static_cast<uint32_t>(row * 64 + piece * 16);
+      if (stage_off(row, piece) != (at ^ ((at >> 3) & 0x30u))) return false;
+    }
+  return true;
+}
+static_assert(stage_is_swizzled_64(), "layout of the staging area");
 
 __device__ __forceinline__ void staged_store64(uint32_t stage, int lane, const uint32_t (&w)[16],
                                                unsigned long long row_ptr) {

@@ -336,7 +336,7 @@ class record_launches:
 
 
 # Argument checks of the host launchers return small negative numbers before any CUDA call is made; failures of CUDA
-# calls come back as minus the cudaError_t value. The two ranges overlap for -2 ... -14, so a message names both readings.
+# calls come back as minus the cudaError_t value. The two ranges overlap for -2 ... -15, so a message names both readings.
 ARG_ERRORS = {-2: "argument out of range", -3: "n must be a multiple of 32", -4: "k-grouped GEMM needs m_per_group % 128 == 0",
               -5: "k must be a multiple of 8", -6: "no kernel for this combination of operand majors and epilogue",
               -7: "cudaSetDevice failed", -8: "the CTA-pair kernel needs m_per_group % 256 == 0 in k-grouped mode",
@@ -347,7 +347,8 @@ ARG_ERRORS = {-2: "argument out of range", -3: "n must be a multiple of 32", -4:
               -12: "the kernel for few rows takes a K-major A operand, 16-bit outputs, no row bound, no narrow tile and no in-place update",
               -13: "the weight-gradient kernel for few rows takes MN-major operands, 16-bit outputs of n columns, no bias and "
                    "m_per_group % 256 == 0",
-              -14: "the rows to be dispatched must begin on a 16-byte boundary"}
+              -14: "the rows to be dispatched must begin on a 16-byte boundary",
+              -15: "the box of a tensor map is 32 or 64 columns wide"}
 
 
 def check(rc: int, what: str):
