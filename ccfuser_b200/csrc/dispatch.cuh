@@ -76,7 +76,7 @@ __device__ __forceinline__ bool mbar_phase_done(uint32_t bar, uint32_t parity) {
 // processed so the atomic's round trip is off the critical path.
 // Not inlined, and one instantiation per direction: the role keeps kChunk rows' worth of pointers and data in registers
 // (the backward form twice as much), which must not be added to the register budget of the GEMM roles it shares a
-// kernel with (168 registers per thread at 320 threads).
+// kernel with (168 registers per thread at 384 threads).
 // `stop_bar`: a barrier in shared memory whose first phase ends the role of this warp (0: none). It finishes the chunk that it has
 // claimed and claims no other; warps without one push whatever is left.
 template <int kChunk, bool kBackward>

@@ -517,6 +517,11 @@ __device__ __forceinline__ CombineDest epilogue_tile(const CcfGemmArgs& args, co
   fetch_aux(chunk0);
   if (!acquire()) return cd;
   cd.here = true;
+  // An accumulator chunk is requested where it is due, in every epilogue: a second chunk in registers, requested ahead, was never faster.
+  // Due / ahead, us: pair kernel, 4 experts of 4096 rows, 1024 x 4096: GELU 122.7 / 124.2, GELU' 128-138 / 141-147, rows combined 105 / 108,
+  // input gradient 116-126 / 109-121 (noise), stored weight gradients 108-116 / 112-116; in place, 16 x 1024 rows, 2048 x 8192: 463 / 465.
+  // One-CTA kernel, 3001 rows, 16 experts of 768 x 3072: ReLU 33.7 / 33.9, ReLU' 32.0 / 32.8, weight gradients 29.2 / 30.3, combined 44.9 / 45.0,
+  // input gradient 34.5 / 36.5; 64 x 256 rows, 1024 x 4096, weight gradients 183-205 / 185-208
   // not unrolled: the body is large and every launch pays for fetching the kernel's code once per SM
 #pragma unroll 1
   for (int c = 0; c < n_chunks; ++c) {

@@ -71,12 +71,18 @@ void set_row_kernel(CcfGemmLaunch& g, const CcfLayer* L, int tokens, int capacit
 
 // Whether a weight-gradient launch of a call that expects `rows` rows per expert runs on gemm_wgrad.cu, which moves its result by TMA,
 // or on the pair kernel: with few rows the reduction is only a handful of k-blocks, and moving the weights decides. In place the
-// weights are read as well as written, and the line lies higher. Both lie on the safe side since gemm_wgrad.cu holds four stages:
-// gemm_wgrad.cu over pair kernel, time, both in alternation:
+// weights are read as well as written, and the line lies higher. The lines were drawn when gemm_wgrad.cu held three stages, and
+// tests/test_row_kernel.py holds them there. With four stages it is the faster one beyond them too; gemm_wgrad.cu over pair kernel, time of
+// single launches, both in alternation:
 //   plain     1024 x 4096, 64 experts: 0.94 at 512 rows, 0.94 at 640, 1.01 at 768; 2048 x 8192, 16: 0.93, 0.95, 1.00, and 1.05 at 1024;
 //             768 x 3072, 16: 0.92, 0.95, 1.02, 1.05; 4096 x 14336, 8: 0.93, 0.92, 0.99
 //   in place  1024 x 4096, 64 experts: 0.83 at 512 rows, 0.94 at 640, 0.99 at 768; 2048 x 8192, 16: 0.79, 0.90, 0.94, and 1.03 at 1024;
 //             4096 x 14336, 8: 0.79, 0.91, 0.97
+// Whole training passes, two runs each, of which those of a millisecond differ by up to 5 % among themselves:
+//   plain     at 400, 450, 512, 580 and 640 rows: 1024 x 4096, 64 experts 0.99, 1.00, 0.96, 1.02, 0.98; 16 experts 0.99 at all five;
+//             2048 x 8192, 16: 1.03, 0.99, 0.95, 1.05, 0.99; 768 x 3072, 16: 0.99, 0.99, 0.99, 1.00, 1.00. About 1 % lies between the lines
+//   in place  at 560, 640 and 768 rows: 1024 x 4096, 64 experts 0.95, 0.98, 0.96; 16 experts 0.96, 0.97, 0.99; 2048 x 8192, 16: 0.92, 0.97,
+//             0.94; 768 x 3072, 16: 0.97, 0.98, 0.99. Here the line at 512 costs a pass 1 to 8 %
 bool wgrad_few(long long rows, bool in_place, int two_cta) { return two_cta && rows <= (in_place ? 512 : 384); }
 
 // Whether the launches of a call may overlap with the end of the ones in front of them (sm100.cuh). A group of ranks leaves it: there a

@@ -55,8 +55,14 @@ inline cudaLaunchAttribute cluster_attribute(unsigned x, unsigned y, unsigned z)
 // Launches of one pass can follow each other without the gap of a stream's order: a kernel with this attribute may be set up while the
 // kernel in front of it still runs, and waits for its end, and its memory, in wait_for_previous().
 // Only for calls of few slots: 16 tokens, 16 experts of 1024 x 4096 92 -> 84 us a pass, 777 tokens, 64 experts of 2048 x 8192 717 -> 714;
-// from 16384 slots, where the gaps are a percent of a pass, passes were 1 to 3 % slower with it (942 -> 952 and 4949 -> 5112 us). Not under
-// capture: the edges of a graph leave 0.4 us, and with the attribute 128 tokens, 4096 x 14336, took 511 us instead of 508.
+// at 16384 slots, where the gaps are a percent of a pass, passes of 4 experts of 1024 x 4096 and of 64 of 2048 x 8192 were 1 to 3 % slower
+// with it (942 -> 952 and 4949 -> 5112 us). In between nothing is slower outside the noise, and small layers gain: the line could lie higher. us
+// without / with at 4096, 6144, 8192, 12288 and 16384 slots:
+//   512 x 2048, 16 experts     inference 86 / 76, 100 / 88, 117 / 107, 130 / 121, 143 / 132; training 246 / 240, 272 / 259, 318 / 300, 364 / 346, 407 / 386
+//   1024 x 4096, 16 experts    inference 131 / 123, 165 / 157, 200 / 191, 255 / 244, 284 / 277; training 375 / 361, 468 / 455, 577 / 560, 736 / 721, 862 / 850
+//   2048 x 8192, 64 experts    inference 724 / 719, 757 / 751, 791 / 786, 902 / 896, 1078 / 1079; training 2445 / 2419, 2547 / 2550, 2750 / 2725,
+//                              3303 and 2913 / 3302 and 3318 (two runs each), 3965 / 4021
+// Not under capture: the edges of a graph leave 0.4 us, and with the attribute 128 tokens, 4096 x 14336, took 511 us instead of 508.
 constexpr long long kEarlySlots = 4096;
 inline int early_launches(long long slots, cudaStream_t stream) {
   if (slots > kEarlySlots) return 0;

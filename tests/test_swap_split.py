@@ -1,4 +1,5 @@
-"""Work split of the kernel with the weights on the M side (csrc/swap_shape.h), on the host with the kernel's own functions."""
+"""Whole tiles of the kernel with the weights on the M side (csrc/swap_shape.h), on the host with the kernel's own functions: one pair sums
+all k-blocks of a tile, and a stage of the pipeline holds it. What becomes of the last round's tiles is test_swap_items.py's."""
 import ctypes as C
 import random
 
@@ -29,21 +30,14 @@ def test_every_k_block_of_every_tile_is_summed_once(wide):
         kb = kseg * ((k + 63) // 64)
         cap = 128 if wide else 256 if max(rows) <= 256 else 320
         tiles = sum((r + cap - 1) // cap for r in rows) * ((n + 255) // 256)
-        seen, slots = {}, set()
-        for pair, tile, k0, k1, first, sharers, half, stages, shared in _segments(rows, n, k, kseg, wide, pairs):
+        seen = {}
+        for pair, tile, k0, k1, first, sharers, half, stages, total in _segments(rows, n, k, kseg, wide, pairs):
             assert 0 <= tile < tiles and 0 <= k0 < k1 <= kb and 0 <= pair < pairs
             assert half % 16 == 0 and half <= 160 and 2 <= stages <= 12
             seen.setdefault(tile, []).append((k0, k1, pair, first, sharers))
-            if (k0, k1) != (0, kb):
-                assert shared <= tile < shared + 2 * pairs      # counters
-                slot = (pair, k0 == 0)                          # each pair has one slot for a tile's start and one for a later run
-                assert slot not in slots
-                slots.add(slot)
+            assert total == tiles and pair == tile % pairs      # the pairs take the tiles in turns
         assert len(seen) == tiles
         for runs in seen.values():
-            runs.sort()
-            assert runs[0][0] == 0 and runs[-1][1] == kb
-            assert all(a[1] == b[0] for a, b in zip(runs, runs[1:]))
-            # every sharer names the same pairs, in the order of the k-blocks, and only the first one's run starts the tile
-            assert {(r[3], r[4]) for r in runs} == {(runs[0][2], len(runs))}
-            assert [r[2] for r in runs] == list(range(runs[0][2], runs[0][2] + len(runs)))
+            assert len(runs) == 1                               # no tile is shared
+            k0, k1, pair, first, sharers = runs[0]
+            assert (k0, k1) == (0, kb) and first == pair and sharers == 1
